@@ -7,10 +7,13 @@
 // nucleus cut and the draw stay with the caller's own `sample` (they are a few dozen flops and keep the
 // draw bit-identical to the host path); greedy decoding keeps using the argmax kernel.
 //
-// One CTA of 1024 threads: a four-pass radix select over the sortable 32-bit keys finds the k-th largest
+// One CTA of 1024 threads. Two sweeps and two sorts serve the common case (topk_kernel); where more than 1024 logits lie
+// above its bound (k near 1024, many ties), a four-pass radix select over the sortable 32-bit keys finds the k-th largest
 // key T and how many logits equal to T belong to the set, a second sweep gathers every key > T plus
 // the first such ties in index order, and a bitonic sort of at most 1024 (key, ~index) words in shared
 // memory puts them in order. The row (<= a few hundred KB) is read from L2 six times.
+#include <cstring>
+
 #include "common.cuh"
 
 namespace {
@@ -22,27 +25,94 @@ __device__ __forceinline__ uint32_t order_key(uint32_t bits) { return bits ^ ((b
 __device__ __forceinline__ uint32_t key_bits(uint32_t key) { return key ^ ((key >> 31) ? 0x80000000u : 0xffffffffu); }
 __device__ __forceinline__ bool is_nan_bits(uint32_t bits) { return (bits & 0x7fffffffu) > 0x7f800000u; }
 
-// sampling.rs:L44-L54: in the order of `recent`; a token listed twice is penalised twice
-__global__ void penalty_kernel(float* __restrict__ l, uint32_t vocab, const int32_t* __restrict__ recent, uint32_t n, float pen) {
-  if (blockIdx.x || threadIdx.x) return;
-  for (uint32_t i = 0; i < n; i++) {
+// Repetition penalty (sampling.rs:L44-L54: in the order of `recent`; a token listed twice is penalised twice). Tokens do
+// not affect one another, so the thread of a token's first listing applies it as often as it is listed, in order.
+__device__ __forceinline__ void penalise(float* l, uint32_t vocab, const int32_t* recent, uint32_t n, float pen) {
+  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
     const int32_t t = recent[i];
-    if (t >= 0 && (uint32_t)t < vocab) {
-      const float v = l[t];
-      l[t] = v > 0.0f ? v / pen : v * pen;
-    }
+    if (t < 0 || (uint32_t)t >= vocab) continue;
+    bool first = true;
+    for (uint32_t j = 0; j < i && first; j++) first = recent[j] != t;
+    if (!first) continue;
+    float v = l[t];
+    for (uint32_t j = i; j < n; j++)
+      if (recent[j] == t) v = v > 0.0f ? v / pen : v * pen;
+    l[t] = v;
   }
 }
 
+// bitonic sort of 1024 words by 1024 threads, descending
+__device__ __forceinline__ void sort_desc(unsigned long long* c) {
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t size = 2; size <= 1024; size <<= 1)
+    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+      const uint32_t j = tid ^ stride;
+      if (j > tid) {
+        const unsigned long long a = c[tid], b = c[j];
+        const bool desc = (tid & size) == 0;
+        if (desc ? a < b : a > b) c[tid] = b, c[j] = a;
+      }
+      if (stride > 16 || stride == 1) // (closer partners are lanes of one warp; the next round may reach across warps)
+        __syncthreads();
+      else
+        __syncwarp();
+    }
+}
+
 __global__ void __launch_bounds__(SEL_THREADS)
-    topk_kernel(const float* __restrict__ l, uint32_t vocab, uint32_t k, int32_t* __restrict__ out_idx, float* __restrict__ out_val,
-                uint32_t* __restrict__ out_n) {
+    topk_kernel(float* l, uint32_t vocab, uint32_t k, const int32_t* __restrict__ recent, uint32_t n_recent, float pen,
+                int32_t* __restrict__ out_idx, float* __restrict__ out_val, uint32_t* __restrict__ out_n) {
   __shared__ uint32_t hist[256];
   __shared__ uint32_t s_prefix, s_need, s_all, s_cnt;
   __shared__ uint32_t scan[SEL_THREADS];
   __shared__ unsigned long long cand[MAX_K];
   const uint32_t tid = threadIdx.x;
   const uint32_t* lb = reinterpret_cast<const uint32_t*>(l);
+  if (n_recent) { // (l is then the launch's own copy of the row)
+    penalise(l, vocab, recent, n_recent, pen);
+    __syncthreads();
+  }
+  // The common case in two sweeps: the k-th largest of the 1024 threads' own maxima bounds the k-th largest logit from
+  // below, and few more than k logits lie above it. (The radix select below takes a sweep per byte, and its histogram
+  // counts nearly all logits in a handful of bins - logits share their exponents - one atomic after the other: 50 us
+  // for 32000 logits.)
+  {
+    uint32_t best = 0; // (0 is no candidate's key: it would be a NaN)
+    for (uint32_t i = tid; i < vocab; i += SEL_THREADS) {
+      const uint32_t b = lb[i];
+      if (!is_nan_bits(b)) best = max(best, order_key(b));
+    }
+    cand[tid] = best;
+    if (tid == 0) s_cnt = 0;
+    __syncthreads();
+    sort_desc(cand);
+    const uint32_t bound = (uint32_t)cand[k - 1];
+    __syncthreads();
+    cand[tid] = 0ull;
+    __syncthreads();
+    if (bound) {
+      for (uint32_t i = tid; i < vocab; i += SEL_THREADS) {
+        const uint32_t b = lb[i];
+        const uint32_t key = is_nan_bits(b) ? 0u : order_key(b);
+        if (key >= bound) {
+          const uint32_t p = atomicAdd(&s_cnt, 1u);
+          if (p < MAX_K) cand[p] = ((unsigned long long)key << 32) | (0xffffffffu - i);
+        }
+      }
+      __syncthreads();
+      if (s_cnt <= MAX_K) { // (at least k: the k maxima themselves)
+        sort_desc(cand);
+        if (tid < k) {
+          const unsigned long long c = cand[tid];
+          out_idx[tid] = (int32_t)(0xffffffffu - (uint32_t)c);
+          out_val[tid] = __uint_as_float(key_bits((uint32_t)(c >> 32)));
+        }
+        if (tid == 0) *out_n = k;
+        return;
+      }
+      __syncthreads();
+    }
+  }
   if (tid == 0) {
     s_prefix = 0;
     s_need = k;
@@ -121,21 +191,7 @@ __global__ void __launch_bounds__(SEL_THREADS)
   }
   __syncthreads();
   const uint32_t n_sel = all ? n_gt : n_gt + min(need_eq, scan[SEL_THREADS - 1]);
-  // bitonic sort, descending, of the 1024 words (unused slots are 0 and sink to the end)
-  for (uint32_t size = 2; size <= MAX_K; size <<= 1) {
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      const uint32_t j = tid ^ stride;
-      if (j > tid) {
-        const unsigned long long a = cand[tid], b2 = cand[j];
-        const bool desc = (tid & size) == 0;
-        if (desc ? a < b2 : a > b2) {
-          cand[tid] = b2;
-          cand[j] = a;
-        }
-      }
-      __syncthreads();
-    }
-  }
+  sort_desc(cand); // (unused slots are 0 and sink to the end)
   if (tid < n_sel) {
     const unsigned long long c = cand[tid];
     out_idx[tid] = (int32_t)(0xffffffffu - (uint32_t)c);
@@ -164,23 +220,26 @@ int k_topk(FcDevice* dev, const float* logits, uint32_t vocab, uint32_t k, float
   int32_t* d_idx = (int32_t*)p;
   float* d_val = (float*)(p + (size_t)k * 4);
   uint32_t* d_n = (uint32_t*)(p + (size_t)k * 8);
-  const float* src = logits;
-  if (rep_penalty != 1.0f && n_recent) {
+  float* src = const_cast<float*>(logits); // (only read, unless penalised in a copy)
+  const bool pen = rep_penalty != 1.0f && n_recent;
+  void* pin; // recent up, the candidates down: one copy and one wait
+  FC_TRY(fc_pinned(dev, (size_t)n_recent * 4 + (size_t)k * 8 + 16, &pin));
+  if (pen) {
+    memcpy(pin, recent_host, (size_t)n_recent * 4);
     FC_CUDA(dev, cudaMemcpyAsync(row, logits, (size_t)vocab * 4, cudaMemcpyDeviceToDevice, dev->stream));
-    FC_CUDA(dev, cudaMemcpyAsync(d_recent, recent_host, (size_t)n_recent * 4, cudaMemcpyHostToDevice, dev->stream));
-    FC_LAUNCH(dev, "sample_penalty", penalty_kernel<<<1, 32, 0, dev->stream>>>(row, vocab, d_recent, n_recent, rep_penalty));
+    FC_CUDA(dev, cudaMemcpyAsync(d_recent, pin, (size_t)n_recent * 4, cudaMemcpyHostToDevice, dev->stream));
     src = row;
   }
-  FC_LAUNCH(dev, "sample_topk", topk_kernel<<<1, SEL_THREADS, 0, dev->stream>>>(src, vocab, k, d_idx, d_val, d_n));
-  uint32_t n = 0;
-  FC_CUDA(dev, cudaMemcpyAsync(&n, d_n, 4, cudaMemcpyDeviceToHost, dev->stream));
+  FC_LAUNCH(dev, "sample_topk", topk_kernel<<<1, SEL_THREADS, 0, dev->stream>>>(src, vocab, k, d_recent, pen ? n_recent : 0u, rep_penalty,
+                                                                               d_idx, d_val, d_n));
+  char* got = (char*)pin + (size_t)n_recent * 4;
+  FC_CUDA(dev, cudaMemcpyAsync(got, d_idx, (size_t)k * 8 + 4, cudaMemcpyDeviceToHost, dev->stream)); // idx | val | n lie together
   FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
+  uint32_t n;
+  memcpy(&n, got + (size_t)k * 8, 4);
   if (n > k) return fc_fail(dev, FC_ERR_DEVICE, "top-k selection returned %u of %u candidates", n, k);
-  if (n) {
-    FC_CUDA(dev, cudaMemcpyAsync(idx_out, d_idx, (size_t)n * 4, cudaMemcpyDeviceToHost, dev->stream));
-    FC_CUDA(dev, cudaMemcpyAsync(val_out, d_val, (size_t)n * 4, cudaMemcpyDeviceToHost, dev->stream));
-    FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
-  }
+  memcpy(idx_out, got, (size_t)n * 4);
+  memcpy(val_out, got + (size_t)k * 4, (size_t)n * 4);
   *n_out = n;
   return FC_OK;
 }
