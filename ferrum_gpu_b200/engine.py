@@ -62,32 +62,18 @@ def sample_candidates(idx, val, p: SampleParams, rng: Rng) -> int:
     if len(idx) == 0:
         return 0
     f = np.float32
-    t = f(p.temperature)
-    probs = [f(math.exp(float((f(v) - f(val[0])) / t))) for v in val]  # expf, correctly rounded
-    total = f(0.0)
-    for x in probs:
-        total = f(total + x)
-    probs = [f(x / total) for x in probs]
-    idx = list(idx)
+    d = ((np.asarray(val, dtype=f) - f(val[0])) / f(p.temperature)).tolist()
+    probs = np.array([math.exp(x) for x in d], dtype=f)  # expf, correctly rounded
+    probs = probs / np.cumsum(probs)[-1]  # (cumsum adds in f32 from left to right, as the reference's loops do)
+    keep = len(probs)
     if p.top_p < 1.0:
-        acc, keep = f(0.0), len(probs)
-        for i, x in enumerate(probs):
-            acc = f(acc + x)
-            if acc >= f(p.top_p):
-                keep = i + 1
-                break
-        idx, probs = idx[:keep], probs[:keep]
-        s2 = f(0.0)
-        for x in probs:
-            s2 = f(s2 + x)
-        probs = [f(x / s2) for x in probs]
-    r = rng.next_f32()
-    acc = f(0.0)
-    for i, x in zip(idx, probs):
-        acc = f(acc + x)
-        if r < acc:
-            return int(i)
-    return int(idx[-1])
+        reached = np.flatnonzero(np.cumsum(probs) >= f(p.top_p))
+        if reached.size:
+            keep = int(reached[0]) + 1
+        probs = probs[:keep]
+        probs = probs / np.cumsum(probs)[-1]
+    drawn = np.flatnonzero(rng.next_f32() < np.cumsum(probs))
+    return int(idx[int(drawn[0]) if drawn.size else keep - 1])
 
 
 def argmax(logits) -> int:
