@@ -28,6 +28,10 @@ struct FcDevice {
   int64_t fail_after = -1; // fault injection: launches left before every launch is refused
   void* pinned = nullptr;  // pinned host staging for results and small inputs
   size_t pinned_bytes = 0;
+  // Workspaces of stand-alone weights come from here, in the order of `stream`: a workspace given back is the next
+  // weight's, without the device-wide allocation and free (300 us of a first product). Holds on to at most
+  // WORKSPACE_POOL_KEEP bytes, goes with the device; null where the device has no memory pools.
+  cudaMemPool_t workspaces = nullptr;
   int* d_flag = nullptr;   // device int for kernels that report a status
   int matvec_choice = 0;   // fc_debug_matvec_kernel: which kernel multiplies 1..8 rows (0: the library's rule)
   // per-kernel timing (off by default): one event pair per launch, summed by name on report
@@ -39,6 +43,11 @@ struct FcDevice {
   std::vector<ProfSpan> spans;
   std::vector<cudaEvent_t> event_pool;
 };
+
+constexpr uint64_t WORKSPACE_POOL_KEEP = 512ull << 20;
+cudaError_t workspace_alloc(FcDevice* dev, void** p, size_t bytes);
+void workspace_free(FcDevice* dev, void* p);
+bool stream_capturing(FcDevice* dev); // the device's stream is being captured into a graph
 
 // Record a message and hand back the status code.
 int fc_fail(FcDevice* dev, int code, const char* fmt, ...);
@@ -117,10 +126,13 @@ struct FcQWeight {
   void* qs_alloc = nullptr;
   void* sc_alloc = nullptr;
   uint64_t bytes = 0;
-  // bf16 GEMM operand descriptors are built lazily by the tensor path
+  // workspace of the products of many rows (fp16 terms of x and of the weight), grown on demand
   void* tc_cache = nullptr;
   size_t tc_cache_bytes = 0;
   void* mma_scratch = nullptr; // scratch of the batched-decode product for stand-alone use
+  // a captured graph may hold the workspace's address: once a call was captured, outgrown workspaces are kept
+  bool captured = false;
+  std::vector<void*> outgrown;
 };
 
 __host__ __device__ constexpr bool kind_is_fp8(int kind) { return kind == FC_FP8_E4M3 || kind == FC_FP8_E5M2; }
@@ -204,6 +216,12 @@ struct Epilogue {
   // device scratch of at least qmatvec_mma_scratch_bytes(k, n): lets products of 9..64 rows run on the
   // tensor-core batched-decode kernel; without it they take the tiled f32 kernel
   void* scratch = nullptr;
+  // a stand-alone product (no norm, nothing pending or deferred) whose width need not be whole 128s: the scratch also
+  // serves qmatvec_mma_ragged_supports
+  bool ragged = false;
+  // device scratch of at least qgemm_pair_scratch_bytes(k, n, m): lets products of more than 64 rows of Q8_0 / Q4_0
+  // weights run on the tensor cores (gemm_pair.cu); without it they take the tiled f32 kernel
+  void* wide_scratch = nullptr;
   // "x is the raw residual stream: normalise each row first" (NORM_RMS: y = x / sqrt(mean(x^2) + eps) * g,
   // NORM_LAYER: (x - mean) / sqrt(var + 1e-5) * g + b). The one-row FMA matvec does it while it stages x
   // in shared memory (one launch less per product); the other kernels run the norm kernel into
@@ -228,6 +246,7 @@ enum { NORM_NONE = 0, NORM_RMS = 1, NORM_LAYER = 2 };
 
 // matvec_mma.cu: 9 <= m <= 64 rows at f32-class accuracy on mma.sync
 bool qmatvec_mma_supports(const QMat& w, uint32_t m);
+bool qmatvec_mma_ragged_supports(const QMat& w, uint32_t m); // 2..64 rows, other whole-block widths (Epilogue::ragged)
 size_t qmatvec_mma_scratch_bytes(uint32_t k, uint32_t n);
 int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, void* scratch);
 // Whether k_qlinear_f32 will take the 9..64-row tensor-core product for (w, m) with this scratch, and where
@@ -270,3 +289,7 @@ int qweight_from_f32(FcDevice* dev, int kind, const float* w_in_out_host, uint32
 int qweight_from_f32_concat(FcDevice* dev, int kind, const float* const* mats_host, const uint32_t* ns, int count,
                             uint32_t k, FcQWeight** out);
 void qweight_free(FcQWeight* w);
+// The weight's product workspace (tc_cache), grown to `bytes` (model_tc.cu). FC_ERR_OOM: there is no room for it, or the
+// stream is being captured and nothing can be allocated - the caller goes on without, where its product can.
+int qweight_workspace(FcQWeight* w, size_t bytes);
+void qweight_workspace_free(FcQWeight* w);

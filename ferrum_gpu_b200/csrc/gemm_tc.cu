@@ -2,7 +2,7 @@
 //   Y[m, n] = A[m, k] (f16) . dequant(W)[n, k]^T (fp16), f32 accumulators in tensor memory.
 // Replaces qlinear_tiled.wgsl for M >= 128 (ferrum_wgpu/src/shaders/quant/qlinear_tiled.wgsl:L93-L128).
 //
-// Two kernel bodies share the packed-weight readers and dequantisers of this file:
+// Kernel bodies that share the packed-weight readers and dequantisers of this file:
 //   - gemm_ts_main.cuh: the weight rows on the tensor-memory lanes. A producer thread owns one weight row = one
 //     lane, dequantises its packed blocks of a 64-k slice and writes them into tensor memory, from where they are
 //     the MMA's A operand; the activations (192 rows x 64 f16 per TMA box) are the B operand. f32 / fp16 /
@@ -10,6 +10,9 @@
 //   - gemm_tc_main.cuh: the activation rows on the lanes, 256 x 128 tiles, both operands in shared memory (the
 //     weight slice dequantised into the swizzled K-major layout TMA produces). The vocabulary head: its epilogue
 //     folds a row of logits into (max, sum-exp, target logit, first argmax) in one thread's registers.
+//   - gemm_tp_main.cuh: with many rows, the weights decoded to fp16 once per launch and both operands read by TMA on CTA
+//     pairs; every epilogue (tp_takes says when).
+//   - gemm_tx_main.cuh: 9..64 rows at f32-class accuracy.
 #include "gemm_tc.cuh"
 #include "tc_ptx.cuh"
 
@@ -45,6 +48,13 @@ constexpr int TS_THREADS = (4 + 4 * PSETS + 8) * 32;
 // the CTA is launched with (checked before the first launch)
 constexpr int TS_REGS_PROD = 64, TS_REGS_EPI = 120;
 constexpr int TS_REGS_NEEDED = 32 * (4 * REGS_CTRL + 4 * PSETS * TS_REGS_PROD + 8 * TS_REGS_EPI);
+
+// The product of many rows on CTA pairs, from decoded weights (gemm_tp_main.cuh)
+constexpr int TP_THREADS = 384, TP_STAGES = 5;
+constexpr uint32_t TP_STAGE_BYTES = 2 * 128 * TC_BK * 2;          // 32 KB: this CTA's 128 rows of A and of B
+constexpr uint32_t TP_STG_OFF = TP_STAGES * TP_STAGE_BYTES + 512; // after the ring and the barriers
+constexpr uint32_t TP_SMEM_BYTES = TP_STG_OFF + 8 * 2 * STG_TILE + 1024 /*alignment slack*/;
+constexpr size_t TP_SLICE_BYTES = (size_t)64 << 20; // decoded weights at once: they stay in the 126 MB L2 beside the activations
 
 // The batched-decode product at f32-class accuracy (gemm_tx_main.cuh)
 constexpr int TX_X_STAGES = 8, TX_W_STAGES = 4, TX_PSETS = 2;
@@ -398,6 +408,7 @@ __device__ __forceinline__ void epilogue_lse(const TcArgs& a, LseState& s, uint3
 #include "gemm_tc_main.cuh"
 #include "gemm_ts_main.cuh"
 #include "gemm_tx_main.cuh"
+#include "gemm_tp_main.cuh"
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point: the library carries no link
 // dependency on libcuda, so it still loads (and exports its symbols) on a machine without a GPU.
@@ -491,6 +502,93 @@ int pick_epi(FcDevice* dev, const CUtensorMap& tmap, const QMat& w, const TcArgs
   return fc_fail(dev, FC_ERR_ARG, "unknown epilogue %d", epi);
 }
 
+template <int EPI>
+int launch_tp(FcDevice* dev, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& to, const TcArgs& a) {
+  auto kern = qgemm_tp_kernel<EPI>;
+  static OncePerDevice attr;
+  if (attr.first(dev->ordinal)) FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TP_SMEM_BYTES));
+  const uint64_t tiles = (uint64_t)((a.n + 255) / 256) * ((a.m + 255) / 256);
+  const uint32_t pairs = (uint32_t)dev->prop.multiProcessorCount / 2;
+  static const char* const names[] = {"qgemm_tc_f32", "qgemm_tc_f16", "qgemm_tc_resid", "qgemm_tc_swiglu", "qgemm_tc_lse"};
+  FC_LAUNCH(dev, names[EPI], kern<<<2 * (unsigned)(tiles < pairs ? tiles : pairs), TP_THREADS, TP_SMEM_BYTES, dev->stream>>>(ta, tb, to, a));
+  return FC_OK;
+}
+
+int half_map(FcDevice* dev, CUtensorMap* map, const __half* p, uint32_t rows, uint32_t k, uint32_t box_rows) {
+  const cuuint64_t dims[2] = {k, rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
+  const cuuint32_t box[2] = {TC_BK, box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult cr = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)p, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (cr != CUDA_SUCCESS) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled failed with %d", (int)cr);
+  return FC_OK;
+}
+
+// weight rows whose decoded values are in the workspace at once: whole 256-row tiles
+uint32_t tp_slice_rows(const QMat& w) {
+  const size_t fit = TP_SLICE_BYTES / ((size_t)w.k * 2) / 256 * 256;
+  const size_t rows = fit < 256 ? 256 : fit;
+  return rows < w.n ? (uint32_t)rows : w.n;
+}
+
+// `handled` stays false where the output cannot leave by TMA and the epilogue has no other way (the ts kernel takes it)
+int k_qgemm_tp(FcDevice* dev, const QMat& w, const __half* x, int epi, const TcArgs& args, bool* handled) {
+  const bool f32 = epi == EPI_F32 || epi == EPI_RESID;
+  uint8_t* out = f32 ? (uint8_t*)args.out_f32 : (uint8_t*)args.out_f16;
+  const uint32_t esize = f32 ? 4 : 2;
+  const uint64_t pitch = (uint64_t)args.ldo * esize;
+  const bool tma = epi != EPI_LSE && out && pitch % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  if (!tma && epi != EPI_LSE && epi != EPI_F32) return FC_OK;
+  *handled = true;
+  __half* wf = (__half*)args.wide;
+  const uint32_t slice = tp_slice_rows(w);
+  CUtensorMap tx, tw;
+  FC_TRY(half_map(dev, &tx, x, args.m, w.k, 128));
+  for (uint32_t n0 = 0; n0 < w.n; n0 += slice) {
+    QMat v = w;
+    v.n = w.n - n0 < slice ? w.n - n0 : slice;
+    v.qs = w.qs + qmat_qs_bytes(w.kind, w.k, n0);
+    v.sc = (const __half*)((const uint8_t*)w.sc + qmat_sc_bytes(w.kind, w.k, n0));
+    const uint32_t bx = w.k / 16 < 64 ? 32 : 64; // (k is a multiple of 64: at least four threads per row)
+    const dim3 block(bx, 256 / bx), grid((w.k / 16 + bx - 1) / bx, (v.n + block.y - 1) / block.y < 65535 ? (v.n + block.y - 1) / block.y : 65535);
+    if (w.kind == FC_Q8_0)
+      FC_LAUNCH(dev, "weights_f16", weights_f16_kernel<FC_Q8_0><<<grid, block, 0, dev->stream>>>(v, wf));
+    else
+      FC_LAUNCH(dev, "weights_f16", weights_f16_kernel<FC_Q4_0><<<grid, block, 0, dev->stream>>>(v, wf));
+    FC_TRY(half_map(dev, &tw, wf, v.n, w.k, 128));
+    TcArgs a = args;
+    a.n = v.n;
+    if (a.bias) a.bias += n0;
+    if (a.out_f32) a.out_f32 += n0;
+    if (a.out_f16) a.out_f16 += epi == EPI_SWIGLU ? n0 / 2 : n0;
+    a.v0 += n0;
+    a.tile0 = n0 / TC_BN;
+    CUtensorMap to = tx;
+    const uint64_t cols = epi == EPI_SWIGLU ? v.n / 2 : v.n;
+    if (tma && cols > 0) { // (a slice starts at a multiple of 256 columns: 16-byte aligned where the whole output is)
+      const cuuint64_t dims[2] = {cols, a.m};
+      const cuuint64_t strides[1] = {pitch};
+      const cuuint32_t box[2] = {epi == EPI_SWIGLU ? 16u : 32u, 32u};
+      const cuuint32_t estr[2] = {1, 1};
+      void* o = f32 ? (void*)a.out_f32 : (void*)a.out_f16;
+      const CUresult cr = encode_fn()(&to, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, o, dims, strides, box,
+                                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      if (cr != CUDA_SUCCESS) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled (output) failed with %d", (int)cr);
+      a.out_tma = 1;
+    }
+    switch (epi) {
+      case EPI_F32: FC_TRY(launch_tp<EPI_F32>(dev, tw, tx, to, a)); break;
+      case EPI_F16: FC_TRY(launch_tp<EPI_F16>(dev, tw, tx, to, a)); break;
+      case EPI_RESID: FC_TRY(launch_tp<EPI_RESID>(dev, tw, tx, to, a)); break;
+      case EPI_SWIGLU: FC_TRY(launch_tp<EPI_SWIGLU>(dev, tw, tx, to, a)); break;
+      default: FC_TRY(launch_tp<EPI_LSE>(dev, tx, tw, to, a)); break;
+    }
+  }
+  return FC_OK;
+}
+
 template <int KIND>
 int launch_tx(FcDevice* dev, const CUtensorMap& txh, const CUtensorMap& txl, const CUtensorMap& tq, const CUtensorMap& tsc,
               const TxArgs& a, dim3 grid) {
@@ -568,6 +666,35 @@ int k_qgemm_tx(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl,
   return launch_tx<FC_Q4_0>(dev, maps[0], maps[1], tq, tsc, a, grid);
 }
 
+// Whether decoding the weights first pays, by the estimated time of both in ns. Constants measured on K 768..4096 x
+// N 768..32000, 128..16384 rows: a K step of a 128 x 192 tile with in-kernel decoding takes 395 (Q4_0) or 530 (Q8_0: a
+// thread reads twice the bytes), of a 256 x 256 pair tile 415, a tile's own overhead about 800; the decoding pass costs a
+// launch and 1.1 (Q4_0) or 0.65 ps per weight; neither form writes more than 2.65 TB/s. (4096 rows of 4096 x 11008 Q8_0:
+// 464 us with in-kernel decoding, 330 decoded first; 256 rows: 71 and 94.)
+bool tp_takes(const FcDevice* dev, const QMat& w, uint32_t m, int epi) {
+  if ((w.kind != FC_Q8_0 && w.kind != FC_Q4_0) || w.k % TC_BK || !m) return false;
+#ifdef TP_ALWAYS
+  return TP_ALWAYS;
+#endif
+  const bool q8 = w.kind == FC_Q8_0;
+  const uint64_t sms = (uint64_t)dev->prop.multiProcessorCount, pairs = sms / 2, steps = w.k / TC_BK;
+  const uint64_t ts_tiles = (uint64_t)((w.n + TC_BN - 1) / TC_BN) * ((m + TS_BX - 1) / TS_BX);
+  uint64_t ts = (ts_tiles + sms - 1) / sms * (steps * (q8 ? 530 : 395) + 800);
+  const uint32_t slice = tp_slice_rows(w);
+  uint64_t waves = 0, launches = 0;
+  for (uint64_t n0 = 0; n0 < w.n; n0 += slice, launches++) {
+    const uint64_t rows = w.n - n0 < slice ? w.n - n0 : slice;
+    waves += ((rows + 255) / 256 * ((m + 255) / 256) + pairs - 1) / pairs;
+  }
+  uint64_t tp = waves * (steps * 415 + 800);
+  const uint64_t out_bytes = (uint64_t)m * w.n * (epi == EPI_LSE ? 0 : epi == EPI_SWIGLU ? 1 : epi == EPI_F16 ? 2 : 4);
+  const uint64_t store = out_bytes / 2650;
+  ts = ts > store ? ts : store;
+  tp = (tp > store ? tp : store) + launches * 4000 + (uint64_t)w.n * w.k / (q8 ? 1540 : 910);
+  return tp < ts;
+}
+size_t tp_workspace_bytes(const QMat& w) { return (size_t)tp_slice_rows(w) * w.k * 2; }
+
 int k_qgemm_tc_f16(FcDevice* dev, const QMat& w, const __half* a_dev, int epi, TcArgs args) {
   if (args.m == 0) return FC_OK;
   args.n = w.n;
@@ -580,6 +707,11 @@ int k_qgemm_tc_f16(FcDevice* dev, const QMat& w, const __half* a_dev, int epi, T
   if ((reinterpret_cast<uintptr_t>(a_dev) & 15) != 0) return fc_fail(dev, FC_ERR_ARG, "the A operand must be 16-byte aligned");
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
+  if (args.wide && tp_takes(dev, w, args.m, epi)) {
+    bool handled = false;
+    FC_TRY(k_qgemm_tp(dev, w, a_dev, epi, args, &handled));
+    if (handled) return FC_OK;
+  }
   // The log-sum-exp head keeps the activation rows on the tensor-memory lanes (a thread folds one row's logits in
   // registers); every other epilogue runs the kernel with the weight rows there.
   const bool on_lanes = epi != EPI_LSE;

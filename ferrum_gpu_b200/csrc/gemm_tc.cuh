@@ -24,6 +24,9 @@ struct TcArgs {
   uint32_t v0 = 0;
   float* partial = nullptr;
   int* err_flag = nullptr;
+  uint32_t tile0 = 0;   // EPI_LSE: 128-column tiles of the head before this launch's weight rows
+  // workspace for the fp16 weights of the pair kernel (tp_workspace_bytes; nullable: the weights are decoded in the product)
+  void* wide = nullptr;
   uint32_t out_tma = 0; // (set by the launch code) results leave through shared memory and TMA
 };
 
@@ -31,6 +34,9 @@ constexpr uint32_t TC_BM = 256, TC_BN = 128, TC_BK = 64; // weight rows per tile
 
 // y = a[m][k] (f16, row-major, device) . W^T with the epilogue `epi`. k % 64 == 0.
 int k_qgemm_tc_f16(FcDevice* dev, const QMat& w, const __half* a, int epi, TcArgs args);
+// Whether that product decodes the weights first, given a workspace, and how much it takes.
+bool tp_takes(const FcDevice* dev, const QMat& w, uint32_t m, int epi);
+size_t tp_workspace_bytes(const QMat& w);
 // Reads and clears the device-side error word the tensor kernels report bounded-wait failures in.
 int tc_check_errors(FcDevice* dev);
 

@@ -29,6 +29,48 @@
 // arrivals / MMA commit) for the weight stages, acc_full / acc_empty for the accumulator buffers. Every wait is
 // bounded and polls the CTA-wide abort word.
 
+// One 32 x 32 chunk of an output tile whose columns lie on the lanes (lane = output column, acc[j] = row j) into a
+// staging tile, as the row-major tile it is (16 columns wide for SwiGLU's halved output): conflict-free, lane = column.
+template <int EPI>
+__device__ __forceinline__ void stage_chunk(const TcArgs& a, uint8_t* st, const uint32_t (&acc)[32], float bias, int lane) {
+  const bool odd = lane & 1;
+  if (EPI == EPI_F32 || EPI == EPI_RESID) {
+    float* t = reinterpret_cast<float*>(st) + lane;
+#pragma unroll
+    for (int j = 0; j < 32; j++) t[j * 32] = __uint_as_float(acc[j]) + bias;
+  } else if (EPI == EPI_F16) {
+    __half* t = reinterpret_cast<__half*>(st) + lane;
+#pragma unroll
+    for (int j = 0; j < 32; j++) {
+      float v = __uint_as_float(acc[j]) + bias;
+      if (a.act == ACT_GELU) v = gelu_f(v);
+      t[j * 32] = __ushort_as_half((unsigned short)(pack_f16(v, 0.0f) & 0xffffu));
+    }
+  } else { // SwiGLU: weight rows 2i / 2i + 1 are gate i / up i; the even lane finishes row j, the odd lane row j + 1
+    __half* t = reinterpret_cast<__half*>(st) + (odd ? 16 : 0) + (lane >> 1);
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? acc[j] : acc[j + 1]), 1);
+      const float gv = odd ? got : __uint_as_float(acc[j]), uv = odd ? __uint_as_float(acc[j + 1]) : got;
+      const float v = __fdividef(gv, 1.0f + ex2f_approx(gv * -1.4426950408889634f)) * uv;
+      t[j * 16] = __ushort_as_half((unsigned short)(pack_f16(v, 0.0f) & 0xffffu));
+    }
+  }
+}
+// One bulk tensor store of the staged tile - for the residual stream a bulk tensor REDUCE (add) -, clipped at the
+// matrix edges by the tensor map. The caller commits the group.
+template <int EPI>
+__device__ __forceinline__ void store_staged(const CUtensorMap* tmap_o, const uint8_t* st, int32_t col, int32_t row) {
+  if (EPI == EPI_RESID)
+    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap_o),
+                 "r"(tc::smem_u32(st)), "r"(col), "r"(row)
+                 : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(tmap_o), "r"(tc::smem_u32(st)),
+                 "r"(col), "r"(row)
+                 : "memory");
+}
+
 template <int KIND, int EPI>
 __global__ void __launch_bounds__(TS_THREADS, 1)
     qgemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_o, const QMat w,
@@ -255,40 +297,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
           sbuf ^= 1;
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           __syncwarp();
-          if (EPI == EPI_F32 || EPI == EPI_RESID) {
-            float* t = reinterpret_cast<float*>(st) + lane;
-#pragma unroll
-            for (int j = 0; j < 32; j++) t[j * 32] = __uint_as_float(acc[j]) + bias;
-          } else if (EPI == EPI_F16) {
-            __half* t = reinterpret_cast<__half*>(st) + lane;
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-              float v = __uint_as_float(acc[j]) + bias;
-              if (a.act == ACT_GELU) v = gelu_f(v);
-              t[j * 32] = __ushort_as_half((unsigned short)(pack_f16(v, 0.0f) & 0xffffu));
-            }
-          } else { // SwiGLU: weight rows 2i / 2i + 1 are gate i / up i; the even lane finishes row j, the odd lane row j + 1
-            __half* t = reinterpret_cast<__half*>(st) + (odd ? 16 : 0) + (lane >> 1);
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? acc[j] : acc[j + 1]), 1);
-              const float gv = odd ? got : __uint_as_float(acc[j]), uv = odd ? __uint_as_float(acc[j + 1]) : got;
-              const float v = __fdividef(gv, 1.0f + ex2f_approx(gv * -1.4426950408889634f)) * uv;
-              t[j * 16] = __ushort_as_half((unsigned short)(pack_f16(v, 0.0f) & 0xffffu));
-            }
-          }
+          stage_chunk<EPI>(a, st, acc, bias, lane);
           tc::fence_async_smem();
           __syncwarp();
           if (lane == 0) {
             const int32_t col = (int32_t)((tile % tiles_n) * TC_BN + quad * 32) >> (EPI == EPI_SWIGLU ? 1 : 0);
-            if (EPI == EPI_RESID)
-              asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&tmap_o),
-                           "r"(tc::smem_u32(st)), "r"(col), "r"((int32_t)x0)
-                           : "memory");
-            else
-              asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(&tmap_o),
-                           "r"(tc::smem_u32(st)), "r"(col), "r"((int32_t)x0)
-                           : "memory");
+            store_staged<EPI>(&tmap_o, st, col, (int32_t)x0);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
         } else if (EPI == EPI_F32 || EPI == EPI_RESID) {

@@ -8,7 +8,7 @@
 // memory) is read once and reused for the R rows. Integer quants are turned into floats with
 // bit tricks (no I2F), the per-block f16 scale multiplies the block's partial sum, accumulation
 // is f32, and the LPR partial sums are combined with warp shuffles.
-#include "common.cuh"
+#include "gemm_pair.cuh"
 #include "ops.cuh"
 
 namespace {
@@ -404,6 +404,12 @@ int k_qlinear_f32(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     if (ep.presplit) return fc_fail(dev, FC_ERR_ARG, "a pre-split x needs the 9..64-row tensor-core product");
     return k_qmatvec1(dev, w, x, y, ep);
   }
+  if (ep.wide_scratch && forced == 0 && !ep.presplit && qgemm_pair_takes(w, m)) { // (its x split takes the norm along)
+    if (ep.pending && ep.pending->splits) FC_TRY(k_flush_deferred(dev, *ep.pending));
+    return k_qgemm_pair(dev, w, x, m, y, ep, ep.wide_scratch);
+  }
+  if (ep.ragged && ep.scratch && forced == 0 && qmatvec_mma_ragged_supports(w, m) && (reinterpret_cast<uintptr_t>(x) & 15) == 0)
+    return k_qmatvec_mma(dev, w, x, m, y, ep, ep.scratch);
   const bool fma_ok = m <= 8 && (size_t)m * w.k * 4 <= 200 * 1024 && w.k % 4 == 0;
   // (the tensor-core kernels stage x with 16-byte asynchronous copies)
   const bool mma_ok = ep.scratch && qmatvec_mma_supports(w, m) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0 || ep.presplit);

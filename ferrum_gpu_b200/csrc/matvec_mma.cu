@@ -14,7 +14,7 @@
 // from shared memory with one 8-byte load per step. x slices (128 k) are staged by cp.async, double
 // buffered. With few output rows the K axis is split across CTAs; partial sums are combined in a
 // fixed order by a second kernel (no atomics: repeated runs are bit-identical).
-#include "common.cuh"
+#include "gemm_pair.cuh"
 
 namespace {
 
@@ -377,7 +377,11 @@ __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
 
-template <int KIND>
+// RAGGED: K in whole blocks of 32 instead of whole slices. The last slice is filled up with zeros, the scales (whose rows
+// then start at any even address) come by two-byte loads one slice ahead, and each row's slice of x is first brought
+// to [2^14, 2^15) by a power of two that the block scales take back, so that the fp16 terms hold any f32 range: the f32
+// kernels that otherwise serve these widths do.
+template <int KIND, bool RAGGED>
 __global__ void __launch_bounds__(128)
     qmatvec_mma8_kernel(QMat w, const float* __restrict__ x, uint32_t m, float* __restrict__ y, float* __restrict__ partial,
                         uint32_t blocks_per_split, Epilogue ep) {
@@ -392,7 +396,21 @@ __global__ void __launch_bounds__(128)
   const uint32_t n = w.n, k = w.k, nblocks = k / QK;
   const uint32_t cta_row0 = blockIdx.x * ROWS_PER_CTA;
   const uint32_t kb_begin = blockIdx.y * blocks_per_split;         // whole 4-block slices; the last split may be shorter
-  const uint32_t n_slices = (min(kb_begin + blocks_per_split, nblocks) - kb_begin) / 4;
+  const uint32_t kb_end = min(kb_begin + blocks_per_split, nblocks);
+  const uint32_t n_slices = (kb_end - kb_begin + (RAGGED ? 3 : 0)) / 4;
+  __shared__ float x_inv[2][8]; // RAGGED: the slice's powers of two, divided out
+  uint32_t sc_lo = 0, sc_hi = 0; // RAGGED: this thread's row of scales, loaded one slice ahead
+  auto load_scales = [&](uint32_t slice) {
+    const uint32_t kb0 = kb_begin + slice * 4, grow = min(cta_row0 + (threadIdx.x & 63u), n - 1);
+    const unsigned short* src = reinterpret_cast<const unsigned short*>(w.sc) + (size_t)grow * nblocks + kb0;
+    uint32_t v[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) v[i] = kb0 + i < kb_end ? (uint32_t)__ldg(src + i) : 0u;
+    sc_lo = v[0] | (v[1] << 16), sc_hi = v[2] | (v[3] << 16);
+  };
+  auto store_scales = [&](uint32_t slice) {
+    *reinterpret_cast<uint2*>(scs + (slice % C::ST) * C::SC_STAGE + threadIdx.x * 8) = make_uint2(sc_lo, sc_hi);
+  };
 
   auto issue = [&](uint32_t slice) {
     const uint32_t st = slice % C::ST, kb0 = kb_begin + slice * 4;
@@ -404,9 +422,15 @@ __global__ void __launch_bounds__(128)
       const uint32_t grow = min(cta_row0 + row, n - 1); // rows past the end are computed and dropped
       const uint8_t* src =
           w.qs + (size_t)grow * (KIND == FC_F16 ? 2 * k : kind_byte_blocks(KIND) ? k : k / 2) + (size_t)kb0 * (C::WBYTES / 4) + ch * 16;
-      cp_async16(smem_u32(wq + st * C::W_STAGE + row * C::WROW + ch * 16), src);
+      const uint32_t dst = smem_u32(wq + st * C::W_STAGE + row * C::WROW + ch * 16);
+      if (RAGGED) {
+        const bool valid = kb0 + ch * 16 / (C::WBYTES / 4) < kb_end;
+        cp_async16_zfill(dst, valid ? src : w.qs, valid);
+      } else {
+        cp_async16(dst, src);
+      }
     }
-    if (KIND != FC_F16 && threadIdx.x < 64) {
+    if (!RAGGED && KIND != FC_F16 && threadIdx.x < 64) {
       const uint32_t grow = min(cta_row0 + threadIdx.x, n - 1);
       cp_async8(smem_u32(scs + st * C::SC_STAGE + threadIdx.x * 8), w.sc + (size_t)grow * nblocks + kb0);
     }
@@ -414,16 +438,19 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
     for (int j = 0; j < 2; j++) {
       const uint32_t c = threadIdx.x + 128 * j, row = c >> 5, ch = c & 31;
-      const bool valid = row < m;
+      const bool valid = row < m && (!RAGGED || kb0 + ch / 8 < kb_end);
       cp_async16_zfill(smem_u32(xf + st * C::XF_STAGE + (row * XS + ch * 4) * 4),
-                       x + (size_t)(valid ? row : 0) * k + (size_t)kb0 * QK + ch * 4, valid);
+                       valid ? x + (size_t)row * k + (size_t)kb0 * QK + ch * 4 : x, valid);
     }
   };
 
   float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int p = 0; p < C::ST - 1; p++) { // one commit group per slice position, empty past the end
-    if ((uint32_t)p < n_slices) issue(p);
+    if ((uint32_t)p < n_slices) {
+      issue(p);
+      if (RAGGED && KIND != FC_F16 && threadIdx.x < 64) load_scales(p), store_scales(p);
+    }
     cp_async_commit();
   }
   const uint32_t r0 = warp * 16 + g, r1 = r0 + 8; // this lane's two weight rows within the CTA
@@ -432,19 +459,41 @@ __global__ void __launch_bounds__(128)
     const uint32_t st = sl % C::ST;
     cp_async_wait<C::ST - 2>();
     __syncthreads(); // slice sl has landed for every thread; everyone is done with slice sl - 1
+    if (RAGGED && KIND != FC_F16 && threadIdx.x < 64) { // (read from the iteration after the next on: two barriers away)
+      if (sl > 0 && sl + C::ST - 2 < n_slices) store_scales(sl + C::ST - 2);
+      if (sl + C::ST - 1 < n_slices) load_scales(sl + C::ST - 1);
+    }
     if (sl + C::ST - 1 < n_slices) issue(sl + C::ST - 1); // into the stage slice sl - 1 used
     cp_async_commit();
     { // split this slice of x into two fp16 terms
       const float* src = reinterpret_cast<const float*>(xf + st * C::XF_STAGE) + xr * XS + xk;
       const float4 xa = *reinterpret_cast<const float4*>(src), xb = *reinterpret_cast<const float4*>(src + 4);
-      const float v[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+      float v[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+      if (RAGGED) { // (an infinity or NaN counts as 2^128: it stays what it is, and nothing finite overflows beside it)
+        uint32_t mx = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) mx = max(mx, __float_as_uint(v[i]) & 0x7fffffffu);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        int sh = mx ? 14 - ((int)(mx >> 23) - 127) : 0;
+        sh = min(126, sh);
+        const float mul = __uint_as_float((uint32_t)(127 + sh) << 23);
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] *= mul;
+        if ((threadIdx.x & 15u) == 0) x_inv[sl & 1][xr] = __uint_as_float((uint32_t)(127 - sh) << 23);
+      }
       __half2 hi[4], lo[4];
 #pragma unroll
       for (int i = 0; i < 4; i++) {
-        const float c0 = fminf(fmaxf(v[2 * i], -65504.0f), 65504.0f), c1 = fminf(fmaxf(v[2 * i + 1], -65504.0f), 65504.0f);
-        hi[i] = __floats2half2_rn(c0, c1); // saturated instead of overflowing to infinity
+        // (not RAGGED: saturated instead of overflowing to infinity)
+        const float c0 = RAGGED ? v[2 * i] : fminf(fmaxf(v[2 * i], -65504.0f), 65504.0f);
+        const float c1 = RAGGED ? v[2 * i + 1] : fminf(fmaxf(v[2 * i + 1], -65504.0f), 65504.0f);
+        hi[i] = __floats2half2_rn(c0, c1);
         const float2 back = __half22float2(hi[i]);
-        lo[i] = __floats2half2_rn(c0 - back.x, c1 - back.y);
+        if (RAGGED)
+          lo[i] = __floats2half2_rn(fabsf(c0) < INFINITY ? c0 - back.x : 0.0f, fabsf(c1) < INFINITY ? c1 - back.y : 0.0f);
+        else
+          lo[i] = __floats2half2_rn(c0 - back.x, c1 - back.y);
       }
       // (rows of 128 halves, the 16-byte chunk index of odd rows XORed with 4: see qmatvec_mma_kernel)
       __half* dst = xs + (size_t)(sl & 1) * 2 * PART + xr * XS + (((xk >> 3) ^ ((xr & 1) << 2)) << 3);
@@ -452,6 +501,7 @@ __global__ void __launch_bounds__(128)
       *reinterpret_cast<uint4*>(dst + PART) = *reinterpret_cast<const uint4*>(lo);
     }
     __syncthreads();
+    const float inv0 = RAGGED ? x_inv[sl & 1][2 * t] : 1.0f, inv1 = RAGGED ? x_inv[sl & 1][2 * t + 1] : 1.0f;
     const __half* xhb = xs + (size_t)(sl & 1) * 2 * PART;
     const __half* xlb = xhb + PART;
     const uint8_t* wst = wq + st * C::W_STAGE;
@@ -518,10 +568,10 @@ __global__ void __launch_bounds__(128)
       mma_16816(c, a[0], bl.x, bl.y);
       mma_16816(c, a[1], bh.z, bh.w);
       mma_16816(c, a[1], bl.z, bl.w);
-      acc[0] = fmaf(dg, c[0], acc[0]);
-      acc[1] = fmaf(dg, c[1], acc[1]);
-      acc[2] = fmaf(dg8, c[2], acc[2]);
-      acc[3] = fmaf(dg8, c[3], acc[3]);
+      acc[0] = fmaf(dg * inv0, c[0], acc[0]);
+      acc[1] = fmaf(dg * inv1, c[1], acc[1]);
+      acc[2] = fmaf(dg8 * inv0, c[2], acc[2]);
+      acc[3] = fmaf(dg8 * inv1, c[3], acc[3]);
     }
   }
   cp_async_wait<0>();
@@ -542,13 +592,15 @@ __global__ void __launch_bounds__(128)
 }
 
 // y = epilogue(sum over splits, ascending split index)
+// (x_scale, nullable: the power of two of each row of x, which the ragged widths' sums still carry)
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, uint32_t splits, uint32_t m, uint32_t n,
-                                     float* __restrict__ y, Epilogue ep) {
+                                     float* __restrict__ y, Epilogue ep, const float* __restrict__ x_scale) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)m * n) return;
   float v = 0.0f;
   for (uint32_t s = 0; s < splits; s++) v += partial[(size_t)s * m * n + i];
   const uint32_t row = (uint32_t)(i % n);
+  if (x_scale) v *= x_scale[i / n];
   if (ep.bias) v += ep.bias[row];
   if (ep.act == ACT_GELU) v = gelu_f(v);
   if (ep.resid) v = ep.resid[i] + v;
@@ -580,24 +632,65 @@ int pick_nb(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, ui
   return launch<KIND, 8>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
 }
 
+int pick_kind(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, uint32_t m, float* y, float* part, uint32_t splits,
+              uint32_t bps, const Epilogue& ep) {
+  switch (w.kind) {
+    case FC_Q8_0: return pick_nb<FC_Q8_0>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+    case FC_FP8_E4M3: return pick_nb<FC_FP8_E4M3>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+    case FC_FP8_E5M2: return pick_nb<FC_FP8_E5M2>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+    case FC_MXFP4: return pick_nb<FC_MXFP4>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+    case FC_F16: return pick_nb<FC_F16>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+  }
+  return pick_nb<FC_Q4_0>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+}
+
+template <int KIND, bool RAGGED>
+int launch_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, float* part, dim3 grid, uint32_t bps, const Epilogue& ep) {
+  auto kern = qmatvec_mma8_kernel<KIND, RAGGED>;
+  static OncePerDevice attr;
+  if (attr.first(dev->ordinal)) FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma8<KIND>::SMEM));
+  FC_LAUNCH(dev, "qmatvec_mma8", kern<<<grid, 128, Mma8<KIND>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
+  return FC_OK;
+}
+template <bool RAGGED>
+int pick_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, float* part, dim3 grid, uint32_t bps, const Epilogue& ep) {
+  switch (w.kind) {
+    case FC_Q8_0: return launch_mma8<FC_Q8_0, RAGGED>(dev, w, x, m, y, part, grid, bps, ep);
+    case FC_FP8_E4M3: return launch_mma8<FC_FP8_E4M3, RAGGED>(dev, w, x, m, y, part, grid, bps, ep);
+    case FC_FP8_E5M2: return launch_mma8<FC_FP8_E5M2, RAGGED>(dev, w, x, m, y, part, grid, bps, ep);
+    case FC_MXFP4: return launch_mma8<FC_MXFP4, RAGGED>(dev, w, x, m, y, part, grid, bps, ep);
+    case FC_F16: return launch_mma8<FC_F16, RAGGED>(dev, w, x, m, y, part, grid, bps, ep);
+  }
+  return launch_mma8<FC_Q4_0, RAGGED>(dev, w, x, m, y, part, grid, bps, ep);
+}
+
 } // namespace
 
 bool qmatvec_mma_supports(const QMat& w, uint32_t m) {
   return (kind_has_scales(w.kind) || w.kind == FC_F16) && m >= 1 && m <= 64 && w.k % XS == 0;
 }
 
-// Device scratch the product needs: the two fp16 terms of x and the split-K partial sums.
+// The same kernels for a width of whole 32-blocks that is not whole slices (Epilogue::ragged: a stand-alone product, whose x
+// terms nobody else writes). Before, these widths took the FMA kernels, which multiply every weight by every row in
+// f32: 8 rows x 4064 x 11008 Q8_0 28 us instead of 162, 40 x 2080 x 11008 Q4_0 51 instead of 181, 2 x 2080 x 3001 Q4_0
+// 13 instead of 27; below one slice they keep them. Error against f64 1.3e-7..1.5e-7 of the result's norm, 1.2e-7..7.7e-7
+// there.
+bool qmatvec_mma_ragged_supports(const QMat& w, uint32_t m) {
+  return (kind_has_scales(w.kind) || w.kind == FC_F16) && m >= 2 && m <= 64 && w.k % QK == 0 && w.k % XS != 0 && w.k >= XS;
+}
+
+// Device scratch the product needs: the two fp16 terms of x (and their scales) and the split-K partial sums.
 size_t qmatvec_mma_scratch_bytes(uint32_t k, uint32_t n) {
   const uint32_t row_ctas = (n + ROWS_PER_CTA - 1) / ROWS_PER_CTA;
   uint32_t splits = 1; // an upper bound of what k_qmatvec_mma picks on any device of up to 160 SMs
   while (splits < 16 && row_ctas * splits < 8 * 160) splits *= 2;
-  return (size_t)2 * 64 * k * 2 + (size_t)splits * 64 * n * 4 + 512;
+  return (size_t)2 * 64 * k * 2 + (size_t)splits * 64 * n * 4 + 1024;
 }
 
 // 1..8 rows: x is converted inside the kernel; more CTAs than the wide variant wants (each holds few
 // bytes in flight), so K is split until the grid covers the SMs about eight times
 static int k_qmatvec_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, void* scratch) {
-  const uint32_t row_ctas = (w.n + ROWS_PER_CTA - 1) / ROWS_PER_CTA, slices = w.k / XS;
+  const uint32_t row_ctas = (w.n + ROWS_PER_CTA - 1) / ROWS_PER_CTA, slices = (w.k + XS - 1) / XS;
   const uint32_t want = 8 * (uint32_t)dev->prop.multiProcessorCount;
   uint32_t splits = (want + row_ctas - 1) / row_ctas;
   splits = splits < 1 ? 1 : splits > 16 ? 16 : splits;
@@ -609,39 +702,14 @@ static int k_qmatvec_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t
   float* partial = (float*)(((uintptr_t)scratch + (size_t)2 * 64 * w.k * 2 + 255) & ~(uintptr_t)255);
   float* part = splits > 1 ? partial : nullptr;
   dim3 grid(row_ctas, splits);
-  static OncePerDevice attr;
-  if (attr.first(dev->ordinal)) {
-    FC_CUDA(dev, cudaFuncSetAttribute(qmatvec_mma8_kernel<FC_Q8_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma8<FC_Q8_0>::SMEM));
-    FC_CUDA(dev, cudaFuncSetAttribute(qmatvec_mma8_kernel<FC_Q4_0>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma8<FC_Q4_0>::SMEM));
-    FC_CUDA(dev, cudaFuncSetAttribute(qmatvec_mma8_kernel<FC_FP8_E4M3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      Mma8<FC_FP8_E4M3>::SMEM));
-    FC_CUDA(dev, cudaFuncSetAttribute(qmatvec_mma8_kernel<FC_FP8_E5M2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      Mma8<FC_FP8_E5M2>::SMEM));
-    FC_CUDA(dev, cudaFuncSetAttribute(qmatvec_mma8_kernel<FC_MXFP4>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma8<FC_MXFP4>::SMEM));
-    FC_CUDA(dev, cudaFuncSetAttribute(qmatvec_mma8_kernel<FC_F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma8<FC_F16>::SMEM));
-  }
-  if (w.kind == FC_Q8_0)
-    FC_LAUNCH(dev, "qmatvec_mma8",
-              qmatvec_mma8_kernel<FC_Q8_0><<<grid, 128, Mma8<FC_Q8_0>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
-  else if (w.kind == FC_FP8_E4M3)
-    FC_LAUNCH(dev, "qmatvec_mma8",
-              qmatvec_mma8_kernel<FC_FP8_E4M3><<<grid, 128, Mma8<FC_FP8_E4M3>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
-  else if (w.kind == FC_FP8_E5M2)
-    FC_LAUNCH(dev, "qmatvec_mma8",
-              qmatvec_mma8_kernel<FC_FP8_E5M2><<<grid, 128, Mma8<FC_FP8_E5M2>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
-  else if (w.kind == FC_MXFP4)
-    FC_LAUNCH(dev, "qmatvec_mma8",
-              qmatvec_mma8_kernel<FC_MXFP4><<<grid, 128, Mma8<FC_MXFP4>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
-  else if (w.kind == FC_F16)
-    FC_LAUNCH(dev, "qmatvec_mma8",
-              qmatvec_mma8_kernel<FC_F16><<<grid, 128, Mma8<FC_F16>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
+  if (w.k % XS)
+    FC_TRY(pick_mma8<true>(dev, w, x, m, y, part, grid, bps, ep));
   else
-    FC_LAUNCH(dev, "qmatvec_mma8",
-              qmatvec_mma8_kernel<FC_Q4_0><<<grid, 128, Mma8<FC_Q4_0>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
+    FC_TRY(pick_mma8<false>(dev, w, x, m, y, part, grid, bps, ep));
   if (splits > 1) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
-              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep));
+              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep, nullptr));
   }
   return FC_OK;
 }
@@ -654,7 +722,7 @@ int k_flush_deferred(FcDevice* dev, const DeferredReduce& d) {
   ep.resid = d.resid;
   const size_t tot = (size_t)d.m * d.n;
   FC_LAUNCH(dev, "splitk_reduce",
-            splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(d.partial, d.splits, d.m, d.n, d.y, ep));
+            splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(d.partial, d.splits, d.m, d.n, d.y, ep, nullptr));
   return FC_OK;
 }
 
@@ -671,6 +739,13 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
   __half *xh, *xl;
   qmatvec_mma_split_ptrs(scratch, m, w.k, &xh, &xl, &mp);
   float* partial = ep.partial_at ? ep.partial_at : (float*)(((uintptr_t)(xl + (size_t)mp * w.k) + 255) & ~(uintptr_t)255);
+  float* x_scale = nullptr;
+  const bool ragged = w.k % XS != 0;
+  if (ragged) { // (a stand-alone product: nothing pending, no norm) every row brought into the fp16 range first
+    x_scale = partial;
+    partial += 64;
+    FC_TRY(k_rows_split(dev, x, m, mp, w.k, xh, xl, x_scale));
+  }
   const size_t total = (size_t)mp * w.k;
   DeferredReduce pend;
   if (ep.pending && ep.pending->splits) {
@@ -683,8 +758,8 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     else
       FC_TRY(k_flush_deferred(dev, d));
   }
-  if (ep.presplit) {
-    // the producer of x wrote xh / xl itself
+  if (ep.presplit || ragged) {
+    // the terms are there: the producer of x wrote them, or the launch above
   } else if (ep.norm != NORM_NONE) // x is the raw residual stream: normalise and split in one launch
     FC_LAUNCH(dev, "norm_split",
               norm_split_kernel<<<mp, 256, 0, dev->stream>>>(x, m, w.k, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, xh, xl, pend));
@@ -693,7 +768,7 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
   if (tx) return k_qgemm_tx(dev, w, xh, xl, mp, m, y, ep);
   // split K until the grid covers the SMs about twice: whole 128-k slices per split, the last split may be
   // shorter (K = 2816 is 22 slices: 11 splits of 2, where a power-of-two rule stops at 2 splits of 11)
-  const uint32_t row_ctas = (w.n + ROWS_PER_CTA - 1) / ROWS_PER_CTA, slices = w.k / XS;
+  const uint32_t row_ctas = (w.n + ROWS_PER_CTA - 1) / ROWS_PER_CTA, slices = (w.k + XS - 1) / XS;
   const uint32_t want = 2 * (uint32_t)dev->prop.multiProcessorCount;
   uint32_t splits = (want + row_ctas - 1) / row_ctas;
   splits = splits < 1 ? 1 : splits > 16 ? 16 : splits;
@@ -701,19 +776,8 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
   const uint32_t slices_per_split = (slices + splits - 1) / splits;
   splits = (slices + slices_per_split - 1) / slices_per_split; // no empty split
   const uint32_t bps = slices_per_split * (XS / QK);
-  float* part = splits > 1 ? partial : nullptr;
-  if (w.kind == FC_Q8_0)
-    FC_TRY(pick_nb<FC_Q8_0>(dev, w, xh, xl, m, y, part, splits, bps, ep));
-  else if (w.kind == FC_FP8_E4M3)
-    FC_TRY(pick_nb<FC_FP8_E4M3>(dev, w, xh, xl, m, y, part, splits, bps, ep));
-  else if (w.kind == FC_FP8_E5M2)
-    FC_TRY(pick_nb<FC_FP8_E5M2>(dev, w, xh, xl, m, y, part, splits, bps, ep));
-  else if (w.kind == FC_MXFP4)
-    FC_TRY(pick_nb<FC_MXFP4>(dev, w, xh, xl, m, y, part, splits, bps, ep));
-  else if (w.kind == FC_F16)
-    FC_TRY(pick_nb<FC_F16>(dev, w, xh, xl, m, y, part, splits, bps, ep));
-  else
-    FC_TRY(pick_nb<FC_Q4_0>(dev, w, xh, xl, m, y, part, splits, bps, ep));
+  float* part = splits > 1 || ragged ? partial : nullptr; // (a ragged width: the reduce takes the rows' scales back)
+  FC_TRY(pick_kind(dev, w, xh, xl, m, y, part, splits, bps, ep));
   if (splits > 1 && ep.defer_out && ep.act == ACT_NONE) { // the consumer's norm + split launch finishes the sum
     DeferredReduce& d = *ep.defer_out;
     d.partial = partial;
@@ -725,10 +789,10 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     d.y = y;
     return FC_OK;
   }
-  if (splits > 1) {
+  if (part) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
-              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep));
+              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep, x_scale));
   }
   return FC_OK;
 }

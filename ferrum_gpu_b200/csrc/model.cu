@@ -11,6 +11,8 @@
 #include <cmath>
 #include <cstring>
 
+#include "gemm_pair.cuh"
+#include "gemm_tc.cuh"
 #include "model.cuh"
 
 namespace {
@@ -199,6 +201,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
                   bool final_norm, DeferredReduce* tail = nullptr, bool embedded = false) {
   FcDevice* dev = m->dev;
   const uint32_t d = m->dim;
+  void* wide = mode != ATTN_DECODE && rows <= m->wide_rows ? m->wide : nullptr;
   if (!embedded) FC_TRY(k_embed(dev, m->tok, m->pos_table, ids, positions, rows, d, b.x)); // (else b.x holds the rows)
   // The two products that write the residual stream (wo, ff2) may leave their split-K sum to the norm
   // launch of the product that reads it next: `pend` is that unfinished sum, consumed (or finished on
@@ -207,6 +210,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
   for (auto& l : m->layers) {
     Epilogue e_qkv;
     e_qkv.scratch = m->mma_scratch;
+    e_qkv.wide_scratch = wide;
     e_qkv.bias = l.qkv.bias;
     e_qkv.pending = &pend;
     norm_before(m, e_qkv, l.norm1_g, l.norm1_b, b.h);
@@ -244,6 +248,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
     else
       FC_TRY(k_attn_prefill_cache_f32(dev, b.qkv, t, start, m->heads, m->kv_heads, m->hd, stream, l.kv, m->ctx, b.attn));
     e_wo.scratch = m->mma_scratch;
+    e_wo.wide_scratch = wide;
     e_wo.bias = l.wo.bias;
     e_wo.resid = b.x;
     made = DeferredReduce();
@@ -252,6 +257,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
     pend = made;
     Epilogue e_ff1;
     e_ff1.scratch = m->mma_scratch;
+    e_ff1.wide_scratch = wide;
     e_ff1.bias = l.ff1.bias;
     e_ff1.act = m->arch == ARCH_GPT2 ? ACT_GELU : ACT_NONE;
     e_ff1.pending = &pend;
@@ -302,24 +308,17 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
   return FC_OK;
 }
 
-int carve_pass(FcModel* m, uint32_t rows, PassBufs* b, size_t extra_bytes) {
+int carve_pass(FcModel* m, uint32_t rows, PassBufs* b, size_t extra_bytes, int mode) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t need = al((size_t)rows * m->dim * 4) * 2 + al((size_t)rows * m->qkv_w() * 4) + al((size_t)rows * m->qd() * 4) +
                       al((size_t)rows * m->ff1_w() * 4) + al((size_t)rows * m->hidden * 4) + al(extra_bytes) + 4096;
-  FC_TRY(arena_reserve(m, need));
+  FC_TRY(arena_reserve_wide(m, need, rows, mode));
   b->x = (float*)arena_take(m, (size_t)rows * m->dim * 4);
   b->h = (float*)arena_take(m, (size_t)rows * m->dim * 4);
   b->qkv = (float*)arena_take(m, (size_t)rows * m->qkv_w() * 4);
   b->attn = (float*)arena_take(m, (size_t)rows * m->qd() * 4);
   b->ff = (float*)arena_take(m, (size_t)rows * m->ff1_w() * 4);
   b->act = (float*)arena_take(m, (size_t)rows * m->hidden * 4);
-  return FC_OK;
-}
-
-int check_ids(FcModel* m, const int32_t* ids, size_t n) {
-  for (size_t i = 0; i < n; i++)
-    if (ids[i] < 0 || (uint32_t)ids[i] >= m->vocab)
-      return fc_fail(m->dev, FC_ERR_RANGE, "index %d is out of range for %u entries", ids[i], m->vocab);
   return FC_OK;
 }
 
@@ -337,8 +336,43 @@ int upload_positions(FcModel* m, uint32_t n_seqs, uint32_t t, uint32_t start, in
 
 } // namespace
 
+int check_ids(FcModel* m, const int32_t* ids, size_t n) {
+  for (size_t i = 0; i < n; i++)
+    if (ids[i] < 0 || (uint32_t)ids[i] >= m->vocab)
+      return fc_fail(m->dev, FC_ERR_RANGE, "index %d is out of range for %u entries", ids[i], m->vocab);
+  return FC_OK;
+}
+
+int arena_reserve_wide(FcModel* m, size_t bytes, size_t rows, int mode) {
+  size_t wide = 0;
+  auto add = [&](const QMat& w) {
+    if (mode == FC_TENSOR_F16) {
+      if (tp_takes(m->dev, w, (uint32_t)rows, EPI_LSE)) wide = tp_workspace_bytes(w) > wide ? tp_workspace_bytes(w) : wide;
+    } else if (qgemm_pair_takes(w, (uint32_t)rows)) {
+      const size_t b = qgemm_pair_scratch_bytes(m->dev, w.k, w.n, (uint32_t)rows);
+      wide = b > wide ? b : wide;
+    }
+  };
+  for (const auto& l : m->layers)
+    for (const FcQWeight* q : {l.qkv.w, l.wo.w, l.ff1.w, l.ff2.w}) add(q->m);
+  add(m->head_view);
+  const size_t at = (bytes + 1023) & ~(size_t)1023;
+  if (wide) {
+    const int rc = arena_reserve(m, at + wide);
+    if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
+    if (rc == FC_OK) {
+      m->wide = m->arena.base + at;
+      m->wide_rows = rows;
+      return FC_OK;
+    }
+  }
+  return arena_reserve(m, bytes);
+}
+
 int arena_reserve(FcModel* m, size_t bytes) {
   m->arena.off = 0;
+  m->wide = nullptr;
+  m->wide_rows = 0;
   if (bytes <= m->arena.cap) return FC_OK;
   FC_CUDA(m->dev, cudaStreamSynchronize(m->dev->stream));
   if (m->arena.base) cudaFree(m->arena.base);
@@ -907,7 +941,7 @@ FC_API int fc_model_prefill(FcModel* m, uint32_t stream_id, const int32_t* ids, 
     if (start != 0)
       return fc_fail(dev, FC_ERR_UNSUPPORTED, "the tensor-core prefill fills an empty stream: stream %u holds %u tokens", stream_id,
                      start);
-    FC_TRY(arena_reserve(m, (size_t)n * 8 + 512 + (size_t)n * m->dim * 2 + 256 + model_tc_trunk_bytes(m, n) + 4096));
+    FC_TRY(arena_reserve_wide(m, (size_t)n * 8 + 512 + (size_t)n * m->dim * 2 + 256 + model_tc_trunk_bytes(m, n) + 4096, n, mode));
     int32_t* t_ids = (int32_t*)arena_take(m, (size_t)n * 4);
     int32_t* t_pos = (int32_t*)arena_take(m, (size_t)n * 4);
     __half* hid = (__half*)arena_take(m, (size_t)n * m->dim * 2);
@@ -929,7 +963,7 @@ FC_API int fc_model_prefill(FcModel* m, uint32_t stream_id, const int32_t* ids, 
     return FC_OK;
   }
   PassBufs b;
-  FC_TRY(carve_pass(m, n, &b, (size_t)n * 12 + 768));
+  FC_TRY(carve_pass(m, n, &b, (size_t)n * 12 + 768, FC_EXACT_F32));
   int32_t* d_ids = (int32_t*)arena_take(m, (size_t)n * 4);
   int32_t* d_pos = (int32_t*)arena_take(m, (size_t)n * 4);
   int32_t* d_slots = (int32_t*)arena_take(m, (size_t)n * 4); // every row writes the same stream's cache
@@ -965,7 +999,7 @@ FC_API int fc_model_forward_all(FcModel* m, const int32_t* ids, uint32_t n, floa
   const size_t extra = (size_t)n * 8 + 512 + (size_t)n * m->vocab * 4 + 256 + (size_t)n * m->dim * 2 + 256 +
                        (mode == FC_TENSOR_F16 ? model_tc_trunk_bytes(m, n) : 0);
   PassBufs b;
-  FC_TRY(carve_pass(m, n, &b, extra));
+  FC_TRY(carve_pass(m, n, &b, extra, mode));
   int32_t* d_ids = (int32_t*)arena_take(m, (size_t)n * 4);
   int32_t* d_pos = (int32_t*)arena_take(m, (size_t)n * 4);
   float* logits = (float*)arena_take(m, (size_t)n * m->vocab * 4);
@@ -973,7 +1007,9 @@ FC_API int fc_model_forward_all(FcModel* m, const int32_t* ids, uint32_t n, floa
   FC_TRY(upload_ids(m, ids, n, d_ids));
   if (mode == FC_EXACT_F32) {
     FC_TRY(run_stack_f32(m, b, d_ids, d_pos, nullptr, n, ATTN_STATELESS, 1, n, 0, 0, true));
-    FC_TRY(k_qlinear_f32(dev, m->head_view, b.h, n, logits, Epilogue()));
+    Epilogue e_head;
+    e_head.wide_scratch = m->wide;
+    FC_TRY(k_qlinear_f32(dev, m->head_view, b.h, n, logits, e_head));
   } else if (mode == FC_TENSOR_F16) {
     __half* hid = (__half*)arena_take(m, (size_t)n * m->dim * 2);
     FC_TRY(model_trunk_tc(m, d_ids, d_pos, 1, n, hid));

@@ -69,6 +69,8 @@ struct FcModel {
   int32_t* d_chain_log = nullptr; // [ctx][max_streams]
   uint32_t* d_chain_cnt = nullptr;
   Arena arena;
+  void* wide = nullptr;   // behind the arena's carved part: workspace of the products of many rows
+  size_t wide_rows = 0;   // rows it is sized for (0: none)
   void* tc = nullptr; // state of the bf16 tensor-core path (built on first use)
   void* dc = nullptr; // state of the one-launch single-stream decode (decode_cluster.cu; probed on first use)
 
@@ -78,9 +80,13 @@ struct FcModel {
   uint32_t ff1_w() const { return arch == ARCH_LLAMA ? 2 * hidden : hidden; }
 };
 
+int check_ids(FcModel* m, const int32_t* ids, size_t n); // every id inside the vocabulary (model.cu)
 // Workspace helpers (model.cu)
 int arena_reserve(FcModel* m, size_t bytes);
 void* arena_take(FcModel* m, size_t bytes);
+// arena_reserve with the products' workspace for passes of up to `rows` rows in `mode` behind it (m->wide); without
+// that workspace where there is no room for it.
+int arena_reserve_wide(FcModel* m, size_t bytes, size_t rows, int mode);
 
 // Batched passes in exact f32 (model.cu).
 // rows = n_seqs * t; ids/positions on the device; writes final-norm hidden states to `hidden_out`

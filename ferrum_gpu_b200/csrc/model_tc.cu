@@ -64,23 +64,53 @@ int model_interleave_gate_up(FcDevice* dev, FcQWeight* w, uint32_t hidden, uint3
   return FC_OK;
 }
 
+void qweight_workspace_free(FcQWeight* w) {
+  for (void* p : w->outgrown) workspace_free(w->dev, p);
+  w->outgrown.clear();
+  if (w->tc_cache) workspace_free(w->dev, w->tc_cache);
+  if (w->mma_scratch) workspace_free(w->dev, w->mma_scratch);
+  w->tc_cache = w->mma_scratch = nullptr;
+  w->tc_cache_bytes = 0;
+}
+
+int qweight_workspace(FcQWeight* w, size_t bytes) {
+  if (!w->captured && stream_capturing(w->dev)) w->captured = true;
+  if (bytes <= w->tc_cache_bytes) return FC_OK;
+  FcDevice* dev = w->dev;
+  if (stream_capturing(dev)) return fc_fail(dev, FC_ERR_OOM, "a %zu-byte product workspace cannot be allocated during a capture", bytes);
+  if (w->tc_cache && w->captured)
+    w->outgrown.push_back(w->tc_cache);
+  else if (w->tc_cache)
+    workspace_free(dev, w->tc_cache);
+  w->tc_cache = nullptr;
+  w->tc_cache_bytes = 0;
+  const cudaError_t e = workspace_alloc(dev, &w->tc_cache, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    w->tc_cache = nullptr;
+    return fc_fail(dev, FC_ERR_OOM, "cannot allocate a %zu-byte product workspace: %s", bytes, cudaGetErrorString(e));
+  }
+  w->tc_cache_bytes = bytes;
+  return FC_OK;
+}
+
 int k_qgemm_tc(FcDevice* dev, FcQWeight* w, const float* x_dev, uint32_t m, float* y_dev) {
   if (m == 0) return FC_OK;
-  const size_t need = (size_t)m * w->m.k * 2;
-  if (need > w->tc_cache_bytes) {
-    FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
-    if (w->tc_cache) cudaFree(w->tc_cache);
-    w->tc_cache = nullptr;
-    w->tc_cache_bytes = 0;
-    FC_CUDA(dev, cudaMalloc(&w->tc_cache, need));
-    w->tc_cache_bytes = need;
+  const size_t a_bytes = al((size_t)m * w->m.k * 2);
+  bool wide = tp_takes(dev, w->m, m, EPI_F32);
+  if (wide) {
+    const int rc = qweight_workspace(w, a_bytes + tp_workspace_bytes(w->m));
+    if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
+    wide = rc == FC_OK; // (no room for the decoded weights: the product decodes them itself)
   }
+  if (!wide) FC_TRY(qweight_workspace(w, a_bytes));
   __half* a = (__half*)w->tc_cache;
   FC_TRY(k_f32_to_f16(dev, x_dev, (size_t)m * w->m.k, a));
   TcArgs t;
   t.m = m;
   t.out_f32 = y_dev;
   t.ldo = w->m.n;
+  if (wide) t.wide = (uint8_t*)w->tc_cache + a_bytes;
   return k_qgemm_tc_f16(dev, w->m, a, EPI_F32, t);
 }
 
@@ -90,6 +120,7 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
   FC_TRY(check_tc_shapes(m));
   if (cache_stream >= 0 && n_seqs != 1) return fc_fail(dev, FC_ERR_ARG, "one sequence fills one stream's cache");
   const uint32_t rows = n_seqs * t, d = m->dim;
+  void* wide = rows <= m->wide_rows ? m->wide : nullptr;
   float* x = (float*)arena_take(m, (size_t)rows * d * 4);
   __half* h = (__half*)arena_take(m, (size_t)rows * d * 2);
   __half* qkv = (__half*)arena_take(m, (size_t)rows * m->qkv_w() * 2);
@@ -100,7 +131,7 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
   for (auto& l : m->layers) {
     FC_TRY(k_norm_f16(dev, ln, x, l.norm1_g, l.norm1_b, rows, d, m->eps, h));
     TcArgs a_qkv;
-    a_qkv.m = rows, a_qkv.bias = l.qkv.bias, a_qkv.out_f16 = qkv, a_qkv.ldo = m->qkv_w();
+    a_qkv.wide = wide, a_qkv.m = rows, a_qkv.bias = l.qkv.bias, a_qkv.out_f16 = qkv, a_qkv.ldo = m->qkv_w();
     // (RoPE fused into this product's epilogue was measured at a third of the plain fp16 store's rate - the
     // table gathers - so the rotation runs as its own 16-byte-vectorised pass over the q and k columns.)
     FC_TRY(k_qgemm_tc_f16(dev, l.qkv.w->m, h, EPI_F16, a_qkv));
@@ -114,7 +145,7 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
     FC_TRY(k_qgemm_tc_f16(dev, l.wo.w->m, attn, EPI_RESID, a_wo));
     FC_TRY(k_norm_f16(dev, ln, x, l.norm2_g, l.norm2_b, rows, d, m->eps, h));
     TcArgs a_ff1;
-    a_ff1.m = rows, a_ff1.bias = l.ff1.bias, a_ff1.out_f16 = act, a_ff1.ldo = m->hidden;
+    a_ff1.wide = wide, a_ff1.m = rows, a_ff1.bias = l.ff1.bias, a_ff1.out_f16 = act, a_ff1.ldo = m->hidden;
     if (m->arch == ARCH_LLAMA) {
       FC_TRY(k_qgemm_tc_f16(dev, l.ff1.w->m, h, EPI_SWIGLU, a_ff1));
     } else {
@@ -122,7 +153,7 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
       FC_TRY(k_qgemm_tc_f16(dev, l.ff1.w->m, h, EPI_F16, a_ff1));
     }
     TcArgs a_ff2;
-    a_ff2.m = rows, a_ff2.bias = l.ff2.bias, a_ff2.out_f32 = x, a_ff2.ldo = d;
+    a_ff2.wide = wide, a_ff2.m = rows, a_ff2.bias = l.ff2.bias, a_ff2.out_f32 = x, a_ff2.ldo = d;
     FC_TRY(k_qgemm_tc_f16(dev, l.ff2.w->m, act, EPI_RESID, a_ff2));
   }
   return k_norm_f16(dev, ln, x, m->normf_g, m->normf_b, rows, d, m->eps, hidden_out);
@@ -132,6 +163,7 @@ int model_head_partial_tc(FcModel* m, const __half* hidden, const int32_t* targe
   const uint32_t tiles = (m->v1 - m->v0 + TC_BN - 1) / TC_BN;
   float* tile_partials = (float*)arena_take(m, (size_t)rows * tiles * 16);
   TcArgs a;
+  if (rows <= m->wide_rows) a.wide = m->wide;
   a.m = rows, a.targets = targets, a.v0 = m->v0, a.partial = tile_partials;
   FC_TRY(k_qgemm_tc_f16(m->dev, m->head_view, hidden, EPI_LSE, a));
   return k_partial_merge(m->dev, tile_partials, tiles, rows, partial);
@@ -139,6 +171,7 @@ int model_head_partial_tc(FcModel* m, const __half* hidden, const int32_t* targe
 
 int model_logits_tc(FcModel* m, const __half* hidden, uint32_t rows, float* logits) {
   TcArgs a;
+  if (rows <= m->wide_rows) a.wide = m->wide;
   a.m = rows, a.out_f32 = logits, a.ldo = m->v1 - m->v0;
   return k_qgemm_tc_f16(m->dev, m->head_view, hidden, EPI_F32, a);
 }

@@ -1,6 +1,6 @@
 // C ABI of the stand-alone quantised weight: upload, read-back, dequantise, product. The
 // counterpart of ferrum_wgpu::ops::quant's public functions (ferrum_wgpu/src/ops/quant.rs).
-#include "common.cuh"
+#include "gemm_pair.cuh"
 
 int k_qgemm_tc(FcDevice* dev, FcQWeight* w, const float* x_dev, uint32_t m, float* y_dev); // model_tc.cu
 int tc_check_errors(FcDevice* dev);                                                            // gemm_tc.cu
@@ -78,8 +78,7 @@ FC_API int fc_qweight_destroy(FcQWeight* w) {
   if (!w) return FC_ERR_ARG;
   cudaSetDevice(w->dev->ordinal);
   cudaStreamSynchronize(w->dev->stream);
-  if (w->tc_cache) cudaFree(w->tc_cache);
-  if (w->mma_scratch) cudaFree(w->mma_scratch);
+  qweight_workspace_free(w);
   qweight_free(w);
   return FC_OK;
 }
@@ -136,9 +135,23 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
   cudaSetDevice(dev->ordinal);
   if (mode == FC_EXACT_F32) {
     Epilogue ep;
-    if (qmatvec_mma_supports(w->m, m)) { // 1..64 rows: the decode tensor product needs scratch
-      if (!w->mma_scratch) FC_CUDA(dev, cudaMalloc(&w->mma_scratch, qmatvec_mma_scratch_bytes(w->m.k, w->m.n)));
+    ep.ragged = true;
+    if ((m > 1 || dev->matvec_choice) && (qmatvec_mma_supports(w->m, m) || qmatvec_mma_ragged_supports(w->m, m))) {
+      // up to 64 rows: the decode tensor product needs scratch (one row takes kernels that need none)
+      // (a first call during a capture, or without room: the f32 kernels need none)
+      if (!w->mma_scratch && !stream_capturing(dev)) {
+        const cudaError_t e = workspace_alloc(dev, &w->mma_scratch, qmatvec_mma_scratch_bytes(w->m.k, w->m.n));
+        if (e != cudaSuccess) {
+          cudaGetLastError();
+          w->mma_scratch = nullptr;
+          if (e != cudaErrorMemoryAllocation) return fc_fail(dev, FC_ERR_DEVICE, "product scratch: %s", cudaGetErrorString(e));
+        }
+      }
       ep.scratch = w->mma_scratch;
+    } else if (qgemm_pair_takes(w->m, m)) {
+      const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m));
+      if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
+      ep.wide_scratch = w->tc_cache; // (no room for it: the tiled f32 kernel needs none)
     }
     return k_qlinear_f32(dev, w->m, x_dev, m, y_dev, ep);
   }

@@ -102,10 +102,29 @@ FC_API int fc_device_open(int ordinal, FcDevice** out) {
   return FC_OK;
 }
 
+cudaError_t workspace_alloc(FcDevice* dev, void** p, size_t bytes) {
+  return dev->workspaces ? cudaMallocFromPoolAsync(p, bytes, dev->workspaces, dev->stream) : cudaMalloc(p, bytes);
+}
+void workspace_free(FcDevice* dev, void* p) {
+  if (dev->workspaces)
+    cudaFreeAsync(p, dev->stream);
+  else
+    cudaFree(p); // (waits for the device)
+}
+bool stream_capturing(FcDevice* dev) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(dev->stream, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return true; // (a capture on another stream forbids the query: allocate nothing)
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
 FC_API int fc_device_close(FcDevice* dev) {
   if (!dev) return FC_ERR_ARG;
   cudaSetDevice(dev->ordinal);
   cudaStreamSynchronize(dev->stream);
+  if (dev->workspaces) cudaMemPoolDestroy(dev->workspaces);
   if (dev->pinned) cudaFreeHost(dev->pinned);
   if (dev->d_flag) cudaFree(dev->d_flag);
   for (auto& s : dev->spans) {

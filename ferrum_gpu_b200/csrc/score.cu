@@ -37,7 +37,9 @@ size_t chunk_bytes(const FcModel* m, size_t rows, int mode) {
 // reduced to per-row partials.
 static int head_partial_f32(FcModel* m, const float* hidden, const int32_t* targets, uint32_t rows, float* logits_ws,
                             float* partial) {
-  FC_TRY(k_qlinear_f32(m->dev, m->head_view, hidden, rows, logits_ws, Epilogue()));
+  Epilogue ep;
+  if (rows <= m->wide_rows) ep.wide_scratch = m->wide;
+  FC_TRY(k_qlinear_f32(m->dev, m->head_view, hidden, rows, logits_ws, ep));
   return k_score_partial(m->dev, logits_ws, targets, rows, m->v1 - m->v0, m->v0, partial);
 }
 
@@ -59,7 +61,7 @@ FC_API int fc_model_score_dev(FcModel* m, const int32_t* ids_dev, uint32_t n_seq
   while (per > 1 && chunk_bytes(m, (size_t)per * t, mode) > cap) per = (per + 1) / 2;
   const size_t rows_max = (size_t)per * t;
   const size_t lp_bytes = logprob_dev ? 0 : al((size_t)n_seqs * t * 4);
-  FC_TRY(arena_reserve(m, chunk_bytes(m, rows_max, mode) + lp_bytes));
+  FC_TRY(arena_reserve_wide(m, chunk_bytes(m, rows_max, mode) + lp_bytes, rows_max, mode));
   float* lp_all = logprob_dev ? logprob_dev : (float*)arena_take(m, (size_t)n_seqs * t * 4);
   int32_t* in_ids = (int32_t*)arena_take(m, rows_max * 4);
   int32_t* targets = (int32_t*)arena_take(m, rows_max * 4);
@@ -117,7 +119,7 @@ FC_API int fc_model_trunk_dev(FcModel* m, const int32_t* ids_dev, uint32_t n_seq
   if (seq_len == 0 || seq_len > m->ctx) return fc_fail(dev, FC_ERR_SHAPE, "sequence length %u must be in 1..=%u", seq_len, m->ctx);
   if (n_seqs == 0) return FC_OK;
   const size_t rows = (size_t)n_seqs * seq_len;
-  FC_TRY(arena_reserve(m, chunk_bytes(m, rows, FC_TENSOR_F16)));
+  FC_TRY(arena_reserve_wide(m, chunk_bytes(m, rows, FC_TENSOR_F16), rows, mode));
   int32_t* positions = (int32_t*)arena_take(m, rows * 4);
   // positions 0..seq_len-1 per sequence (score_prep with a virtual extra token would drop the
   // last row; here every row is kept)
@@ -140,7 +142,7 @@ FC_API int fc_model_head_partial_dev(FcModel* m, const void* hidden_dev, const i
   cudaSetDevice(dev->ordinal);
   if (rows == 0) return FC_OK;
   if (mode == FC_TENSOR_F16) {
-    FC_TRY(arena_reserve(m, model_tc_head_bytes(m, rows)));
+    FC_TRY(arena_reserve_wide(m, model_tc_head_bytes(m, rows), rows, mode));
     return model_head_partial_tc(m, (const __half*)hidden_dev, targets_dev, rows, partial_dev);
   }
   if (mode != FC_EXACT_F32) return fc_fail(dev, FC_ERR_ARG, "unknown arithmetic mode %d", mode);
@@ -148,7 +150,7 @@ FC_API int fc_model_head_partial_dev(FcModel* m, const void* hidden_dev, const i
   const size_t vs = m->v1 - m->v0;
   size_t per = rows;
   while (per > 1 && per * vs * 4 > ((size_t)2 << 30)) per = (per + 1) / 2;
-  FC_TRY(arena_reserve(m, al(per * vs * 4) + 4096));
+  FC_TRY(arena_reserve_wide(m, al(per * vs * 4) + 4096, per, mode));
   float* logits_ws = (float*)arena_take(m, per * vs * 4);
   for (size_t r0 = 0; r0 < rows; r0 += per) {
     const uint32_t nr = (uint32_t)(rows - r0 < per ? rows - r0 : per);

@@ -1,0 +1,125 @@
+"""The products of many rows on CTA pairs and the decode products at widths that are not whole 128s, at the sizes where
+they can go wrong: tile edges, K tails, one column, splits of K; and the tiled exact attention. References are float64.
+
+Bounds of the exact class: the two fp16 terms leave 2^-22 of each factor and the dropped cross term 2^-22 of the
+product, f32 sums of 128 k (rounded toward zero, one unit of 2^-23 per 16 k) are added in f32: below 16 x 2^-23 = 2e-6
+of sum |x w| whatever the width."""
+import numpy as np
+import pytest
+
+from ferrum_gpu_b200 import CudaGpt2, CudaLlama, Mode, QKind, linear_q, upload_quantised
+from ferrum_gpu_b200.hostmodel import Gpt2Config, LlamaConfig, random_gpt2, random_llama, random_tokens
+from oracle import oracle as orc
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+
+EXACT = 2e-6  # of sum |x w|
+
+
+def _problem(dev, kind, m, k, n, seed=1, mag=1.0):
+    rng = np.random.default_rng(seed)
+    qw = upload_quantised(dev, kind, (rng.standard_normal(k * n) * 0.02).astype(np.float32), k, n)
+    x = (rng.standard_normal((m, k)) * mag).astype(np.float32)
+    w = qw.dequantised().reshape(n, k).astype(np.float64)
+    return qw, x, x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0])
+@pytest.mark.parametrize("m,k,n", [(65, 32, 1), (65, 64, 255), (127, 96, 256), (128, 4096, 257), (129, 160, 40), (192, 800, 1000),
+                                   (300, 2080, 513), (70, 1024, 9000), (1500, 128, 300), (600, 96, 3000), (300, 32, 20000)])
+@pytest.mark.parametrize("mag", [1.0, 1e-30, 1e30])
+def test_exact_products_of_many_rows(dev, kind, m, k, n, mag):
+    qw, x, want, scale = _problem(dev, kind, m, k, n, mag=mag)
+    got = linear_q(dev, x, qw, m).reshape(m, n)
+    assert np.all(np.abs(got - want) <= EXACT * scale), (kind, m, k, n, np.max(np.abs(got - want) / scale))
+    assert np.array_equal(got, linear_q(dev, x, qw, m).reshape(m, n)), "repeated runs are bit-identical"
+    qw.close()
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0])
+@pytest.mark.parametrize("m,k", [(100, 256), (80, 2048)])
+def test_rows_with_infinities_and_nans_and_zero_rows(dev, kind, m, k):
+    n = 300
+    qw, x, _, _ = _problem(dev, kind, m, k, n)
+    clean = linear_q(dev, x, qw, m).reshape(m, n)
+    x[3, 5], x[7, k - 1], x[11, 0], x[20], x[30, 1] = np.inf, -np.inf, np.nan, 0.0, 3e38
+    w = qw.dequantised().reshape(n, k).astype(np.float64)
+    got = linear_q(dev, x, qw, m).reshape(m, n)
+    bad = [3, 7, 11]
+    with np.errstate(invalid="ignore", over="ignore"):
+        want = (x.astype(np.float64)[bad][:, None, :] * w[None]).sum(-1)
+    for i, r in enumerate(bad):
+        assert np.array_equal(np.isnan(got[r]), np.isnan(want[i])) and np.array_equal(got[r][~np.isnan(want[i])], want[i][~np.isnan(want[i])])
+    assert np.all(got[20] == 0)
+    others = [r for r in range(m) if r not in bad + [20, 30]]
+    assert np.array_equal(got[others], clean[others]), "other rows do not change"
+    qw.close()
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0, QKind.F16, QKind.FP8_E4M3, QKind.MXFP4])
+@pytest.mark.parametrize("m,k,n", [(2, 160, 5), (3, 224, 64), (8, 4064, 130), (5, 1056, 3000), (9, 160, 70), (16, 288, 65), (33, 2080, 300),
+                                   (64, 1120, 1000), (40, 4064, 20)])
+@pytest.mark.parametrize("mag", [1.0, 1e-20, 1e20])
+def test_decode_products_at_ragged_widths(dev, kind, m, k, n, mag):
+    qw, x, want, scale = _problem(dev, kind, m, k, n, mag=mag)
+    got = linear_q(dev, x, qw, m).reshape(m, n)
+    assert np.all(np.abs(got - want) <= EXACT * scale), (kind, m, k, n, np.max(np.abs(got - want) / scale))
+    qw.close()
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0])
+@pytest.mark.parametrize("m,k,n", [(1024, 64, 256), (1025, 192, 257), (1300, 768, 1000), (2049, 128, 8)])
+def test_tensor_products_of_many_rows(dev, kind, m, k, n):
+    """fp16 operands, one rounding each (2^-11), products exact, f32 sums: 2^-10 of sum |x w| bounds them."""
+    qw, x, want, scale = _problem(dev, kind, m, k, n)
+    got = linear_q(dev, x, qw, m, Mode.TENSOR_F16).reshape(m, n)
+    assert np.all(np.abs(got - want) <= 2.0 ** -10 * scale), (kind, m, k, n, np.max(np.abs(got - want) / scale))
+    # the rows that a smaller call has too: the same operands through the kernel that decodes the weights itself
+    few = linear_q(dev, x[:200], qw, 200, Mode.TENSOR_F16).reshape(200, n)
+    assert np.all(np.abs(got[:200] - few) <= 1e-5 * scale[:200] + 1e-30)
+    qw.close()
+
+
+@pytest.mark.parametrize("arch", ["llama", "gpt2"])
+@pytest.mark.parametrize("t", [31, 32, 64, 65, 130, 200])
+def test_exact_prefill_and_scoring_match_the_oracle(dev, arch, t):
+    if arch == "llama":
+        cfg = LlamaConfig(vocab=300, ctx=256, dim=128, heads=4, kv_heads=2, head_dim=64, layers=2, hidden=160, rope_dim=64)
+        m = random_llama(cfg, seed=3, std=0.05)
+        oracle = orc.OracleLlama(orc.dequantised_llama(m, int(QKind.Q8_0), snap_embedding=False), threads=4)
+        g = CudaLlama(dev, m, QKind.Q8_0)
+    else:
+        cfg = Gpt2Config(vocab=300, ctx=256, dim=128, heads=2, layers=2, hidden=160)
+        m = random_gpt2(cfg, seed=3, std=0.05)
+        oracle = orc.OracleGpt2(orc.dequantised_gpt2(m, int(QKind.Q8_0), snap_embedding=False), threads=4)
+        g = CudaGpt2(dev, m, QKind.Q8_0)
+    ids = random_tokens(t, t, cfg.vocab)
+    whole = g.prefill(ids)
+    g.reset(0)
+    head = max(1, t - 40)
+    g.prefill(ids[:head])
+    assert orc.max_rel_err(g.prefill(ids[head:]), whole) < 2e-5, "a prompt in two passes"
+    lp, _, _ = g.score_batch(np.stack([ids, ids[::-1]]), Mode.EXACT_F32)
+    for s, seq in enumerate([ids, np.ascontiguousarray(ids[::-1])]):
+        want, _ = oracle.score(seq)
+        assert np.max(np.abs(lp[s] - want)) < 5e-5
+    g.close()
+
+
+@pytest.mark.parametrize("poison", [np.inf, np.nan])
+def test_a_later_row_with_infinities_does_not_reach_earlier_rows(dev, poison):
+    """Causality at the bit level: a token whose embedding overflows changes nothing before its position, also inside the
+    same tile of the tiled attention."""
+    cfg = LlamaConfig(vocab=64, ctx=128, dim=128, heads=2, kv_heads=1, head_dim=64, layers=1, hidden=128, rope_dim=64)
+    m = random_llama(cfg, seed=7, std=0.05)
+    tok = np.asarray(m.tok, dtype=np.float32).reshape(cfg.vocab, cfg.dim).copy()
+    tok[63, 0] = poison
+    m.tok = tok.reshape(np.asarray(m.tok).shape)
+    g = CudaLlama(dev, m, QKind.Q8_0)
+    ids = (np.arange(100) % 60).astype(np.int32)
+    clean = g.forward_all(ids)
+    ids[70] = 63
+    got = g.forward_all(ids)
+    assert np.array_equal(got[:70], clean[:70]) and np.all(np.isnan(got[70]))
+    g.close()
