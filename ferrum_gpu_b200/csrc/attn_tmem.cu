@@ -75,25 +75,31 @@ constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint64_t desc_at(uint32_t smem_addr) { return ((uint64_t)DESC_HI << 32) | (smem_addr >> 4); }
 
 struct Item { // one (sequence, head, 256-row query block)
-  uint32_t qb, h, seq, n0, n1, n_max;
+  uint32_t qb, h, row0, t, n0, n1, n_max; // row0, t: the sequence's first row in the buffer and its length
 };
-__device__ __forceinline__ Item item_at(uint32_t w, uint32_t nqb, uint32_t heads, uint32_t n_seqs, uint32_t t) {
+__device__ __forceinline__ Item item_at(uint32_t w, uint32_t nqb, uint32_t heads, uint32_t n_seqs, uint32_t t, const uint4* blocks) {
   Item it;
-  const uint32_t per = heads * n_seqs;
-  it.qb = nqb - 1 - w / per; // heaviest (latest) query blocks first
-  const uint32_t hs = w % per;
-  it.seq = hs / heads;
-  it.h = hs % heads;
+  if (blocks) { // sequences of unequal length: the caller's list of query blocks, heaviest first
+    const uint4 b = __ldg(blocks + w / heads);
+    it.row0 = b.x, it.t = b.y, it.qb = b.z;
+    it.h = w % heads;
+  } else {
+    const uint32_t per = heads * n_seqs;
+    it.qb = nqb - 1 - w / per; // heaviest (latest) query blocks first
+    const uint32_t hs = w % per;
+    it.row0 = hs / heads * t, it.t = t;
+    it.h = hs % heads;
+  }
   // key tiles of each half: through its diagonal tile; half 1 is idle when it holds no row of the sequence
   it.n0 = 2 * it.qb + 1;
-  it.n1 = (it.qb * 256 + 128 < t) ? 2 * it.qb + 2 : 0;
+  it.n1 = (it.qb * 256 + 128 < it.t) ? 2 * it.qb + 2 : 0;
   it.n_max = it.n0 > it.n1 ? it.n0 : it.n1;
   return it;
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
     attn_tmem_kernel(const __grid_constant__ CUtensorMap tmap, uint32_t n_seqs, uint32_t t, uint32_t heads, uint32_t kv_heads,
-                     __half* __restrict__ out, int* __restrict__ err_flag) {
+                     const uint4* __restrict__ blocks, uint32_t n_blocks, __half* __restrict__ out, int* __restrict__ err_flag) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (tc::smem_u32(smem_raw) + 1023u) & ~1023u; // swizzle phase follows the absolute address
   uint8_t* smem = smem_raw + (base - tc::smem_u32(smem_raw));
@@ -114,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t qd = heads * 64, kvd = kv_heads * 64, group = heads / kv_heads;
   const uint32_t nqb = (t + 255) / 256;
-  const uint32_t n_items = nqb * heads * n_seqs;
+  const uint32_t n_items = blocks ? n_blocks * heads : nqb * heads * n_seqs;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; i++) {
@@ -155,8 +161,8 @@ __global__ void __launch_bounds__(THREADS, 1)
         uint32_t qi[2] = {0, 0};     // Q halves loaded so far
         bool ok = true;
         for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-          const Item it = item_at(w, nqb, heads, n_seqs, t);
-          const uint32_t row_base = it.seq * t, q0 = it.qb * 256, kvh = it.h / group;
+          const Item it = item_at(w, nqb, heads, n_seqs, t, blocks);
+          const uint32_t row_base = it.row0, q0 = it.qb * 256, kvh = it.h / group;
           for (uint32_t half = 0; half < 2; half++) {
             if (half == 1 && !it.n1) break;
             if (!wait_or_abort(&q_empty[half], (qi[half] & 1) ^ 1, abort_word)) { // the previous item's S reads are done
@@ -242,7 +248,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         __syncwarp();
       };
       for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-        const Item it = item_at(w, nqb, heads, n_seqs, t);
+        const Item it = item_at(w, nqb, heads, n_seqs, t, blocks);
         // the first scores of both halves
         if (!wait(&q_full[0], ci[0]++ & 1)) break;
         if (it.n1 && !wait(&q_full[1], ci[1]++ & 1)) break;
@@ -290,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint32_t c = 0;                                  // key tiles of this half since the kernel began
     bool ok = !*abort_word;
     for (uint32_t w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-      const Item it = item_at(w, nqb, heads, n_seqs, t);
+      const Item it = item_at(w, nqb, heads, n_seqs, t, blocks);
       const uint32_t n_tiles = half ? it.n1 : it.n0;
       const uint32_t diag = 2 * it.qb + half;        // the one key tile that needs the causal mask
       float m_run = -INFINITY, l_run = 0.0f;
@@ -387,9 +393,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         tc::tmem_ld_32x32(o_addr + 32, ov + 32);
         tc::tmem_ld_wait();
         const uint32_t qrow = it.qb * 256 + half * 128 + r;
-        if (qrow < t) {
+        if (qrow < it.t) {
           const float inv = 1.0f / l_run;
-          uint4* dst = reinterpret_cast<uint4*>(out + ((size_t)it.seq * t + qrow) * qd + it.h * 64);
+          uint4* dst = reinterpret_cast<uint4*>(out + ((size_t)it.row0 + qrow) * qd + it.h * 64);
 #pragma unroll
           for (int q = 0; q < 8; q++) {
             float f[8];
@@ -432,18 +438,15 @@ bool attn_tmem_supports(uint32_t n_seqs, uint32_t t, uint32_t heads, uint32_t kv
          (uint64_t)n_seqs * t < 0x7fffff00ull;
 }
 
-int k_attn_causal_tmem(FcDevice* dev, const __half* qkv, uint32_t n_seqs, uint32_t t, uint32_t heads, uint32_t kv_heads,
-                       uint32_t hd, __half* out) {
-  if (!n_seqs || !t) return FC_OK;
-  if (!attn_tmem_supports(n_seqs, t, heads, kv_heads, hd))
-    return fc_fail(dev, FC_ERR_UNSUPPORTED, "the tensor-memory attention needs head_dim 64 and at most 65535 sequences");
+static int launch_tmem(FcDevice* dev, const __half* qkv, uint32_t n_seqs, uint32_t t, const uint4* blocks, uint32_t n_blocks, uint32_t rows,
+                       uint32_t heads, uint32_t kv_heads, __half* out) {
   if ((reinterpret_cast<uintptr_t>(qkv) & 15) || (reinterpret_cast<uintptr_t>(out) & 15))
     return fc_fail(dev, FC_ERR_ARG, "attention buffers must be 16-byte aligned");
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
   const uint64_t width = (uint64_t)(heads + 2 * kv_heads) * 64;
   CUtensorMap tmap;
-  const cuuint64_t dims[2] = {width, (cuuint64_t)n_seqs * t};
+  const cuuint64_t dims[2] = {width, rows};
   const cuuint64_t strides[1] = {width * 2};
   const cuuint32_t box[2] = {64, 128};
   const cuuint32_t estr[2] = {1, 1};
@@ -462,11 +465,27 @@ int k_attn_causal_tmem(FcDevice* dev, const __half* qkv, uint32_t n_seqs, uint32
     attr.first(dev->ordinal);
   }
   // persistent: one CTA per SM walks the (query block, sequence, head) items, heaviest blocks first
-  const uint64_t items = (uint64_t)((t + 255) / 256) * heads * n_seqs;
+  const uint64_t items = blocks ? (uint64_t)n_blocks * heads : (uint64_t)((t + 255) / 256) * heads * n_seqs;
   if (items > 0x7fffffffull) return fc_fail(dev, FC_ERR_UNSUPPORTED, "too many attention work items for one launch");
   const uint32_t sms = (uint32_t)dev->prop.multiProcessorCount;
   dim3 grid((unsigned)(items < sms ? items : sms));
   FC_LAUNCH(dev, "attn_causal_tmem",
-            attn_tmem_kernel<<<grid, THREADS, SMEM_BYTES, dev->stream>>>(tmap, n_seqs, t, heads, kv_heads, out, dev->d_flag));
+            attn_tmem_kernel<<<grid, THREADS, SMEM_BYTES, dev->stream>>>(tmap, n_seqs, t, heads, kv_heads, blocks, n_blocks, out, dev->d_flag));
   return FC_OK;
+}
+
+int k_attn_causal_tmem(FcDevice* dev, const __half* qkv, uint32_t n_seqs, uint32_t t, uint32_t heads, uint32_t kv_heads,
+                       uint32_t hd, __half* out) {
+  if (!n_seqs || !t) return FC_OK;
+  if (!attn_tmem_supports(n_seqs, t, heads, kv_heads, hd))
+    return fc_fail(dev, FC_ERR_UNSUPPORTED, "the tensor-memory attention needs head_dim 64 and at most 65535 sequences");
+  return launch_tmem(dev, qkv, n_seqs, t, nullptr, 0, n_seqs * t, heads, kv_heads, out);
+}
+
+int k_attn_causal_ragged(FcDevice* dev, const __half* qkv, const uint4* blocks, uint32_t n_blocks, uint32_t rows, uint32_t heads,
+                         uint32_t kv_heads, uint32_t hd, __half* out) {
+  if (!n_blocks || !rows) return FC_OK;
+  if (!attn_tmem_supports(1, rows, heads, kv_heads, hd))
+    return fc_fail(dev, FC_ERR_UNSUPPORTED, "the tensor-memory attention needs head_dim 64");
+  return launch_tmem(dev, qkv, 0, 0, blocks, n_blocks, rows, heads, kv_heads, out);
 }

@@ -50,6 +50,10 @@ int k_kv_store_f16(FcDevice* dev, const __half* qkv, uint32_t t, uint32_t heads,
                    uint32_t start, uint32_t ctx, float* k_cache, float* v_cache);
 int k_attn_causal_f16(FcDevice* dev, const __half* qkv, uint32_t n_seqs, uint32_t t, uint32_t heads,
                        uint32_t kv_heads, uint32_t hd, __half* out);
+// The same over sequences of unequal length, packed one after another: `blocks` (on the device) lists every block of 256
+// query rows as (first row of its sequence, length of its sequence, block number), the heaviest (latest) blocks first.
+int k_attn_causal_ragged(FcDevice* dev, const __half* qkv, const uint4* blocks, uint32_t n_blocks, uint32_t rows, uint32_t heads,
+                         uint32_t kv_heads, uint32_t hd, __half* out);
 int k_partial_merge(FcDevice* dev, const float* tiles, uint32_t n_tiles, uint32_t rows, float* out);
 int k_permute_rows(FcDevice* dev, const uint8_t* src, uint8_t* dst, uint32_t rows, uint32_t row_bytes, uint32_t half,
                    uint32_t group);

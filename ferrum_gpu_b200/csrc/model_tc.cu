@@ -115,7 +115,7 @@ int k_qgemm_tc(FcDevice* dev, FcQWeight* w, const float* x_dev, uint32_t m, floa
 }
 
 int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uint32_t n_seqs, uint32_t t,
-                   __half* hidden_out, int32_t cache_stream) {
+                   __half* hidden_out, int32_t cache_stream, const uint4* blocks, uint32_t n_blocks) {
   FcDevice* dev = m->dev;
   FC_TRY(check_tc_shapes(m));
   if (cache_stream >= 0 && n_seqs != 1) return fc_fail(dev, FC_ERR_ARG, "one sequence fills one stream's cache");
@@ -139,9 +139,12 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
                        positions));
     if (cache_stream >= 0)
       FC_TRY(k_kv_store_f16(dev, qkv, t, m->heads, m->kv_heads, m->hd, (uint32_t)cache_stream, 0, m->ctx, l.kv.k, l.kv.v));
-    FC_TRY(k_attn_causal_f16(dev, qkv, n_seqs, t, m->heads, m->kv_heads, m->hd, attn));
+    if (blocks)
+      FC_TRY(k_attn_causal_ragged(dev, qkv, blocks, n_blocks, rows, m->heads, m->kv_heads, m->hd, attn));
+    else
+      FC_TRY(k_attn_causal_f16(dev, qkv, n_seqs, t, m->heads, m->kv_heads, m->hd, attn));
     TcArgs a_wo;
-    a_wo.m = rows, a_wo.bias = l.wo.bias, a_wo.out_f32 = x, a_wo.ldo = d;
+    a_wo.wide = wide, a_wo.m = rows, a_wo.bias = l.wo.bias, a_wo.out_f32 = x, a_wo.ldo = d;
     FC_TRY(k_qgemm_tc_f16(dev, l.wo.w->m, attn, EPI_RESID, a_wo));
     FC_TRY(k_norm_f16(dev, ln, x, l.norm2_g, l.norm2_b, rows, d, m->eps, h));
     TcArgs a_ff1;

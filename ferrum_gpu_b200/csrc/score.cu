@@ -2,6 +2,10 @@
 // over many sequences, in chunks that bound the workspace, plus the pieces of the
 // vocabulary-split head (trunk / head partials / combine) that the multi-GPU driver strings
 // together around its collectives.
+#include <algorithm>
+#include <cstring>
+
+#include "gemm_tc.cuh"
 #include "model.cuh"
 
 namespace {
@@ -170,5 +174,95 @@ FC_API int fc_score_combine_dev(FcDevice* dev, const float* partials_dev, uint32
   const uint32_t rows = n_seqs * rows_per_seq;
   FC_TRY(k_score_combine(dev, partials_dev, n_shards, rows, targets_dev, logprob_dev, greedy_dev));
   if (nll_sum_dev) FC_TRY(k_nll_sums(dev, logprob_dev, n_seqs, rows_per_seq, nll_sum_dev));
+  return FC_OK;
+}
+
+// Sequences of unequal length on the tensor cores: their rows packed one after another without padding, as many whole
+// sequences per pass as the workspace bound allows, and one attention launch per layer over a list of query blocks.
+// Results stay on the device until all passes are enqueued: one wait per call. (Groups of similar length, each padded
+// and run as a pass of its own with its copies and waits, kept the tensor pipe idle: a server's batch is a few hundred
+// rows per group. 23 sequences of 250..1000 ids on the GPT-2-124M shape: 13.3 ms so, 5.7 now.)
+int model_score_packed(FcModel* m, const int32_t* ids, const uint32_t* offsets, uint32_t n_seqs, float* logprob_out, uint8_t* greedy_out) {
+  FcDevice* dev = m->dev;
+  const size_t cap = (size_t)6 << 30;
+  const size_t total = (size_t)offsets[n_seqs] - n_seqs; // rows: every position but each sequence's last
+  // whole sequences per pass, in the caller's order
+  std::vector<uint32_t> first(1, 0);
+  size_t rows_max = 0, blocks_max = 0;
+  for (uint32_t s = 0; s < n_seqs;) {
+    size_t rows = 0, blocks = 0;
+    uint32_t e = s;
+    while (e < n_seqs) {
+      const size_t t = offsets[e + 1] - offsets[e] - 1;
+      if (rows && chunk_bytes(m, rows + t, FC_TENSOR_F16) > cap) break;
+      rows += t, blocks += (t + 255) / 256;
+      e++;
+    }
+    rows_max = rows > rows_max ? rows : rows_max;
+    blocks_max = blocks > blocks_max ? blocks : blocks_max;
+    first.push_back(e);
+    s = e;
+  }
+  const size_t b_in = al(total * 4);
+  FC_TRY(arena_reserve_wide(m, chunk_bytes(m, rows_max, FC_TENSOR_F16) + 3 * b_in + al(total * 4) + al(total) + al(total * 16) + 8192, rows_max,
+                            FC_TENSOR_F16));
+  // everything the passes read, built once and sent in one copy: ids, targets, positions, block lists
+  const size_t n_blocks_all = [&] {
+    size_t b = 0;
+    for (uint32_t s = 0; s < n_seqs; s++) b += (offsets[s + 1] - offsets[s] - 1 + 255) / 256;
+    return b;
+  }();
+  const size_t in_bytes = 3 * b_in + al(n_blocks_all * 16);
+  void* pin;
+  FC_TRY(fc_pinned(dev, in_bytes + al(total * 4) + al(total), &pin));
+  int32_t* h_ids = (int32_t*)pin;
+  int32_t* h_tgt = (int32_t*)((char*)pin + b_in);
+  int32_t* h_pos = (int32_t*)((char*)pin + 2 * b_in);
+  uint4* h_blk = (uint4*)((char*)pin + 3 * b_in);
+  for (uint32_t s = 0; s < n_seqs; s++) {
+    const size_t t = offsets[s + 1] - offsets[s] - 1, at = (size_t)offsets[s] - s;
+    std::copy(ids + offsets[s], ids + offsets[s] + t, h_ids + at);
+    std::copy(ids + offsets[s] + 1, ids + offsets[s] + 1 + t, h_tgt + at);
+    for (size_t i = 0; i < t; i++) h_pos[at + i] = (int32_t)i;
+  }
+  std::vector<size_t> blk_at(1, 0);
+  {
+    size_t b = 0;
+    for (size_t c = 0; c + 1 < first.size(); c++) {
+      const size_t b0 = b, row0 = (size_t)offsets[first[c]] - first[c];
+      for (uint32_t s = first[c]; s < first[c + 1]; s++) {
+        const uint32_t t = offsets[s + 1] - offsets[s] - 1;
+        for (uint32_t q = 0; q < (t + 255) / 256; q++) h_blk[b++] = make_uint4((uint32_t)((size_t)offsets[s] - s - row0), t, q, 0);
+      }
+      std::stable_sort(h_blk + b0, h_blk + b, [](const uint4& x, const uint4& y) { return x.z > y.z; });
+      blk_at.push_back(b);
+    }
+  }
+  char* d_in = (char*)arena_take(m, in_bytes);
+  float* d_lp = (float*)arena_take(m, total * 4);
+  uint8_t* d_gr = (uint8_t*)arena_take(m, total);
+  float* partial = (float*)arena_take(m, rows_max * 16);
+  __half* hidden = (__half*)arena_take(m, rows_max * m->dim * 2);
+  FC_CUDA(dev, cudaMemcpyAsync(d_in, pin, in_bytes, cudaMemcpyHostToDevice, dev->stream));
+  const size_t mark = m->arena.off;
+  for (size_t c = 0; c + 1 < first.size(); c++) {
+    m->arena.off = mark;
+    const size_t row0 = (size_t)offsets[first[c]] - first[c], row1 = (size_t)offsets[first[c + 1]] - first[c + 1];
+    const uint32_t rows = (uint32_t)(row1 - row0);
+    const int32_t* c_ids = (const int32_t*)d_in + row0;
+    const int32_t* c_tgt = (const int32_t*)(d_in + b_in) + row0;
+    const int32_t* c_pos = (const int32_t*)(d_in + 2 * b_in) + row0;
+    const uint4* c_blk = (const uint4*)(d_in + 3 * b_in) + blk_at[c];
+    FC_TRY(model_trunk_tc(m, c_ids, c_pos, 1, rows, hidden, -1, c_blk, (uint32_t)(blk_at[c + 1] - blk_at[c])));
+    FC_TRY(model_head_partial_tc(m, hidden, c_tgt, rows, partial));
+    FC_TRY(k_score_combine(dev, partial, 1, rows, c_tgt, d_lp + row0, d_gr + row0));
+  }
+  FC_TRY(tc_check_errors(dev));
+  char* h_out = (char*)pin + in_bytes;
+  FC_CUDA(dev, cudaMemcpyAsync(h_out, d_lp, total * 4, cudaMemcpyDeviceToHost, dev->stream));
+  FC_CUDA(dev, cudaMemcpyAsync(h_out + al(total * 4), d_gr, total, cudaMemcpyDeviceToHost, dev->stream));
+  FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
+  memcpy(logprob_out, h_out, total * 4);
+  memcpy(greedy_out, h_out + al(total * 4), total);
   return FC_OK;
 }

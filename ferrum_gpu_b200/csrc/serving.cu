@@ -52,6 +52,28 @@ FC_API int fc_model_score_ragged(FcModel* m, const int32_t* ids, const uint32_t*
     order[s] = s;
   }
   auto len_of = [&](uint32_t s) { return offsets[s + 1] - offsets[s]; };
+  if (mode == FC_TENSOR_F16 && m->n_shards == 1) { // one packed pass (or a few), no padding
+    cudaSetDevice(dev->ordinal);
+    FC_TRY(check_ids(m, ids + offsets[0], offsets[n_seqs] - offsets[0]));
+    const size_t total = (size_t)(offsets[n_seqs] - offsets[0]) - n_seqs;
+    std::vector<uint32_t> off(n_seqs + 1); // (the caller's first offset need not be 0)
+    for (uint32_t s = 0; s <= n_seqs; s++) off[s] = offsets[s] - offsets[0];
+    std::vector<float> lp_all(total);
+    std::vector<uint8_t> gr_all(total);
+    FC_TRY(model_score_packed(m, ids + offsets[0], off.data(), n_seqs, lp_all.data(), gr_all.data()));
+    for (uint32_t s = 0; s < n_seqs; s++) {
+      const uint32_t n = len_of(s) - 1;
+      const size_t src = (size_t)off[s] - s, dst = (size_t)offsets[s] - s;
+      if (logprob_out) std::copy(lp_all.begin() + src, lp_all.begin() + src + n, logprob_out + dst);
+      if (greedy_out) std::copy(gr_all.begin() + src, gr_all.begin() + src + n, greedy_out + dst);
+      if (nll_sum_out) { // serving/decoder.rs:L69-L83: f64, ascending position
+        double acc = 0.0;
+        for (uint32_t p = 0; p < n; p++) acc += (double)lp_all[src + p];
+        nll_sum_out[s] = -acc;
+      }
+    }
+    return FC_OK;
+  }
   std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return len_of(a) > len_of(b); });
   std::vector<int32_t> padded;
   std::vector<float> lp;
