@@ -21,7 +21,7 @@
 namespace {
 
 constexpr int HD = 64;
-// NW warps per CTA (4, or 8 for the one-CTA-per-(row, kv-head) form that needs no merge launch): a CTA consumes
+// NW warps per CTA (4, or 8 for the one-CTA-per-(row, kv-head) form that needs no merge): a CTA consumes
 // NW x 16 positions per loop iteration (4 lane groups x 4 positions per warp)
 template <int NW>
 struct Tile {
@@ -29,6 +29,8 @@ struct Tile {
   static constexpr size_t BYTES = (size_t)2 * 2 * POS * HD * 4; // two stages of a K and a V tile
 };
 constexpr int POS_PER_ITER = Tile<4>::POS;
+// one arrival counter per (row, kv-head): a cache is only split while all CTAs are resident at once, far fewer than this
+constexpr uint32_t ATTN_COUNTERS = 4096;
 
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -61,28 +63,74 @@ struct QkvFinish {
   bool on = false;
   DeferredReduce pend; // splits == 0: the row is already summed
   RopeParams rope;
+  // where the finished slice goes: the qkv buffer itself after a pending sum (built from the partial sums, which nobody
+  // modifies), another buffer of its shape for a finished row - the splits of a (row, kv-head) each rotate it, and a
+  // rotation in place would not be repeatable
+  float* to = nullptr;
 };
 
-// partial layout per (row, kv-head, split): [G] max (log2 domain), [G] sum, [G][64] weighted output
+// partial layout per (row, kv-head, split): [G] max (log2 domain), [G] sum, padding to whole 16 bytes, [G][64] weighted output
+template <int G>
+struct Part {
+  static constexpr int HEAD = (2 * G + 3) & ~3;
+  static constexpr int FLOATS = HEAD + G * HD;
+};
 template <int G, int NW>
 __global__ void __launch_bounds__(NW * 32)
     attn_decode_split_kernel(const float* qkv, uint32_t q_stride, uint32_t heads, uint32_t kv_heads,
                              const int32_t* __restrict__ positions, const int32_t* __restrict__ streams, KvLayer kv,
-                             uint32_t ctx, uint32_t n_splits, float* __restrict__ partial, DecodeOut dst, bool append, QkvFinish fin) {
+                             uint32_t ctx, uint32_t n_splits, float* partial, uint32_t* arrived, DecodeOut dst, bool append, QkvFinish fin) {
   constexpr int POS_PER_ITER = Tile<NW>::POS; // (this kernel's own step; the host's split rule keeps the 4-warp one)
   __shared__ float sm_m[NW][G], sm_l[NW][G];
   __shared__ __align__(16) float sm_o[NW][G][HD];
+  // One stream: launched under the tail of the qkv product (programmatic dependent launch), and the output product may
+  // start its weight stream on the SMs this launch leaves free. Nothing is read before the wait.
+  if (NW == 4) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
   const uint32_t split = blockIdx.x, kvh = blockIdx.y, r = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
   const uint32_t len = (uint32_t)positions[r] + 1;
   const uint32_t split_len = ((len + n_splits - 1) / n_splits + POS_PER_ITER - 1) / POS_PER_ITER * POS_PER_ITER;
   const uint32_t p0 = min(len, split * split_len), p1 = min(len, p0 + split_len);
+  // ranges that hold positions at the row's current length: the others leave at once (a short text in a long cache)
+  const uint32_t n_used = (len + split_len - 1) / split_len;
   if (dst.xh && split == 0 && r + 1 == gridDim.z) // the padding rows of the product's n-block are zero
     for (uint32_t i = threadIdx.x; i < (dst.mp - gridDim.z) * G * HD; i += blockDim.x) {
       const size_t at = (size_t)(gridDim.z + i / (G * HD)) * heads * HD + (size_t)kvh * G * HD + i % (G * HD);
       dst.xh[at] = dst.xl[at] = __float2half_rn(0.0f);
     }
+  if (NW == 4 && split >= n_used) return;
   const uint32_t slot = streams ? (uint32_t)streams[r] : 0;
+  // K and V tiles of 64 positions travel through two shared-memory stages by cp.async: the loads of the next
+  // tile are in flight while this one is multiplied, and the lanes of a group can all read the same row
+  // (a shared-memory broadcast) instead of each holding a slice of it in registers. The first tile is requested before
+  // the row itself is finished; of it only the row's own k and v, which are not in the cache yet, follow later.
+  extern __shared__ __align__(16) float tiles[]; // [2 stages][K, V][64 positions][64]
+  constexpr uint32_t TILE = POS_PER_ITER * HD;
+  const float* kcache = kv.k + ((size_t)slot * kv_heads + kvh) * ctx * HD;
+  const float* vcache = kv.v + ((size_t)slot * kv_heads + kvh) * ctx * HD;
+  // what this thread's c-th piece of the tile at j0 is: 2 tensors x POS positions x 16 chunks over NW x 32 threads
+  auto piece = [&](int c, uint32_t j0, uint32_t buf, uint32_t& tensor, uint32_t& jj, uint32_t& ch, float*& dst) {
+    const uint32_t id = threadIdx.x + NW * 32 * c, pos = (id >> 4) % POS_PER_ITER, j = j0 + pos;
+    tensor = id / (POS_PER_ITER * 16), ch = id & 15;
+    jj = j < p1 ? j : p0; // past the range: any valid row (its scores are masked)
+    dst = tiles + (buf * 2 + tensor) * TILE + pos * HD + ch * 4;
+  };
+  auto copy16 = [](float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+  };
+  if (p0 < p1) {
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+      uint32_t tensor, jj, ch;
+      float* dst;
+      piece(c, p0, 0, tensor, jj, ch, dst);
+      if (!(append && jj + 1 == len)) copy16(dst, (tensor ? vcache : kcache) + (size_t)jj * HD + ch * 4);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   if (fin.on) {
     // This CTA's slice of the row: its G query heads, its k head and its v head (every split of the same
     // (row, kv-head) computes and writes the same values).
@@ -99,10 +147,17 @@ __global__ void __launch_bounds__(NW * 32)
       if (fin.pend.splits) {
         v = 0.0f;
         const float* p = fin.pend.partial + (size_t)r * w + col;
-        for (uint32_t sp = 0; sp < fin.pend.splits; sp++) v += p[(size_t)sp * fin.pend.m * w];
+        const size_t stride = (size_t)fin.pend.m * w;
+        for (uint32_t sp = 0; sp < fin.pend.splits; sp += 8) { // eight loads in flight; added in ascending order
+          float t[8];
+#pragma unroll
+          for (uint32_t j = 0; j < 8; j++) t[j] = sp + j < fin.pend.splits ? p[(sp + j) * stride] : 0.0f;
+#pragma unroll
+          for (uint32_t j = 0; j < 8; j++) v += t[j];
+        }
         if (fin.pend.bias) v += fin.pend.bias[col];
       } else {
-        v = grow[col]; // (host code folds the launch only with a pending sum: see attn_decode_folds_rope)
+        v = grow[col];
       }
       slice[idx] = v;
     }
@@ -121,7 +176,9 @@ __global__ void __launch_bounds__(NW * 32)
       }
       __syncthreads();
     }
-    for (uint32_t idx = threadIdx.x; idx < (G + 2) * HD; idx += blockDim.x) grow[col_of(idx)] = slice[idx];
+    float* out_row = fin.to + (size_t)r * q_stride;
+    for (uint32_t idx = threadIdx.x; idx < (G + 2) * HD; idx += blockDim.x) out_row[col_of(idx)] = slice[idx];
+    qkv = fin.to;
     __threadfence(); // (the tiles below fetch the row's k and v with cp.async, past this SM's L1)
     __syncthreads();
   }
@@ -162,15 +219,8 @@ __global__ void __launch_bounds__(NW * 32)
     for (int c = 0; c < CH; c++) acc[h][c] = 0.0f;
   }
 
-  // K and V tiles of 64 positions travel through two shared-memory stages by cp.async: the loads of the next
-  // tile are in flight while this one is multiplied, and the lanes of a group can all read the same row
-  // (a shared-memory broadcast) instead of each holding a slice of it in registers.
-  extern __shared__ __align__(16) float tiles[]; // [2 stages][K, V][64 positions][64]
-  constexpr uint32_t TILE = POS_PER_ITER * HD;
   const float* krow_new = qkv + (size_t)r * q_stride + (size_t)(heads + kvh) * HD;
   const float* vrow_new = qkv + (size_t)r * q_stride + (size_t)(heads + kv_heads + kvh) * HD;
-  const float* kcache = kv.k + ((size_t)slot * kv_heads + kvh) * ctx * HD;
-  const float* vcache = kv.v + ((size_t)slot * kv_heads + kvh) * ctx * HD;
   if (append && p0 < len && p1 == len) {
     // the row's own k and v (models without RoPE) are not in the cache yet: this CTA's range ends with them,
     // so it stores them; the tiles below take that position from the qkv row
@@ -181,18 +231,24 @@ __global__ void __launch_bounds__(NW * 32)
   }
   auto stage = [&](uint32_t j0, uint32_t buf) {
 #pragma unroll
-    for (int c = 0; c < 16; c++) { // 2 tensors x POS positions x 16 chunks over NW x 32 threads
-      const uint32_t id = threadIdx.x + NW * 32 * c, tensor = id / (POS_PER_ITER * 16), pos = (id >> 4) % POS_PER_ITER, ch = id & 15;
-      const uint32_t j = j0 + pos;
-      const uint32_t jj = j < p1 ? j : p0; // past the range: any valid row (its scores are masked)
+    for (int c = 0; c < 16; c++) {
+      uint32_t tensor, jj, ch;
+      float* dst;
+      piece(c, j0, buf, tensor, jj, ch, dst);
       const bool fresh = append && jj + 1 == len;
-      const float* src = tensor ? (fresh ? vrow_new : vcache + (size_t)jj * HD) : (fresh ? krow_new : kcache + (size_t)jj * HD);
-      const uint32_t dst_addr = (uint32_t)__cvta_generic_to_shared(tiles + (buf * 2 + tensor) * TILE + pos * HD + ch * 4);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst_addr), "l"(src + ch * 4) : "memory");
+      copy16(dst, (tensor ? (fresh ? vrow_new : vcache + (size_t)jj * HD) : (fresh ? krow_new : kcache + (size_t)jj * HD)) + ch * 4);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (p0 < p1) stage(p0, 0);
+  if (append && p1 == len && p1 - p0 <= (uint32_t)POS_PER_ITER) { // the row's own k and v, where the first tile holds them
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+      uint32_t tensor, jj, ch;
+      float* dst;
+      piece(c, p0, 0, tensor, jj, ch, dst);
+      if (jj + 1 == len) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>((tensor ? vrow_new : krow_new) + ch * 4);
+    }
+  }
   uint32_t buf = 0;
   for (uint32_t j0 = p0; j0 < p1; j0 += POS_PER_ITER, buf ^= 1) {
     if (j0 + POS_PER_ITER < p1) {
@@ -304,31 +360,74 @@ __global__ void __launch_bounds__(NW * 32)
     if (n_splits == 1) {
       dst.put((size_t)r * heads * HD + (size_t)(kvh * G + g) * HD + c, o / ll);
     } else {
-      float* p = partial + (((size_t)r * kv_heads + kvh) * n_splits + split) * (size_t)(G * (2 + HD));
+      float* p = partial + (((size_t)r * kv_heads + kvh) * n_splits + split) * (size_t)Part<G>::FLOATS;
       if (c == 0) p[g] = mm, p[G + g] = ll;
-      p[2 * G + g * HD + c] = o;
+      p[Part<G>::HEAD + g * HD + c] = o;
     }
   }
-}
-
-// out[row][head][c] = merge over splits, ascending
-template <int G>
-__global__ void attn_decode_merge_kernel(const float* __restrict__ partial, uint32_t heads, uint32_t kv_heads,
-                                         uint32_t n_splits, DecodeOut dst) {
-  const uint32_t kvh = blockIdx.x, r = blockIdx.y;
-  const float* base = partial + ((size_t)r * kv_heads + kvh) * n_splits * (size_t)(G * (2 + HD));
-  for (int idx = threadIdx.x; idx < G * HD; idx += blockDim.x) {
-    const int g = idx / HD, c = idx % HD;
-    float mm = -INFINITY;
-    for (uint32_t s = 0; s < n_splits; s++) mm = fmaxf(mm, base[(size_t)s * G * (2 + HD) + g]);
-    float ll = 0.0f, o = 0.0f;
-    for (uint32_t s = 0; s < n_splits; s++) {
-      const float* p = base + (size_t)s * G * (2 + HD);
-      const float sc = p[g] == -INFINITY ? 0.0f : ex2(p[g] - mm);
-      ll = fmaf(p[G + g], sc, ll);
-      o = fmaf(p[2 * G + g * HD + c], sc, o);
+  if (NW != 4 || n_splits == 1) return; // (the eight-warp form is never split)
+  // The CTA of a (row, kv-head) that finishes last merges its splits, in ascending order whoever that is. (A merge
+  // launch of its own took 4 us of launch and, at the 32 splits of a lone stream's 2048-position cache, 21 us of
+  // loads one behind the other.)
+  __shared__ uint32_t s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t* cnt = arrived + r * kv_heads + kvh;
+    s_last = atomicAdd(cnt, 1u) == n_used - 1;
+    if (s_last) *cnt = 0; // for the next launch
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const float* base = partial + ((size_t)r * kv_heads + kvh) * n_splits * (size_t)Part<G>::FLOATS;
+  float* sw = tiles; // [split][G], over the K / V stages: everyone is done with them
+  for (uint32_t i = threadIdx.x; i < n_used * G; i += blockDim.x) sw[i] = __ldcg(base + (size_t)(i / G) * Part<G>::FLOATS + i % G);
+  __syncthreads();
+  for (int g = warp; g < G; g += NW) {
+    float mm = -INFINITY, ll = 0.0f;
+    for (uint32_t s = lane; s < n_used; s += 32) mm = fmaxf(mm, sw[s * G + g]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    for (uint32_t s = lane; s < n_used; s += 32) {
+      const float ms = sw[s * G + g], sc = ms == -INFINITY ? 0.0f : ex2(ms - mm);
+      ll = fmaf(__ldcg(base + (size_t)s * Part<G>::FLOATS + G + g), sc, ll);
+      sw[s * G + g] = sc;
     }
-    dst.put((size_t)r * heads * HD + (size_t)(kvh * G + g) * HD + c, o / ll);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
+    if (lane == 0) sm_l[0][g] = ll;
+  }
+  __syncthreads();
+  // four channels per thread; with few heads, groups of threads take the splits in turn
+  constexpr int QUADS = G * HD / 4, FIT = NW * 32 / QUADS, GROUPS = FIT < 1 ? 1 : FIT > NW ? NW : FIT;
+  static_assert(QUADS <= NW * 32 || NW != 4, "one float4 of the result per thread");
+  float4* part_o = reinterpret_cast<float4*>(&sm_o[0][0][0]); // [GROUPS][QUADS]: at most what sm_o holds
+  const int quad = threadIdx.x % QUADS, group = threadIdx.x / QUADS, g = quad * 4 / HD;
+  float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (group < GROUPS) {
+    const float* p = base + Part<G>::HEAD + quad * 4;
+#pragma unroll 8
+    for (uint32_t s = group; s < n_used; s += GROUPS) {
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(p + (size_t)s * Part<G>::FLOATS));
+      const float wt = sw[s * G + g];
+      o.x = fmaf(v.x, wt, o.x), o.y = fmaf(v.y, wt, o.y), o.z = fmaf(v.z, wt, o.z), o.w = fmaf(v.w, wt, o.w);
+    }
+  }
+  if (GROUPS > 1) {
+    if (group < GROUPS) part_o[group * QUADS + quad] = o;
+    __syncthreads();
+    if (group != 0) return;
+#pragma unroll
+    for (int q = 1; q < GROUPS; q++) {
+      const float4 v = part_o[q * QUADS + quad];
+      o.x += v.x, o.y += v.y, o.z += v.z, o.w += v.w;
+    }
+  }
+  if (group == 0) {
+    const size_t at = (size_t)r * heads * HD + (size_t)kvh * G * HD + quad * 4;
+    const float ll = sm_l[0][g];
+    dst.put(at, o.x / ll), dst.put(at + 1, o.y / ll), dst.put(at + 2, o.z / ll), dst.put(at + 3, o.w / ll);
   }
 }
 
@@ -336,6 +435,9 @@ template <int G>
 int launch(FcDevice* dev, const float* qkv, uint32_t q_stride, uint32_t rows, uint32_t heads, uint32_t kv_heads,
            const int32_t* positions, const int32_t* streams, const KvLayer& kv, uint32_t ctx, uint32_t n_splits,
            float* scratch, const DecodeOut& dst, bool append, const QkvFinish& fin) {
+  uint32_t* arrived = (uint32_t*)scratch; // counters first (zero between launches), then the partial results
+  float* partial = scratch + ATTN_COUNTERS;
+  if (n_splits > 1 && rows * kv_heads > ATTN_COUNTERS) return fc_fail(dev, FC_ERR_UNSUPPORTED, "too many rows for a split cache");
   static OncePerDevice attr;
   if (attr.first(dev->ordinal)) {
     FC_CUDA(dev, cudaFuncSetAttribute(attn_decode_split_kernel<G, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<4>::BYTES));
@@ -348,18 +450,18 @@ int launch(FcDevice* dev, const float* qkv, uint32_t q_stride, uint32_t rows, ui
     dim3 grid(1, kv_heads, rows);
     FC_LAUNCH(dev, "attn_decode",
               attn_decode_split_kernel<G, 8><<<grid, 256, Tile<8>::BYTES, dev->stream>>>(qkv, q_stride, heads, kv_heads, positions, streams,
-                                                                                      kv, ctx, 1, scratch, dst, append, fin));
+                                                                                      kv, ctx, 1, partial, arrived, dst, append, fin));
     return FC_OK;
   }
-  dim3 grid(n_splits, kv_heads, rows);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n_splits, kv_heads, rows), cfg.blockDim = dim3(128), cfg.dynamicSmemBytes = Tile<4>::BYTES, cfg.stream = dev->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at, cfg.numAttrs = rows == 1 ? 1 : 0; // (between the launches of a batched step it costs more than it hides)
   FC_LAUNCH(dev, "attn_decode",
-            attn_decode_split_kernel<G, 4><<<grid, 128, Tile<4>::BYTES, dev->stream>>>(qkv, q_stride, heads, kv_heads, positions, streams, kv,
-                                                                                    ctx, n_splits, scratch, dst, append, fin));
-  if (n_splits > 1) {
-    dim3 mg(kv_heads, rows);
-    FC_LAUNCH(dev, "attn_decode_merge",
-              attn_decode_merge_kernel<G><<<mg, 128, 0, dev->stream>>>(scratch, heads, kv_heads, n_splits, dst));
-  }
+            cudaLaunchKernelEx(&cfg, attn_decode_split_kernel<G, 4>, qkv, q_stride, heads, kv_heads, positions, streams, kv, ctx, n_splits,
+                               partial, arrived, dst, append, fin));
   return FC_OK;
 }
 
@@ -395,14 +497,16 @@ static uint32_t attn_decode_splits(const FcDevice* dev, uint32_t rows, uint32_t 
   uint32_t s = slots / (rows * kv_heads);
   const uint32_t max_s = (ctx + POS_PER_ITER - 1) / POS_PER_ITER;
   if (s > max_s) s = max_s;
-  if (ctx <= 512) s = 1; // a short cache is a microsecond for one CTA: the merge launch would cost more
+  if (ctx <= 512) s = 1; // a short cache is a microsecond for one CTA: the merge would cost more
   return s < 1 ? 1 : s;
 }
 
-// Partial results of every split.
+// Arrival counters (the caller zeroes them once: attn_decode_zero_bytes) and the partial results of every split.
+size_t attn_decode_zero_bytes() { return ATTN_COUNTERS * 4; }
 size_t attn_decode_scratch_bytes(const FcDevice* dev, uint32_t rows, uint32_t heads, uint32_t kv_heads, uint32_t ctx) {
   const uint32_t ns = attn_decode_splits(dev, rows, heads, kv_heads, ctx);
-  return (size_t)rows * kv_heads * ns * (heads / kv_heads) * (2 + HD) * 4 + 256;
+  const uint32_t g = heads / kv_heads;
+  return ATTN_COUNTERS * 4 + (size_t)rows * kv_heads * ns * (((2 * g + 3) & ~3u) + g * HD) * 4 + 256;
 }
 
 bool attn_decode_split_supports(uint32_t heads, uint32_t kv_heads, uint32_t hd) {
@@ -413,7 +517,7 @@ bool attn_decode_split_supports(uint32_t heads, uint32_t kv_heads, uint32_t hd) 
 int k_attn_decode_split(FcDevice* dev, const float* qkv, uint32_t q_stride, uint32_t rows, uint32_t heads, uint32_t kv_heads,
                         const int32_t* positions, const int32_t* streams, const KvLayer& kv, uint32_t ctx, float* scratch,
                         float* out, __half* xh, __half* xl, uint32_t mp, bool append, const DeferredReduce* qkv_pending,
-                        const RopeParams* rope) {
+                        const RopeParams* rope, float* rotated) {
   if (!rows) return FC_OK;
   const uint32_t ns = attn_decode_splits(dev, rows, heads, kv_heads, ctx);
   DecodeOut dst;
@@ -423,6 +527,8 @@ int k_attn_decode_split(FcDevice* dev, const float* qkv, uint32_t q_stride, uint
     fin.on = true;
     fin.rope = *rope;
     if (qkv_pending) fin.pend = *qkv_pending;
+    fin.to = fin.pend.splits ? const_cast<float*>(qkv) : rotated;
+    if (!fin.to) return fc_fail(dev, FC_ERR_ARG, "rotating a finished row needs a second buffer");
   }
   switch (heads / kv_heads) {
     case 1: return launch<1>(dev, qkv, q_stride, rows, heads, kv_heads, positions, streams, kv, ctx, ns, scratch, dst, append, fin);

@@ -231,6 +231,10 @@ struct Epilogue {
   const float* norm_b = nullptr;
   float norm_eps = 0.0f;
   float* norm_tmp = nullptr;
+  // x is the fused gate / up row (2 k wide, the layout of k_swiglu's `group`) and the product is fed silu(gate) * up: only
+  // where qlinear_takes_swiglu says so
+  bool swiglu = false;
+  uint32_t swiglu_group = 0;
   // the producer of x has already written its two fp16 terms where the 9..64-row tensor-core product
   // stages them (qmatvec_mma_split_ptrs): the product skips its split launch and ignores `x`
   bool presplit = false;
@@ -251,8 +255,10 @@ size_t qmatvec_mma_scratch_bytes(uint32_t k, uint32_t n);
 int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, void* scratch);
 // Whether k_qlinear_f32 will take the 9..64-row tensor-core product for (w, m) with this scratch, and where
 // that product expects the two fp16 terms of x ([mp][k] each, rows >= m zero).
+bool qlinear_takes_swiglu(const FcDevice* dev, const QMat& w); // one row, the streamed product (matvec1.cu)
 bool qlinear_takes_wide_mma(const QMat& w, uint32_t m, const void* scratch);
 int k_flush_deferred(FcDevice* dev, const DeferredReduce& d);
+int k_norm_pending(FcDevice* dev, const DeferredReduce& d, int norm, const float* g, const float* b, float eps, float* h);
 void qmatvec_mma_split_ptrs(void* scratch, uint32_t m, uint32_t k, __half** xh, __half** xl, uint32_t* mp);
 
 // ---- kernels' host entry points (each enqueues on dev->stream) --------------------------------

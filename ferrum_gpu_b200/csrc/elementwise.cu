@@ -82,12 +82,25 @@ __global__ void layernorm_kernel(const float* __restrict__ x, const float* __res
 // `group` > 0: the fused product's columns come as `group` gate columns followed by the matching
 // `group` up columns (the layout the tensor-core SwiGLU epilogue wants); 0: all gate, then all up.
 __global__ void swiglu_kernel(const float* __restrict__ gu, uint32_t rows, uint32_t hidden, uint32_t group,
-                              float* __restrict__ act) {
+                              float* __restrict__ act, DeferredReduce pend) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)rows * hidden) return;
   const size_t r = i / hidden, c = i % hidden;
-  const size_t gi = group ? (c / group) * 2 * group + c % group : c;
-  const float g = gu[r * 2 * hidden + gi], u = gu[r * 2 * hidden + gi + (group ? group : hidden)];
+  const size_t gi = group ? (c / group) * 2 * group + c % group : c, ui = gi + (group ? group : hidden);
+  float g, u;
+  if (pend.splits) { // the gate / up product's unfinished sum, in the order of its own reduce
+    const size_t stride = (size_t)pend.m * 2 * hidden;
+    const float* p = pend.partial + r * 2 * hidden;
+    g = 0.0f, u = 0.0f;
+#pragma unroll 4
+    for (uint32_t s = 0; s < pend.splits; s++) {
+      g += p[s * stride + gi];
+      u += p[s * stride + ui];
+    }
+    if (pend.bias) g += pend.bias[gi], u += pend.bias[ui];
+  } else {
+    g = gu[r * 2 * hidden + gi], u = gu[r * 2 * hidden + ui];
+  }
   act[i] = g / (1.0f + expf(-g)) * u;
 }
 
@@ -282,6 +295,7 @@ __global__ void swiglu_split_kernel(const float* __restrict__ gu, uint32_t rows,
       const size_t stride = (size_t)pend.m * 2 * hidden;
       const float* p = pend.partial + r * 2 * hidden;
       g = 0.0f, u = 0.0f;
+#pragma unroll 4
       for (uint32_t s = 0; s < pend.splits; s++) {
         g += p[s * stride + gi];
         u += p[s * stride + ui];
@@ -337,10 +351,18 @@ int k_layernorm(FcDevice* dev, const float* x, const float* g, const float* b, u
   return FC_OK;
 }
 
-int k_swiglu(FcDevice* dev, const float* gate_up, uint32_t rows, uint32_t hidden, uint32_t group, float* act) {
+int k_swiglu(FcDevice* dev, const float* gate_up, uint32_t rows, uint32_t hidden, uint32_t group, float* act,
+             const DeferredReduce* pending) {
   const size_t total = (size_t)rows * hidden;
+  DeferredReduce pend;
+  if (pending && pending->splits) {
+    if (total && pending->y == gate_up && pending->m == rows && pending->n == 2 * hidden && !pending->resid)
+      pend = *pending;
+    else
+      FC_TRY(k_flush_deferred(dev, *pending));
+  }
   if (!total) return FC_OK;
-  FC_LAUNCH(dev, "swiglu", swiglu_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(gate_up, rows, hidden, group, act));
+  FC_LAUNCH(dev, "swiglu", swiglu_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(gate_up, rows, hidden, group, act, pend));
   return FC_OK;
 }
 

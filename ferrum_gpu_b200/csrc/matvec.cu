@@ -393,6 +393,8 @@ bool qlinear_takes_wide_mma(const QMat& w, uint32_t m, const void* scratch) {
   return scratch && m > 8 && qmatvec_mma_supports(w, m); // (x lives in the library's own aligned buffers there)
 }
 
+bool qlinear_takes_swiglu(const FcDevice* dev, const QMat& w) { return dev->matvec_choice == 0 && qmatvec1_supports(dev, w); }
+
 int k_qlinear_f32(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep_in) {
   if (m == 0) return FC_OK;
   const int forced = dev->matvec_choice; // 0: the rule above; 1: FMA kernel; 2: small-batch mma.sync kernel
@@ -404,6 +406,7 @@ int k_qlinear_f32(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     if (ep.presplit) return fc_fail(dev, FC_ERR_ARG, "a pre-split x needs the 9..64-row tensor-core product");
     return k_qmatvec1(dev, w, x, y, ep);
   }
+  if (ep.swiglu) return fc_fail(dev, FC_ERR_ARG, "only the streamed one-row product applies SwiGLU");
   if (ep.wide_scratch && forced == 0 && !ep.presplit && qgemm_pair_takes(w, m)) { // (its x split takes the norm along)
     if (ep.pending && ep.pending->splits) FC_TRY(k_flush_deferred(dev, *ep.pending));
     return k_qgemm_pair(dev, w, x, m, y, ep, ep.wide_scratch);
@@ -416,11 +419,21 @@ int k_qlinear_f32(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
   if (ep.presplit && !(mma_ok && m > 8)) return fc_fail(dev, FC_ERR_ARG, "a pre-split x needs the 9..64-row tensor-core product");
   const bool use_fma = fma_ok && (!mma_ok || forced == 1 || (forced == 0 && m < 2));
   const bool use_mma_wide = !use_fma && mma_ok && m > 8; // its x split takes the norm along
+  const bool use_mma8 = !use_fma && mma_ok && m <= 8;
+  // 2..8 rows: the norm launch in front of the product finishes the pending sum of its rows
+  const bool norm_finishes = use_mma8 && ep.norm != NORM_NONE && ep.norm_tmp && ep.pending && ep.pending->splits && ep.pending->y == x &&
+                             ep.pending->m == m && ep.pending->n == w.k;
+  if (norm_finishes) {
+    FC_TRY(k_norm_pending(dev, *ep.pending, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, ep.norm_tmp));
+    x = ep.norm_tmp;
+    ep.norm = NORM_NONE;
+    ep.pending = nullptr;
+  }
   if (ep.pending && ep.pending->splits && !use_mma_wide) { // only that split can finish a producer's split-K sum
     FC_TRY(k_flush_deferred(dev, *ep.pending));
     ep.pending = nullptr;
   }
-  if (!use_mma_wide) ep.defer_out = nullptr;
+  if (!use_mma_wide && !use_mma8) ep.defer_out = nullptr;
   if (ep.norm != NORM_NONE && !use_fma && !use_mma_wide) { // the FMA matvec normalises while it stages x
     if (!ep.norm_tmp) return fc_fail(dev, FC_ERR_ARG, "a fused norm needs a temporary for the kernels that cannot fuse it");
     if (ep.norm == NORM_RMS)

@@ -133,7 +133,8 @@ __device__ __forceinline__ float store_split(__half* xh, __half* xl, uint32_t i,
 }
 
 // NW warps per CTA; a stage is one TMA box of 16 rows x LINES 128-byte lines of packed quants.
-template <int KIND, int NW, int LINES>
+// SWIGLU: x is a fused gate / up row and the product is fed silu(gate) * up (Epilogue::swiglu).
+template <int KIND, int NW, int LINES, bool SWIGLU>
 __global__ void __launch_bounds__(NW * 32, 1)
     qmatvec1_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_s, const uint32_t k,
                     const uint32_t n, const float* __restrict__ x, float* y, const Epilogue ep, const Plan pl, int* err_flag) {
@@ -227,7 +228,22 @@ __global__ void __launch_bounds__(NW * 32, 1)
   float* stat = norm_red + 32; // [0] 1/rms or 1/std, [1] mean, [2..] per-warp maxima
   float* xsum = reinterpret_cast<float*>(smem + pl.xs_off); // per block: -offset * sum of the staged x
   float* xf = reinterpret_cast<float*>(xh); // x as it is, over the place of the two terms, until they are written
-  for (uint32_t i = threadIdx.x; i < k; i += THREADS) xf[i] = x[i];
+  if (SWIGLU) { // silu(gate) * up as swiglu_kernel computes it
+    const uint32_t gr = ep.swiglu_group;
+    for (uint32_t i = threadIdx.x; i < k; i += THREADS) {
+      float gv, uv;
+      if (gr == 1) {
+        const float2 p = reinterpret_cast<const float2*>(x)[i];
+        gv = p.x, uv = p.y;
+      } else {
+        const uint32_t gi = gr ? (i / gr) * 2 * gr + i % gr : i;
+        gv = x[gi], uv = x[gi + (gr ? gr : k)];
+      }
+      xf[i] = gv / (1.0f + expf(-gv)) * uv;
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < k; i += THREADS) xf[i] = x[i];
+  }
   __syncthreads();
   if (ep.norm != NORM_NONE && threadIdx.x < 256) {
     // statistics by the first 256 threads, which sum in the order of the stand-alone norm kernels (256-thread CTAs)
@@ -548,7 +564,7 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-template <int KIND, int NW, int LINES>
+template <int KIND, int NW, int LINES, bool SWIGLU>
 int launch_cfg(FcDevice* dev, const QMat& w, const float* x, float* y, const Epilogue& ep, const Plan& p) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
@@ -575,7 +591,7 @@ int launch_cfg(FcDevice* dev, const QMat& w, const float* x, float* y, const Epi
                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled (scales) failed with %d", (int)cr);
   }
-  auto kern = qmatvec1_kernel<KIND, NW, LINES>;
+  auto kern = qmatvec1_kernel<KIND, NW, LINES, SWIGLU>;
   static OncePerDevice attr;
   if (attr.first(dev->ordinal)) FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_LIMIT));
   cudaLaunchConfig_t cfg = {};
@@ -590,7 +606,8 @@ int launch_cfg(FcDevice* dev, const QMat& w, const float* x, float* y, const Epi
 
 template <int KIND>
 int launch(FcDevice* dev, const QMat& w, const float* x, float* y, const Epilogue& ep, const Plan& p) {
-  return launch_cfg<KIND, Cfg<KIND>::NW, Cfg<KIND>::LINES>(dev, w, x, y, ep, p);
+  if (ep.swiglu) return launch_cfg<KIND, Cfg<KIND>::NW, Cfg<KIND>::LINES, true>(dev, w, x, y, ep, p);
+  return launch_cfg<KIND, Cfg<KIND>::NW, Cfg<KIND>::LINES, false>(dev, w, x, y, ep, p);
 }
 
 } // namespace

@@ -78,7 +78,7 @@ __device__ __forceinline__ float block_sum_mma(float v, float* red) {
 __global__ void __launch_bounds__(256)
     norm_split_kernel(const float* x, uint32_t m, uint32_t k, int norm, const float* __restrict__ g,
                       const float* __restrict__ b, float eps, __half* __restrict__ xh, __half* __restrict__ xl,
-                      DeferredReduce pend) {
+                      DeferredReduce pend, float* __restrict__ yf) { // yf set: the f32 rows instead of the terms
   __shared__ float red[32];
   const uint32_t r = blockIdx.x;
   __half* oh = xh + (size_t)r * k;
@@ -134,6 +134,10 @@ __global__ void __launch_bounds__(256)
   }
   for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) {
     float v = norm == NORM_RMS ? row[i] * inv * g[i] : (row[i] - mean) * inv * g[i] + b[i];
+    if (yf) {
+      yf[(size_t)r * k + i] = v;
+      continue;
+    }
     v = fminf(fmaxf(v, -65504.0f), 65504.0f);
     const __half h = __float2half_rn(v);
     oh[i] = h;
@@ -706,11 +710,21 @@ static int k_qmatvec_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t
     FC_TRY(pick_mma8<true>(dev, w, x, m, y, part, grid, bps, ep));
   else
     FC_TRY(pick_mma8<false>(dev, w, x, m, y, part, grid, bps, ep));
+  if (splits > 1 && ep.defer_out && ep.act == ACT_NONE) { // the consumer finishes the sum
+    *ep.defer_out = DeferredReduce{partial, splits, m, w.n, ep.bias, ep.resid, y};
+    return FC_OK;
+  }
   if (splits > 1) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
               splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep, nullptr));
   }
+  return FC_OK;
+}
+
+// Finish a pending sum and normalise its rows into `h` (f32): one launch where a reduce and a norm would be two.
+int k_norm_pending(FcDevice* dev, const DeferredReduce& d, int norm, const float* g, const float* b, float eps, float* h) {
+  FC_LAUNCH(dev, "norm_pending", norm_split_kernel<<<d.m, 256, 0, dev->stream>>>(d.y, d.m, d.n, norm, g, b, eps, nullptr, nullptr, d, h));
   return FC_OK;
 }
 
@@ -762,7 +776,7 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     // the terms are there: the producer of x wrote them, or the launch above
   } else if (ep.norm != NORM_NONE) // x is the raw residual stream: normalise and split in one launch
     FC_LAUNCH(dev, "norm_split",
-              norm_split_kernel<<<mp, 256, 0, dev->stream>>>(x, m, w.k, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, xh, xl, pend));
+              norm_split_kernel<<<mp, 256, 0, dev->stream>>>(x, m, w.k, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, xh, xl, pend, nullptr));
   else
     FC_LAUNCH(dev, "x_split", x_split_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(x, m, mp, w.k, xh, xl));
   if (tx) return k_qgemm_tx(dev, w, xh, xl, mp, m, y, ep);

@@ -104,7 +104,7 @@ uint64_t plan_bytes(const Shape& s, int qkind, uint64_t streams) {
   per += 2 * streams * s.ctx * kvd * 4;                              // K and V caches
   b += per * s.layers;
   b += 2 * d * 4 + matrix_bytes(qkind, d, s.vocab);                  // final norm, head
-  b += streams * (2 * d + (qd + 2 * kvd) + qd + ff1 + hid + s.vocab) * 4 + streams * 16; // decode scratch
+  b += streams * (2 * d + 2 * (qd + 2 * kvd) + qd + ff1 + hid + s.vocab) * 4 + streams * 16; // decode scratch
   return b;
 }
 
@@ -131,6 +131,7 @@ int alloc_common(FcModel* m) {
   FC_TRY(dev_alloc(m, (size_t)s * m->dim * 4, (void**)&m->x));
   FC_TRY(dev_alloc(m, (size_t)s * m->dim * 4, (void**)&m->h));
   FC_TRY(dev_alloc(m, (size_t)s * m->qkv_w() * 4, (void**)&m->qkv));
+  if (m->rope.cos) FC_TRY(dev_alloc(m, (size_t)s * m->qkv_w() * 4, (void**)&m->qkv_rot));
   FC_TRY(dev_alloc(m, (size_t)s * m->qd() * 4, (void**)&m->attn));
   FC_TRY(dev_alloc(m, (size_t)s * m->ff1_w() * 4, (void**)&m->ff));
   FC_TRY(dev_alloc(m, (size_t)s * m->hidden * 4, (void**)&m->act));
@@ -151,6 +152,7 @@ int alloc_common(FcModel* m) {
       need = b > need ? b : need;
     }
     FC_TRY(dev_alloc(m, need, (void**)&m->attn_scratch));
+    FC_CUDA(m->dev, cudaMemsetAsync(m->attn_scratch, 0, attn_decode_zero_bytes(), m->dev->stream));
   }
   // scratch of the decode tensor product (x split + split-K partials), sized for the widest matrix
   {
@@ -220,12 +222,11 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
     pend = DeferredReduce();
     const bool to_cache = mode != ATTN_STATELESS;
     // Without RoPE the launch below would only copy k and v into the cache: the decode attention does that itself.
-    const bool attn_appends =
-        mode == ATTN_DECODE && !m->rope.cos && attn_decode_appends(m->heads, m->kv_heads, m->hd, m->attn_scratch);
-    // With RoPE, the decode attention can take the rotation, the pending sum and the cache append along as well:
-    // one launch less per layer.
-    const bool attn_folds = mode == ATTN_DECODE && m->rope.cos &&
+    // It also takes the rotation and a pending sum of the qkv product along: one launch less per layer.
+    const bool attn_folds = mode == ATTN_DECODE && (m->rope.cos || qkv_sum.splits) &&
                             attn_decode_folds_rope(m->heads, m->kv_heads, m->hd, m->attn_scratch, qkv_sum, b.qkv, rows);
+    const bool attn_appends = mode == ATTN_DECODE && !m->rope.cos && !attn_folds &&
+                              attn_decode_appends(m->heads, m->kv_heads, m->hd, m->attn_scratch);
     if (attn_appends)
       FC_TRY(k_flush_deferred(dev, qkv_sum));
     else if (!attn_folds)
@@ -242,7 +243,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
       }
       FC_TRY(k_attn_decode(dev, b.qkv, m->qkv_w(), rows, m->heads, m->kv_heads, m->hd, positions, streams, l.kv, m->ctx,
                            b.attn, m->attn_scratch, xh, xl, mp, attn_appends || attn_folds, attn_folds ? &qkv_sum : nullptr,
-                           attn_folds ? &m->rope : nullptr));
+                           attn_folds ? &m->rope : nullptr, m->qkv_rot));
     } else if (mode == ATTN_STATELESS)
       FC_TRY(k_attn_causal_f32(dev, b.qkv, n_seqs, t, m->heads, m->kv_heads, m->hd, b.attn));
     else
@@ -266,8 +267,8 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
     // partial sums then sit behind the widest x terms, clear of the ones SwiGLU writes.
     const bool swiglu_splits = m->arch == ARCH_LLAMA && qlinear_takes_wide_mma(l.ff2.w->m, rows, m->mma_scratch);
     DeferredReduce gu_sum;
+    if (m->arch == ARCH_LLAMA) e_ff1.defer_out = &gu_sum; // (either SwiGLU launch finishes it)
     if (swiglu_splits) {
-      e_ff1.defer_out = &gu_sum;
       const size_t widest = m->hidden > d ? m->hidden : d;
       e_ff1.partial_at = (float*)(((uintptr_t)m->mma_scratch + (size_t)2 * 64 * widest * 2 + 255) & ~(uintptr_t)255);
     }
@@ -283,11 +284,15 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
         FC_TRY(k_swiglu_split(dev, b.ff, rows, mp, m->hidden, m->gu_group, xh, xl, &gu_sum));
         e_ff2.presplit = true;
       } else {
-        FC_TRY(k_swiglu(dev, b.ff, rows, m->hidden, m->gu_group, b.act));
+        // (one row: the streamed product takes SwiGLU along while it stages x)
+        e_ff2.swiglu = rows == 1 && qlinear_takes_swiglu(dev, l.ff2.w->m);
+        e_ff2.swiglu_group = m->gu_group;
+        if (!e_ff2.swiglu) FC_TRY(k_swiglu(dev, b.ff, rows, m->hidden, m->gu_group, b.act, &gu_sum));
       }
-      ff2_in = b.act;
+      ff2_in = e_ff2.swiglu ? b.ff : b.act;
     }
     e_ff2.scratch = m->mma_scratch;
+    e_ff2.wide_scratch = wide;
     e_ff2.bias = l.ff2.bias;
     e_ff2.resid = b.x;
     made = DeferredReduce();

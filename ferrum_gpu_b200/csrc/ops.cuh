@@ -20,7 +20,8 @@ int k_embed(FcDevice* dev, const float* tok, const float* pos_table /*nullable*/
             const int32_t* positions /*nullable unless pos_table*/, uint32_t rows, uint32_t d, float* x);
 int k_rmsnorm(FcDevice* dev, const float* x, const float* g, uint32_t rows, uint32_t d, float eps, float* y);
 int k_layernorm(FcDevice* dev, const float* x, const float* g, const float* b, uint32_t rows, uint32_t d, float* y);
-int k_swiglu(FcDevice* dev, const float* gate_up /*[rows][2*hidden]*/, uint32_t rows, uint32_t hidden, uint32_t group, float* act);
+int k_swiglu(FcDevice* dev, const float* gate_up /*[rows][2*hidden]*/, uint32_t rows, uint32_t hidden, uint32_t group, float* act,
+             const DeferredReduce* pending = nullptr); // gate_up's unfinished split-K sum: finished here
 int k_swiglu_split(FcDevice* dev, const float* gate_up, uint32_t rows, uint32_t mp, uint32_t hidden, uint32_t group, __half* xh,
                    __half* xl, const DeferredReduce* pending = nullptr); // gate_up's unfinished split-K sum: finished here
 // Rotate q and k of the fused qkv rows in place (rope.type/rope_dim; skipped when rope.cos is
@@ -51,17 +52,19 @@ int k_attn_decode(FcDevice* dev, const float* qkv, uint32_t q_stride, uint32_t r
                   uint32_t mp = 0, bool append_kv = false,
                   // the context-split kernel only: fold the RoPE / cache launch into this one - finish the qkv
                   // product's pending split-K sum (nullable: none), rotate q and k by `rope`, append k and v
-                  const DeferredReduce* qkv_pending = nullptr, const RopeParams* rope = nullptr);
+                  // (`rotated`: a buffer like qkv, for rows without a pending sum)
+                  const DeferredReduce* qkv_pending = nullptr, const RopeParams* rope = nullptr, float* rotated = nullptr);
 // Whether k_attn_decode can store the rows' own k and v into the cache itself (`append_kv`): the
 // context-split kernel does, for models whose k needs no rotation first.
 bool attn_decode_appends(uint32_t heads, uint32_t kv_heads, uint32_t hd, const float* scratch);
 // attn_decode.cu
 bool attn_decode_split_supports(uint32_t heads, uint32_t kv_heads, uint32_t hd);
+size_t attn_decode_zero_bytes(); // leading bytes of the scratch that must be zero before its first use
 size_t attn_decode_scratch_bytes(const FcDevice* dev, uint32_t rows, uint32_t heads, uint32_t kv_heads, uint32_t ctx);
 int k_attn_decode_split(FcDevice* dev, const float* qkv, uint32_t q_stride, uint32_t rows, uint32_t heads, uint32_t kv_heads,
                         const int32_t* positions, const int32_t* streams, const KvLayer& kv, uint32_t ctx, float* scratch,
                         float* out, __half* xh, __half* xl, uint32_t mp, bool append, const DeferredReduce* qkv_pending = nullptr,
-                        const RopeParams* rope = nullptr);
+                        const RopeParams* rope = nullptr, float* rotated = nullptr);
 // Whether the launch can take the qkv product's pending sum and the rotation along (attn_decode.cu).
 bool attn_decode_folds_rope(uint32_t heads, uint32_t kv_heads, uint32_t hd, const float* scratch, const DeferredReduce& pending,
                             const float* qkv, uint32_t rows);
