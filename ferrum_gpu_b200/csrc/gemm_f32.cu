@@ -1,6 +1,6 @@
 // Exact-f32 batched product y[m, n] = x[m, k] . W[n, k]^T for any m: the f32-accumulated path
-// behind forward_all / scoring when FC_EXACT_F32 is asked for, and behind decode batches wider
-// than the matvec kernel takes. Replaces qlinear_tiled.wgsl and matmul_blocked4.wgsl
+// behind forward_all / scoring when FC_EXACT_F32 is asked for, for the formats and sizes that the
+// tensor-core products at f32-class accuracy (gemm_pair.cu, matvec_mma.cu) do not take. Replaces qlinear_tiled.wgsl and matmul_blocked4.wgsl
 // (ferrum_wgpu/src/shaders/quant/qlinear_tiled.wgsl:L93-L128, shaders/matmul).
 //
 // 64 x 64 output tile per CTA of 256 threads (4 x 4 outputs per thread), K walked in slices of 32
