@@ -45,6 +45,7 @@ struct FcDevice {
 };
 
 constexpr uint64_t WORKSPACE_POOL_KEEP = 512ull << 20;
+constexpr uint64_t WORKSPACE_POOL_WARM = 64ull << 20; // mapped when the device is opened
 cudaError_t workspace_alloc(FcDevice* dev, void** p, size_t bytes);
 void workspace_free(FcDevice* dev, void* p);
 bool stream_capturing(FcDevice* dev); // the device's stream is being captured into a graph

@@ -98,6 +98,24 @@ FC_API int fc_device_open(int ordinal, FcDevice** out) {
     return rc;
   }
   cudaMemsetAsync(dev->d_flag, 0, sizeof(int), dev->stream);
+  {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ordinal;
+    uint64_t keep = WORKSPACE_POOL_KEEP;
+    if (cudaMemPoolCreate(&dev->workspaces, &props) != cudaSuccess) {
+      dev->workspaces = nullptr;
+    } else if (cudaMemPoolSetAttribute(dev->workspaces, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaMemPoolDestroy(dev->workspaces);
+      dev->workspaces = nullptr;
+    } else { // the first workspaces find their memory mapped (half a millisecond of a first product)
+      void* p = nullptr;
+      if (workspace_alloc(dev, &p, WORKSPACE_POOL_WARM) == cudaSuccess) workspace_free(dev, p);
+    }
+    cudaGetLastError();
+  }
   *out = dev;
   return FC_OK;
 }
