@@ -989,6 +989,7 @@ FC_API int fc_model_prefill(FcModel* m, uint32_t stream_id, const int32_t* ids, 
     if (logits_out)
       FC_CUDA(dev, cudaMemcpyAsync(logits_out, m->logits, (size_t)m->vocab * 4, cudaMemcpyDeviceToHost, dev->stream));
   }
+  if (n > 64) FC_TRY(tc_check_errors(dev)); // (the products of many rows have bounded waits)
   FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
   m->pos[stream_id] = start + n;
   return FC_OK;
@@ -1015,6 +1016,7 @@ FC_API int fc_model_forward_all(FcModel* m, const int32_t* ids, uint32_t n, floa
     Epilogue e_head;
     e_head.wide_scratch = m->wide;
     FC_TRY(k_qlinear_f32(dev, m->head_view, b.h, n, logits, e_head));
+    if (n > 64) FC_TRY(tc_check_errors(dev));
   } else if (mode == FC_TENSOR_F16) {
     __half* hid = (__half*)arena_take(m, (size_t)n * m->dim * 2);
     FC_TRY(model_trunk_tc(m, d_ids, d_pos, 1, n, hid));
@@ -1067,7 +1069,7 @@ FC_API int fc_model_score(FcModel* m, const int32_t* ids, uint32_t n_seqs, uint3
   if (cudaMemcpyAsync(d_ids, ids, (size_t)n_seqs * seq_len * 4, cudaMemcpyHostToDevice, dev->stream) != cudaSuccess)
     rc = fc_fail(dev, FC_ERR_DEVICE, "upload of ids failed");
   if (rc == FC_OK) rc = fc_model_score_dev(m, d_ids, n_seqs, seq_len, mode, d_lp, d_gr, d_nll);
-  if (rc == FC_OK && mode == FC_TENSOR_F16) rc = tc_check_errors(dev);
+  if (rc == FC_OK) rc = tc_check_errors(dev);
   if (rc == FC_OK) {
     if (logprob_out) cudaMemcpyAsync(logprob_out, d_lp, rows * 4, cudaMemcpyDeviceToHost, dev->stream);
     if (greedy_out) cudaMemcpyAsync(greedy_out, d_gr, rows, cudaMemcpyDeviceToHost, dev->stream);

@@ -176,7 +176,7 @@ FC_API int fc_qmatmul(FcQWeight* w, const float* x, uint32_t m, float* y, int mo
   if (cudaMemcpyAsync(dx, x, (size_t)m * w->m.k * 4, cudaMemcpyHostToDevice, dev->stream) != cudaSuccess)
     rc = fc_fail(dev, FC_ERR_DEVICE, "upload of x failed");
   if (rc == FC_OK) rc = fc_qmatmul_dev(w, dx, m, dy, mode);
-  if (rc == FC_OK && mode == FC_TENSOR_F16) rc = tc_check_errors(dev);
+  if (rc == FC_OK && m > 1) rc = tc_check_errors(dev);
   if (rc == FC_OK && cudaMemcpyAsync(y, dy, (size_t)m * w->m.n * 4, cudaMemcpyDeviceToHost, dev->stream) != cudaSuccess)
     rc = fc_fail(dev, FC_ERR_DEVICE, "read-back of y failed");
   if (rc == FC_OK && cudaStreamSynchronize(dev->stream) != cudaSuccess) {
