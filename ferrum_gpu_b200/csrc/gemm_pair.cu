@@ -571,7 +571,9 @@ int launch(FcDevice* dev, const CUtensorMap* maps, const PairArgs& a) {
 // Against the tiled f32 kernel: 512 x 2048 x 32000 Q8_0 294 us instead of 2523, 1536 x 1024 x 5632 Q8_0 69 instead of 677,
 // 100 x 768 x 1280 Q4_0 21 instead of 46, 65 x 512 x 512 19 instead of 33, 128 x 320 x 1000 19 instead of 21; short widths
 // with few tiles, where three launches cost more than they save (128 x 64 x 512: 17.5 instead of 7.8, 333 x 96 x 1000: 17
-// instead of 10), keep the tiled kernel (TILED_KEEPS). Bound by L2: 48 KB per 64 k and CTA for the 128-row tile, 9 TB/s over all SMs.
+// instead of 10), keep the tiled kernel (TILED_KEEPS). At 1536 x 1024 x 5632 the tensor pipe is
+// active 47 %, L2 33 %: 264 tiles take 4 waves of pairs (3.6 full), and every 128 k the accumulator changes hands between
+// the MMA thread and the epilogues of two SMs.
 // Error against f64 on N(0, 1) x N(0, 0.02), of the result's norm: 1.2e-7 (K 96) to 2.2e-7 (K 4096); the f32 chain
 // 1.8e-7 to 1.15e-6.
 bool qgemm_pair_takes(const QMat& w, uint32_t m) {
