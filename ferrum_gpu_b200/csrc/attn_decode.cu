@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(NW * 32)
   // K and V tiles of 64 positions travel through two shared-memory stages by cp.async: the loads of the next
   // tile are in flight while this one is multiplied, and the lanes of a group can all read the same row
   // (a shared-memory broadcast) instead of each holding a slice of it in registers. The first tile is requested before
-  // the row itself is finished; of it only the row's own k and v, which are not in the cache yet, follow later.
+  // the row itself is finished (fin.on); of it only the row's own k and v, which are not in the cache yet, follow later.
   extern __shared__ __align__(16) float tiles[]; // [2 stages][K, V][64 positions][64]
   constexpr uint32_t TILE = POS_PER_ITER * HD;
   const float* kcache = kv.k + ((size_t)slot * kv_heads + kvh) * ctx * HD;
@@ -127,14 +127,19 @@ __global__ void __launch_bounds__(NW * 32)
       uint32_t tensor, jj, ch;
       float* dst;
       piece(c, p0, 0, tensor, jj, ch, dst);
-      if (!(append && jj + 1 == len)) copy16(dst, (tensor ? vcache : kcache) + (size_t)jj * HD + ch * 4);
+      const float* src = (tensor ? vcache : kcache) + (size_t)jj * HD;
+      if (append && jj + 1 == len) {
+        if (fin.on) continue;
+        src = qkv + (size_t)r * q_stride + (size_t)(heads + (tensor ? kv_heads : 0) + kvh) * HD;
+      }
+      copy16(dst, src + ch * 4);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+  __shared__ __align__(16) float slice[(G + 2) * HD];
   if (fin.on) {
     // This CTA's slice of the row: its G query heads, its k head and its v head (every split of the same
     // (row, kv-head) computes and writes the same values).
-    __shared__ float slice[(G + 2) * HD];
     const uint32_t qd = heads * HD, kvd = kv_heads * HD, w = qd + 2 * kvd;
     float* grow = const_cast<float*>(qkv) + (size_t)r * q_stride;
     auto col_of = [&](uint32_t idx) {
@@ -240,13 +245,13 @@ __global__ void __launch_bounds__(NW * 32)
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (append && p1 == len && p1 - p0 <= (uint32_t)POS_PER_ITER) { // the row's own k and v, where the first tile holds them
+  if (fin.on && append && p0 < p1 && p1 == len && p1 - p0 <= (uint32_t)POS_PER_ITER) { // the row's own k and v, where the first tile holds them
 #pragma unroll
     for (int c = 0; c < 16; c++) {
       uint32_t tensor, jj, ch;
       float* dst;
       piece(c, p0, 0, tensor, jj, ch, dst);
-      if (jj + 1 == len) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>((tensor ? vrow_new : krow_new) + ch * 4);
+      if (jj + 1 == len) *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(slice + (G + tensor) * HD + ch * 4);
     }
   }
   uint32_t buf = 0;
