@@ -444,7 +444,8 @@ __global__ void __launch_bounds__(128)
       const uint32_t c = threadIdx.x + 128 * j, row = c >> 5, ch = c & 31;
       const bool valid = row < m && (!RAGGED || kb0 + ch / 8 < kb_end);
       cp_async16_zfill(smem_u32(xf + st * C::XF_STAGE + (row * XS + ch * 4) * 4),
-                       valid ? x + (size_t)row * k + (size_t)kb0 * QK + ch * 4 : x, valid);
+                       RAGGED ? (valid ? x + (size_t)row * k + (size_t)kb0 * QK + ch * 4 : x)
+                              : x + (size_t)(valid ? row : 0) * k + (size_t)kb0 * QK + ch * 4, valid);
     }
   };
 
