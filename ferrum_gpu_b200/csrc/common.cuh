@@ -220,9 +220,11 @@ struct Epilogue {
   // a stand-alone product (no norm, nothing pending or deferred) whose width need not be whole 128s: the scratch also
   // serves qmatvec_mma_ragged_supports
   bool ragged = false;
-  // device scratch of at least qgemm_pair_scratch_bytes(k, n, m): lets products of more than 64 rows of Q8_0 / Q4_0
-  // weights run on the tensor cores (gemm_pair.cu); without it they take the tiled f32 kernel
+  // device scratch that lets products of more than 64 rows of Q8_0 / Q4_0 weights run on the tensor cores (gemm_pair.cu;
+  // qgemm_pair_scratch_bytes(k, n, m) is what the best cut takes); without it, or where it is too small, they take the
+  // tiled f32 kernel
   void* wide_scratch = nullptr;
+  size_t wide_bytes = 0;
   // "x is the raw residual stream: normalise each row first" (NORM_RMS: y = x / sqrt(mean(x^2) + eps) * g,
   // NORM_LAYER: (x - mean) / sqrt(var + 1e-5) * g + b). The one-row FMA matvec does it while it stages x
   // in shared memory (one launch less per product); the other kernels run the norm kernel into

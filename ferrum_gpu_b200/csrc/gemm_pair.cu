@@ -526,7 +526,14 @@ struct Plan {
   uint32_t kp, steps, bn, splits, per_split, slice; // slice: weight rows whose terms are in the workspace at once
 };
 constexpr size_t W_TERMS_BYTES = (size_t)64 << 20;
-Plan make_plan(uint32_t sms, uint32_t k, uint32_t n, uint32_t m) {
+size_t al(size_t v) { return (v + 1023) & ~(size_t)1023; }
+size_t plan_bytes(const Plan& p, uint32_t m) {
+  return 2 * al((size_t)m * p.kp * 2) + 2 * al((size_t)p.slice * p.kp * 2) + al((size_t)m * 4) + al((size_t)p.slice * 4) +
+         al((size_t)p.splits * m * p.slice * 4) + 1024;
+}
+// The best cut whose workspace fits into `limit` bytes; splits == 0 where not even the smallest does. (Fewer rows may ask
+// for more than many: they leave the chip idle without a split of K, and every split has sums of its own.)
+Plan make_plan(uint32_t sms, uint32_t k, uint32_t n, uint32_t m, size_t limit) {
   Plan p;
   p.kp = (k + BK - 1) / BK * BK;
   p.steps = p.kp / BK;
@@ -537,19 +544,19 @@ Plan make_plan(uint32_t sms, uint32_t k, uint32_t n, uint32_t m) {
   // 700 (64 rows) cycles each, and for a split of K its second launch and the sums' way through L2 (2 KB a cycle).
   const uint64_t pairs = sms / 2, tiles_n = (p.slice + 255) / 256;
   uint64_t best = ~0ull;
-  uint32_t s = 1;
+  p.bn = p.splits = p.per_split = 0;
   for (uint32_t bn : {128u, 64u})
     for (uint32_t c = 1; c <= 8 && c <= p.steps; c++) {
       const uint64_t items = tiles_n * ((m + bn - 1) / bn) * c, per = (p.steps + c - 1) / c;
       const uint64_t cost = (items + pairs - 1) / pairs * (per * (bn == 128 ? 1000 : 700) + 3000) +
                             (c > 1 ? 5000 + (uint64_t)m * p.slice * 4 * (2 * c + 1) / 2048 : 0);
-      if (cost < best) best = cost, p.bn = bn, s = c;
+      if (cost >= best) continue;
+      Plan q = p;
+      q.bn = bn, q.per_split = (uint32_t)per, q.splits = (uint32_t)((p.steps + per - 1) / per);
+      if (plan_bytes(q, m) <= limit) best = cost, p = q;
     }
-  p.per_split = (p.steps + s - 1) / s;
-  p.splits = (p.steps + p.per_split - 1) / p.per_split;
   return p;
 }
-size_t al(size_t v) { return (v + 1023) & ~(size_t)1023; }
 
 template <int KIND, int BN>
 int launch(FcDevice* dev, const CUtensorMap* maps, const PairArgs& a) {
@@ -583,14 +590,21 @@ bool qgemm_pair_takes(const QMat& w, uint32_t m) {
 }
 
 size_t qgemm_pair_scratch_bytes(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m) {
-  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m);
-  return 2 * al((size_t)m * p.kp * 2) + 2 * al((size_t)p.slice * p.kp * 2) + al((size_t)m * 4) + al((size_t)p.slice * 4) +
-         al((size_t)p.splits * m * p.slice * 4) + 1024;
+  return plan_bytes(make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m, SIZE_MAX), m);
+}
+bool qgemm_pair_fits(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m, size_t bytes) {
+  return make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m, bytes).splits != 0;
+}
+FC_API uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, uint32_t m, uint64_t limit) {
+  if (sm_count < 2 || !k || k % QK || !n || !m) return 0;
+  const Plan p = make_plan(sm_count, k, n, m, (size_t)limit);
+  return p.splits ? plan_bytes(p, m) : 0;
 }
 
-int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, void* scratch) {
+int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, void* scratch, size_t bytes) {
   if (m == 0) return FC_OK;
-  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, w.k, w.n, m);
+  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, w.k, w.n, m, bytes);
+  if (!p.splits) return fc_fail(dev, FC_ERR_ARG, "a %zu-byte workspace is too small for this product", bytes);
   uint8_t* at = (uint8_t*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
   auto take = [&](size_t bytes) {
     uint8_t* r = at;

@@ -25,8 +25,10 @@ struct TcArgs {
   float* partial = nullptr;
   int* err_flag = nullptr;
   uint32_t tile0 = 0;   // EPI_LSE: 128-column tiles of the head before this launch's weight rows
-  // workspace for the fp16 weights of the pair kernel (tp_workspace_bytes; nullable: the weights are decoded in the product)
+  // workspace for the fp16 weights of the pair kernel (tp_workspace_bytes; missing or too small: the weights are decoded in
+  // the product)
   void* wide = nullptr;
+  size_t wide_bytes = 0;
   uint32_t out_tma = 0; // (set by the launch code) results leave through shared memory and TMA
 };
 

@@ -151,7 +151,7 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
     } else if (qgemm_pair_takes(w->m, m)) {
       const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m));
       if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
-      ep.wide_scratch = w->tc_cache; // (no room for it: the tiled f32 kernel needs none)
+      ep.wide_scratch = w->tc_cache, ep.wide_bytes = w->tc_cache_bytes; // (no room for it: the tiled f32 kernel needs none)
     }
     return k_qlinear_f32(dev, w->m, x_dev, m, y_dev, ep);
   }

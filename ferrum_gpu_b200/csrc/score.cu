@@ -35,14 +35,23 @@ size_t chunk_bytes(const FcModel* m, size_t rows, int mode) {
   return b;
 }
 
+// What one pass may take: whole sequences as long as it fits (2 GiB exact, 6 GiB tensor path).
+size_t pass_cap(const FcModel* m, int mode) { return m->pass_bytes ? m->pass_bytes : (size_t)(mode == FC_EXACT_F32 ? 2 : 6) << 30; }
+
 } // namespace
+
+FC_API int fc_debug_score_pass_bytes(FcModel* m, uint64_t bytes) {
+  if (!m) return FC_ERR_ARG;
+  m->pass_bytes = (size_t)bytes;
+  return FC_OK;
+}
 
 // Exact-f32 head over this rank's vocabulary rows: logits of the chunk are materialised, then
 // reduced to per-row partials.
 static int head_partial_f32(FcModel* m, const float* hidden, const int32_t* targets, uint32_t rows, float* logits_ws,
                             float* partial) {
   Epilogue ep;
-  if (rows <= m->wide_rows) ep.wide_scratch = m->wide;
+  ep.wide_scratch = m->wide, ep.wide_bytes = m->wide_bytes;
   FC_TRY(k_qlinear_f32(m->dev, m->head_view, hidden, rows, logits_ws, ep));
   return k_score_partial(m->dev, logits_ws, targets, rows, m->v1 - m->v0, m->v0, partial);
 }
@@ -59,8 +68,7 @@ FC_API int fc_model_score_dev(FcModel* m, const int32_t* ids_dev, uint32_t n_seq
     return fc_fail(dev, FC_ERR_UNSUPPORTED, "this model holds one vocabulary shard: use the trunk / head_partial / combine calls");
   if (n_seqs == 0) return FC_OK;
   const uint32_t t = seq_len - 1;
-  // chunk size: whole sequences, workspace bounded (2 GiB exact / 6 GiB tensor path)
-  const size_t cap = mode == FC_EXACT_F32 ? ((size_t)2 << 30) : ((size_t)6 << 30);
+  const size_t cap = pass_cap(m, mode);
   uint32_t per = n_seqs;
   while (per > 1 && chunk_bytes(m, (size_t)per * t, mode) > cap) per = (per + 1) / 2;
   const size_t rows_max = (size_t)per * t;
@@ -153,7 +161,7 @@ FC_API int fc_model_head_partial_dev(FcModel* m, const void* hidden_dev, const i
   // chunk the rows so the materialised logits stay under 2 GiB
   const size_t vs = m->v1 - m->v0;
   size_t per = rows;
-  while (per > 1 && per * vs * 4 > ((size_t)2 << 30)) per = (per + 1) / 2;
+  while (per > 1 && per * vs * 4 > pass_cap(m, mode)) per = (per + 1) / 2;
   FC_TRY(arena_reserve_wide(m, al(per * vs * 4) + 4096, per, mode));
   float* logits_ws = (float*)arena_take(m, per * vs * 4);
   for (size_t r0 = 0; r0 < rows; r0 += per) {
@@ -184,7 +192,7 @@ FC_API int fc_score_combine_dev(FcDevice* dev, const float* partials_dev, uint32
 // rows per group. 23 sequences of 250..1000 ids on the GPT-2-124M shape: 13.3 ms so, 5.7 now.)
 int model_score_packed(FcModel* m, const int32_t* ids, const uint32_t* offsets, uint32_t n_seqs, float* logprob_out, uint8_t* greedy_out) {
   FcDevice* dev = m->dev;
-  const size_t cap = (size_t)6 << 30;
+  const size_t cap = pass_cap(m, FC_TENSOR_F16);
   const size_t total = (size_t)offsets[n_seqs] - n_seqs; // rows: every position but each sequence's last
   // whole sequences per pass, in the caller's order
   std::vector<uint32_t> first(1, 0);

@@ -106,6 +106,10 @@ int fc_debug_fail_after(FcDevice* dev, int64_t n_launches);
  * 1 = the f32 FMA kernel, 2 = the small-batch mma.sync kernel. Measurement hook; results stay within the
  * exact path's tolerance whichever runs. */
 int fc_debug_matvec_kernel(FcDevice* dev, int choice);
+/* Workspace bytes of the exact product of `m` > 64 rows by an [n, k] weight on a device of `sm_count` multiprocessors
+ * when at most `limit` bytes are there; 0 when none of its forms fits (the tiled f32 kernel, which needs none, then
+ * runs). Needs no device. Test hook. */
+uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, uint32_t m, uint64_t limit);
 /* Per-kernel device timing, the counterpart of the reference's one-kernel-at-a-time profiler
  * (ferrum_wgpu/benches/profile_train.rs:L15-L25): while enabled every launch is bracketed by a pair
  * of CUDA events on the device's stream. The report is a JSON object
@@ -365,6 +369,9 @@ int fc_model_score(FcModel* m, const int32_t* ids, uint32_t n_seqs, uint32_t seq
  * `logprob_dev` / `greedy_dev` nullable. Enqueues without synchronising. */
 int fc_model_score_dev(FcModel* m, const int32_t* ids_dev, uint32_t n_seqs, uint32_t seq_len,
                        int mode, float* logprob_dev, uint8_t* greedy_dev, double* nll_sum_dev);
+/* Bound of the workspace of one scoring pass (a call whose sequences need more runs several passes): `bytes` instead of
+ * the library's own, 0 for the library's own. Results do not depend on it beyond rounding. Test hook. */
+int fc_debug_score_pass_bytes(FcModel* m, uint64_t bytes);
 
 /* ---- vocabulary-split head (multi-GPU scoring) --------------------------------------------
  * Precedent: Lin::Sharded splits a `[k, n]` weight by output columns, each block quantised and

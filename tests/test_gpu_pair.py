@@ -7,7 +7,7 @@ of sum |x w| whatever the width."""
 import numpy as np
 import pytest
 
-from ferrum_gpu_b200 import CudaGpt2, CudaLlama, Mode, QKind, linear_q, upload_quantised
+from ferrum_gpu_b200 import CudaGpt2, CudaLlama, Mode, QKind, _ffi, linear_q, upload_quantised
 from ferrum_gpu_b200.hostmodel import Gpt2Config, LlamaConfig, random_gpt2, random_llama, random_tokens
 from oracle import oracle as orc
 from tests import helpers
@@ -122,4 +122,22 @@ def test_a_later_row_with_infinities_does_not_reach_earlier_rows(dev, poison):
     ids[70] = 63
     got = g.forward_all(ids)
     assert np.array_equal(got[:70], clean[:70]) and np.all(np.isnan(got[70]))
+    g.close()
+
+
+def test_exact_scoring_in_unequal_passes(dev):
+    """A call in two passes whose shorter one would, cut for itself, take more workspace than the longer one reserved."""
+    lib = _ffi.load()
+    cfg = LlamaConfig(vocab=1000, ctx=64, dim=128, heads=2, kv_heads=1, head_dim=64, layers=2, hidden=768, rope_dim=64)
+    if dev.props()[0] == 148:  # (`down` is the only matrix here that is not left to the tiled kernel)
+        need = [lib.fc_debug_pair_bytes(148, 768, 128, seqs * 60, 2**64 - 1) for seqs in (11, 10)]
+        assert need[0] < need[1]
+    g = CudaLlama(dev, random_llama(cfg, seed=3, std=0.05), QKind.Q8_0)
+    ids = np.stack([random_tokens(i, 61, cfg.vocab) for i in range(21)])
+    whole = g.score_batch(ids, Mode.EXACT_F32)
+    dev.check(lib.fc_debug_score_pass_bytes(g._h, 15 << 20))  # 16 KB a row: 21 x 60 rows are passes of 11 and 10 sequences
+    parts = g.score_batch(ids, Mode.EXACT_F32)
+    assert np.max(np.abs(parts[0] - whole[0])) < 2e-5 and np.mean(parts[1] != whole[1]) < 0.002
+    again = g.score_batch(ids, Mode.EXACT_F32)
+    assert np.array_equal(again[0], parts[0])
     g.close()
