@@ -151,7 +151,8 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
     } else if (qgemm_pair_takes(w->m, m)) {
       const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m));
       if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
-      ep.wide_scratch = w->tc_cache, ep.wide_bytes = w->tc_cache_bytes; // (no room for it: the tiled f32 kernel needs none)
+// (no room for more, or a capture: the product is cut to the workspace that is there, or takes the tiled f32 kernel)
+      ep.wide_scratch = w->tc_cache, ep.wide_bytes = w->tc_cache_bytes;
     }
     return k_qlinear_f32(dev, w->m, x_dev, m, y_dev, ep);
   }

@@ -141,3 +141,41 @@ def test_exact_scoring_in_unequal_passes(dev):
     again = g.score_batch(ids, Mode.EXACT_F32)
     assert np.array_equal(again[0], parts[0])
     g.close()
+
+
+@pytest.mark.parametrize("mode,eager_rows", [(Mode.EXACT_F32, 0), (Mode.EXACT_F32, 100), (Mode.EXACT_F32, 3000), (Mode.TENSOR_F16, 3000)])
+def test_products_captured_into_a_graph(dev, mode, eager_rows):
+    """A captured call works in memory of its own size, whatever an earlier call of the same weight had, and replays read
+    the operands of the moment."""
+    import torch
+    lib = _ffi.load()
+    m, k, n = 2000, 512, 1024
+    rng = np.random.default_rng(5)
+    qw = upload_quantised(dev, QKind.Q8_0, (rng.standard_normal(k * n) * 0.02).astype(np.float32), k, n)
+    w = torch.from_numpy(qw.dequantised().reshape(n, k)).cuda().double()
+    x, y = torch.randn(max(m, eager_rows), k, device="cuda"), torch.zeros(max(m, eager_rows), n, device="cuda")
+    call = lambda rows: dev.check(lib.fc_qmatmul_dev(qw.handle, x.data_ptr(), rows, y.data_ptr(), int(mode)))
+    call(70)  # (the kernels' one-time settings)
+    if eager_rows:
+        call(eager_rows)
+    dev.sync()
+    other = upload_quantised(dev, QKind.Q8_0, (rng.standard_normal(k * n) * 0.02).astype(np.float32), k, n)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(dev.stream())):
+        call(m)
+    bound = EXACT if mode == Mode.EXACT_F32 else 2.0 ** -10
+    for seed in range(2):
+        x.copy_(torch.randn(x.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(seed)))
+        y.zero_()
+        # work of other weights between the replays does not disturb them
+        dev.check(lib.fc_qmatmul_dev(other.handle, x.data_ptr(), m, y.data_ptr(), int(mode)))
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        dev.sync()
+        xd = x[:m].double()
+        assert bool(((y[:m].double() - xd @ w.T).abs() <= bound * (xd.abs() @ w.abs().T)).all())
+        assert not bool(y[m:].any())
+    del graph
+    qw.close()
+    other.close()
