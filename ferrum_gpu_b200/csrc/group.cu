@@ -274,7 +274,7 @@ FC_API int fc_group_score(FcGroup* g, const int32_t* ids, uint32_t n_seqs, uint3
   cudaEventRecord(g->ev[5], dev->stream);
   FC_CUDA(dev, cudaMemcpyAsync(nll_sum_out, d_out, (size_t)n_seqs * 8, cudaMemcpyDeviceToHost, dev->stream));
   FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
-  if (mode == FC_TENSOR_F16) FC_TRY(tc_check_errors(dev));
+  FC_TRY(tc_check_errors(dev)); // (the products of both modes have bounded waits)
   if (timed_split) {
     cudaEventElapsedTime(&g->last_ms[0], g->ev[0], g->ev[1]);
     cudaEventElapsedTime(&g->last_ms[1], g->ev[2], g->ev[3]);

@@ -3,7 +3,7 @@ CPU oracle, window by window), and a one-rank group of the C ABI (the NCCL path 
 import numpy as np
 import pytest
 
-from ferrum_gpu_b200 import CudaLlama, Mode, QKind
+from ferrum_gpu_b200 import CudaError, CudaLlama, Mode, QKind
 from ferrum_gpu_b200 import _ffi
 from ferrum_gpu_b200.group import GroupScorer
 from ferrum_gpu_b200.hostmodel import LlamaConfig, random_llama, random_tokens
@@ -91,4 +91,19 @@ def test_a_one_rank_group_scores_like_the_model(dev):
     got = gs.score(ids)
     assert np.array_equal(got, want)
     assert len(gs.exchange_ms()) == 3
+    gs.close()
+
+
+@pytest.mark.parametrize("mode", [Mode.EXACT_F32, Mode.TENSOR_F16])
+def test_a_given_up_wait_ends_a_group_call_with_an_error(dev, mode):
+    """The products of both modes have bounded waits. The status word such a wait leaves is set from the host here."""
+    cfg, m = _model(ctx=40)
+    ids = np.stack([random_tokens(50 + i, 33, cfg.vocab) for i in range(6)])
+    gs = GroupScorer(m, QKind.Q4_0, vocab_shards=1, mode=mode)
+    want = gs.score(ids)
+    gs.dev.check(_ffi.load().fc_debug_raise_status(gs.dev.handle, 3))
+    with pytest.raises(CudaError) as e:
+        gs.score(ids)
+    assert e.value.code == _ffi.FC_ERR_TIMEOUT
+    assert np.array_equal(gs.score(ids), want), "the status is cleared once reported"
     gs.close()
