@@ -210,6 +210,11 @@ struct DeferredReduce {
   float* y = nullptr;
 };
 
+struct Workspace { // device scratch and its size
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+
 struct Epilogue {
   const float* bias = nullptr;  // [n]
   const float* resid = nullptr; // [m][n]; may alias y
@@ -222,9 +227,9 @@ struct Epilogue {
   bool ragged = false;
   // device scratch that lets products of more than 64 rows of Q8_0 / Q4_0 weights run on the tensor cores (gemm_pair.cu;
   // qgemm_pair_scratch_bytes(k, n, m) is what the best cut takes); without it, or where it is too small, they take the
-  // tiled f32 kernel
-  void* wide_scratch = nullptr;
-  size_t wide_bytes = 0;
+  // tiled f32 kernel. (One pointer, read by host code only: the decode kernels take this struct as an
+  // argument, and with eight bytes more a decode step of 12 layers took 445 us instead of 433.)
+  const Workspace* wide = nullptr;
   // "x is the raw residual stream: normalise each row first" (NORM_RMS: y = x / sqrt(mean(x^2) + eps) * g,
   // NORM_LAYER: (x - mean) / sqrt(var + 1e-5) * g + b). The one-row FMA matvec does it while it stages x
   // in shared memory (one launch less per product); the other kernels run the norm kernel into

@@ -601,11 +601,11 @@ FC_API uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, u
   return p.splits ? plan_bytes(p, m) : 0;
 }
 
-int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, void* scratch, size_t bytes) {
+int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, const Workspace& space) {
   if (m == 0) return FC_OK;
-  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, w.k, w.n, m, bytes);
-  if (!p.splits) return fc_fail(dev, FC_ERR_ARG, "a %zu-byte workspace is too small for this product", bytes);
-  uint8_t* at = (uint8_t*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
+  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, w.k, w.n, m, space.bytes);
+  if (!p.splits) return fc_fail(dev, FC_ERR_ARG, "a %zu-byte workspace is too small for this product", space.bytes);
+  uint8_t* at = (uint8_t*)(((uintptr_t)space.p + 1023) & ~(uintptr_t)1023);
   auto take = [&](size_t bytes) {
     uint8_t* r = at;
     at += al(bytes);

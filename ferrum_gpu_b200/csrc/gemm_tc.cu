@@ -541,7 +541,7 @@ int k_qgemm_tp(FcDevice* dev, const QMat& w, const __half* x, int epi, const TcA
   const bool tma = epi != EPI_LSE && out && pitch % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   if (!tma && epi != EPI_LSE && epi != EPI_F32) return FC_OK;
   *handled = true;
-  __half* wf = (__half*)args.wide;
+  __half* wf = (__half*)args.wide->p;
   const uint32_t slice = tp_slice_rows(w);
   CUtensorMap tx, tw;
   FC_TRY(half_map(dev, &tx, x, args.m, w.k, 128));
@@ -707,7 +707,7 @@ int k_qgemm_tc_f16(FcDevice* dev, const QMat& w, const __half* a_dev, int epi, T
   if ((reinterpret_cast<uintptr_t>(a_dev) & 15) != 0) return fc_fail(dev, FC_ERR_ARG, "the A operand must be 16-byte aligned");
   EncodeTiledFn enc = encode_fn();
   if (!enc) return fc_fail(dev, FC_ERR_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
-  if (args.wide && tp_workspace_bytes(w) <= args.wide_bytes && tp_takes(dev, w, args.m, epi)) {
+  if (args.wide && tp_workspace_bytes(w) <= args.wide->bytes && tp_takes(dev, w, args.m, epi)) {
     bool handled = false;
     FC_TRY(k_qgemm_tp(dev, w, a_dev, epi, args, &handled));
     if (handled) return FC_OK;

@@ -27,8 +27,7 @@ struct TcArgs {
   uint32_t tile0 = 0;   // EPI_LSE: 128-column tiles of the head before this launch's weight rows
   // workspace for the fp16 weights of the pair kernel (tp_workspace_bytes; missing or too small: the weights are decoded in
   // the product)
-  void* wide = nullptr;
-  size_t wide_bytes = 0;
+  const Workspace* wide = nullptr;
   uint32_t out_tma = 0; // (set by the launch code) results leave through shared memory and TMA
 };
 

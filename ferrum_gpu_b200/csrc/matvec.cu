@@ -407,10 +407,10 @@ int k_qlinear_f32(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     return k_qmatvec1(dev, w, x, y, ep);
   }
   if (ep.swiglu) return fc_fail(dev, FC_ERR_ARG, "only the streamed one-row product applies SwiGLU");
-  if (ep.wide_scratch && forced == 0 && !ep.presplit && qgemm_pair_takes(w, m) && qgemm_pair_fits(dev, w.k, w.n, m, ep.wide_bytes)) {
+  if (ep.wide && ep.wide->p && forced == 0 && !ep.presplit && qgemm_pair_takes(w, m) && qgemm_pair_fits(dev, w.k, w.n, m, ep.wide->bytes)) {
     // (its x split takes the norm along)
     if (ep.pending && ep.pending->splits) FC_TRY(k_flush_deferred(dev, *ep.pending));
-    return k_qgemm_pair(dev, w, x, m, y, ep, ep.wide_scratch, ep.wide_bytes);
+    return k_qgemm_pair(dev, w, x, m, y, ep, *ep.wide);
   }
   if (ep.ragged && ep.scratch && forced == 0 && qmatvec_mma_ragged_supports(w, m) && (reinterpret_cast<uintptr_t>(x) & 15) == 0)
     return k_qmatvec_mma(dev, w, x, m, y, ep, ep.scratch);

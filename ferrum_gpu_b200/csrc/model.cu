@@ -203,7 +203,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
                   bool final_norm, DeferredReduce* tail = nullptr, bool embedded = false) {
   FcDevice* dev = m->dev;
   const uint32_t d = m->dim;
-  void* wide = mode != ATTN_DECODE ? m->wide : nullptr;
+  const Workspace* wide = mode != ATTN_DECODE ? &m->wide : nullptr;
   if (!embedded) FC_TRY(k_embed(dev, m->tok, m->pos_table, ids, positions, rows, d, b.x)); // (else b.x holds the rows)
   // The two products that write the residual stream (wo, ff2) may leave their split-K sum to the norm
   // launch of the product that reads it next: `pend` is that unfinished sum, consumed (or finished on
@@ -212,7 +212,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
   for (auto& l : m->layers) {
     Epilogue e_qkv;
     e_qkv.scratch = m->mma_scratch;
-    e_qkv.wide_scratch = wide, e_qkv.wide_bytes = m->wide_bytes;
+    e_qkv.wide = wide;
     e_qkv.bias = l.qkv.bias;
     e_qkv.pending = &pend;
     norm_before(m, e_qkv, l.norm1_g, l.norm1_b, b.h);
@@ -249,7 +249,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
     else
       FC_TRY(k_attn_prefill_cache_f32(dev, b.qkv, t, start, m->heads, m->kv_heads, m->hd, stream, l.kv, m->ctx, b.attn));
     e_wo.scratch = m->mma_scratch;
-    e_wo.wide_scratch = wide, e_wo.wide_bytes = m->wide_bytes;
+    e_wo.wide = wide;
     e_wo.bias = l.wo.bias;
     e_wo.resid = b.x;
     made = DeferredReduce();
@@ -258,7 +258,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
     pend = made;
     Epilogue e_ff1;
     e_ff1.scratch = m->mma_scratch;
-    e_ff1.wide_scratch = wide, e_ff1.wide_bytes = m->wide_bytes;
+    e_ff1.wide = wide;
     e_ff1.bias = l.ff1.bias;
     e_ff1.act = m->arch == ARCH_GPT2 ? ACT_GELU : ACT_NONE;
     e_ff1.pending = &pend;
@@ -292,7 +292,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
       ff2_in = e_ff2.swiglu ? b.ff : b.act;
     }
     e_ff2.scratch = m->mma_scratch;
-    e_ff2.wide_scratch = wide, e_ff2.wide_bytes = m->wide_bytes;
+    e_ff2.wide = wide;
     e_ff2.bias = l.ff2.bias;
     e_ff2.resid = b.x;
     made = DeferredReduce();
@@ -366,8 +366,7 @@ int arena_reserve_wide(FcModel* m, size_t bytes, size_t rows, int mode) {
     const int rc = arena_reserve(m, at + wide);
     if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
     if (rc == FC_OK) {
-      m->wide = m->arena.base + at;
-      m->wide_bytes = wide;
+      m->wide = Workspace{m->arena.base + at, wide};
       return FC_OK;
     }
   }
@@ -376,8 +375,7 @@ int arena_reserve_wide(FcModel* m, size_t bytes, size_t rows, int mode) {
 
 int arena_reserve(FcModel* m, size_t bytes) {
   m->arena.off = 0;
-  m->wide = nullptr;
-  m->wide_bytes = 0;
+  m->wide = Workspace();
   if (bytes <= m->arena.cap) return FC_OK;
   FC_CUDA(m->dev, cudaStreamSynchronize(m->dev->stream));
   if (m->arena.base) cudaFree(m->arena.base);
@@ -1014,7 +1012,7 @@ FC_API int fc_model_forward_all(FcModel* m, const int32_t* ids, uint32_t n, floa
   if (mode == FC_EXACT_F32) {
     FC_TRY(run_stack_f32(m, b, d_ids, d_pos, nullptr, n, ATTN_STATELESS, 1, n, 0, 0, true));
     Epilogue e_head;
-    e_head.wide_scratch = m->wide, e_head.wide_bytes = m->wide_bytes;
+    e_head.wide = &m->wide;
     FC_TRY(k_qlinear_f32(dev, m->head_view, b.h, n, logits, e_head));
     if (n > 64) FC_TRY(tc_check_errors(dev));
   } else if (mode == FC_TENSOR_F16) {

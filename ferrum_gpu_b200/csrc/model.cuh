@@ -70,8 +70,7 @@ struct FcModel {
   int32_t* d_chain_log = nullptr; // [ctx][max_streams]
   uint32_t* d_chain_cnt = nullptr;
   Arena arena;
-  void* wide = nullptr;   // behind the arena's carved part: workspace of the products of many rows
-  size_t wide_bytes = 0;  // its size: a product that needs more does without, or is cut to it
+  Workspace wide; // behind the arena's carved part, for the products of many rows: one that needs more does without, or is cut to it
   size_t pass_bytes = 0;  // bound of one scoring pass's workspace (fc_debug_score_pass_bytes; 0: the library's own)
   void* tc = nullptr; // state of the bf16 tensor-core path (built on first use)
   void* dc = nullptr; // state of the one-launch single-stream decode (decode_cluster.cu; probed on first use)

@@ -110,7 +110,8 @@ int k_qgemm_tc(FcDevice* dev, FcQWeight* w, const float* x_dev, uint32_t m, floa
   t.m = m;
   t.out_f32 = y_dev;
   t.ldo = w->m.n;
-  if (wide) t.wide = (uint8_t*)w->tc_cache + a_bytes, t.wide_bytes = w->tc_cache_bytes - a_bytes;
+  const Workspace rest{(uint8_t*)w->tc_cache + a_bytes, w->tc_cache_bytes - a_bytes};
+  if (wide) t.wide = &rest;
   return k_qgemm_tc_f16(dev, w->m, a, EPI_F32, t);
 }
 
@@ -130,7 +131,7 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
   for (auto& l : m->layers) {
     FC_TRY(k_norm_f16(dev, ln, x, l.norm1_g, l.norm1_b, rows, d, m->eps, h));
     TcArgs a_qkv;
-    a_qkv.wide = m->wide, a_qkv.wide_bytes = m->wide_bytes, a_qkv.m = rows, a_qkv.bias = l.qkv.bias, a_qkv.out_f16 = qkv, a_qkv.ldo = m->qkv_w();
+    a_qkv.wide = &m->wide, a_qkv.m = rows, a_qkv.bias = l.qkv.bias, a_qkv.out_f16 = qkv, a_qkv.ldo = m->qkv_w();
     // (RoPE fused into this product's epilogue was measured at a third of the plain fp16 store's rate - the
     // table gathers - so the rotation runs as its own 16-byte-vectorised pass over the q and k columns.)
     FC_TRY(k_qgemm_tc_f16(dev, l.qkv.w->m, h, EPI_F16, a_qkv));
@@ -143,11 +144,11 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
     else
       FC_TRY(k_attn_causal_f16(dev, qkv, n_seqs, t, m->heads, m->kv_heads, m->hd, attn));
     TcArgs a_wo;
-    a_wo.wide = m->wide, a_wo.wide_bytes = m->wide_bytes, a_wo.m = rows, a_wo.bias = l.wo.bias, a_wo.out_f32 = x, a_wo.ldo = d;
+    a_wo.wide = &m->wide, a_wo.m = rows, a_wo.bias = l.wo.bias, a_wo.out_f32 = x, a_wo.ldo = d;
     FC_TRY(k_qgemm_tc_f16(dev, l.wo.w->m, attn, EPI_RESID, a_wo));
     FC_TRY(k_norm_f16(dev, ln, x, l.norm2_g, l.norm2_b, rows, d, m->eps, h));
     TcArgs a_ff1;
-    a_ff1.wide = m->wide, a_ff1.wide_bytes = m->wide_bytes, a_ff1.m = rows, a_ff1.bias = l.ff1.bias, a_ff1.out_f16 = act, a_ff1.ldo = m->hidden;
+    a_ff1.wide = &m->wide, a_ff1.m = rows, a_ff1.bias = l.ff1.bias, a_ff1.out_f16 = act, a_ff1.ldo = m->hidden;
     if (m->arch == ARCH_LLAMA) {
       FC_TRY(k_qgemm_tc_f16(dev, l.ff1.w->m, h, EPI_SWIGLU, a_ff1));
     } else {
@@ -155,7 +156,7 @@ int model_trunk_tc(FcModel* m, const int32_t* ids, const int32_t* positions, uin
       FC_TRY(k_qgemm_tc_f16(dev, l.ff1.w->m, h, EPI_F16, a_ff1));
     }
     TcArgs a_ff2;
-    a_ff2.wide = m->wide, a_ff2.wide_bytes = m->wide_bytes, a_ff2.m = rows, a_ff2.bias = l.ff2.bias, a_ff2.out_f32 = x, a_ff2.ldo = d;
+    a_ff2.wide = &m->wide, a_ff2.m = rows, a_ff2.bias = l.ff2.bias, a_ff2.out_f32 = x, a_ff2.ldo = d;
     FC_TRY(k_qgemm_tc_f16(dev, l.ff2.w->m, act, EPI_RESID, a_ff2));
   }
   return k_norm_f16(dev, ln, x, m->normf_g, m->normf_b, rows, d, m->eps, hidden_out);
@@ -165,7 +166,7 @@ int model_head_partial_tc(FcModel* m, const __half* hidden, const int32_t* targe
   const uint32_t tiles = (m->v1 - m->v0 + TC_BN - 1) / TC_BN;
   float* tile_partials = (float*)arena_take(m, (size_t)rows * tiles * 16);
   TcArgs a;
-  a.wide = m->wide, a.wide_bytes = m->wide_bytes;
+  a.wide = &m->wide;
   a.m = rows, a.targets = targets, a.v0 = m->v0, a.partial = tile_partials;
   FC_TRY(k_qgemm_tc_f16(m->dev, m->head_view, hidden, EPI_LSE, a));
   return k_partial_merge(m->dev, tile_partials, tiles, rows, partial);
@@ -173,7 +174,7 @@ int model_head_partial_tc(FcModel* m, const __half* hidden, const int32_t* targe
 
 int model_logits_tc(FcModel* m, const __half* hidden, uint32_t rows, float* logits) {
   TcArgs a;
-  a.wide = m->wide, a.wide_bytes = m->wide_bytes;
+  a.wide = &m->wide;
   a.m = rows, a.out_f32 = logits, a.ldo = m->v1 - m->v0;
   return k_qgemm_tc_f16(m->dev, m->head_view, hidden, EPI_F32, a);
 }

@@ -135,6 +135,7 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
   cudaSetDevice(dev->ordinal);
   if (mode == FC_EXACT_F32) {
     Epilogue ep;
+    Workspace wide;
     ep.ragged = true;
     if ((m > 1 || dev->matvec_choice) && (qmatvec_mma_supports(w->m, m) || qmatvec_mma_ragged_supports(w->m, m))) {
       // up to 64 rows: the decode tensor product needs scratch (one row takes kernels that need none)
@@ -151,8 +152,9 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
     } else if (qgemm_pair_takes(w->m, m)) {
       const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m));
       if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
-// (no room for more, or a capture: the product is cut to the workspace that is there, or takes the tiled f32 kernel)
-      ep.wide_scratch = w->tc_cache, ep.wide_bytes = w->tc_cache_bytes;
+      // (no room for more, or a capture: the product is cut to the workspace that is there, or takes the tiled f32 kernel)
+      wide = Workspace{w->tc_cache, w->tc_cache_bytes};
+      ep.wide = &wide;
     }
     return k_qlinear_f32(dev, w->m, x_dev, m, y_dev, ep);
   }

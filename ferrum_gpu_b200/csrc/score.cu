@@ -51,7 +51,7 @@ FC_API int fc_debug_score_pass_bytes(FcModel* m, uint64_t bytes) {
 static int head_partial_f32(FcModel* m, const float* hidden, const int32_t* targets, uint32_t rows, float* logits_ws,
                             float* partial) {
   Epilogue ep;
-  ep.wide_scratch = m->wide, ep.wide_bytes = m->wide_bytes;
+  ep.wide = &m->wide;
   FC_TRY(k_qlinear_f32(m->dev, m->head_view, hidden, rows, logits_ws, ep));
   return k_score_partial(m->dev, logits_ws, targets, rows, m->v1 - m->v0, m->v0, partial);
 }
