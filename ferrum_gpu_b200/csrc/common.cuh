@@ -194,6 +194,65 @@ __device__ __forceinline__ float fp8_to_f32(uint32_t code) {
   const uint32_t h2 = fp8x2_to_f16x2<KIND>(code & 0xffu);
   return __half2float(__ushort_as_half((unsigned short)(h2 & 0xffffu)));
 }
+// Elements i .. i + 7 (i a multiple of 8) of weight row `row`, d * q rounded as the decoder rounds it.
+template <int KIND>
+__device__ __forceinline__ void qmat_eight(const QMat& w, uint32_t row, uint32_t i, float (&v)[8]) {
+  const uint32_t k = w.k;
+  if (KIND == FC_Q8_0) {
+    const uint2 q = *reinterpret_cast<const uint2*>(w.qs + (size_t)row * k + i);
+    const float d = __half2float(w.sc[(size_t)row * (k / QK) + i / QK]);
+    const uint32_t qw[2] = {q.x, q.y};
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __fmul_rn(d, (float)(int8_t)((qw[j >> 2] >> (8 * (j & 3))) & 0xff));
+  } else if (KIND == FC_Q2_K) { // (d * sc) * q - dmin * m, as the decoder rounds it
+    const uint32_t sub = i / 16;
+    const uint8_t* rec = reinterpret_cast<const uint8_t*>(w.sc) + ((size_t)row * (k / QK_K) + i / QK_K) * 20;
+    const uint32_t word = reinterpret_cast<const uint32_t*>(w.qs)[(size_t)row * (k / 16) + sub] >> (2 * (i % 16));
+    const uint8_t sc = rec[sub % 16];
+    const float dl = __fmul_rn(__half2float(*reinterpret_cast<const __half*>(rec + 16)), (float)(sc & 15));
+    const float ml = __fmul_rn(__half2float(*reinterpret_cast<const __half*>(rec + 18)), (float)(sc >> 4));
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __fsub_rn(__fmul_rn(dl, (float)((word >> (2 * j)) & 3)), ml);
+  } else if (KIND == FC_MXFP4) {
+    const uint32_t q = *reinterpret_cast<const uint32_t*>(w.qs + (size_t)row * (k / 2) + i / 2);
+    const float d = block_scale_f32<KIND>(w.sc[(size_t)row * (k / QK) + i / QK]);
+    uint32_t h[4];
+    e2m1x8_to_f16x2(q, h);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[j]));
+      v[2 * j] = __fmul_rn(d, f.x);
+      v[2 * j + 1] = __fmul_rn(d, f.y);
+    }
+  } else if (kind_is_fp8(KIND)) {
+    const uint2 q = *reinterpret_cast<const uint2*>(w.qs + (size_t)row * k + i);
+    const float d = __half2float(w.sc[(size_t)row * (k / QK) + i / QK]);
+    const uint32_t qw[2] = {q.x, q.y};
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __fmul_rn(d, fp8_to_f32<KIND>(qw[j >> 2] >> (8 * (j & 3))));
+  } else if (KIND == FC_Q4_0) {
+    const uint32_t q = *reinterpret_cast<const uint32_t*>(w.qs + (size_t)row * (k / 2) + i / 2);
+    const float d = __half2float(w.sc[(size_t)row * (k / QK) + i / QK]);
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      const int pos = (j >> 1) + 4 * (j & 1);
+      v[j] = __fmul_rn(d, (float)((q >> (4 * pos)) & 0xf) - 8.0f);
+    }
+  } else if (KIND == FC_F16) {
+    const uint4 q = *reinterpret_cast<const uint4*>(w.qs + ((size_t)row * k + i) * 2);
+    const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&qw[j]));
+      v[2 * j] = f.x;
+      v[2 * j + 1] = f.y;
+    }
+  } else {
+    const float* src = reinterpret_cast<const float*>(w.qs) + (size_t)row * k;
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = i + j < k ? src[i + j] : 0.0f;
+  }
+}
 #endif
 
 // Epilogue of a matrix product: y = act(x W + bias) (+ resid). All pointers device, nullable.

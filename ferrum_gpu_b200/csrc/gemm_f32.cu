@@ -48,63 +48,7 @@ __global__ void __launch_bounds__(256)
       const uint32_t row = n0 + r;
       float v[8];
       if (row < n) {
-        if (KIND == FC_Q8_0) {
-          const uint2 q = *reinterpret_cast<const uint2*>(w.qs + (size_t)row * k + k0 + part * 8);
-          const float d = __half2float(w.sc[(size_t)row * (k / QK) + k0 / QK]);
-          const uint32_t qw[2] = {q.x, q.y};
-#pragma unroll
-          for (int j = 0; j < 8; j++) v[j] = __fmul_rn(d, (float)(int8_t)((qw[j >> 2] >> (8 * (j & 3))) & 0xff));
-        } else if (KIND == FC_Q2_K) { // (d * sc) * q - dmin * m, as the decoder rounds it
-          const uint32_t kk = k0 + part * 8, sub = kk / 16;
-          const uint8_t* rec = reinterpret_cast<const uint8_t*>(w.sc) + ((size_t)row * (k / QK_K) + kk / QK_K) * 20;
-          const uint32_t word = reinterpret_cast<const uint32_t*>(w.qs)[(size_t)row * (k / 16) + sub] >> (2 * (kk % 16));
-          const uint8_t sc = rec[sub % 16];
-          const float dl = __fmul_rn(__half2float(*reinterpret_cast<const __half*>(rec + 16)), (float)(sc & 15));
-          const float ml = __fmul_rn(__half2float(*reinterpret_cast<const __half*>(rec + 18)), (float)(sc >> 4));
-#pragma unroll
-          for (int j = 0; j < 8; j++) v[j] = __fsub_rn(__fmul_rn(dl, (float)((word >> (2 * j)) & 3)), ml);
-        } else if (KIND == FC_MXFP4) {
-          const uint32_t q = *reinterpret_cast<const uint32_t*>(w.qs + (size_t)row * (k / 2) + (k0 / QK) * 16 + part * 4);
-          const float d = block_scale_f32<KIND>(w.sc[(size_t)row * (k / QK) + k0 / QK]);
-          uint32_t h[4];
-          e2m1x8_to_f16x2(q, h);
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[j]));
-            v[2 * j] = __fmul_rn(d, f.x);
-            v[2 * j + 1] = __fmul_rn(d, f.y);
-          }
-        } else if (kind_is_fp8(KIND)) {
-          const uint2 q = *reinterpret_cast<const uint2*>(w.qs + (size_t)row * k + k0 + part * 8);
-          const float d = __half2float(w.sc[(size_t)row * (k / QK) + k0 / QK]);
-          const uint32_t qw[2] = {q.x, q.y};
-#pragma unroll
-          for (int j = 0; j < 8; j++) v[j] = __fmul_rn(d, fp8_to_f32<KIND>(qw[j >> 2] >> (8 * (j & 3))));
-        } else if (KIND == FC_Q4_0) {
-          const uint32_t q = *reinterpret_cast<const uint32_t*>(w.qs + (size_t)row * (k / 2) + (k0 / QK) * 16 + part * 4);
-          const float d = __half2float(w.sc[(size_t)row * (k / QK) + k0 / QK]);
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const int pos = (j >> 1) + 4 * (j & 1);
-            v[j] = __fmul_rn(d, (float)((q >> (4 * pos)) & 0xf) - 8.0f);
-          }
-        } else if (KIND == FC_F16) {
-          const uint4 q = *reinterpret_cast<const uint4*>(w.qs + ((size_t)row * k + k0 + part * 8) * 2);
-          const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&qw[j]));
-            v[2 * j] = f.x;
-            v[2 * j + 1] = f.y;
-          }
-        } else {
-          const float* src = reinterpret_cast<const float*>(w.qs) + (size_t)row * k;
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const uint32_t kk = k0 + part * 8 + j;
-            v[j] = kk < k ? src[kk] : 0.0f;
-          }
-        }
+        qmat_eight<KIND>(w, row, k0 + part * 8, v);
       } else {
 #pragma unroll
         for (int j = 0; j < 8; j++) v[j] = 0.0f;

@@ -3,12 +3,16 @@
 //   y[r, n] = sum_k x[r, k] * d[n, k / 32] * q[n, k]
 //
 // Both factors become two fp16 terms, written once per call by two preparation kernels (gemm_pair.cu: rows_split,
-// weights_split) and read by TMA: x 2^s = xh + xl, d q 2^t = wh + wl, s per row of x and t per weight row, powers of
-// two that put the row's largest magnitude next to the top of the fp16 range, so that the low terms keep their bits
-// however small the values are; the epilogue takes 2^-s 2^-t back. Three of the four cross terms are multiplied
-// (wl . xl is below 2^-22 of the product, a quarter of an f32 rounding), all into one f32 accumulator, the small ones
-// first. The tensor cores' f32 accumulation rounds toward zero, so tensor memory only ever holds the sum of 128 k
-// (64 k at short widths): then the epilogue warps add the finished sum into f32 registers.
+// weights_split) and read by TMA: x 2^s = xh + xl 2^-11, d q 2^t = wh + wl 2^-11, s per row of x and t per weight row,
+// powers of two that put the row's largest magnitude next to the top of the fp16 range; the epilogue takes 2^-s 2^-t back.
+// The low terms are kept 2^11 larger than what they stand for, at the magnitude of the high ones, so that they are as far
+// from fp16's subnormals: an element of x has 22 bits down to 2^-28 of its row's largest, and d q (19 bits, and no f16
+// scale is below 2^-24) is always exact. A row that reaches further down with a part of its sum that counts is multiplied
+// by the f32 chain instead, as are rows with infinities and NaNs (row_is_wide). Three of the four cross terms are
+// multiplied (wl . xl is below 2^-22 of the product, a quarter of an f32 rounding), all into one f32 accumulator, the small
+// ones first; the first large one brings their sum down by 2^-11 (the MMA's own scaling of D). The tensor cores' f32
+// accumulation rounds toward zero, so tensor memory only ever holds the sum of 128 k (64 k at short widths): then the
+// epilogue warps add the finished sum into f32 registers.
 //
 // The pair: two CTAs on neighbouring SMs work on one tile of 256 weight rows x 128 or 64 rows of x
 // (tcgen05.mma.cta_group::2): each holds its 128 weight rows (tensor-memory lanes) and half of the x rows in shared
@@ -34,6 +38,7 @@ namespace {
 constexpr uint32_t BK = 64;                        // k per stage: one 128-byte swizzle row of fp16
 constexpr int PAIR_THREADS = 384;
 constexpr uint32_t A_TERM = 128 * BK * 2;          // 16 KB: this CTA's 128 weight rows, one term
+constexpr int LOW_SHIFT = 11;                      // low terms are stored times 2^11
 constexpr uint32_t NACC = 4;                       // accumulator buffers: the hand-over between SMs takes about a chunk's MMA time
 template <int BN>
 struct Shape {
@@ -80,7 +85,7 @@ struct PairArgs {
   uint32_t ldy = 0;
   const float* bias = nullptr;  // [w.n]
   const float* resid = nullptr; // [m][ldy]; may alias y
-  const float* x_scale = nullptr; // [m] 2^-s; 0: the row holds an infinity or NaN
+  const float* x_scale = nullptr; // [m] 2^-s; 0: the fp16 terms do not hold the row
   const float* w_scale = nullptr; // [w.n] 2^-t; 0: a block scale of the row is not finite
   float* partial = nullptr;       // [splits][m][w.n]: the sums without bias, activation and residual
   int* err_flag = nullptr;
@@ -88,18 +93,16 @@ struct PairArgs {
 
 // One output by the f32 chain, ascending k: rows of x or W with values that the fp16 terms cannot hold.
 template <int KIND>
-__device__ __noinline__ float exact_dot(const float* xr, const uint8_t* qs, const __half* sc, uint32_t width) {
+__device__ __noinline__ float exact_dot(const float* x, const uint8_t* qs, const __half* sc, uint32_t k, uint32_t n) {
+  const QMat w{KIND, k, 0, qs, sc}; // (by reference, the kernel's whole argument block would be copied to the stack)
   float acc = 0.0f;
-  for (uint32_t k = 0; k < width; k++) {
-    const float d = __half2float(sc[k / QK]);
-    int q;
-    if (KIND == FC_Q8_0) {
-      q = (int)(int8_t)qs[k];
-    } else { // element j of a word of eight sits at nibble (j >> 1) + 4 (j & 1)
-      const uint32_t word = reinterpret_cast<const uint32_t*>(qs)[k / 8], j = k % 8;
-      q = (int)((word >> (4 * ((j >> 1) + 4 * (j & 1)))) & 15u) - 8;
-    }
-    acc = fmaf(xr[k], __fmul_rn(d, (float)q), acc);
+#pragma unroll 4
+  for (uint32_t i = 0; i < k; i += 8) {
+    float v[8];
+    qmat_eight<KIND>(w, n, i, v);
+    const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
+    acc = fmaf(a.x, v[0], acc), acc = fmaf(a.y, v[1], acc), acc = fmaf(a.z, v[2], acc), acc = fmaf(a.w, v[3], acc);
+    acc = fmaf(b.x, v[4], acc), acc = fmaf(b.y, v[5], acc), acc = fmaf(b.z, v[6], acc), acc = fmaf(b.w, v[7], acc);
   }
   return acc;
 }
@@ -229,7 +232,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
             const uint32_t s = (it + c) % S::STAGES, st = base + s * S::STAGE;
             const uint64_t dwh = hi | (st >> 4), dxh = hi | ((st + 2 * A_TERM) >> 4);
 #pragma unroll
-            for (uint32_t ks = 0; ks < BK / 16; ks++) tc::mma_f16_pair(d, dwh + 2 * ks, dxh + 2 * ks, idesc, 1u);
+            for (uint32_t ks = 0; ks < BK / 16; ks++) {
+              if (ks == 0 && c == 0)
+                tc::mma_f16_pair_shifted<LOW_SHIFT>(d, dwh, dxh, idesc); // what is there so far are the low terms' products
+              else
+                tc::mma_f16_pair(d, dwh + 2 * ks, dxh + 2 * ks, idesc, 1u);
+            }
             tc::mma_commit_pair(&empty[s]);
           }
           it += n_st;
@@ -305,13 +313,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           }
         }
         if (bad) {
-          const uint32_t k = a.w.k;
 #pragma unroll 1
           for (uint32_t row = xr; row < min(xr + COLS, a.m); row++) {
             if (ws != 0.0f && a.x_scale[row] != 0.0f) continue;
             float v = 0.0f; // (of several splits the first has the whole sum)
-            if (k0 == 0)
-              v = exact_dot<KIND>(a.x + (size_t)row * k, a.w.qs + (size_t)n * (KIND == FC_Q8_0 ? k : k / 2), a.w.sc + (size_t)n * (k / QK), k);
+            if (k0 == 0) v = exact_dot<KIND>(a.x + (size_t)row * a.w.k, a.w.qs, a.w.sc, a.w.k, n);
             if (!a.partial) v += bias;
             if (res) v = res[(size_t)row * ldo + n] + v;
             out[(size_t)row * ldo + n] = v;
@@ -371,6 +377,21 @@ __device__ __forceinline__ void pow2_to(float mx, int e, float& mul, float& inv)
   inv = __uint_as_float((uint32_t)(127 - s) << 23);
 }
 
+// Whether the two terms of a row lose what an f32 sum would keep. `lost` is what this thread's elements lose beyond 2^-22
+// of themselves (elements below 2^-28 of the row's largest: their low terms are subnormal, or both terms are zero), `sum`
+// the sum of its elements' magnitudes. One such element among ordinary ones is far below a rounding of the result; it
+// counts where the row's large elements meet weights of zero and only small ones remain. So the row is held as long as
+// 2^-22 of what is left covers the loss even without any `few` threads' parts (so many large elements at least): where
+// few + 1 threads each have as much, or few + a quarter of the threads their share of it. No element loses more than 2^-50
+// of the row's largest: ordinary rows, whose other elements sum to far more than k 2^-28 of it, are never refused.
+__device__ __forceinline__ bool row_is_wide(float lost, float sum, uint32_t k, float* red) {
+  if (!__syncthreads_or(lost > 0.0f)) return false;
+  const float covered = block_sum(lost, red) * 0x1p22f;
+  const int few = (int)min(15u, k / 8 - 1), quarter = (int)min(256u, k / 2) / 4;
+  const int have = __syncthreads_count(sum >= covered), share = __syncthreads_count(sum * (float)quarter >= covered);
+  return have < few + 1 && share < few + quarter;
+}
+
 // One CTA per row: norm (the sums in the order of the stand-alone norm kernels: the same bits), the row's power of
 // two, the two fp16 terms, zeros up to the padded width. `normed` (with a norm) gets the f32 row.
 __global__ void __launch_bounds__(256)
@@ -420,18 +441,31 @@ __global__ void __launch_bounds__(256)
   const bool finite = s_max < 0x7f800000u;
   float mul, back;
   pow2_to(__uint_as_float(s_max), 14, mul, back);
-  // a row with an infinity or NaN: flagged for the kernel's own f32 chain, or (`carry`) kept in the high term
-  if (threadIdx.x == 0) x_scale[r] = finite || carry ? back : 0.0f;
+  const float up = carry ? 1.0f : (float)(1 << LOW_SHIFT);
+  float lost = 0.0f, sum = 0.0f;
   for (uint32_t i = threadIdx.x * 2; i < kp; i += blockDim.x * 2) { // (k and kp are even)
     float v0 = 0.0f, v1 = 0.0f;
     if ((finite || carry) && i < k) v0 = value(i) * mul, v1 = value(i + 1) * mul;
     const __half2 h = __floats2half2_rn(v0, v1);
     float2 f = __half22float2(h);
     *reinterpret_cast<__half2*>(xh + (size_t)r * kp + i) = h;
-    float l0 = v0 - f.x, l1 = v1 - f.y;
+    float l0 = (v0 - f.x) * up, l1 = (v1 - f.y) * up;
     if (!finite) l0 = fabsf(v0) < INFINITY ? l0 : 0.0f, l1 = fabsf(v1) < INFINITY ? l1 : 0.0f;
-    *reinterpret_cast<__half2*>(xl + (size_t)r * kp + i) = __floats2half2_rn(l0, l1);
+    const __half2 l = __floats2half2_rn(l0, l1);
+    *reinterpret_cast<__half2*>(xl + (size_t)r * kp + i) = l;
+    const float a0 = fabsf(v0), a1 = fabsf(v1);
+    if (fminf(a0, a1) < 0x1p-14f) { // (only there can the terms be short)
+      const float2 lf = __half22float2(l);
+      const float e0 = fabsf(l0 - lf.x), e1 = fabsf(l1 - lf.y); // the errors, times 2^11
+      if (e0 > a0 * 0x1p-11f) lost += e0 * 0x1p-11f;
+      if (e1 > a1 * 0x1p-11f) lost += e1 * 0x1p-11f;
+    }
+    sum += a0 + a1;
   }
+  // a row that the terms do not hold: flagged for the product's own f32 chain, or (`carry`) left to the terms, the
+  // infinities and NaNs in the high one
+  const bool held = carry || (finite && !row_is_wide(lost, sum, k, red));
+  if (threadIdx.x == 0) x_scale[r] = held ? back : 0.0f;
 }
 
 // One warp per weight row: the row's power of two from its block scales, then eight elements per lane and step: the
@@ -474,7 +508,7 @@ __global__ void __launch_bounds__(256)
     for (int j = 0; j < 4; j++) {
       const __half2 hh = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
       const float2 f = __half22float2(hh);
-      const __half2 ll = __floats2half2_rn(v[2 * j] - f.x, v[2 * j + 1] - f.y);
+      const __half2 ll = __floats2half2_rn((v[2 * j] - f.x) * (float)(1 << LOW_SHIFT), (v[2 * j + 1] - f.y) * (float)(1 << LOW_SHIFT));
       h[j] = *reinterpret_cast<const uint32_t*>(&hh);
       l[j] = *reinterpret_cast<const uint32_t*>(&ll);
     }
@@ -582,7 +616,9 @@ int launch(FcDevice* dev, const CUtensorMap* maps, const PairArgs& a) {
 // active 47 %, L2 33 %: 264 tiles take 4 waves of pairs (3.6 full), and every 128 k the accumulator changes hands between
 // the MMA thread and the epilogues of two SMs.
 // Error against f64 on N(0, 1) x N(0, 0.02), of the result's norm: 1.2e-7 (K 96) to 2.2e-7 (K 4096); the f32 chain
-// 1.8e-7 to 1.15e-6.
+// 1.8e-7 to 1.15e-6. With two elements of 2^20 or 2^26 in every row, the largest error of an output against its own
+// sum |x w|: 0.9e-6..1.3e-6 (the chain 2.3e-6..7.7e-6; with low terms at their own magnitude 2^26 came to 1e-5, beyond 2^34
+// to a thousandth and more). The check of the rows costs 1 us a call.
 bool qgemm_pair_takes(const QMat& w, uint32_t m) {
   const uint64_t tiles = (uint64_t)((w.n + 63) / 64) * ((m + 63) / 64); // the tiled kernel's CTAs
   if (w.k * (tiles > TILED_WAVE ? tiles : TILED_WAVE) < TILED_KEEPS) return false;

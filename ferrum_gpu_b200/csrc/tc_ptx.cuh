@@ -228,6 +228,15 @@ __device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t desc_a, u
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// D = A . B + D 2^-SHIFT
+template <int SHIFT>
+__device__ __forceinline__ void mma_f16_pair_shifted(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
+  static_assert(SHIFT >= 0 && SHIFT <= 15, "scale-input-d");
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.eq.b32 p, 0, 0;\ntcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, %4;\n}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "n"(SHIFT)
+      : "memory");
+}
 // Arrive on the barrier at this offset in both CTAs once every MMA this thread issued so far has finished.
 __device__ __forceinline__ void mma_commit_pair(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),

@@ -52,9 +52,51 @@ def test_rows_with_infinities_and_nans_and_zero_rows(dev, kind, m, k):
     for i, r in enumerate(bad):
         assert np.array_equal(np.isnan(got[r]), np.isnan(want[i])) and np.array_equal(got[r][~np.isnan(want[i])], want[i][~np.isnan(want[i])])
     assert np.all(got[20] == 0)
+    # 3e38 among values about 1: an f32 chain rounds k times at most; where its weight is zero the others count in full
+    big = x[30].astype(np.float64)
+    assert np.all(np.abs(got[30] - big @ w.T) <= k * 2.0 ** -24 * (np.abs(big) @ np.abs(w).T)) and np.any(w[:, 1] == 0)
     others = [r for r in range(m) if r not in bad + [20, 30]]
     assert np.array_equal(got[others], clean[others]), "other rows do not change"
     qw.close()
+
+
+def _spread_rows(spread, m, k):
+    """Rows whose magnitudes are far apart."""
+    rng = np.random.default_rng(9)
+    x = rng.standard_normal((m, k))
+    if spread == "ramp":
+        x *= 2.0 ** (-60 * np.arange(k) / k)
+    elif spread == "lognormal":
+        x *= np.exp(4 * rng.standard_normal((m, k)))
+    elif spread == "one small":
+        x[:, 3] *= 2.0 ** -45
+    else:  # two large elements, whose weights are zero in half of the outputs
+        x[:, 7], x[:, k - 2] = 2.0 ** spread, -2.0 ** (spread - 1)
+    return x.astype(np.float32)
+
+
+def _spread_check(dev, kind, m, k, n, spread):
+    w = np.random.default_rng(4).standard_normal((k, n)).astype(np.float32) * 0.02
+    w[7, ::2] = w[k - 2, ::2] = 0.0
+    qw = upload_quantised(dev, kind, w.reshape(-1), k, n)
+    w = qw.dequantised().reshape(n, k).astype(np.float64)
+    x = _spread_rows(spread, m, k)
+    want, scale = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    got = linear_q(dev, x, qw, m).reshape(m, n)
+    # the terms hold elements down to 2^-28 of the largest; beyond, the f32 chain: k roundings at most
+    bound = k * 2.0 ** -24 if not isinstance(spread, str) and spread > 26 else EXACT
+    assert np.all(np.abs(got - want) <= bound * scale), (kind, m, k, n, spread, np.max(np.abs(got - want) / scale))
+    qw.close()
+
+
+SPREADS = [8, 20, 26, 34, 60, 127, "ramp", "lognormal", "one small"]
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0])
+@pytest.mark.parametrize("m,k,n", [(100, 512, 300), (300, 96, 3000), (200, 2080, 513)])
+@pytest.mark.parametrize("spread", SPREADS)
+def test_exact_products_of_many_rows_keep_small_elements_beside_large_ones(dev, kind, m, k, n, spread):
+    _spread_check(dev, kind, m, k, n, spread)
 
 
 @pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0, QKind.F16, QKind.FP8_E4M3, QKind.MXFP4])
