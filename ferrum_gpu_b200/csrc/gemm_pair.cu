@@ -38,7 +38,6 @@ namespace {
 constexpr uint32_t BK = 64;                        // k per stage: one 128-byte swizzle row of fp16
 constexpr int PAIR_THREADS = 384;
 constexpr uint32_t A_TERM = 128 * BK * 2;          // 16 KB: this CTA's 128 weight rows, one term
-constexpr int LOW_SHIFT = 11;                      // low terms are stored times 2^11
 constexpr uint32_t NACC = 4;                       // accumulator buffers: the hand-over between SMs takes about a chunk's MMA time
 template <int BN>
 struct Shape {
@@ -90,22 +89,6 @@ struct PairArgs {
   float* partial = nullptr;       // [splits][m][w.n]: the sums without bias, activation and residual
   int* err_flag = nullptr;
 };
-
-// One output by the f32 chain, ascending k: rows of x or W with values that the fp16 terms cannot hold.
-template <int KIND>
-__device__ __noinline__ float exact_dot(const float* x, const uint8_t* qs, const __half* sc, uint32_t k, uint32_t n) {
-  const QMat w{KIND, k, 0, qs, sc}; // (by reference, the kernel's whole argument block would be copied to the stack)
-  float acc = 0.0f;
-#pragma unroll 4
-  for (uint32_t i = 0; i < k; i += 8) {
-    float v[8];
-    qmat_eight<KIND>(w, n, i, v);
-    const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
-    acc = fmaf(a.x, v[0], acc), acc = fmaf(a.y, v[1], acc), acc = fmaf(a.z, v[2], acc), acc = fmaf(a.w, v[3], acc);
-    acc = fmaf(b.x, v[4], acc), acc = fmaf(b.y, v[5], acc), acc = fmaf(b.z, v[6], acc), acc = fmaf(b.w, v[7], acc);
-  }
-  return acc;
-}
 
 template <int KIND, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
@@ -317,7 +300,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
           for (uint32_t row = xr; row < min(xr + COLS, a.m); row++) {
             if (ws != 0.0f && a.x_scale[row] != 0.0f) continue;
             float v = 0.0f; // (of several splits the first has the whole sum)
-            if (k0 == 0) v = exact_dot<KIND>(a.x + (size_t)row * a.w.k, a.w.qs, a.w.sc, a.w.k, n);
+            if (k0 == 0) v = exact_dot<KIND>(a.x + (size_t)row * a.w.k, a.w.qs, a.w.sc, a.w.k, n, 0, a.w.k);
             if (!a.partial) v += bias;
             if (res) v = res[(size_t)row * ldo + n] + v;
             out[(size_t)row * ldo + n] = v;
@@ -395,7 +378,7 @@ __device__ __forceinline__ bool row_is_wide(float lost, float sum, uint32_t k, f
 // One CTA per row: norm (the sums in the order of the stand-alone norm kernels: the same bits), the row's power of
 // two, the two fp16 terms, zeros up to the padded width. `normed` (with a norm) gets the f32 row.
 __global__ void __launch_bounds__(256)
-    rows_split_kernel(const float* __restrict__ x, uint32_t m, uint32_t k, uint32_t kp, bool carry, int norm, const float* __restrict__ g,
+    rows_split_kernel(const float* __restrict__ x, uint32_t m, uint32_t k, uint32_t kp, int norm, const float* __restrict__ g,
                       const float* __restrict__ b, float eps, float* __restrict__ normed, __half* __restrict__ xh,
                       __half* __restrict__ xl, float* __restrict__ x_scale) {
   __shared__ float red[32];
@@ -441,16 +424,15 @@ __global__ void __launch_bounds__(256)
   const bool finite = s_max < 0x7f800000u;
   float mul, back;
   pow2_to(__uint_as_float(s_max), 14, mul, back);
-  const float up = carry ? 1.0f : (float)(1 << LOW_SHIFT);
+  constexpr float UP = (float)(1 << LOW_SHIFT);
   float lost = 0.0f, sum = 0.0f;
   for (uint32_t i = threadIdx.x * 2; i < kp; i += blockDim.x * 2) { // (k and kp are even)
     float v0 = 0.0f, v1 = 0.0f;
-    if ((finite || carry) && i < k) v0 = value(i) * mul, v1 = value(i + 1) * mul;
+    if (finite && i < k) v0 = value(i) * mul, v1 = value(i + 1) * mul;
     const __half2 h = __floats2half2_rn(v0, v1);
     float2 f = __half22float2(h);
     *reinterpret_cast<__half2*>(xh + (size_t)r * kp + i) = h;
-    float l0 = (v0 - f.x) * up, l1 = (v1 - f.y) * up;
-    if (!finite) l0 = fabsf(v0) < INFINITY ? l0 : 0.0f, l1 = fabsf(v1) < INFINITY ? l1 : 0.0f;
+    const float l0 = (v0 - f.x) * UP, l1 = (v1 - f.y) * UP;
     const __half2 l = __floats2half2_rn(l0, l1);
     *reinterpret_cast<__half2*>(xl + (size_t)r * kp + i) = l;
     const float a0 = fabsf(v0), a1 = fabsf(v1);
@@ -462,9 +444,7 @@ __global__ void __launch_bounds__(256)
     }
     sum += a0 + a1;
   }
-  // a row that the terms do not hold: flagged for the product's own f32 chain, or (`carry`) left to the terms, the
-  // infinities and NaNs in the high one
-  const bool held = carry || (finite && !row_is_wide(lost, sum, k, red));
+  const bool held = finite && !row_is_wide(lost, sum, k, red); // (else: the product's own f32 chain)
   if (threadIdx.x == 0) x_scale[r] = held ? back : 0.0f;
 }
 
@@ -656,7 +636,7 @@ int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float
   float* partial = p.splits > 1 || ep.act != ACT_NONE ? (float*)take((size_t)p.splits * m * p.slice * 4) : nullptr;
   if (ep.norm != NORM_NONE && !ep.norm_tmp) return fc_fail(dev, FC_ERR_ARG, "a fused norm needs a temporary");
   FC_LAUNCH(dev, "rows_split",
-            rows_split_kernel<<<m, 256, 0, dev->stream>>>(x, m, w.k, p.kp, false, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, ep.norm_tmp, xh, xl, xs));
+            rows_split_kernel<<<m, 256, 0, dev->stream>>>(x, m, w.k, p.kp, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, ep.norm_tmp, xh, xl, xs));
   if (ep.norm != NORM_NONE) x = ep.norm_tmp;
   CUtensorMap maps[4];
   FC_TRY(make_map(dev, &maps[2], xh, m, p.kp, p.bn / 2));
@@ -692,7 +672,7 @@ int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float
 }
 
 int k_rows_split(FcDevice* dev, const float* x, uint32_t m, uint32_t mp, uint32_t k, __half* xh, __half* xl, float* x_scale) {
-  FC_LAUNCH(dev, "rows_split", rows_split_kernel<<<mp, 256, 0, dev->stream>>>(x, m, k, k, true, NORM_NONE, nullptr, nullptr, 0.0f,
+  FC_LAUNCH(dev, "rows_split", rows_split_kernel<<<mp, 256, 0, dev->stream>>>(x, m, k, k, NORM_NONE, nullptr, nullptr, 0.0f,
                                                                               nullptr, xh, xl, x_scale));
   return FC_OK;
 }

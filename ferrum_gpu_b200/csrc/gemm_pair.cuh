@@ -13,5 +13,7 @@ size_t qgemm_pair_scratch_bytes(const FcDevice* dev, uint32_t k, uint32_t n, uin
 bool qgemm_pair_fits(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m, size_t bytes);
 int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, const Workspace& ws);
 // x[m][k] as its two fp16 terms [mp][k] (rows m.. zero), each row times a power of two that brings its largest
-// magnitude to [2^14, 2^15); x_scale[mp] takes it back. Infinities and NaNs stay what they are in the high term.
+// magnitude to [2^14, 2^15), the low term times 2^LOW_SHIFT; x_scale[mp] takes the power of two back, or is 0 for a row
+// that the terms do not hold (infinities, NaNs, small elements that count beside far larger ones).
+constexpr int LOW_SHIFT = 11;
 int k_rows_split(FcDevice* dev, const float* x, uint32_t m, uint32_t mp, uint32_t k, __half* xh, __half* xl, float* x_scale);

@@ -18,6 +18,7 @@
 
 namespace {
 
+constexpr float LOW_DOWN = 1.0f / (float)(1 << LOW_SHIFT);
 constexpr int XS = 128;        // k per staged x slice
 constexpr int XSTRIDE = XS + 16; // halves per staged row (+32 bytes: conflict-free 8-byte reads)
 constexpr int ROWS_PER_CTA = 64;
@@ -232,7 +233,8 @@ __device__ __forceinline__ void block_frags(const BlockRegs<KIND>& r, uint32_t a
 // loads and rows padded by 32 bytes half of all shared-memory wavefronts of the kernel were bank conflicts).
 // RW: 16-row tiles of the weight a warp holds at once. Two tiles share every load of x from shared memory (the
 // kernel's busiest unit at one tile): used for the long outputs that need no split of K, the vocabulary head.
-template <int KIND, int NB, int RW>
+// RAGGED: the terms are k_rows_split's, low ones 2^LOW_SHIFT larger, which their products have to come down by.
+template <int KIND, int NB, int RW, bool RAGGED>
 __global__ void __launch_bounds__(128)
     qmatvec_mma_kernel(QMat w, const __half* __restrict__ xh, const __half* __restrict__ xl, uint32_t m, float* __restrict__ y,
                        float* __restrict__ partial, uint32_t blocks_per_split, Epilogue ep) {
@@ -320,10 +322,27 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
         for (int i = 0; i < RW; i++) {
           float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-          mma_16816(c, a[i][0], bh.x, bh.y);
-          mma_16816(c, a[i][0], bl.x, bl.y);
-          mma_16816(c, a[i][1], bh.z, bh.w);
-          mma_16816(c, a[i][1], bl.z, bl.w);
+          if (RAGGED && RW == 2) {
+            float low[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            mma_16816(low, a[i][0], bl.x, bl.y);
+            mma_16816(c, a[i][0], bh.x, bh.y);
+            mma_16816(low, a[i][1], bl.z, bl.w);
+            mma_16816(c, a[i][1], bh.z, bh.w);
+#pragma unroll
+            for (int j = 0; j < 4; j++) c[j] = fmaf(low[j], LOW_DOWN, c[j]);
+          } else if (RAGGED) { // (one row tile per warp: 64 x 4064 x 11008 Q8_0 85 us so, 90 in the form above, which RW 2 wants)
+            mma_16816(c, a[i][0], bl.x, bl.y);
+            mma_16816(c, a[i][1], bl.z, bl.w);
+#pragma unroll
+            for (int j = 0; j < 4; j++) c[j] *= LOW_DOWN;
+            mma_16816(c, a[i][0], bh.x, bh.y);
+            mma_16816(c, a[i][1], bh.z, bh.w);
+          } else {
+            mma_16816(c, a[i][0], bh.x, bh.y);
+            mma_16816(c, a[i][0], bl.x, bl.y);
+            mma_16816(c, a[i][1], bh.z, bh.w);
+            mma_16816(c, a[i][1], bl.z, bl.w);
+          }
           acc[i][nb][0] = fmaf(dg[i], c[0], acc[i][nb][0]);
           acc[i][nb][1] = fmaf(dg[i], c[1], acc[i][nb][1]);
           acc[i][nb][2] = fmaf(dg8[i], c[2], acc[i][nb][2]);
@@ -383,8 +402,10 @@ __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
 
 // RAGGED: K in whole blocks of 32 instead of whole slices. The last slice is filled up with zeros, the scales (whose rows
 // then start at any even address) come by two-byte loads one slice ahead, and each row's slice of x is first brought
-// to [2^14, 2^15) by a power of two that the block scales take back, so that the fp16 terms hold any f32 range: the f32
-// kernels that otherwise serve these widths do.
+// to [2^14, 2^15) by a power of two that the block scales take back, its low terms 2^LOW_SHIFT larger: 22 bits of every
+// element down to 2^-28 of the slice's largest. A slice that the terms do not hold - infinities, NaNs, small elements that
+// count beside far larger ones (by the rule of rows_split) - turns its row's sums into NaN, and every sum that is not
+// finite at the end is taken again by the f32 chain, which is what served these widths before.
 template <int KIND, bool RAGGED>
 __global__ void __launch_bounds__(128)
     qmatvec_mma8_kernel(QMat w, const float* __restrict__ x, uint32_t m, float* __restrict__ y, float* __restrict__ partial,
@@ -474,7 +495,9 @@ __global__ void __launch_bounds__(128)
       const float* src = reinterpret_cast<const float*>(xf + st * C::XF_STAGE) + xr * XS + xk;
       const float4 xa = *reinterpret_cast<const float4*>(src), xb = *reinterpret_cast<const float4*>(src + 4);
       float v[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-      if (RAGGED) { // (an infinity or NaN counts as 2^128: it stays what it is, and nothing finite overflows beside it)
+      float inv = 1.0f, least = INFINITY;
+      bool held = true, blank = false;
+      if (RAGGED) {
         uint32_t mx = 0;
 #pragma unroll
         for (int i = 0; i < 8; i++) mx = max(mx, __float_as_uint(v[i]) & 0x7fffffffu);
@@ -485,7 +508,8 @@ __global__ void __launch_bounds__(128)
         const float mul = __uint_as_float((uint32_t)(127 + sh) << 23);
 #pragma unroll
         for (int i = 0; i < 8; i++) v[i] *= mul;
-        if ((threadIdx.x & 15u) == 0) x_inv[sl & 1][xr] = __uint_as_float((uint32_t)(127 - sh) << 23);
+        inv = __uint_as_float((uint32_t)(127 - sh) << 23);
+        held = mx < 0x7f800000u, blank = mx == 0;
       }
       __half2 hi[4], lo[4];
 #pragma unroll
@@ -495,10 +519,30 @@ __global__ void __launch_bounds__(128)
         const float c1 = RAGGED ? v[2 * i + 1] : fminf(fmaxf(v[2 * i + 1], -65504.0f), 65504.0f);
         hi[i] = __floats2half2_rn(c0, c1);
         const float2 back = __half22float2(hi[i]);
-        if (RAGGED)
-          lo[i] = __floats2half2_rn(fabsf(c0) < INFINITY ? c0 - back.x : 0.0f, fabsf(c1) < INFINITY ? c1 - back.y : 0.0f);
-        else
-          lo[i] = __floats2half2_rn(c0 - back.x, c1 - back.y);
+        constexpr float UP = RAGGED ? (float)(1 << LOW_SHIFT) : 1.0f;
+        lo[i] = __floats2half2_rn((c0 - back.x) * UP, (c1 - back.y) * UP);
+        if (RAGGED) least = fminf(least, fminf(fabsf(c0), fabsf(c1)));
+      }
+      if (RAGGED) {
+        if (__any_sync(0xffffffffu, least < 0x1p-14f && !blank)) { // only there can the terms be short: see rows_split_kernel
+          float lost = 0.0f, sum = 0.0f;
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            const float h = __half2float(i & 1 ? __high2half(hi[i / 2]) : __low2half(hi[i / 2]));
+            const float l = __half2float(i & 1 ? __high2half(lo[i / 2]) : __low2half(lo[i / 2]));
+            const float e = fabsf((v[i] - h) * (float)(1 << LOW_SHIFT) - l), a = fabsf(v[i]);
+            if (e > a * LOW_DOWN) lost += e * LOW_DOWN;
+            sum += a;
+          }
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) lost += __shfl_xor_sync(0xffffffffu, lost, o); // a row's slice is half a warp
+          const float covered = lost * 0x1p22f;
+          const uint32_t half = 0xffffu << (threadIdx.x & 16u);
+          const int have = __popc(__ballot_sync(0xffffffffu, sum >= covered) & half);
+          const int share = __popc(__ballot_sync(0xffffffffu, sum * 4.0f >= covered) & half);
+          held = held && (lost == 0.0f || have >= 4 || share >= 7);
+        }
+        if ((threadIdx.x & 15u) == 0) x_inv[sl & 1][xr] = held ? inv : __int_as_float(0x7fffffff);
       }
       // (rows of 128 halves, the 16-byte chunk index of odd rows XORed with 4: see qmatvec_mma_kernel)
       __half* dst = xs + (size_t)(sl & 1) * 2 * PART + xr * XS + (((xk >> 3) ^ ((xr & 1) << 2)) << 3);
@@ -569,10 +613,20 @@ __global__ void __launch_bounds__(128)
       const uint32_t off = g * XS + (((bi * 4 + t) ^ ((g & 1) << 2)) * 8);
       const uint4 bh = *reinterpret_cast<const uint4*>(xhb + off);
       const uint4 bl = *reinterpret_cast<const uint4*>(xlb + off);
-      mma_16816(c, a[0], bh.x, bh.y);
-      mma_16816(c, a[0], bl.x, bl.y);
-      mma_16816(c, a[1], bh.z, bh.w);
-      mma_16816(c, a[1], bl.z, bl.w);
+      if (RAGGED) {
+        float low[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_16816(low, a[0], bl.x, bl.y);
+        mma_16816(c, a[0], bh.x, bh.y);
+        mma_16816(low, a[1], bl.z, bl.w);
+        mma_16816(c, a[1], bh.z, bh.w);
+#pragma unroll
+        for (int j = 0; j < 4; j++) c[j] = fmaf(low[j], LOW_DOWN, c[j]);
+      } else {
+        mma_16816(c, a[0], bh.x, bh.y);
+        mma_16816(c, a[0], bl.x, bl.y);
+        mma_16816(c, a[1], bh.z, bh.w);
+        mma_16816(c, a[1], bl.z, bl.w);
+      }
       acc[0] = fmaf(dg * inv0, c[0], acc[0]);
       acc[1] = fmaf(dg * inv1, c[1], acc[1]);
       acc[2] = fmaf(dg8 * inv0, c[2], acc[2]);
@@ -585,6 +639,7 @@ __global__ void __launch_bounds__(128)
     const uint32_t row = cta_row0 + warp * 16 + g + (j >> 1) * 8, col = 2 * t + (j & 1);
     if (row >= n || col >= m) continue;
     float v = acc[j];
+    if (RAGGED && !(fabsf(v) < INFINITY)) v = exact_dot<KIND>(x + (size_t)col * k, w.qs, w.sc, k, row, kb_begin * QK, kb_end * QK);
     if (partial) {
       partial[((size_t)blockIdx.y * m + col) * n + row] = v;
     } else {
@@ -596,26 +651,40 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// The same at a ragged width: the sums still carry their row's power of two, and what is not finite, or belongs to a row
+// that the fp16 terms do not hold (x_scale 0), is taken again by the f32 chain.
+template <int KIND>
+__global__ void ragged_reduce_kernel(const float* __restrict__ partial, uint32_t splits, uint32_t m, QMat w, const float* __restrict__ x,
+                                     const float* __restrict__ x_scale, float* __restrict__ y, const float* __restrict__ bias) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (size_t)m * w.n) return;
+  float v = 0.0f;
+  for (uint32_t s = 0; s < splits; s++) v += partial[(size_t)s * m * w.n + i];
+  const uint32_t row = (uint32_t)(i / w.n), col = (uint32_t)(i % w.n);
+  const float scale = x_scale[row];
+  v *= scale;
+  if (scale == 0.0f || !(fabsf(v) < INFINITY)) v = exact_dot<KIND>(x + (size_t)row * w.k, w.qs, w.sc, w.k, col, 0, w.k);
+  y[i] = bias ? v + bias[col] : v;
+}
+
 // y = epilogue(sum over splits, ascending split index)
-// (x_scale, nullable: the power of two of each row of x, which the ragged widths' sums still carry)
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, uint32_t splits, uint32_t m, uint32_t n,
-                                     float* __restrict__ y, Epilogue ep, const float* __restrict__ x_scale) {
+                                     float* __restrict__ y, Epilogue ep) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)m * n) return;
   float v = 0.0f;
   for (uint32_t s = 0; s < splits; s++) v += partial[(size_t)s * m * n + i];
   const uint32_t row = (uint32_t)(i % n);
-  if (x_scale) v *= x_scale[i / n];
   if (ep.bias) v += ep.bias[row];
   if (ep.act == ACT_GELU) v = gelu_f(v);
   if (ep.resid) v = ep.resid[i] + v;
   y[i] = v;
 }
 
-template <int KIND, int NB, int RW = 1>
+template <int KIND, int NB, int RW = 1, bool RAGGED = false>
 int launch(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, uint32_t m, float* y, float* partial,
            uint32_t splits, uint32_t bps, const Epilogue& ep) {
-  auto kern = qmatvec_mma_kernel<KIND, NB, RW>;
+  auto kern = qmatvec_mma_kernel<KIND, NB, RW, RAGGED>;
   const size_t smem = (size_t)2 * 2 * NB * 8 * XS * sizeof(__half);
   static OncePerDevice attr;
   if (attr.first(dev->ordinal)) {
@@ -629,11 +698,17 @@ int launch(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, uin
 template <int KIND>
 int pick_nb(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, uint32_t m, float* y, float* partial,
             uint32_t splits, uint32_t bps, const Epilogue& ep) {
+  // an output long enough to fill the device many times over without a split of K: two row tiles per warp
+  const bool two = m > 32 && splits == 1 && (w.n + 127) / 128 >= 4 * (uint32_t)dev->prop.multiProcessorCount;
+  if (w.k % XS) {
+    if (m <= 16) return launch<KIND, 2, 1, true>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
+    if (m <= 32) return launch<KIND, 4, 1, true>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
+    if (two) return launch<KIND, 8, 2, true>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
+    return launch<KIND, 8, 1, true>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
+  }
   if (m <= 16) return launch<KIND, 2>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
   if (m <= 32) return launch<KIND, 4>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
-  // an output long enough to fill the device many times over without a split of K: two row tiles per warp
-  if (splits == 1 && (w.n + 127) / 128 >= 4 * (uint32_t)dev->prop.multiProcessorCount)
-    return launch<KIND, 8, 2>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
+  if (two) return launch<KIND, 8, 2>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
   return launch<KIND, 8>(dev, w, xh, xl, m, y, partial, splits, bps, ep);
 }
 
@@ -647,6 +722,27 @@ int pick_kind(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, 
     case FC_F16: return pick_nb<FC_F16>(dev, w, xh, xl, m, y, part, splits, bps, ep);
   }
   return pick_nb<FC_Q4_0>(dev, w, xh, xl, m, y, part, splits, bps, ep);
+}
+
+template <int KIND>
+int ragged_reduce(FcDevice* dev, const QMat& w, const float* x, uint32_t m, const float* partial, uint32_t splits, const float* x_scale,
+                  float* y, const Epilogue& ep) {
+  if (ep.act != ACT_NONE || ep.resid) return fc_fail(dev, FC_ERR_ARG, "a product of a ragged width stands alone");
+  const size_t tot = (size_t)m * w.n;
+  FC_LAUNCH(dev, "splitk_reduce",
+            ragged_reduce_kernel<KIND><<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w, x, x_scale, y, ep.bias));
+  return FC_OK;
+}
+int pick_ragged_reduce(FcDevice* dev, const QMat& w, const float* x, uint32_t m, const float* partial, uint32_t splits, const float* x_scale,
+                       float* y, const Epilogue& ep) {
+  switch (w.kind) {
+    case FC_Q8_0: return ragged_reduce<FC_Q8_0>(dev, w, x, m, partial, splits, x_scale, y, ep);
+    case FC_FP8_E4M3: return ragged_reduce<FC_FP8_E4M3>(dev, w, x, m, partial, splits, x_scale, y, ep);
+    case FC_FP8_E5M2: return ragged_reduce<FC_FP8_E5M2>(dev, w, x, m, partial, splits, x_scale, y, ep);
+    case FC_MXFP4: return ragged_reduce<FC_MXFP4>(dev, w, x, m, partial, splits, x_scale, y, ep);
+    case FC_F16: return ragged_reduce<FC_F16>(dev, w, x, m, partial, splits, x_scale, y, ep);
+  }
+  return ragged_reduce<FC_Q4_0>(dev, w, x, m, partial, splits, x_scale, y, ep);
 }
 
 template <int KIND, bool RAGGED>
@@ -677,9 +773,11 @@ bool qmatvec_mma_supports(const QMat& w, uint32_t m) {
 
 // The same kernels for a width of whole 32-blocks that is not whole slices (Epilogue::ragged: a stand-alone product, whose x
 // terms nobody else writes). Before, these widths took the FMA kernels, which multiply every weight by every row in
-// f32: 8 rows x 4064 x 11008 Q8_0 28 us instead of 162, 40 x 2080 x 11008 Q4_0 51 instead of 181, 2 x 2080 x 3001 Q4_0
-// 13 instead of 27; below one slice they keep them. Error against f64 1.3e-7..1.5e-7 of the result's norm, 1.2e-7..7.7e-7
-// there.
+// f32: 8 rows x 4064 x 11008 Q8_0 29 us instead of 162, 40 x 2080 x 11008 Q4_0 49 instead of 181, 2 x 2080 x 3001 Q4_0
+// 10 instead of 27; below one slice they keep them. Error against f64 0.9e-7..1.1e-7 of the result's norm on Gaussian rows,
+// 1.0e-7..7.7e-7 there; with two elements of 2^20 or 2^26 in every row at most 6e-7 of an output's own sum |x w| (there up to
+// 4.6e-6). Holding small elements beside large ones costs 0..7 % (rows whose terms all lie at the largest one's magnitude:
+// 26.7 us for the first shape, and at 2^34 a thousandth of the sum lost).
 bool qmatvec_mma_ragged_supports(const QMat& w, uint32_t m) {
   return (kind_has_scales(w.kind) || w.kind == FC_F16) && m >= 2 && m <= 64 && w.k % QK == 0 && w.k % XS != 0 && w.k >= XS;
 }
@@ -718,7 +816,7 @@ static int k_qmatvec_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t
   if (splits > 1) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
-              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep, nullptr));
+              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep));
   }
   return FC_OK;
 }
@@ -737,7 +835,7 @@ int k_flush_deferred(FcDevice* dev, const DeferredReduce& d) {
   ep.resid = d.resid;
   const size_t tot = (size_t)d.m * d.n;
   FC_LAUNCH(dev, "splitk_reduce",
-            splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(d.partial, d.splits, d.m, d.n, d.y, ep, nullptr));
+            splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(d.partial, d.splits, d.m, d.n, d.y, ep));
   return FC_OK;
 }
 
@@ -804,10 +902,11 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     d.y = y;
     return FC_OK;
   }
+  if (ragged) return pick_ragged_reduce(dev, w, x, m, partial, splits, x_scale, y, ep);
   if (part) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
-              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep, x_scale));
+              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep));
   }
   return FC_OK;
 }

@@ -7,7 +7,7 @@ of sum |x w| whatever the width."""
 import numpy as np
 import pytest
 
-from ferrum_gpu_b200 import CudaGpt2, CudaLlama, Mode, QKind, _ffi, linear_q, upload_quantised
+from ferrum_gpu_b200 import CudaGpt2, CudaLlama, Mode, QKind, _ffi, linear_q, upload_quantised, upload_qweight
 from ferrum_gpu_b200.hostmodel import Gpt2Config, LlamaConfig, random_gpt2, random_llama, random_tokens
 from oracle import oracle as orc
 from tests import helpers
@@ -107,6 +107,39 @@ def test_decode_products_at_ragged_widths(dev, kind, m, k, n, mag):
     qw, x, want, scale = _problem(dev, kind, m, k, n, mag=mag)
     got = linear_q(dev, x, qw, m).reshape(m, n)
     assert np.all(np.abs(got - want) <= EXACT * scale), (kind, m, k, n, np.max(np.abs(got - want) / scale))
+    qw.close()
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0, QKind.F16, QKind.FP8_E4M3, QKind.MXFP4])
+@pytest.mark.parametrize("m,k,n", [(2, 160, 70), (5, 1056, 3000), (8, 4064, 130), (9, 160, 70), (40, 1056, 300), (64, 2080, 1000)])
+@pytest.mark.parametrize("spread", SPREADS)
+def test_decode_products_at_ragged_widths_keep_small_elements_beside_large_ones(dev, kind, m, k, n, spread):
+    _spread_check(dev, kind, m, k, n, spread)
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0])
+@pytest.mark.parametrize("m,k,n", [(5, 160, 70), (7, 4064, 600), (12, 160, 70), (50, 2080, 300), (100, 2080, 300)])
+def test_infinities_and_nans_go_where_an_f32_chain_puts_them(dev, kind, m, k, n):
+    rng = np.random.default_rng(2)
+    clean = upload_quantised(dev, kind, (rng.standard_normal(k * n) * 0.02).astype(np.float32), k, n)
+    raw = clean.blocks().reshape(n, k // 32, -1)
+    raw[3, 1, :2] = np.array([np.inf], dtype=np.float16).view(np.uint8)
+    raw[5, 2, :2] = np.array([np.nan], dtype=np.float16).view(np.uint8)
+    clean.close()
+    qw = upload_qweight(dev, kind, raw.reshape(-1), k, n)
+    w = qw.dequantised().reshape(n, k).astype(np.float64)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[0, 5], x[1, k - 1], x[2, 40] = np.inf, np.nan, -np.inf
+    x[3] = 0.0
+    got = linear_q(dev, x, qw, m).reshape(m, n)
+    with np.errstate(invalid="ignore"):
+        want = np.stack([(row.astype(np.float64)[None] * w).sum(-1) for row in x])
+        scale = np.abs(x).astype(np.float64) @ np.nan_to_num(np.abs(w), posinf=0.0).T
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    inf = np.isinf(want)
+    assert inf.any() and np.array_equal(got[inf], want[inf])
+    ok = np.isfinite(want)
+    assert np.all(np.abs(got[ok] - want[ok]) <= EXACT * scale[ok])
     qw.close()
 
 
