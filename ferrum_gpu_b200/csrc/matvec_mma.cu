@@ -627,10 +627,11 @@ __global__ void __launch_bounds__(128)
         mma_16816(c, a[1], bh.z, bh.w);
         mma_16816(c, a[1], bl.z, bl.w);
       }
-      acc[0] = fmaf(dg * inv0, c[0], acc[0]);
-      acc[1] = fmaf(dg * inv1, c[1], acc[1]);
-      acc[2] = fmaf(dg8 * inv0, c[2], acc[2]);
-      acc[3] = fmaf(dg8 * inv1, c[3], acc[3]);
+      // (the power of two meets the sum first: beside a block scale of ordinary size it could be subnormal)
+      acc[0] = fmaf(dg, c[0] * inv0, acc[0]);
+      acc[1] = fmaf(dg, c[1] * inv1, acc[1]);
+      acc[2] = fmaf(dg8, c[2] * inv0, acc[2]);
+      acc[3] = fmaf(dg8, c[3] * inv1, acc[3]);
     }
   }
   cp_async_wait<0>();

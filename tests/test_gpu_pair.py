@@ -102,11 +102,12 @@ def test_exact_products_of_many_rows_keep_small_elements_beside_large_ones(dev, 
 @pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0, QKind.F16, QKind.FP8_E4M3, QKind.MXFP4])
 @pytest.mark.parametrize("m,k,n", [(2, 160, 5), (3, 224, 64), (8, 4064, 130), (5, 1056, 3000), (9, 160, 70), (16, 288, 65), (33, 2080, 300),
                                    (64, 1120, 1000), (40, 4064, 20)])
-@pytest.mark.parametrize("mag", [1.0, 1e-20, 1e20])
+@pytest.mark.parametrize("mag", [1.0, 1e-20, 1e20, 1e-35, 1e36])
 def test_decode_products_at_ragged_widths(dev, kind, m, k, n, mag):
     qw, x, want, scale = _problem(dev, kind, m, k, n, mag=mag)
     got = linear_q(dev, x, qw, m).reshape(m, n)
-    assert np.all(np.abs(got - want) <= EXACT * scale), (kind, m, k, n, np.max(np.abs(got - want) / scale))
+    # (at 1e-35 block sums come near the smallest normal number: 2^-149 for each of their roundings and splits)
+    assert np.all(np.abs(got - want) <= EXACT * scale + (k // 32 + 16) * 2.0 ** -149), (kind, m, k, n, np.max(np.abs(got - want) / scale))
     qw.close()
 
 
