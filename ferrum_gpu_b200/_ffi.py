@@ -161,7 +161,7 @@ def load() -> C.CDLL:
         "fc_debug_profile": (C.c_int, [vp, C.c_int]),
         "fc_debug_matvec_kernel": (C.c_int, [vp, C.c_int]),
         "fc_debug_raise_status": (C.c_int, [vp, C.c_int]),
-        "fc_debug_pair_bytes": (u64, [u32, u32, u32, u32, u64]),
+        "fc_debug_pair_bytes": (u64, [u32, u32, u32, u32, C.c_int, u64]),
         "fc_debug_score_pass_bytes": (C.c_int, [vp, u64]),
         "fc_debug_profile_report": (C.c_int, [vp, C.c_char_p, sz]),
         "fc_model_topk": (C.c_int, [vp, u32, u32, C.c_float, vp, u32, vp, vp, P(u32)]),

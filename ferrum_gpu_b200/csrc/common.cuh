@@ -302,7 +302,7 @@ struct Epilogue {
   // serves qmatvec_mma_ragged_supports
   bool ragged = false;
   // device scratch that lets products of more than 64 rows of Q8_0 / Q4_0 weights run on the tensor cores (gemm_pair.cu;
-  // qgemm_pair_scratch_bytes(k, n, m) is what the best cut takes); without it, or where it is too small, they take the
+  // qgemm_pair_scratch_bytes is what the best cut takes); without it, or where it is too small, they take the
   // tiled f32 kernel. (One pointer, read by host code only: the decode kernels take this struct as an
   // argument, and with eight bytes more a decode step of 12 layers took 445 us instead of 433.)
   const Workspace* wide = nullptr;

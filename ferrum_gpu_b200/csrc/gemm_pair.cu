@@ -541,13 +541,14 @@ struct Plan {
 };
 constexpr size_t W_TERMS_BYTES = (size_t)64 << 20;
 size_t al(size_t v) { return (v + 1023) & ~(size_t)1023; }
-size_t plan_bytes(const Plan& p, uint32_t m) {
+// sums: the result leaves through pair_reduce_kernel even without a split of K (an activation)
+size_t plan_bytes(const Plan& p, uint32_t m, bool sums) {
   return 2 * al((size_t)m * p.kp * 2) + 2 * al((size_t)p.slice * p.kp * 2) + al((size_t)m * 4) + al((size_t)p.slice * 4) +
-         al((size_t)p.splits * m * p.slice * 4) + 1024;
+         (p.splits > 1 || sums ? al((size_t)p.splits * m * p.slice * 4) : 0) + 1024;
 }
 // The best cut whose workspace fits into `limit` bytes; splits == 0 where not even the smallest does. (Fewer rows may ask
 // for more than many: they leave the chip idle without a split of K, and every split has sums of its own.)
-Plan make_plan(uint32_t sms, uint32_t k, uint32_t n, uint32_t m, size_t limit) {
+Plan make_plan(uint32_t sms, uint32_t k, uint32_t n, uint32_t m, bool sums, size_t limit) {
   Plan p;
   p.kp = (k + BK - 1) / BK * BK;
   p.steps = p.kp / BK;
@@ -567,7 +568,7 @@ Plan make_plan(uint32_t sms, uint32_t k, uint32_t n, uint32_t m, size_t limit) {
       if (cost >= best) continue;
       Plan q = p;
       q.bn = bn, q.per_split = (uint32_t)per, q.splits = (uint32_t)((p.steps + per - 1) / per);
-      if (plan_bytes(q, m) <= limit) best = cost, p = q;
+      if (plan_bytes(q, m, sums) <= limit) best = cost, p = q;
     }
   return p;
 }
@@ -605,21 +606,21 @@ bool qgemm_pair_takes(const QMat& w, uint32_t m) {
   return (w.kind == FC_Q8_0 || w.kind == FC_Q4_0) && m > 64 && w.k % QK == 0 && w.k > 0 && w.n > 0;
 }
 
-size_t qgemm_pair_scratch_bytes(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m) {
-  return plan_bytes(make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m, SIZE_MAX), m);
+size_t qgemm_pair_scratch_bytes(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m, int act) {
+  return plan_bytes(make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m, act != ACT_NONE, SIZE_MAX), m, act != ACT_NONE);
 }
-bool qgemm_pair_fits(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m, size_t bytes) {
-  return make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m, bytes).splits != 0;
+bool qgemm_pair_fits(const FcDevice* dev, uint32_t k, uint32_t n, uint32_t m, int act, size_t bytes) {
+  return make_plan((uint32_t)dev->prop.multiProcessorCount, k, n, m, act != ACT_NONE, bytes).splits != 0;
 }
-FC_API uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, uint32_t m, uint64_t limit) {
+FC_API uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, uint32_t m, int gelu, uint64_t limit) {
   if (sm_count < 2 || !k || k % QK || !n || !m) return 0;
-  const Plan p = make_plan(sm_count, k, n, m, (size_t)limit);
-  return p.splits ? plan_bytes(p, m) : 0;
+  const Plan p = make_plan(sm_count, k, n, m, gelu != 0, (size_t)limit);
+  return p.splits ? plan_bytes(p, m, gelu != 0) : 0;
 }
 
 int k_qgemm_pair(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float* y, const Epilogue& ep, const Workspace& space) {
   if (m == 0) return FC_OK;
-  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, w.k, w.n, m, space.bytes);
+  const Plan p = make_plan((uint32_t)dev->prop.multiProcessorCount, w.k, w.n, m, ep.act != ACT_NONE, space.bytes);
   if (!p.splits) return fc_fail(dev, FC_ERR_ARG, "a %zu-byte workspace is too small for this product", space.bytes);
   uint8_t* at = (uint8_t*)(((uintptr_t)space.p + 1023) & ~(uintptr_t)1023);
   auto take = [&](size_t bytes) {

@@ -407,7 +407,7 @@ int k_qlinear_f32(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     return k_qmatvec1(dev, w, x, y, ep);
   }
   if (ep.swiglu) return fc_fail(dev, FC_ERR_ARG, "only the streamed one-row product applies SwiGLU");
-  if (ep.wide && ep.wide->p && forced == 0 && !ep.presplit && qgemm_pair_takes(w, m) && qgemm_pair_fits(dev, w.k, w.n, m, ep.wide->bytes)) {
+  if (ep.wide && ep.wide->p && forced == 0 && !ep.presplit && qgemm_pair_takes(w, m) && qgemm_pair_fits(dev, w.k, w.n, m, ep.act, ep.wide->bytes)) {
     // (its x split takes the norm along)
     if (ep.pending && ep.pending->splits) FC_TRY(k_flush_deferred(dev, *ep.pending));
     return k_qgemm_pair(dev, w, x, m, y, ep, *ep.wide);

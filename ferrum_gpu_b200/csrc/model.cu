@@ -350,17 +350,17 @@ int check_ids(FcModel* m, const int32_t* ids, size_t n) {
 
 int arena_reserve_wide(FcModel* m, size_t bytes, size_t rows, int mode) {
   size_t wide = 0;
-  auto add = [&](const QMat& w) {
+  auto add = [&](const QMat& w, int act) {
     if (mode == FC_TENSOR_F16) {
       if (tp_takes(m->dev, w, (uint32_t)rows, EPI_LSE)) wide = tp_workspace_bytes(w) > wide ? tp_workspace_bytes(w) : wide;
     } else if (qgemm_pair_takes(w, (uint32_t)rows)) {
-      const size_t b = qgemm_pair_scratch_bytes(m->dev, w.k, w.n, (uint32_t)rows);
+      const size_t b = qgemm_pair_scratch_bytes(m->dev, w.k, w.n, (uint32_t)rows, act);
       wide = b > wide ? b : wide;
     }
   };
   for (const auto& l : m->layers)
-    for (const FcQWeight* q : {l.qkv.w, l.wo.w, l.ff1.w, l.ff2.w}) add(q->m);
-  add(m->head_view);
+    for (const FcQWeight* q : {l.qkv.w, l.wo.w, l.ff1.w, l.ff2.w}) add(q->m, q == l.ff1.w && m->arch == ARCH_GPT2 ? ACT_GELU : ACT_NONE);
+  add(m->head_view, ACT_NONE);
   const size_t at = (bytes + 1023) & ~(size_t)1023;
   if (wide) {
     const int rc = arena_reserve(m, at + wide);

@@ -150,7 +150,7 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
       }
       ep.scratch = w->mma_scratch;
     } else if (qgemm_pair_takes(w->m, m)) {
-      const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m));
+      const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m, ACT_NONE));
       if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
       // (no room for more, or a capture: the product is cut to the workspace that is there, or takes the tiled f32 kernel)
       wide = Workspace{w->tc_cache, w->tc_cache_bytes};

@@ -106,10 +106,10 @@ int fc_debug_fail_after(FcDevice* dev, int64_t n_launches);
  * 1 = the f32 FMA kernel, 2 = the small-batch mma.sync kernel. Measurement hook; results stay within the
  * exact path's tolerance whichever runs. */
 int fc_debug_matvec_kernel(FcDevice* dev, int choice);
-/* Workspace bytes of the exact product of `m` > 64 rows by an [n, k] weight on a device of `sm_count` multiprocessors
- * when at most `limit` bytes are there; 0 when none of its forms fits (the tiled f32 kernel, which needs none, then
+/* Workspace bytes of the exact product of `m` > 64 rows by an [n, k] weight (with a GELU behind it or without) on a
+ * device of `sm_count` multiprocessors when at most `limit` bytes are there; 0 when none of its forms fits (the tiled f32 kernel, which needs none, then
  * runs). Needs no device. Test hook. */
-uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, uint32_t m, uint64_t limit);
+uint64_t fc_debug_pair_bytes(uint32_t sm_count, uint32_t k, uint32_t n, uint32_t m, int gelu, uint64_t limit);
 /* Per-kernel device timing, the counterpart of the reference's one-kernel-at-a-time profiler
  * (ferrum_wgpu/benches/profile_train.rs:L15-L25): while enabled every launch is bracketed by a pair
  * of CUDA events on the device's stream. The report is a JSON object

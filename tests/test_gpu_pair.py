@@ -206,7 +206,7 @@ def test_exact_scoring_in_unequal_passes(dev):
     lib = _ffi.load()
     cfg = LlamaConfig(vocab=1000, ctx=64, dim=128, heads=2, kv_heads=1, head_dim=64, layers=2, hidden=768, rope_dim=64)
     if dev.props()[0] == 148:  # (`down` is the only matrix here that is not left to the tiled kernel)
-        need = [lib.fc_debug_pair_bytes(148, 768, 128, seqs * 60, 2**64 - 1) for seqs in (11, 10)]
+        need = [lib.fc_debug_pair_bytes(148, 768, 128, seqs * 60, 0, 2**64 - 1) for seqs in (11, 10)]
         assert need[0] < need[1]
     g = CudaLlama(dev, random_llama(cfg, seed=3, std=0.05), QKind.Q8_0)
     ids = np.stack([random_tokens(i, 61, cfg.vocab) for i in range(21)])

@@ -14,7 +14,7 @@ WIDTHS = [(128, 256, 768, 1000), (768, 1280, 2048, 32000), (1024, 1280, 2816, 15
 @pytest.fixture(scope="module")
 def pair():
     lib = _ffi.load()
-    return lambda k, n, m, limit=NO_LIMIT, sms=SMS: lib.fc_debug_pair_bytes(sms, k, n, m, limit)
+    return lambda k, n, m, limit=NO_LIMIT, sms=SMS, gelu=0: lib.fc_debug_pair_bytes(sms, k, n, m, gelu, limit)
 
 
 def _matrices(d, qkv, hid, vocab):
@@ -37,6 +37,14 @@ def test_no_run_of_rows_leaves_what_a_pass_reserved(pair, widths):
             for k, n in mats:
                 need = pair(k, n, rows, reserved)
                 assert 0 < need <= reserved, (widths, most, rows, k, n)
+
+
+def test_sums_are_reserved_where_they_are_written(pair):
+    """One split of K and no activation: the result goes straight to y, and the workspace is the terms and scales."""
+    k, n, m = 4096, 11008, 4096
+    terms, kib = 2 * m * k * 2 + 2 * 4096 * k * 2, 1024  # x, and 64 MB of weight rows at once
+    assert terms < pair(k, n, m) < terms + 64 * kib
+    assert pair(k, n, m, gelu=1) >= terms + m * 4096 * 4
 
 
 @pytest.mark.parametrize("sms", [148, 132, 60, 2])
