@@ -18,6 +18,11 @@
 
 constexpr int QK = 32; // elements per quantisation block (ferrum_gguf/src/lib.rs:L55)
 
+struct Workspace { // device scratch and its size
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+
 struct FcDevice {
   int ordinal = 0;
   cudaStream_t stream = nullptr;
@@ -28,9 +33,11 @@ struct FcDevice {
   int64_t fail_after = -1; // fault injection: launches left before every launch is refused
   void* pinned = nullptr;  // pinned host staging for results and small inputs
   size_t pinned_bytes = 0;
-  // Workspaces of stand-alone weights come from here, in the order of `stream`: a workspace given back is the next
-  // weight's, without the device-wide allocation and free (300 us of a first product). Holds on to at most
-  // WORKSPACE_POOL_KEEP bytes, goes with the device; null where the device has no memory pools.
+  // Scratch of the stand-alone products (qweight_scratch), and where it comes from: a pool in the order of `stream` that
+  // holds on to at most WORKSPACE_POOL_KEEP bytes, so that a first product finds its memory mapped (mapping took 300 us);
+  // null where the device has no memory pools.
+  Workspace scratch;
+  uint32_t weights = 0; // stand-alone weights alive
   cudaMemPool_t workspaces = nullptr;
   int* d_flag = nullptr;   // device int for kernels that report a status
   int matvec_choice = 0;   // fc_debug_matvec_kernel: which kernel multiplies 1..8 rows (0: the library's rule)
@@ -127,14 +134,19 @@ struct FcQWeight {
   void* qs_alloc = nullptr;
   void* sc_alloc = nullptr;
   uint64_t bytes = 0;
-  // workspace of the products of many rows (fp16 terms of x and of the weight), grown on demand
-  void* tc_cache = nullptr;
-  size_t tc_cache_bytes = 0;
-  void* mma_scratch = nullptr; // scratch of the batched-decode product for stand-alone use
-  // a captured graph may hold the workspace's address: once a call was captured, outgrown workspaces are kept
-  bool captured = false;
+  // scratch of products captured into graphs, and what they outgrew (a graph may still hold its address): see qweight_scratch
+  Workspace graph_ws;
   std::vector<void*> outgrown;
 };
+
+// Scratch for one product of a stand-alone weight. All products of a device handle run one behind the other on its stream
+// and share one buffer, as large as the largest of them asked for; it goes back with the last of the weights, or when
+// memory is short. (An allocation of the call's own, from the pool and back in stream order, left 2 us between the kernels
+// of neighbouring calls: 5 x 1056 x 1500 10.3 us instead of 8.2.) Inside a stream capture the scratch is the weight's own,
+// for the graph to replay with on any stream, until the weight is destroyed.
+// FC_ERR_OOM: there is no room (a smaller request, or a kernel without scratch, may do).
+int qweight_scratch(FcQWeight* w, size_t bytes, Workspace* out);
+void release_scratch(FcDevice* dev);
 
 __host__ __device__ constexpr bool kind_is_fp8(int kind) { return kind == FC_FP8_E4M3 || kind == FC_FP8_E5M2; }
 // one byte per element and an f16 scale per 32: Q8_0 and the FP8 formats share planes, loads and addressing
@@ -286,11 +298,6 @@ struct DeferredReduce {
   float* y = nullptr;
 };
 
-struct Workspace { // device scratch and its size
-  void* p = nullptr;
-  size_t bytes = 0;
-};
-
 struct Epilogue {
   const float* bias = nullptr;  // [n]
   const float* resid = nullptr; // [m][n]; may alias y
@@ -379,7 +386,3 @@ int qweight_from_f32(FcDevice* dev, int kind, const float* w_in_out_host, uint32
 int qweight_from_f32_concat(FcDevice* dev, int kind, const float* const* mats_host, const uint32_t* ns, int count,
                             uint32_t k, FcQWeight** out);
 void qweight_free(FcQWeight* w);
-// The weight's product workspace (tc_cache), grown to `bytes` (model_tc.cu). FC_ERR_OOM: there is no room for it, or the
-// stream is being captured and nothing can be allocated - the caller goes on without, where its product can.
-int qweight_workspace(FcQWeight* w, size_t bytes);
-void qweight_workspace_free(FcQWeight* w);

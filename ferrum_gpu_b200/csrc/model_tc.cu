@@ -64,53 +64,24 @@ int model_interleave_gate_up(FcDevice* dev, FcQWeight* w, uint32_t hidden, uint3
   return FC_OK;
 }
 
-void qweight_workspace_free(FcQWeight* w) {
-  for (void* p : w->outgrown) workspace_free(w->dev, p);
-  w->outgrown.clear();
-  if (w->tc_cache) workspace_free(w->dev, w->tc_cache);
-  if (w->mma_scratch) workspace_free(w->dev, w->mma_scratch);
-  w->tc_cache = w->mma_scratch = nullptr;
-  w->tc_cache_bytes = 0;
-}
-
-int qweight_workspace(FcQWeight* w, size_t bytes) {
-  if (!w->captured && stream_capturing(w->dev)) w->captured = true;
-  if (bytes <= w->tc_cache_bytes) return FC_OK;
-  FcDevice* dev = w->dev;
-  if (stream_capturing(dev)) return fc_fail(dev, FC_ERR_OOM, "a %zu-byte product workspace cannot be allocated during a capture", bytes);
-  if (w->tc_cache && w->captured)
-    w->outgrown.push_back(w->tc_cache);
-  else if (w->tc_cache)
-    workspace_free(dev, w->tc_cache);
-  w->tc_cache = nullptr;
-  w->tc_cache_bytes = 0;
-  const cudaError_t e = workspace_alloc(dev, &w->tc_cache, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    w->tc_cache = nullptr;
-    return fc_fail(dev, FC_ERR_OOM, "cannot allocate a %zu-byte product workspace: %s", bytes, cudaGetErrorString(e));
-  }
-  w->tc_cache_bytes = bytes;
-  return FC_OK;
-}
-
 int k_qgemm_tc(FcDevice* dev, FcQWeight* w, const float* x_dev, uint32_t m, float* y_dev) {
   if (m == 0) return FC_OK;
   const size_t a_bytes = al((size_t)m * w->m.k * 2);
+  Workspace scratch;
   bool wide = tp_takes(dev, w->m, m, EPI_F32);
   if (wide) {
-    const int rc = qweight_workspace(w, a_bytes + tp_workspace_bytes(w->m));
+    const int rc = qweight_scratch(w, a_bytes + tp_workspace_bytes(w->m), &scratch);
     if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
     wide = rc == FC_OK; // (no room for the decoded weights: the product decodes them itself)
   }
-  if (!wide) FC_TRY(qweight_workspace(w, a_bytes));
-  __half* a = (__half*)w->tc_cache;
+  if (!wide) FC_TRY(qweight_scratch(w, a_bytes, &scratch));
+  __half* a = (__half*)scratch.p;
   FC_TRY(k_f32_to_f16(dev, x_dev, (size_t)m * w->m.k, a));
   TcArgs t;
   t.m = m;
   t.out_f32 = y_dev;
   t.ldo = w->m.n;
-  const Workspace rest{(uint8_t*)w->tc_cache + a_bytes, w->tc_cache_bytes - a_bytes};
+  const Workspace rest{(uint8_t*)scratch.p + a_bytes, scratch.bytes - a_bytes};
   if (wide) t.wide = &rest;
   return k_qgemm_tc_f16(dev, w->m, a, EPI_F32, t);
 }

@@ -25,7 +25,9 @@ FC_API int fc_qweight_create(FcDevice* dev, int kind, const float* w_in_out, uin
   if (k == 0 || n == 0 || (kind != FC_F32 && k % QK))
     return fc_fail(dev, FC_ERR_SHAPE, "cannot quantise %llu elements as a %u x %u weight in whole 32-blocks",
                    (unsigned long long)k * n, k, n);
-  return qweight_from_f32(dev, kind, w_in_out, k, n, out);
+  FC_TRY(qweight_from_f32(dev, kind, w_in_out, k, n, out));
+  dev->weights++;
+  return FC_OK;
 }
 
 FC_API int fc_qweight_create_from_blocks(FcDevice* dev, int kind, const uint8_t* blocks, size_t n_bytes, uint32_t k,
@@ -71,15 +73,17 @@ FC_API int fc_qweight_create_from_blocks(FcDevice* dev, int kind, const uint8_t*
     return rc;
   }
   *out = w;
+  dev->weights++;
   return FC_OK;
 }
 
 FC_API int fc_qweight_destroy(FcQWeight* w) {
   if (!w) return FC_ERR_ARG;
-  cudaSetDevice(w->dev->ordinal);
-  cudaStreamSynchronize(w->dev->stream);
-  qweight_workspace_free(w);
+  FcDevice* dev = w->dev;
+  cudaSetDevice(dev->ordinal);
+  cudaStreamSynchronize(dev->stream);
   qweight_free(w);
+  if (--dev->weights == 0) release_scratch(dev);
   return FC_OK;
 }
 
@@ -135,26 +139,21 @@ FC_API int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y
   cudaSetDevice(dev->ordinal);
   if (mode == FC_EXACT_F32) {
     Epilogue ep;
-    Workspace wide;
     ep.ragged = true;
+    Workspace scratch;
+    // (without room the f32 kernels run, which need none; one row takes kernels that need none either)
     if ((m > 1 || dev->matvec_choice) && (qmatvec_mma_supports(w->m, m) || qmatvec_mma_ragged_supports(w->m, m))) {
-      // up to 64 rows: the decode tensor product needs scratch (one row takes kernels that need none)
-      // (a first call during a capture, or without room: the f32 kernels need none)
-      if (!w->mma_scratch && !stream_capturing(dev)) {
-        const cudaError_t e = workspace_alloc(dev, &w->mma_scratch, qmatvec_mma_scratch_bytes(w->m.k, w->m.n));
-        if (e != cudaSuccess) {
-          cudaGetLastError();
-          w->mma_scratch = nullptr;
-          if (e != cudaErrorMemoryAllocation) return fc_fail(dev, FC_ERR_DEVICE, "product scratch: %s", cudaGetErrorString(e));
-        }
-      }
-      ep.scratch = w->mma_scratch;
+      const int rc = qweight_scratch(w, qmatvec_mma_scratch_bytes(w->m.k, w->m.n), &scratch);
+      if (rc == FC_OK)
+        ep.scratch = scratch.p;
+      else if (rc != FC_ERR_OOM)
+        return rc;
     } else if (qgemm_pair_takes(w->m, m)) {
-      const int rc = qweight_workspace(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m, ACT_NONE));
-      if (rc != FC_OK && rc != FC_ERR_OOM) return rc;
-      // (no room for more, or a capture: the product is cut to the workspace that is there, or takes the tiled f32 kernel)
-      wide = Workspace{w->tc_cache, w->tc_cache_bytes};
-      ep.wide = &wide;
+      const int rc = qweight_scratch(w, qgemm_pair_scratch_bytes(dev, w->m.k, w->m.n, m, ACT_NONE), &scratch);
+      if (rc == FC_OK)
+        ep.wide = &scratch;
+      else if (rc != FC_ERR_OOM)
+        return rc;
     }
     return k_qlinear_f32(dev, w->m, x_dev, m, y_dev, ep);
   }

@@ -129,6 +129,42 @@ void workspace_free(FcDevice* dev, void* p) {
   else
     cudaFree(p); // (waits for the device)
 }
+void release_scratch(FcDevice* dev) {
+  if (dev->scratch.p) workspace_free(dev, dev->scratch.p);
+  dev->scratch = Workspace();
+}
+int qweight_scratch(FcQWeight* w, size_t bytes, Workspace* out) {
+  FcDevice* dev = w->dev;
+  void* p = nullptr;
+  cudaError_t e;
+  if (!stream_capturing(dev)) {
+    if (bytes <= dev->scratch.bytes) {
+      *out = dev->scratch;
+      return FC_OK;
+    }
+    release_scratch(dev);
+    e = workspace_alloc(dev, &p, bytes);
+    if (e == cudaSuccess) *out = dev->scratch = Workspace{p, bytes};
+  } else {
+    if (bytes <= w->graph_ws.bytes) {
+      *out = w->graph_ws;
+      return FC_OK;
+    }
+    // (no stream operation: nothing that a capture would record or, in this mode, forbid)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    e = cudaMalloc(&p, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) {
+      if (w->graph_ws.p) w->outgrown.push_back(w->graph_ws.p);
+      *out = w->graph_ws = Workspace{p, bytes};
+    }
+  }
+  if (e == cudaSuccess) return FC_OK;
+  cudaGetLastError();
+  return fc_fail(dev, e == cudaErrorMemoryAllocation ? FC_ERR_OOM : FC_ERR_DEVICE, "cannot allocate a %zu-byte product workspace: %s", bytes,
+                 cudaGetErrorString(e));
+}
 bool stream_capturing(FcDevice* dev) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(dev->stream, &st) != cudaSuccess) {
@@ -142,6 +178,7 @@ FC_API int fc_device_close(FcDevice* dev) {
   if (!dev) return FC_ERR_ARG;
   cudaSetDevice(dev->ordinal);
   cudaStreamSynchronize(dev->stream);
+  release_scratch(dev);
   if (dev->workspaces) cudaMemPoolDestroy(dev->workspaces);
   if (dev->pinned) cudaFreeHost(dev->pinned);
   if (dev->d_flag) cudaFree(dev->d_flag);
@@ -269,6 +306,8 @@ void qweight_free(FcQWeight* w) {
   if (!w) return;
   if (w->qs_alloc) cudaFree(w->qs_alloc);
   if (w->sc_alloc) cudaFree(w->sc_alloc);
+  for (void* p : w->outgrown) cudaFree(p);
+  if (w->graph_ws.p) cudaFree(w->graph_ws.p);
   delete w;
 }
 

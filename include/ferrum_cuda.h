@@ -162,14 +162,15 @@ int fc_dequant(FcQWeight* w, float* out_n_k, size_t out_elems);
 int fc_qmatmul(FcQWeight* w, const float* x, uint32_t m, float* y, int mode);
 /* The same on device buffers, enqueued on the device's stream, no synchronisation. `x_dev` and `y_dev` must be
  * 16-byte aligned (the kernels move 16-byte pieces; a misaligned pointer is refused with FC_ERR_ARG before any
- * launch). A kernel that gives up a bounded wait is reported by the next fc_device_sync, not here. */
+ * launch). A kernel that gives up a bounded wait is reported by the next fc_device_sync, not here.
+ * Scratch belongs to the device handle: all its weights share it, and it grows with the largest product. Under stream
+ * capture the weight allocates scratch of its own, kept for the replays until it is destroyed: replays of graphs that hold products of one
+ * weight must not overlap. */
 int fc_qmatmul_dev(FcQWeight* w, const float* x_dev, uint32_t m, float* y_dev, int mode);
 
 /* The tensor-core product of fc_qmatmul_dev (mode FC_TENSOR_F16) for callers that must not trigger a
- * device allocation. This entry point has no counterpart in the reference. fc_qmatmul_dev keeps its
- * fp16 copy of `x` in a buffer it cudaMalloc's and grows per weight; that is unusable from inside a
- * stream capture, under a memory plan that was checked once and may not grow, or in a loop that
- * cannot afford the device-wide synchronisation an allocation implies. Here the copy lives in a
+ * device allocation. This entry point has no counterpart in the reference. fc_qmatmul_dev takes scratch
+ * (the fp16 copy of `x`, decoded weights) that grows with the products, under stream capture too; that is unusable under a memory plan that was checked once and may not grow. Here the copy lives in a
  * fixed 8 MiB array inside the library's device image (every GPU that loads the library carries it
  * until the process exits), so `m * k` may be at most 4 Mi elements (4 194 304); larger products are
  * refused with FC_ERR_SHAPE. `x_dev` and `y_dev` are the caller's. The first call on a device looks

@@ -219,13 +219,14 @@ def test_exact_scoring_in_unequal_passes(dev):
     g.close()
 
 
-@pytest.mark.parametrize("mode,eager_rows", [(Mode.EXACT_F32, 0), (Mode.EXACT_F32, 100), (Mode.EXACT_F32, 3000), (Mode.TENSOR_F16, 3000)])
-def test_products_captured_into_a_graph(dev, mode, eager_rows):
-    """A captured call works in memory of its own size, whatever an earlier call of the same weight had, and replays read
-    the operands of the moment."""
+@pytest.mark.parametrize("eager_rows", [0, 100, 3000])
+@pytest.mark.parametrize("mode,m,k", [(Mode.EXACT_F32, 2000, 512), (Mode.EXACT_F32, 40, 512), (Mode.EXACT_F32, 5, 480), (Mode.TENSOR_F16, 2000, 512)])
+def test_products_captured_into_a_graph(dev, mode, m, k, eager_rows):
+    """A captured call works in memory of its own, whatever earlier calls of the same weight had, and replays read the
+    operands of the moment while eager work of this and other weights goes on between them."""
     import torch
     lib = _ffi.load()
-    m, k, n = 2000, 512, 1024
+    n = 1024
     rng = np.random.default_rng(5)
     qw = upload_quantised(dev, QKind.Q8_0, (rng.standard_normal(k * n) * 0.02).astype(np.float32), k, n)
     w = torch.from_numpy(qw.dequantised().reshape(n, k)).cuda().double()
@@ -242,9 +243,11 @@ def test_products_captured_into_a_graph(dev, mode, eager_rows):
     bound = EXACT if mode == Mode.EXACT_F32 else 2.0 ** -10
     for seed in range(2):
         x.copy_(torch.randn(x.shape, device="cuda", generator=torch.Generator("cuda").manual_seed(seed)))
-        y.zero_()
-        # work of other weights between the replays does not disturb them
+        torch.cuda.synchronize()
         dev.check(lib.fc_qmatmul_dev(other.handle, x.data_ptr(), m, y.data_ptr(), int(mode)))
+        call(m)
+        dev.sync()
+        y.zero_()
         torch.cuda.synchronize()
         graph.replay()
         torch.cuda.synchronize()
@@ -255,3 +258,25 @@ def test_products_captured_into_a_graph(dev, mode, eager_rows):
     del graph
     qw.close()
     other.close()
+
+
+@pytest.mark.parametrize("mode", [Mode.EXACT_F32, Mode.TENSOR_F16])
+def test_weights_share_their_scratch(dev, mode):
+    """Products of many weights leave no workspace behind with each."""
+    import torch
+    lib = _ffi.load()
+    m, k, n = 1500, 2048, 4096
+    w = (np.random.default_rng(1).standard_normal(k * n) * 0.02).astype(np.float32)
+    weights = [upload_quantised(dev, QKind.Q8_0, w, k, n) for _ in range(24)]
+    x, y = torch.randn(m, k, device="cuda"), torch.empty(m, n, device="cuda")
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    want = None
+    for qw in weights:
+        dev.check(lib.fc_qmatmul_dev(qw.handle, x.data_ptr(), m, y.data_ptr(), int(mode)))
+        dev.sync()
+        want = y.clone() if want is None else want
+        assert torch.equal(y, want)
+    assert free - torch.cuda.mem_get_info()[0] < 256 << 20  # one workspace is 28..46 MB
+    for qw in weights:
+        qw.close()
