@@ -8,6 +8,7 @@
 //   norm -> qkv(+bias) -> rope+cache -> attention -> wo(+bias)+residual -> norm -> ff1(+bias, GELU)
 //   [-> swiglu] -> ff2(+bias)+residual;   final norm -> head.
 // That is 9 (Llama) / 8 (GPT-2) launches per layer against the reference's 18-21 / 15.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -104,7 +105,8 @@ uint64_t plan_bytes(const Shape& s, int qkind, uint64_t streams) {
   per += 2 * streams * s.ctx * kvd * 4;                              // K and V caches
   b += per * s.layers;
   b += 2 * d * 4 + matrix_bytes(qkind, d, s.vocab);                  // final norm, head
-  b += streams * (2 * d + 2 * (qd + 2 * kvd) + qd + ff1 + hid + s.vocab) * 4 + streams * 16; // decode scratch
+  const uint64_t qkv = qd + 2 * kvd, ff = s.rope_dim && qkv > ff1 ? qkv : ff1;
+  b += streams * (2 * d + qkv + qd + ff + hid + s.vocab) * 4 + streams * 16; // decode scratch
   return b;
 }
 
@@ -131,9 +133,9 @@ int alloc_common(FcModel* m) {
   FC_TRY(dev_alloc(m, (size_t)s * m->dim * 4, (void**)&m->x));
   FC_TRY(dev_alloc(m, (size_t)s * m->dim * 4, (void**)&m->h));
   FC_TRY(dev_alloc(m, (size_t)s * m->qkv_w() * 4, (void**)&m->qkv));
-  if (m->rope.cos) FC_TRY(dev_alloc(m, (size_t)s * m->qkv_w() * 4, (void**)&m->qkv_rot));
   FC_TRY(dev_alloc(m, (size_t)s * m->qd() * 4, (void**)&m->attn));
-  FC_TRY(dev_alloc(m, (size_t)s * m->ff1_w() * 4, (void**)&m->ff));
+  // (between two feed-forward parts the decode attention of models with RoPE keeps the rotated qkv rows there)
+  FC_TRY(dev_alloc(m, (size_t)s * (m->rope.cos ? std::max(m->ff1_w(), m->qkv_w()) : m->ff1_w()) * 4, (void**)&m->ff));
   FC_TRY(dev_alloc(m, (size_t)s * m->hidden * 4, (void**)&m->act));
   FC_TRY(dev_alloc(m, (size_t)s * m->vocab * 4, (void**)&m->logits));
   FC_TRY(dev_alloc(m, (size_t)s * 4, (void**)&m->d_ids));
@@ -243,7 +245,7 @@ int run_stack_f32(FcModel* m, const PassBufs& b, const int32_t* ids, const int32
       }
       FC_TRY(k_attn_decode(dev, b.qkv, m->qkv_w(), rows, m->heads, m->kv_heads, m->hd, positions, streams, l.kv, m->ctx,
                            b.attn, m->attn_scratch, xh, xl, mp, attn_appends || attn_folds, attn_folds ? &qkv_sum : nullptr,
-                           attn_folds ? &m->rope : nullptr, m->qkv_rot));
+                           attn_folds ? &m->rope : nullptr, b.ff));
     } else if (mode == ATTN_STATELESS)
       FC_TRY(k_attn_causal_f32(dev, b.qkv, n_seqs, t, m->heads, m->kv_heads, m->hd, b.attn));
     else

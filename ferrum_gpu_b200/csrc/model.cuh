@@ -47,7 +47,6 @@ struct FcModel {
   uint64_t weight_bytes = 0;
   std::vector<void*> allocs;  // everything cudaMalloc'ed for this model except QWeights
   // decode scratch, sized for max_streams rows
-  float* qkv_rot = nullptr; // the qkv rows after RoPE (models with RoPE), written by the decode attention
   float *x = nullptr, *h = nullptr, *qkv = nullptr, *attn = nullptr, *ff = nullptr, *act = nullptr, *logits = nullptr;
   int32_t *d_ids = nullptr, *d_pos = nullptr, *d_streams = nullptr, *d_argmax = nullptr;
   void* argmax_scratch = nullptr; // keys and counters of the multi-CTA argmax, zero between launches

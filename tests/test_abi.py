@@ -59,6 +59,21 @@ def test_plan_bytes_without_a_device(lib):
     assert plan_bytes(config_c1(), QKind.Q8_0) > 0
 
 
+@pytest.mark.parametrize("name", ["config_c1", "config_c3", "config_c4", "config_c5"])
+def test_a_stream_plans_its_caches_and_one_row_of_each_decode_buffer(lib, name):
+    """What every further stream adds: K and V, a row each of the residual stream, its norm, qkv, the attention, both
+    feed-forward parts and the logits, and 16 bytes of inputs. The rotated qkv rows lie in the feed-forward buffer."""
+    from ferrum_gpu_b200 import QKind, hostmodel, plan_bytes
+    cfg = getattr(hostmodel, name)()
+    llama = isinstance(cfg, hostmodel.LlamaConfig)
+    qd, kvd = (cfg.q_dim, cfg.kv_dim) if llama else (cfg.dim, cfg.dim)
+    ff1 = 2 * cfg.hidden if llama else cfg.hidden
+    row = 2 * cfg.dim + qd + 2 * kvd + qd + ff1 + cfg.hidden + cfg.vocab
+    for streams in (1, 7):
+        grown = plan_bytes(cfg, QKind.Q8_0, streams + 1) - plan_bytes(cfg, QKind.Q8_0, streams)
+        assert grown == cfg.layers * 2 * cfg.ctx * kvd * 4 + row * 4 + 16
+
+
 def test_null_handles_are_refused_not_dereferenced(lib):
     assert lib.fc_device_close(None) == _ffi.FC_ERR_ARG
     assert lib.fc_qweight_destroy(None) == _ffi.FC_ERR_ARG

@@ -8,7 +8,7 @@ import pytest
 from ferrum_gpu_b200 import (CudaBackend, CudaError, CudaGpt2, CudaLlama, GenOpts, Mode, QKind, generate_with,
                              plan_bytes)
 from ferrum_gpu_b200 import _ffi
-from ferrum_gpu_b200.hostmodel import Gpt2Config, config_c1, random_gpt2, random_llama, random_tokens
+from ferrum_gpu_b200.hostmodel import Gpt2Config, LlamaConfig, config_c1, random_gpt2, random_llama, random_tokens
 from oracle import oracle as orc
 from tests import helpers
 
@@ -495,3 +495,25 @@ def test_chained_greedy_decode_returns_the_picks_of_step_by_step_decode(dev, str
     assert rc == _ffi.FC_ERR_CONTEXT_FULL and dev.launch_count() == before
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("ctx", [64, 1024])
+@pytest.mark.parametrize("hidden", [96, 512])
+def test_decode_with_a_feed_forward_narrower_and_wider_than_qkv(dev, hidden, ctx):
+    """The decode attention keeps the rotated qkv rows in the feed-forward buffer; the wider of the two sizes it."""
+    cfg = LlamaConfig(vocab=120, ctx=ctx, dim=128, heads=4, kv_heads=2, head_dim=64, layers=3, hidden=hidden, rope_dim=64)
+    m = random_llama(cfg, seed=11, std=0.1)
+    o = orc.OracleLlama(orc.dequantised_llama(m, int(QKind.Q8_0), snap_embedding=False))
+    g = CudaLlama(dev, m, QKind.Q8_0, max_streams=3)
+    ids = random_tokens(5, 40, cfg.vocab)
+    for i, t in enumerate(ids):
+        want = o.feed(int(t))
+        assert orc.max_rel_err(g.feed(int(t)), want) < 2 * FORWARD, i
+    # the same prompt on another stream, then both in one step
+    g.prefill(ids[:-1], stream=1)
+    g.reset(0)
+    g.prefill(ids[:-1], stream=0)
+    _, both = g.feed_batch([int(ids[-1])] * 2, streams=[0, 1], want_logits=True)
+    for row in both:
+        assert orc.max_rel_err(row, want) < 2 * FORWARD
+    g.close()
