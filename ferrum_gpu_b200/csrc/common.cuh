@@ -55,6 +55,10 @@ constexpr uint64_t WORKSPACE_POOL_KEEP = 512ull << 20;
 constexpr uint64_t WORKSPACE_POOL_WARM = 64ull << 20; // mapped when the device is opened
 cudaError_t workspace_alloc(FcDevice* dev, void** p, size_t bytes);
 void workspace_free(FcDevice* dev, void* p);
+// cudaMalloc that gives the scratch and the pool's cached memory back and tries again where there is no room (not under
+// capture, nor between asking for scratch and launching with it); and that release by itself.
+cudaError_t device_malloc(FcDevice* dev, void** p, size_t bytes);
+void release_cached(FcDevice* dev);
 bool stream_capturing(FcDevice* dev); // the device's stream is being captured into a graph
 
 // Record a message and hand back the status code.

@@ -204,7 +204,7 @@ FC_API int fc_group_score(FcGroup* g, const int32_t* ids, uint32_t n_seqs, uint3
     FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
     if (g->ws) cudaFree(g->ws);
     g->ws = nullptr, g->ws_bytes = 0;
-    FC_CUDA(dev, cudaMalloc(&g->ws, need));
+    FC_CUDA(dev, device_malloc(dev, &g->ws, need));
     g->ws_bytes = need;
   }
   uint8_t* p = (uint8_t*)g->ws;

@@ -21,7 +21,7 @@ namespace {
 int dev_alloc(FcModel* m, size_t bytes, void** out) {
   *out = nullptr;
   if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc(out, bytes);
+  cudaError_t e = device_malloc(m->dev, out, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fc_fail(m->dev, FC_ERR_OOM, "cannot allocate %zu bytes: %s", bytes, cudaGetErrorString(e));
@@ -113,6 +113,10 @@ uint64_t plan_bytes(const Shape& s, int qkind, uint64_t streams) {
 int check_budget(FcDevice* dev, uint64_t need, uint64_t budget) {
   size_t free_b = 0, total_b = 0;
   FC_CUDA(dev, cudaMemGetInfo(&free_b, &total_b));
+  if (!budget && need > free_b) {
+    release_cached(dev);
+    FC_CUDA(dev, cudaMemGetInfo(&free_b, &total_b));
+  }
   const uint64_t limit = budget ? budget : (uint64_t)free_b;
   if (need > limit)
     return fc_fail(dev, FC_ERR_OOM, "the model needs %llu bytes on the device, over the budget of %llu bytes",
@@ -383,7 +387,7 @@ int arena_reserve(FcModel* m, size_t bytes) {
   if (m->arena.base) cudaFree(m->arena.base);
   m->arena.base = nullptr;
   m->arena.cap = 0;
-  cudaError_t e = cudaMalloc((void**)&m->arena.base, bytes);
+  cudaError_t e = device_malloc(m->dev, (void**)&m->arena.base, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fc_fail(m->dev, FC_ERR_OOM, "cannot allocate a %zu-byte workspace: %s", bytes, cudaGetErrorString(e));
@@ -1053,7 +1057,7 @@ FC_API int fc_model_score(FcModel* m, const int32_t* ids, uint32_t n_seqs, uint3
     if (m->score_stage) cudaFree(m->score_stage);
     m->score_stage = nullptr;
     m->score_stage_bytes = 0;
-    const cudaError_t e = cudaMalloc(&m->score_stage, need);
+    const cudaError_t e = device_malloc(dev, &m->score_stage, need);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fc_fail(dev, FC_ERR_OOM, "cannot allocate scoring buffers: %s", cudaGetErrorString(e));

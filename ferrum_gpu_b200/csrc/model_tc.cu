@@ -40,8 +40,8 @@ int model_interleave_gate_up(FcDevice* dev, FcQWeight* w, uint32_t hidden, uint3
   const QMat& q = w->m;
   const size_t qs_row = qmat_qs_bytes(q.kind, q.k, 1), sc_row = qmat_sc_bytes(q.kind, q.k, 1);
   void *nqs = nullptr, *nsc = nullptr;
-  cudaError_t e = cudaMalloc(&nqs, qs_row * q.n);
-  if (e == cudaSuccess && sc_row) e = cudaMalloc(&nsc, sc_row * q.n);
+  cudaError_t e = device_malloc(dev, &nqs, qs_row * q.n);
+  if (e == cudaSuccess && sc_row) e = device_malloc(dev, &nsc, sc_row * q.n);
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (nqs) cudaFree(nqs);

@@ -46,9 +46,9 @@ FC_API int fc_qweight_create_from_blocks(FcDevice* dev, int kind, const uint8_t*
   w->dev = dev;
   const size_t qs_bytes = qmat_qs_bytes(kind, k, n), sc_bytes = qmat_sc_bytes(kind, k, n);
   uint8_t* stage = nullptr;
-  cudaError_t e = cudaMalloc(&w->qs_alloc, qs_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&w->sc_alloc, sc_bytes);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&stage, n_bytes);
+  cudaError_t e = device_malloc(dev, &w->qs_alloc, qs_bytes);
+  if (e == cudaSuccess) e = device_malloc(dev, &w->sc_alloc, sc_bytes);
+  if (e == cudaSuccess) e = device_malloc(dev, (void**)&stage, n_bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     qweight_free(w);
@@ -104,7 +104,7 @@ FC_API int fc_qweight_blocks(FcQWeight* w, uint8_t* out, size_t out_bytes) {
   const size_t want = fc_block_bytes(w->m.kind, (size_t)w->m.k * w->m.n);
   if (out_bytes != want) return fc_fail(dev, FC_ERR_SHAPE, "output holds %zu bytes, the blocks are %zu", out_bytes, want);
   uint8_t* d = nullptr;
-  FC_CUDA(dev, cudaMalloc((void**)&d, want));
+  FC_CUDA(dev, device_malloc(dev, (void**)&d, want));
   int rc = k_export_blocks(dev, w->m, d);
   if (rc == FC_OK && cudaMemcpyAsync(out, d, want, cudaMemcpyDeviceToHost, dev->stream) != cudaSuccess)
     rc = fc_fail(dev, FC_ERR_DEVICE, "block read-back failed");
@@ -120,7 +120,7 @@ FC_API int fc_dequant(FcQWeight* w, float* out, size_t out_elems) {
   const size_t want = (size_t)w->m.k * w->m.n;
   if (out_elems != want) return fc_fail(dev, FC_ERR_SHAPE, "output holds %zu elements, the weight has %zu", out_elems, want);
   float* d = nullptr;
-  FC_CUDA(dev, cudaMalloc((void**)&d, want * 4));
+  FC_CUDA(dev, device_malloc(dev, (void**)&d, want * 4));
   int rc = k_dequant(dev, w->m, d);
   if (rc == FC_OK && cudaMemcpyAsync(out, d, want * 4, cudaMemcpyDeviceToHost, dev->stream) != cudaSuccess)
     rc = fc_fail(dev, FC_ERR_DEVICE, "dequant read-back failed");
@@ -167,8 +167,8 @@ FC_API int fc_qmatmul(FcQWeight* w, const float* x, uint32_t m, float* y, int mo
   cudaSetDevice(dev->ordinal);
   if (m == 0) return FC_OK;
   float *dx = nullptr, *dy = nullptr;
-  cudaError_t e = cudaMalloc((void**)&dx, (size_t)m * w->m.k * 4);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&dy, (size_t)m * w->m.n * 4);
+  cudaError_t e = device_malloc(dev, (void**)&dx, (size_t)m * w->m.k * 4);
+  if (e == cudaSuccess) e = device_malloc(dev, (void**)&dy, (size_t)m * w->m.n * 4);
   if (e != cudaSuccess) {
     cudaGetLastError();
     if (dx) cudaFree(dx);

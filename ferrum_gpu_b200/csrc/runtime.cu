@@ -133,6 +133,19 @@ void release_scratch(FcDevice* dev) {
   if (dev->scratch.p) workspace_free(dev, dev->scratch.p);
   dev->scratch = Workspace();
 }
+void release_cached(FcDevice* dev) {
+  release_scratch(dev);
+  cudaStreamSynchronize(dev->stream);
+  if (dev->workspaces) cudaMemPoolTrimTo(dev->workspaces, 0);
+  cudaGetLastError();
+}
+cudaError_t device_malloc(FcDevice* dev, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  release_cached(dev);
+  return cudaMalloc(p, bytes);
+}
 int qweight_scratch(FcQWeight* w, size_t bytes, Workspace* out) {
   FcDevice* dev = w->dev;
   void* p = nullptr;
@@ -345,9 +358,9 @@ int qweight_from_parts(FcDevice* dev, int kind, const WeightSrc* parts, const ui
   w->dev = dev;
   const size_t qs_bytes = qmat_qs_bytes(kind, k, n), sc_bytes = qmat_sc_bytes(kind, k, n);
   uint8_t* stage = nullptr;
-  cudaError_t e = cudaMalloc(&w->qs_alloc, qs_bytes);
-  if (e == cudaSuccess && sc_bytes) e = cudaMalloc(&w->sc_alloc, sc_bytes);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&stage, stage_bytes);
+  cudaError_t e = device_malloc(dev, &w->qs_alloc, qs_bytes);
+  if (e == cudaSuccess && sc_bytes) e = device_malloc(dev, &w->sc_alloc, sc_bytes);
+  if (e == cudaSuccess) e = device_malloc(dev, (void**)&stage, stage_bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     qweight_free(w);

@@ -249,7 +249,7 @@ FC_API int fc_topk_dev(FcDevice* dev, const float* logits_dev, uint32_t vocab, u
   if (!dev || !logits_dev || !idx_out || !val_out || !n_out || (n_recent && !recent)) return FC_ERR_ARG;
   cudaSetDevice(dev->ordinal);
   void* scratch = nullptr;
-  FC_CUDA(dev, cudaMalloc(&scratch, topk_scratch_bytes(vocab, k ? k : 1, n_recent)));
+  FC_CUDA(dev, device_malloc(dev, &scratch, topk_scratch_bytes(vocab, k ? k : 1, n_recent)));
   const int rc = k_topk(dev, logits_dev, vocab, k, repetition_penalty, recent, n_recent, scratch, idx_out, val_out, n_out);
   cudaFree(scratch);
   return rc;

@@ -280,3 +280,31 @@ def test_weights_share_their_scratch(dev, mode):
     assert free - torch.cuda.mem_get_info()[0] < 256 << 20  # one workspace is 28..46 MB
     for qw in weights:
         qw.close()
+
+
+def test_cached_scratch_makes_room_for_weights(dev):
+    """What products left in the device handle's pool goes back when a weight finds no room beside it."""
+    import torch
+    lib = _ffi.load()
+    m, k, n = 6000, 8192, 1024
+    zeros = np.zeros(k * n, dtype=np.float32)
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    qw = upload_quantised(dev, QKind.Q8_0, zeros, k, n)
+    x, y = torch.randn(m, k, device="cuda"), torch.empty(m, n, device="cuda")
+    torch.cuda.synchronize()
+    dev.check(lib.fc_qmatmul_dev(qw.handle, x.data_ptr(), m, y.data_ptr(), 0))
+    dev.sync()
+    qw.close()
+    del x, y
+    torch.cuda.empty_cache()
+    cached = before - torch.cuda.mem_get_info()[0]
+    assert cached > 128 << 20, "the pool holds on to the workspace (197 MB of terms)"
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] < 80 << 20
+        big = upload_quantised(dev, QKind.Q8_0, np.zeros(4096 * 4096, dtype=np.float32), 4096, 4096)  # 18 MB and 67 of staging
+        big.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
