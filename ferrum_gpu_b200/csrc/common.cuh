@@ -270,7 +270,7 @@ __device__ __forceinline__ void qmat_eight(const QMat& w, uint32_t row, uint32_t
   }
 }
 // One output (or its part over [i0, i1), whole blocks) by an f32 chain in ascending k: what the products on fp16 terms of x
-// do with rows that such terms cannot hold. `x` is 16-byte aligned.
+// do with rows that such terms cannot hold.
 template <int KIND>
 __device__ __noinline__ float exact_dot(const float* x, const uint8_t* qs, const __half* sc, uint32_t k, uint32_t row, uint32_t i0,
                                         uint32_t i1) {
@@ -280,9 +280,8 @@ __device__ __noinline__ float exact_dot(const float* x, const uint8_t* qs, const
   for (uint32_t i = i0; i < i1; i += 8) {
     float v[8];
     qmat_eight<KIND>(w, row, i, v);
-    const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
-    acc = fmaf(a.x, v[0], acc), acc = fmaf(a.y, v[1], acc), acc = fmaf(a.z, v[2], acc), acc = fmaf(a.w, v[3], acc);
-    acc = fmaf(b.x, v[4], acc), acc = fmaf(b.y, v[5], acc), acc = fmaf(b.z, v[6], acc), acc = fmaf(b.w, v[7], acc);
+#pragma unroll
+    for (int j = 0; j < 8; j++) acc = fmaf(x[i + j], v[j], acc); // (x: a caller's pointer, aligned to nothing but floats)
   }
   return acc;
 }

@@ -308,3 +308,24 @@ def test_cached_scratch_makes_room_for_weights(dev):
     finally:
         del hog
         torch.cuda.empty_cache()
+
+
+def test_hidden_states_at_any_float_address(dev):
+    """The exact head takes hidden states where they lie, also rows that its fp16 terms do not hold."""
+    import torch
+    cfg = LlamaConfig(vocab=1000, ctx=64, dim=256, heads=4, kv_heads=2, head_dim=64, layers=1, hidden=256, rope_dim=64)
+    g = CudaLlama(dev, random_llama(cfg, seed=3, std=0.05), QKind.Q8_0)
+    rows = 200
+    h = torch.randn(rows, cfg.dim, device="cuda")
+    h[7, 3], h[9, 0], h[11] = 1e30, float("inf"), h[11] * 2.0 ** (-60 * torch.arange(cfg.dim, device="cuda") / cfg.dim)
+    moved = torch.empty(rows * cfg.dim + 1, device="cuda")
+    moved[1:] = h.reshape(-1)
+    targets = torch.arange(rows, device="cuda", dtype=torch.int32)
+    out = torch.zeros(2, rows, 4, device="cuda")
+    torch.cuda.synchronize()
+    g.head_partial_dev(h.data_ptr(), targets.data_ptr(), rows, Mode.EXACT_F32, out[0].data_ptr())
+    g.head_partial_dev(moved.data_ptr() + 4, targets.data_ptr(), rows, Mode.EXACT_F32, out[1].data_ptr())
+    dev.sync()
+    a, b = out.cpu().numpy()
+    assert np.array_equal(a, b, equal_nan=True) and np.all(np.isfinite(np.delete(a, 9, axis=0)))
+    g.close()
