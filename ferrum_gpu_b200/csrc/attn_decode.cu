@@ -13,8 +13,8 @@
 // all CTAs are resident at once: a second, partly filled wave costs more than longer ranges (64 streams
 // x 2 kv-heads at 1550 positions: 2 splits 0.60 ms per step of 24 layers, 3 splits 0.70). The range
 // of a split is not fixed: each row's current length is cut into equal parts, so the CTAs of a row
-// carry the same load whatever the length. The merge launch writes f32 rows or, for a following
-// 9..64-row tensor-core product, directly that product's two fp16 terms.
+// carry the same load whatever the length. The CTA of a (row, kv-head) that arrives last merges its splits and
+// writes f32 rows or, for a following 9..64-row tensor-core product, directly that product's two fp16 terms.
 // Replaces attn_gqd_probs.wgsl + attn_gqd_pv.wgsl (ferrum_wgpu/src/ops/llama.rs:L150-L179).
 #include "ops.cuh"
 
@@ -448,9 +448,9 @@ int launch(FcDevice* dev, const float* qkv, uint32_t q_stride, uint32_t rows, ui
     FC_CUDA(dev, cudaFuncSetAttribute(attn_decode_split_kernel<G, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<4>::BYTES));
     FC_CUDA(dev, cudaFuncSetAttribute(attn_decode_split_kernel<G, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile<8>::BYTES));
   }
-  // Two splits of four-warp CTAs, two CTAs per SM, and a merge launch - or, where every (row, kv-head) can have
-  // an SM of its own, one eight-warp CTA over the whole context: the same eight warps per SM stream the same
-  // positions, and the partial results and the merge launch (about 4 us of a 64-row step's layer) fall away.
+  // Two splits of four-warp CTAs, two CTAs per SM, and a merge of their results - or, where every (row, kv-head) can
+  // have an SM of its own, one eight-warp CTA over the whole context: the same eight warps per SM stream the same
+  // positions, without partial results (as a launch of its own the merge took about 4 us of a 64-row step's layer).
   if (n_splits == 2 && rows * kv_heads <= (uint32_t)dev->prop.multiProcessorCount) {
     dim3 grid(1, kv_heads, rows);
     FC_LAUNCH(dev, "attn_decode",

@@ -32,6 +32,7 @@
 // Phases run on across items. Every wait is bounded and raises a CTA-wide abort word.
 #include "gemm_tc.cuh"
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -414,21 +415,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     __syncwarp();
     tc::tmem_dealloc(tmem_base, TMEM_COLS);
   }
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
-  return fn;
 }
 
 } // namespace

@@ -29,9 +29,8 @@
 // acc_empty[b] (leader: 16 epilogue warps). Every wait is bounded and polls the CTA's abort word.
 #include "gemm_pair.cuh"
 
-#include <cuda.h>
-
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -496,21 +495,6 @@ __global__ void __launch_bounds__(256)
     *reinterpret_cast<uint4*>(wh + at) = make_uint4(h[0], h[1], h[2], h[3]);
     *reinterpret_cast<uint4*>(wl + at) = make_uint4(l[0], l[1], l[2], l[3]);
   }
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link dependency on libcuda)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-                    q == cudaDriverEntryPointSuccess;
-    return ok ? (EncodeTiledFn)p : nullptr;
-  }();
-  return fn;
 }
 
 // [rows][kp] fp16, boxes of `box` rows x 64 k under the 128-byte swizzle; rows past the end read as zeros

@@ -15,6 +15,7 @@
 //   - gemm_tx_main.cuh: 9..64 rows at f32-class accuracy.
 #include "gemm_tc.cuh"
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -410,24 +411,6 @@ __device__ __forceinline__ void epilogue_lse(const TcArgs& a, LseState& s, uint3
 #include "gemm_tx_main.cuh"
 #include "gemm_tp_main.cuh"
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point: the library carries no link
-// dependency on libcuda, so it still loads (and exports its symbols) on a machine without a GPU.
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
-  return fn;
-}
-
 template <int KIND, int EPI>
 int launch_tc(FcDevice* dev, const CUtensorMap& tmap, const QMat& w, const TcArgs& a, dim3 grid) {
   auto kern = qgemm_tc_kernel<KIND, EPI>;
@@ -673,9 +656,6 @@ int k_qgemm_tx(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl,
 // 464 us with in-kernel decoding, 330 decoded first; 256 rows: 71 and 94.)
 bool tp_takes(const FcDevice* dev, const QMat& w, uint32_t m, int epi) {
   if ((w.kind != FC_Q8_0 && w.kind != FC_Q4_0) || w.k % TC_BK || !m) return false;
-#ifdef TP_ALWAYS
-  return TP_ALWAYS;
-#endif
   const bool q8 = w.kind == FC_Q8_0;
   const uint64_t sms = (uint64_t)dev->prop.multiProcessorCount, pairs = sms / 2, steps = w.k / TC_BK;
   const uint64_t ts_tiles = (uint64_t)((w.n + TC_BN - 1) / TC_BN) * ((m + TS_BX - 1) / TS_BX);

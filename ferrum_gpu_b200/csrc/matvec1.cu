@@ -28,11 +28,10 @@
 //     sum exactly as the reference applies it.
 //
 // Every wait is bounded; a wait that gives up raises the device status flag and its warp returns.
-#include <cuda.h>
-
 #include "common.cuh"
 #include "ops.cuh"
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -546,22 +545,6 @@ bool make_plan(const FcDevice* dev, const QMat& w, Plan& p) {
   p.sc_off = p.ring_off + nw * p.n_stages * w_stage;
   p.smem = (size_t)p.sc_off + (size_t)nw * p.n_stages * p.sc_stage + 1024; // (+ the alignment slack)
   return true;
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link dependency on libcuda)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiledFn)p;
-  }
-  return fn;
 }
 
 template <int KIND, int NW, int LINES, bool SWIGLU>

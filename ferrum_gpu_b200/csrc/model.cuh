@@ -100,8 +100,8 @@ int model_trunk_f32(FcModel* m, const int32_t* ids_dev, const int32_t* pos_dev, 
 // `blocks` (k_attn_causal_ragged): n_seqs * t packed rows of sequences of unequal length instead of n_seqs equal ones.
 int model_trunk_tc(FcModel* m, const int32_t* ids_dev, const int32_t* pos_dev, uint32_t n_seqs, uint32_t t,
                    __half* hidden_out, int32_t cache_stream = -1, const uint4* blocks = nullptr, uint32_t n_blocks = 0);
-// Tensor-core scoring of sequences of unequal length in packed passes (score.cu): sequence order[i] is
-// ids[offsets[order[i]] ..]; the results go to the places fc_model_score_ragged documents.
+// Tensor-core scoring of sequences of unequal length in packed passes (score.cu): sequence s is ids[offsets[s] ..
+// offsets[s + 1]), offsets[0] is 0; the results go to the places fc_model_score_ragged documents.
 int model_score_packed(FcModel* m, const int32_t* ids, const uint32_t* offsets, uint32_t n_seqs, float* logprob_out, uint8_t* greedy_out);
 int model_head_partial_tc(FcModel* m, const __half* hidden, const int32_t* targets_dev, uint32_t rows,
                           float* partial);

@@ -196,18 +196,17 @@ int model_score_packed(FcModel* m, const int32_t* ids, const uint32_t* offsets, 
   const size_t total = (size_t)offsets[n_seqs] - n_seqs; // rows: every position but each sequence's last
   // whole sequences per pass, in the caller's order
   std::vector<uint32_t> first(1, 0);
-  size_t rows_max = 0, blocks_max = 0;
+  size_t rows_max = 0;
   for (uint32_t s = 0; s < n_seqs;) {
-    size_t rows = 0, blocks = 0;
+    size_t rows = 0;
     uint32_t e = s;
     while (e < n_seqs) {
       const size_t t = offsets[e + 1] - offsets[e] - 1;
       if (rows && chunk_bytes(m, rows + t, FC_TENSOR_F16) > cap) break;
-      rows += t, blocks += (t + 255) / 256;
+      rows += t;
       e++;
     }
     rows_max = rows > rows_max ? rows : rows_max;
-    blocks_max = blocks > blocks_max ? blocks : blocks_max;
     first.push_back(e);
     s = e;
   }

@@ -34,10 +34,11 @@ FC_API uint32_t fc_score_windows(uint32_t n_ids, uint32_t from, uint32_t ctx, ui
   return n;
 }
 
-// Sequences of unequal length: sequence s is ids[offsets[s] .. offsets[s + 1]). They are scored in groups of
-// similar length, each group padded with id 0 to its longest member - causal attention keeps a padded tail from
-// touching the positions before it - and one batched pass per group. Results are packed: sequence s owns
-// offsets[s] - s .. offsets[s + 1] - (s + 1) of logprob_out / greedy_out (len - 1 entries each).
+// Sequences of unequal length: sequence s is ids[offsets[s] .. offsets[s + 1]). On the tensor cores their rows are packed
+// one after another without padding, as many whole sequences per pass as fit (model_score_packed). In exact arithmetic
+// they are scored in groups of similar length, each group padded with id 0 to its longest member - causal attention keeps
+// a padded tail from touching the positions before it - and one batched pass per group. Results are packed: sequence s
+// owns offsets[s] - s .. offsets[s + 1] - (s + 1) of logprob_out / greedy_out (len - 1 entries each).
 FC_API int fc_model_score_ragged(FcModel* m, const int32_t* ids, const uint32_t* offsets, uint32_t n_seqs, int mode,
                                  float* logprob_out, uint8_t* greedy_out, double* nll_sum_out) {
   if (!m || !ids || !offsets) return FC_ERR_ARG;
