@@ -37,12 +37,11 @@ N_SEQS, SEQ_LEN = 256, 1024
 METRIC, UNIT = "scoring tok/s", "scored tokens/s"
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch of the largest product (gate/up with the
-# SwiGLU epilogue, M = 131072 rows, K = 768, N = 4096) from an ncu capture of a quarter-size launch
-# (32 x 1024 rows: 52.2 MB read + 80.3 MB written), scaled by 4; see profiles/.
-NCU_TRAFFIC_BYTES = 4 * (52.16e6 + 80.28e6)
-NCU_TRAFFIC_NOTE = ("gate/up product, per launch; algorithmic bytes are 740 MB (201 MB f16 rows in, 537 MB f16 out, "
-                    "1.8 MB weights) - part of the output is still in L2 when the launch ends")
+# DRAM traffic of the products' kernels (dram__bytes_read.sum + dram__bytes_write.sum): not captured for the form that decodes
+# the weights first; the figure of the kernels before it is in profiles/qgemm_c3_chunk_32x1024.md
+NCU_TRAFFIC_BYTES = None
+NCU_TRAFFIC_NOTE = ("not captured; algorithmic bytes of the gate/up product are 740 MB per launch (201 MB f16 rows in, 537 MB f16 out, "
+                    "1.8 MB weights), and its decoded weights are 6.3 MB more, written and read through L2")
 
 def peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
