@@ -107,3 +107,25 @@ def test_a_given_up_wait_ends_a_group_call_with_an_error(dev, mode):
     assert e.value.code == _ffi.FC_ERR_TIMEOUT
     assert np.array_equal(gs.score(ids), want), "the status is cleared once reported"
     gs.close()
+
+
+@pytest.mark.parametrize("pass_bytes", [0, 3 << 20, 1])
+def test_packed_scoring_in_several_passes_and_query_blocks(dev, pass_bytes):
+    """Tensor-core scoring of texts of 1 to 599 rows (one to three query blocks of 256), packed into one pass, several, or
+    one per text, against the exact path text by text."""
+    cfg, _ = _model(ctx=640)
+    m = random_llama(cfg, seed=21, std=0.05)  # logits of order 1, for which the scoring path is held to 2e-2 each
+    g = CudaLlama(dev, m, QKind.Q4_0)
+    seqs = [random_tokens(70 + i, n, cfg.vocab) for i, n in enumerate([2, 600, 3, 257, 258, 130, 17, 513, 129, 33, 256, 514])]
+    dev.check(_ffi.load().fc_debug_score_pass_bytes(g._h, pass_bytes))
+    lp, greedy, nll = g.score_ragged(seqs, Mode.TENSOR_F16)
+    differ = 0
+    for s, ids in enumerate(seqs):
+        want, want_greedy, want_nll = g.score_batch(ids[None], Mode.EXACT_F32)
+        assert lp[s].shape == (ids.size - 1,)
+        assert np.max(np.abs(lp[s] - want[0])) <= 4e-2, (s, ids.size)  # a log-probability is two logits' difference: 2 x 2e-2
+        assert abs(nll[s] - want_nll[0]) / (ids.size - 1) <= (1e-3 if ids.size > 16 else 4e-2)
+        assert abs(nll[s] + np.sum(lp[s].astype(np.float64))) <= 1e-9 * abs(nll[s])
+        differ += int(np.sum(greedy[s] != want_greedy[0]))
+    assert differ <= 0.01 * sum(ids.size for ids in seqs)
+    g.close()
