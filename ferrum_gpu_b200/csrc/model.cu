@@ -62,6 +62,7 @@ void model_free(FcModel* m) {
   cudaStreamSynchronize(m->dev->stream);
   model_tc_free(m);
   decode_cluster_free(m);
+  decode_grid_free(m);
   for (cudaGraphExec_t g : m->chain_graphs)
     if (g) cudaGraphExecDestroy(g);
   for (cudaGraphExec_t g : m->graphs)
@@ -669,6 +670,19 @@ FC_API int fc_model_info(FcModel* m, uint32_t* vocab, uint32_t* ctx, uint32_t* m
   return FC_OK;
 }
 
+// The end of a run of one-kernel steps (decode_grid.cu): the last picks and the status of its waits, one wait of the host.
+static int finish_grid_steps(FcModel* m, uint32_t n, int32_t* picks, float* logits_out) {
+  FcDevice* dev = m->dev;
+  int32_t* p = m->pin_dec;
+  FC_CUDA(dev, cudaMemcpyAsync(p, decode_grid_out(m), 36, cudaMemcpyDeviceToHost, dev->stream));
+  if (logits_out)
+    FC_CUDA(dev, cudaMemcpyAsync(logits_out, m->logits, (size_t)n * m->vocab * 4, cudaMemcpyDeviceToHost, dev->stream));
+  FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
+  if (p[8]) FC_TRY(tc_check_errors(dev));
+  if (picks) memcpy(picks, p, (size_t)n * 4);
+  return FC_OK;
+}
+
 FC_API int fc_model_feed_batch(FcModel* m, uint32_t n, const uint32_t* stream_ids, const int32_t* tokens,
                                float* logits_out, int32_t* argmax_out) {
   if (!m || !stream_ids || !tokens) return FC_ERR_ARG;
@@ -690,7 +704,7 @@ FC_API int fc_model_feed_batch(FcModel* m, uint32_t n, const uint32_t* stream_id
   // one eager step per batch width it is captured into a CUDA graph and replayed (a decode step is
   // ~50-220 dependent launches of a few microseconds each, so launch overhead, not bandwidth, sets
   // its time at small widths). Fault injection and per-kernel profiling use the eager path.
-  if (!m->pin_dec) FC_CUDA(dev, cudaMallocHost((void**)&m->pin_dec, (size_t)m->max_streams * 16));
+  if (!m->pin_dec) FC_CUDA(dev, cudaMallocHost((void**)&m->pin_dec, (size_t)m->max_streams * 16 + 64));
   int32_t* p = m->pin_dec;
   for (uint32_t i = 0; i < n; i++) {
     p[i] = tokens[i];
@@ -708,6 +722,15 @@ FC_API int fc_model_feed_batch(FcModel* m, uint32_t n, const uint32_t* stream_id
     FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
     if (argmax_out) argmax_out[0] = p[3];
     m->pos[stream_ids[0]]++;
+    return FC_OK;
+  }
+  // One to eight streams: the whole step is one persistent kernel (decode_grid.cu).
+  if (decode_grid_ready(m, n)) {
+    uint32_t positions[8];
+    for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]];
+    FC_TRY(k_decode_grid(m, n, stream_ids, positions, tokens, nullptr));
+    FC_TRY(finish_grid_steps(m, n, argmax_out, logits_out));
+    for (uint32_t i = 0; i < n; i++) m->pos[stream_ids[i]]++;
     return FC_OK;
   }
   auto enqueue_step = [&]() -> int {
@@ -851,6 +874,18 @@ FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream
     FC_CUDA(dev, cudaMemcpyAsync(tokens_out + (steps - 1), m->d_argmax, 4, cudaMemcpyDeviceToHost, dev->stream));
     FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
     m->pos[stream_ids[0]] += steps - 1;
+    return FC_OK;
+  }
+  if (decode_grid_ready(m, n)) { // a launch per step, each taking the picks of the one before
+    uint32_t positions[8];
+    for (uint32_t s = 1; s < steps; s++) {
+      for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]] + s - 1;
+      FC_TRY(k_decode_grid(m, n, stream_ids, positions, nullptr, m->d_chain_log + (size_t)s * n));
+    }
+    if (steps > 2) // the log holds the tokens the steps consumed: the picks of steps 0 .. steps - 2
+      FC_CUDA(dev, cudaMemcpyAsync(tokens_out + n, m->d_chain_log + 2 * (size_t)n, (size_t)(steps - 2) * n * 4, cudaMemcpyDeviceToHost, dev->stream));
+    FC_TRY(finish_grid_steps(m, n, tokens_out + (size_t)(steps - 1) * n, nullptr));
+    for (uint32_t i = 0; i < n; i++) m->pos[stream_ids[i]] += steps - 1;
     return FC_OK;
   }
   const bool graph_mode = m->graph_ok && dev->fail_after < 0 && !dev->profiling;
