@@ -1,4 +1,4 @@
-// Decode step of one to eight streams as ONE persistent kernel over all SMs: embedding, every layer (norm, q/k/v
+// Decode step of one to 64 streams as ONE persistent kernel over all SMs: embedding, every layer (norm, q/k/v
 // product, rotation and cache append, attention, output product, norm, gate/up or fc product, activation, down product),
 // final norm, head and the greedy pick. Op order of GpuLlama::feed / GpuGpt2::feed
 // (ferrum_wgpu/src/models/llama/forward.rs:L18-L72, models/gpt2.rs:L192-L265).
@@ -11,8 +11,9 @@
 //     (launch, layer); consumers poll the very words they need (a 64-bit access is single, so a matching tag vouches for
 //     its value). Producer and consumer are one store and one load apart.
 //   * The weight stream never waits for activations: one producer warp per CTA runs ahead through the CTA's tiles of all
-//     stages and fills a ring in shared memory with bulk copies; the K/V tiles of the CTA's attention items likewise. What a
-//     stage needs is there when its input arrives.
+//     stages and fills a ring in shared memory; the K/V tiles of the CTA's attention items likewise. What a stage needs is
+//     there when its input arrives. A slot is one TMA box of 16 rows x up to 1024 bytes, 128-byte swizzled so that the lanes'
+//     reads fall into different banks (a bulk copy per row, to a padded pitch, took 110 cycles each: 1900 per tile).
 //   * A product gives every CTA tiles of 16 weight rows. Its warps poll x, eight elements per lane, and leave it in shared
 //     memory as two fp16 terms (22 bits, every 32-block at a power of two of its own); then they share out the tiles' units
 //     of 128 k (mma.sync m16n8k16, the block scale applied to the f32 sum of a block), and the units' sums meet in shared
@@ -21,6 +22,8 @@
 //     One row uses the eight MMA columns as (block, term) pairs, four blocks at a time: a lane's k slots all come from one
 //     block, and its column pair carries that block's x and zeros elsewhere. More rows take a column each (up to four rows:
 //     two, one per term).
+//   * More than eight rows: the SMs split into as many grids as there are groups of eight rows, each a whole step of its own
+//     over all weights, which come from L2 once per group.
 //   * Attention: an item is (row, heads of a group, part of the positions); parts merge through the same tagged words.
 //
 // The code of a layer has to stay below the 32 KB or so that an SM's instruction cache holds: beyond it straight-line code
@@ -32,9 +35,11 @@
 // of the old one having finished its stage. All CTAs are resident (cooperative launch) and every wait is bounded: one
 // that gives up raises the device's status word, everybody's waits end at once, and the step reports it.
 #include <algorithm>
+#include <cstring>
 
 #include "model.cuh"
 #include "tc_ptx.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -46,23 +51,25 @@ constexpr int CONS = WARPS * 32;
 constexpr int THREADS = CONS + 128;
 constexpr uint32_t MAX_K = 3072;
 constexpr uint32_t TASKS = MAX_K / 256; // 256-element parts of a row of x
-constexpr uint32_t SLOT_ROW = 1024;     // bytes of a weight row per ring slot, at most
+constexpr uint32_t MAX_GROUPS = 8;      // groups of eight rows
+// 128-byte lines of a weight row per ring slot, at most
+__host__ __device__ constexpr uint32_t slot_lines(int mt) { return mt == 8 ? 4 : 8; }
 // tiles between two barriers, at most: their 16 x mt results take a thread each
-constexpr uint32_t tile_group(int mt) { return mt == 8 ? 3 : 4; }
+__host__ __device__ constexpr uint32_t tile_group(int mt) { return mt == 8 ? 3 : 4; }
 constexpr uint32_t SLOTS = 16;          // ring slots outstanding, at most
 constexpr uint32_t KV_POS = 64;         // positions of a K/V tile
 constexpr uint32_t KV_TILE = KV_POS * 64 * 4;
 constexpr uint32_t MAX_KV = 4;          // K/V tiles in flight
 constexpr uint32_t MAX_SPLITS = 16;
-constexpr uint32_t MAX_ITEMS = 8;       // attention items per CTA
-constexpr uint32_t MAX_RESID = 2;       // 16-row tiles of the residual stream per CTA
+constexpr uint32_t MAX_ITEMS = 24;      // attention items per CTA
+constexpr uint32_t MAX_RESID = 11;      // 16-row tiles of the residual stream per CTA
 constexpr uint32_t ITEM_HEADS = 4;      // heads of an attention item, at most
 constexpr uint32_t PART = 66;           // max, sum, 64 channels
 constexpr uint32_t SMEM_MAX = 227 * 1024;
 constexpr uint32_t POLL_LIMIT = 1u << 21; // tries of a poll (about 0.7 us each)
 
 struct DgMat {
-  const uint8_t* qs;
+  const void *map_w, *map_s; // tensor maps of the codes, [line][row][128 bytes], and of the scales
   const __half* sc;
   const float *bias, *gain, *beta; // (gain: its input is normed)
 };
@@ -71,12 +78,12 @@ struct DgLayer {
   float *kc, *vc;
 };
 // What the four matrices have in common over the layers (the fifth is the head), derived so that no stage divides:
-// 256-element parts of a row of x and 2^16 / that, 128-element units, ring slots per tile, pitch of the weight rows and
-// (halves) of the scales in a slot, size of a slot, tiles between two barriers.
+// 256-element parts of a row of x and 2^16 / that, 128-element units, ring slots per tile; of a slot the place of the scales,
+// their pitch (halves) and bytes, its size; tiles between two barriers.
 struct DgShape {
   const unsigned long long* src; // tagged words of its input and its result
   unsigned long long* dst;
-  uint32_t k, n, tpr, tpr_inv, nu, nch, pitch, sc_pitch, size, group, dst_stride;
+  uint32_t k, n, tpr, tpr_inv, nu, nch, sc_off, sc_pitch, sc_bytes, size, group, dst_stride;
   float k_inv;
 };
 struct DgArgs {
@@ -92,14 +99,16 @@ struct DgArgs {
   // every split
   unsigned long long *b_qkv, *b_attn, *b_x1, *b_x2, *b_act, *b_part;
   uint32_t x_stride, attn_stride, act_stride; // words of a row
-  uint32_t* state;          // [0] the last tag of the launches before, [1] CTAs that are through
-  unsigned long long* keys; // [8] best (logit, index) of a row; zero between launches
-  int32_t* out;             // [8] picks, [8] the status word
+  uint32_t group_words;     // (of one group of rows)
+  uint32_t* state;          // per group: [0] the last tag of the launches before, [1] CTAs that are through
+  unsigned long long* keys; // [64] best (logit, index) of a row; zero between launches
+  int32_t* out;             // [64] picks, [8] the groups' status words
   float* logits;
   int* err_flag;
   int32_t* log;             // where the consumed tokens go (nullable)
-  int32_t tok_in[8], pos[8], stream[8];
-  uint32_t rows, chained, splits, item_heads, kv_log; // (2^kv_log K/V tiles in flight)
+  int32_t tok_in[64], pos[64], stream[64];
+  uint32_t rows, group_rows, sub; // rows of a group, CTAs of a group
+  uint32_t chained, splits, item_heads, kv_log; // (2^kv_log K/V tiles in flight)
   uint32_t off_desc, off_red, off_x, off_ys, off_kv, off_ring, ring_bytes;
 };
 
@@ -111,7 +120,7 @@ struct Misc { // small per-CTA state
   float slice[(ITEM_HEADS + 2) * 64]; // q heads (scaled), k, v of the attention item's own position
   float pw[AWARPS][8][ITEM_HEADS], cw[AWARPS][ITEM_HEADS];
   float wm[AWARPS][ITEM_HEADS], wl[AWARPS][ITEM_HEADS];
-  int32_t ids[8];
+  int32_t ids[8], pos[8], stream[8];
   uint32_t used[8];            // parts that a row's positions are in
   struct Item {
     uint32_t r, h0, kvh, s, c0, c1, append; // row, first head, split, its K/V tiles; whether it appends k and v to the cache
@@ -219,10 +228,10 @@ __device__ __forceinline__ void item_range(uint32_t len, uint32_t splits, uint32
 // head's score), then the 16 four-channel columns x two halves of the positions for the weighted sum of V.
 template <int GP>
 __device__ __forceinline__ void attn_item(const DgArgs& a, const DgLayer& L, Misc& ms, float* wpart, float* kv_tiles, uint32_t& kvn,
-                                          Ctl ctl, uint32_t tag, const Misc::Item& im) {
+                                          Ctl ctl, uint32_t tag, uint32_t words, const Misc::Item& im) {
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), grp = lane >> 3, sub = lane & 7;
   const uint32_t r = im.r, h0 = im.h0, kvh = im.kvh, c0 = im.c0, c1 = im.c1;
-  const uint32_t G = GP == 1 ? 1u : a.item_heads, len = (uint32_t)a.pos[r] + 1;
+  const uint32_t G = GP == 1 ? 1u : a.item_heads, len = (uint32_t)ms.pos[r] + 1;
   // q, k, v of the row's own position: two channels per thread, rotated on the way in
   if (tid < (int)(G + 2) * 32) {
     const uint32_t hs = tid >> 5, pp = tid & 31, half = a.rope_dim / 2, p = len - 1;
@@ -231,7 +240,7 @@ __device__ __forceinline__ void attn_item(const DgArgs& a, const DgLayer& L, Mis
     const uint32_t ia = neox ? pp : 2 * pp, ib = neox ? pp + half : 2 * pp + 1;
     const float cs = rot ? a.cos[(size_t)p * half + pp] : 1.0f, sn = rot ? a.sin[(size_t)p * half + pp] : 0.0f;
     const uint32_t col = (hs < G ? h0 + hs : a.heads + kvh + (hs == G ? 0u : a.kv_heads)) * 64;
-    const unsigned long long* src = a.b_qkv + r * a.sh[0].dst_stride + col;
+    const unsigned long long* src = a.b_qkv + words + r * a.sh[0].dst_stride + col;
     unsigned long long w0, w1;
     uint32_t tries = 0;
     do {
@@ -246,7 +255,7 @@ __device__ __forceinline__ void attn_item(const DgArgs& a, const DgLayer& L, Mis
     ms.slice[hs * 64 + ia] = x * qs;
     ms.slice[hs * 64 + ib] = y * qs;
     if (hs >= G && im.append) {
-      float* dst = (hs == G ? L.kc : L.vc) + (((size_t)a.stream[r] * a.kv_heads + kvh) * a.ctx + p) * 64;
+      float* dst = (hs == G ? L.kc : L.vc) + (((size_t)ms.stream[r] * a.kv_heads + kvh) * a.ctx + p) * 64;
       dst[ia] = x, dst[ib] = y;
     }
   }
@@ -374,9 +383,9 @@ __device__ __forceinline__ void attn_item(const DgArgs& a, const DgLayer& L, Mis
 #pragma unroll
     for (int i = 0; i < AWARPS; i++) o = fmaf(__shfl_sync(0xffffffffu, f, i), wpart[((size_t)i * GP + h) * 64 + ch], o);
     if (ms.used[r] == 1) {
-      ll_st(a.b_attn + r * a.attn_stride + ll_at((h0 + h) * 64 + ch), o / l, tag);
+      ll_st(a.b_attn + words + r * a.attn_stride + ll_at((h0 + h) * 64 + ch), o / l, tag);
     } else {
-      unsigned long long* dst = a.b_part + (r * a.heads + h0 + h) * a.splits * PART;
+      unsigned long long* dst = a.b_part + words + (r * a.heads + h0 + h) * a.splits * PART;
       ll_st(dst + ((ch >> 3) * a.splits + im.s) * 8 + (ch & 7), o, tag);
       if (ch < 2) ll_st(dst + a.splits * 64 + 2 * im.s + ch, ch ? l : M, tag);
     }
@@ -385,24 +394,17 @@ __device__ __forceinline__ void attn_item(const DgArgs& a, const DgLayer& L, Mis
 }
 
 __host__ __device__ constexpr uint32_t al(uint32_t v, uint32_t a) { return (v + a - 1) / a * a; }
-// Pitch of a weight row in a slot: the lanes of a load (one row of x: 16 bytes of a block each, four blocks x two rows at a
-// time; more rows: 8 or 4 bytes, four lanes to a block) fall into different banks.
-constexpr uint32_t slot_pitch(bool q8, bool one, uint32_t bytes) { return al(bytes, 128) + (q8 ? (one ? 16 : 32) : (one ? 64 : 16)); }
-// Weight rows of `bytes`, then their scales.
-constexpr uint32_t slot_bytes(bool q8, bool one, uint32_t bytes) {
-  return al(16 * slot_pitch(q8, one, bytes) + 16 * (bytes / (q8 ? 32 : 16)) * 2, 128);
-}
-
 // MT: rows, padded to 1, 2, 4 or 8. GP: heads of an attention item, 1 or up to 4.
 template <int KIND, int MT, bool LLAMA, int GP>
 __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_constant__ DgArgs a) {
-  extern __shared__ __align__(128) uint8_t smem[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   constexpr bool Q8 = KIND == FC_Q8_0, ONE = MT == 1;
   constexpr bool WIDE = MT == 8;           // (else the low terms of x take columns 4 .. 7)
   constexpr uint32_t BLK = Q8 ? 32 : 16;   // bytes of a block's codes
-  constexpr uint32_t UPC = SLOT_ROW / (4 * BLK); // units of a full slot
+  constexpr uint32_t UPC = slot_lines(MT) * 128 / (4 * BLK); // units of a full slot
   constexpr uint32_t XBLK = 2 * MT * 64;   // bytes of a block of x: both terms of every row
   constexpr uint32_t PIECE = MT * 16;      // floats of a piece: a warp's sums of a tile
+  uint8_t* smem = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u); // (the swizzle is a function of the address)
   Misc& ms = *reinterpret_cast<Misc*>(smem);
   DgLayer* layers = reinterpret_cast<DgLayer*>(smem + a.off_desc);
   float* red = reinterpret_cast<float*>(smem + a.off_red);
@@ -411,7 +413,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   float* kv_tiles = reinterpret_cast<float*>(smem + a.off_kv);
   uint8_t* ring = smem + a.off_ring;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31; // (uniform, and known to be)
-  const uint32_t grid = gridDim.x, cta = blockIdx.x, M = ONE ? 1 : a.rows;
+  // this CTA's group of rows, and the grid that works on it
+  const uint32_t grp = WIDE ? blockIdx.x / a.sub : 0, grid = a.sub, cta = blockIdx.x - grp * grid, r0 = grp * a.group_rows;
+  const uint32_t M = ONE ? 1 : min(a.group_rows, a.rows - r0), words = grp * a.group_words;
   Ctl ctl{&ms.dead, a.err_flag};
 
   if (tid == 0) {
@@ -422,12 +426,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     for (uint32_t i = 0; i < MAX_KV; i++) tc::mbar_init(&ms.kv_full[i], 1), tc::mbar_init(&ms.kv_empty[i], AWARPS);
     tc::fence_barrier_init();
   }
-  if (tid < (int)M) ms.ids[tid] = a.chained ? *(volatile int32_t*)(a.out + tid) : a.tok_in[tid];
+  if (tid < (int)M) {
+    ms.ids[tid] = a.chained ? *(volatile int32_t*)(a.out + r0 + tid) : a.tok_in[r0 + tid];
+    ms.pos[tid] = a.pos[r0 + tid], ms.stream[tid] = a.stream[r0 + tid];
+  }
   // (the descriptors are read at every stage: from global memory each would be a trip to L2 in the stage's chain)
 #pragma unroll 1
   for (uint32_t i = tid; i < a.n_layers * (uint32_t)(sizeof(DgLayer) / 8); i += THREADS)
     reinterpret_cast<uint64_t*>(layers)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
-  const uint32_t tag0 = *(volatile uint32_t*)a.state + 1; // (words start out as zeros: 0 is no tag)
+  const uint32_t tag0 = *(volatile uint32_t*)(a.state + 2 * grp) + 1; // (words start out as zeros: 0 is no tag)
   // Tile T of a stage belongs to CTA (T + start) mod grid; the starts follow one another so that the small stages land on
   // different CTAs. wo and ff2 share theirs: the CTA of a tile keeps its rows of the residual stream.
   if (tid < 5) {
@@ -442,7 +449,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
 #pragma unroll 1
     for (uint32_t item = cta; item < M * head_groups * a.splits; item += grid) {
       const uint32_t s = item % a.splits, hg = item / a.splits % head_groups, r = item / (a.splits * head_groups);
-      const uint32_t h0 = hg * a.item_heads, len = (uint32_t)a.pos[r] + 1;
+      const uint32_t h0 = hg * a.item_heads, len = (uint32_t)a.pos[r0 + r] + 1;
       uint32_t c0, c1, used;
       item_range(len, a.splits, s, c0, c1, used);
       // (one of the items that hold the row's own position appends it)
@@ -451,7 +458,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     ms.n_items = n;
   } else if (tid >= 64 && tid < 64 + (int)M) {
     uint32_t c0, c1;
-    item_range((uint32_t)a.pos[tid - 64] + 1, a.splits, 0, c0, c1, ms.used[tid - 64]);
+    item_range((uint32_t)a.pos[r0 + tid - 64] + 1, a.splits, 0, c0, c1, ms.used[tid - 64]);
   }
   __syncthreads();
 
@@ -459,6 +466,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   if (warp >= WARPS) { // ---- the producer warp ----
     asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     if (warp > WARPS) return;
+    if (lane != 0) return; // (one thread issues all copies)
     // The ring: slots of the sizes that their matrices need, one behind the other, freed in the same order.
     uint32_t it = 0, tail = 0, head = 0, kvn = 0;
     bool on = true; // (nothing is requested any more once somebody gave up: a slot may still be in flight)
@@ -471,23 +479,20 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
 #pragma unroll 1
       for (uint32_t i = 0; i < ms.n_items; i++) {
         const Misc::Item& im = ms.items[i];
-        const uint32_t len = (uint32_t)a.pos[im.r] + 1;
-        const size_t at = ((size_t)a.stream[im.r] * a.kv_heads + im.kvh) * a.ctx * 64;
+        const uint32_t len = (uint32_t)ms.pos[im.r] + 1;
+        const size_t at = ((size_t)ms.stream[im.r] * a.kv_heads + im.kvh) * a.ctx * 64;
 #pragma unroll 1
         for (uint32_t c = im.c0; c < im.c1; c++, kvn++) {
           const uint32_t buf = kvn & ((1u << a.kv_log) - 1), p0 = c * KV_POS, cnt = min(KV_POS, len - 1 - p0); // (the new position is not in the cache yet)
           if (kvn >> a.kv_log) ctl.mbar(&ms.kv_empty[buf], ((kvn >> a.kv_log) - 1) & 1);
-          on = __all_sync(0xffffffffu, *ctl.dead == 0);
+          on = *ctl.dead == 0;
           if (!on) return;
-          if (lane == 0) {
-            tc::mbar_arrive_expect_tx(&ms.kv_full[buf], cnt * 512);
-            const uint32_t to = tc::smem_u32(kv_tiles) + buf * 2 * KV_TILE;
-            if (cnt) {
-              copy(to, L.kc + at + (size_t)p0 * 64, cnt * 256, &ms.kv_full[buf]);
-              copy(to + KV_TILE, L.vc + at + (size_t)p0 * 64, cnt * 256, &ms.kv_full[buf]);
-            }
+          tc::mbar_arrive_expect_tx(&ms.kv_full[buf], cnt * 512);
+          const uint32_t to = tc::smem_u32(kv_tiles) + buf * 2 * KV_TILE;
+          if (cnt) {
+            copy(to, L.kc + at + (size_t)p0 * 64, cnt * 256, &ms.kv_full[buf]);
+            copy(to + KV_TILE, L.vc + at + (size_t)p0 * 64, cnt * 256, &ms.kv_full[buf]);
           }
-          __syncwarp();
         }
       }
     };
@@ -496,7 +501,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
       const uint32_t mi = si == 4 * a.n_layers ? 4 : si & 3;
       const DgMat& W = mi == 4 ? a.head : layers[si >> 2].m[mi];
       const DgShape& sh = a.sh[mi];
-      const uint32_t row_bytes = Q8 ? sh.k : sh.k / 2, nblk = sh.k / 32, nch = sh.nch, pitch = sh.pitch, size = sh.size;
+      const uint32_t nch = sh.nch, size = sh.size;
       uint32_t T = ms.first[mi];
 #pragma unroll 1
       for (uint32_t left = ms.tiles[mi]; left && on; left--, T += grid)
@@ -518,26 +523,28 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
             if (fits && it - tail < SLOTS) break;
             ctl.mbar(&ms.empty[tail % SLOTS], (tail / SLOTS) & 1);
             tail++;
-            on = __all_sync(0xffffffffu, *ctl.dead == 0);
+            on = *ctl.dead == 0;
             if (!on) break;
           }
           if (!on) break;
           head = at + size;
           uint64_t* bar = &ms.full[it % SLOTS];
-          const uint32_t rows = min(16u, sh.n - T * 16), cb = min(SLOT_ROW, row_bytes - c * SLOT_ROW);
-          const uint32_t sb = nch == 1 ? nblk * 2 : cb / BLK * 2; // scale bytes of a row
-          if (lane == 0) {
-            ms.slot_at[it % SLOTS] = at;
-            tc::mbar_arrive_expect_tx(bar, rows * (cb + sb));
-          }
-          __syncwarp();
+          ms.slot_at[it % SLOTS] = at;
+          // (a box counts in full, rows and lines past the matrix's end are zeros; scales in one piece: valid rows only)
+          const uint32_t sb = nch == 1 ? min(16u, sh.n - T * 16) * sh.sc_pitch * 2 : sh.sc_bytes;
+          tc::mbar_arrive_expect_tx(bar, sh.sc_off + sb);
           const uint32_t to = tc::smem_u32(ring) + at;
-          if (lane < (int)rows) {
-            const size_t row = (size_t)T * 16 + lane;
-            copy(to + lane * pitch, W.qs + row * row_bytes + c * SLOT_ROW, cb, bar);
-            if (nch != 1) copy(to + 16 * pitch + lane * (SLOT_ROW / BLK * 2), W.sc + row * nblk + c * (SLOT_ROW / BLK), sb, bar);
-          }
-          if (nch == 1 && lane == 16) copy(to + 16 * pitch, W.sc + (size_t)T * 16 * nblk, rows * sb, bar);
+          asm volatile(
+              "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(to),
+              "l"(W.map_w), "r"(tc::smem_u32(bar)), "r"(0), "r"((int32_t)(T * 16)), "r"((int32_t)(c * slot_lines(MT)))
+              : "memory");
+          if (nch == 1)
+            copy(to + sh.sc_off, W.sc + (size_t)T * 16 * sh.sc_pitch, sb, bar);
+          else
+            asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
+                             to + sh.sc_off),
+                         "l"(W.map_s), "r"(tc::smem_u32(bar)), "r"((int32_t)(c * sh.sc_pitch)), "r"((int32_t)(T * 16))
+                         : "memory");
         }
       if (mi == 0 && on) kv_tiles_of(layers[si >> 2]);
     }
@@ -560,18 +567,23 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   const uint32_t ewarp = (uint32_t)(WARPS - 1 - warp), etid = ewarp * 32 + lane, e_row = lane & 15;
   const uint32_t e_ti = ONE ? ewarp : etid / PIECE, e_col = ONE ? 0 : (etid >> 4) & (MT - 1);
   // the embedding, by the CTAs that keep the residual stream: its words carry the tag before the first layer's
-  static_assert(MAX_RESID <= tile_group(MT) && tile_group(MT) * (ONE ? 32 : PIECE) <= CONS, "a thread per result of a group");
-  {
-    const uint32_t o = (cta + e_ti * grid) * 16 + e_row;
-    if (e_ti < MAX_RESID && o < a.dim && e_col < M) {
+  static_assert(tile_group(MT) * (ONE ? 32 : PIECE) <= CONS, "a thread per result of a group");
+#pragma unroll 1
+  for (uint32_t li = e_ti; li < MAX_RESID && e_ti < tile_group(MT); li += tile_group(MT)) {
+    const uint32_t o = (cta + li * grid) * 16 + e_row;
+    if (o < a.dim && e_col < M) {
       float v = a.tok[(size_t)ms.ids[e_col] * a.dim + o];
-      if (a.pos_table) v += a.pos_table[(size_t)a.pos[e_col] * a.dim + o];
-      ms.resid[(e_ti * MT + e_col) * 16 + e_row] = v;
-      ll_st(a.b_x2 + e_col * a.x_stride + ll_at(o), v, tag0);
+      if (a.pos_table) v += a.pos_table[(size_t)ms.pos[e_col] * a.dim + o];
+      ms.resid[(li * MT + e_col) * 16 + e_row] = v;
+      ll_st(a.b_x2 + words + e_col * a.x_stride + ll_at(o), v, tag0);
     }
   }
 
   const int g = lane >> 2, t = lane & 3;
+  // Fragment row g is tile row rho: a row's 16-byte chunks are XORed with its low three bits, and the rows whose lanes read
+  // together are to differ where their chunks then do (one row, Q8_0: two rows, every second chunk; Q4_0: two rows, four
+  // neighbouring chunks; more rows, Q8_0: four rows, two neighbouring chunks; Q4_0: eight rows, one chunk).
+  const uint32_t rho = ONE ? (Q8 ? g : (g >> 1) | ((g & 1) << 2)) : (Q8 ? ((g & 3) << 1) | (g >> 2) : g);
   uint32_t it = 0, kvn = 0, red_par = 0;
   unsigned long long best = 0; // head: the best (logit, index) of this thread's row
   uint32_t mi = 0, l = 0;      // matrix 0 .. 3 of layer l; 4: the head
@@ -607,27 +619,30 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
             const uint32_t c = kg / UPC, si = it + u_ti * sh.nch + c, b0 = (kg - c * UPC) * 4; // (first block, within the slot)
             ctl.mbar(&ms.full[si % SLOTS], (si / SLOTS) & 1);
             const uint8_t* slot = ring + ms.slot_at[si % SLOTS];
-            const uint32_t pitch = sh.pitch, sc_pitch = sh.sc_pitch;
-            const __half* sp = reinterpret_cast<const __half*>(slot + 16 * pitch) + g * sc_pitch + b0;
+            const uint32_t sc_pitch = sh.sc_pitch;
+            const __half* sp = reinterpret_cast<const __half*>(slot + sh.sc_off) + rho * sc_pitch + b0;
+            const uint8_t* wp = slot + (b0 / (128 / BLK)) * 2048 + rho * 128; // the unit's line (Q4_0: half a line) of row rho
+            const uint32_t h4 = Q8 ? 0 : b0 & 4;
             if (ONE) {
-              const uint8_t* wp = slot + g * pitch + (b0 + t) * BLK;
 #pragma unroll
               for (int h = 0; h < (Q8 ? 2 : 1); h++) {
-                const uint4 va = *reinterpret_cast<const uint4*>(wp + h * 16), vb = *reinterpret_cast<const uint4*>(wp + 8 * pitch + h * 16);
+                const uint8_t* p = wp + ((Q8 ? 2 * t + h : h4 + t) ^ (rho & 7)) * 16;
+                const uint4 va = *reinterpret_cast<const uint4*>(p), vb = *reinterpret_cast<const uint4*>(p + 1024);
                 wraw[h * 8] = va.x, wraw[h * 8 + 1] = va.y, wraw[h * 8 + 2] = va.z, wraw[h * 8 + 3] = va.w;
                 wraw[h * 8 + 4] = vb.x, wraw[h * 8 + 5] = vb.y, wraw[h * 8 + 6] = vb.z, wraw[h * 8 + 7] = vb.w;
               }
               sraw[0] = __half_as_ushort(sp[t]), sraw[1] = __half_as_ushort(sp[8 * sc_pitch + t]);
             } else {
-              const uint8_t* wp = slot + g * pitch + b0 * BLK + t * (BLK / 4);
 #pragma unroll
               for (int bb = 0; bb < 4; bb++) {
                 if (Q8) {
-                  const uint2 va = *reinterpret_cast<const uint2*>(wp + bb * BLK), vb = *reinterpret_cast<const uint2*>(wp + 8 * pitch + bb * BLK);
+                  const uint8_t* p = wp + ((2 * bb + (t >> 1)) ^ (rho & 7)) * 16 + (t & 1) * 8;
+                  const uint2 va = *reinterpret_cast<const uint2*>(p), vb = *reinterpret_cast<const uint2*>(p + 1024);
                   wraw[(bb * 4) % NW] = va.x, wraw[(bb * 4 + 1) % NW] = va.y, wraw[(bb * 4 + 2) % NW] = vb.x, wraw[(bb * 4 + 3) % NW] = vb.y;
                 } else {
-                  wraw[bb * 2] = *reinterpret_cast<const uint32_t*>(wp + bb * BLK);
-                  wraw[bb * 2 + 1] = *reinterpret_cast<const uint32_t*>(wp + 8 * pitch + bb * BLK);
+                  const uint8_t* p = wp + ((h4 + bb) ^ (rho & 7)) * 16 + t * 4;
+                  wraw[bb * 2] = *reinterpret_cast<const uint32_t*>(p);
+                  wraw[bb * 2 + 1] = *reinterpret_cast<const uint32_t*>(p + 1024);
                 }
               }
               const uint2 sa = *reinterpret_cast<const uint2*>(sp), sb = *reinterpret_cast<const uint2*>(sp + 8 * sc_pitch);
@@ -639,7 +654,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
             staged = true;
             const uint32_t n_tasks = M * tpr, want = mi == 0 || mi == 4 ? tag - 1 : tag;
             auto row_of = [&](uint32_t task) { return ONE ? 0u : (task * sh.tpr_inv) >> 16; };
-            const unsigned long long* src = sh.src + lane * 2;
+            const unsigned long long* src = sh.src + words + lane * 2;
             unsigned long long q[8];
             auto request = [&](uint32_t task) {
               const unsigned long long* p = src + task * 256; // (a row is whole tasks)
@@ -844,14 +859,14 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
 #pragma unroll
             for (int s = 1; s < 4; s <<= 1)
               acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], s), acc[2] += __shfl_xor_sync(0xffffffffu, acc[2], s);
-            if (t == 0) rw[g] = acc[0], rw[g + 8] = acc[2];
+            if (t == 0) rw[rho] = acc[0], rw[rho + 8] = acc[2];
           } else {
             if (!WIDE) { // columns 4 .. 7 are the low terms of columns 0 .. 3
 #pragma unroll
               for (int s = 0; s < 4; s++) acc[s] += __shfl_xor_sync(0xffffffffu, acc[s], 2);
             }
-            if (2 * t < MT) rw[2 * t * 16 + g] = acc[0], rw[2 * t * 16 + g + 8] = acc[2];
-            if (2 * t + 1 < MT) rw[(2 * t + 1) * 16 + g] = acc[1], rw[(2 * t + 1) * 16 + g + 8] = acc[3];
+            if (2 * t < MT) rw[2 * t * 16 + rho] = acc[0], rw[2 * t * 16 + rho + 8] = acc[2];
+            if (2 * t + 1 < MT) rw[(2 * t + 1) * 16 + rho] = acc[1], rw[(2 * t + 1) * 16 + rho + 8] = acc[3];
           }
         }
         const bool busy = (ONE ? ewarp : (etid & ~31u) / PIECE) < ntg; // (uniform in the warp)
@@ -894,7 +909,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
           }
           if (mine) {
             if (mi == 4) {
-              a.logits[(size_t)e_col * sh.n + o] = v;
+              a.logits[(size_t)(r0 + e_col) * sh.n + o] = v;
               // first maximum; NaN and -inf never win; -0 equals 0
               if (v > -INFINITY) {
                 const uint32_t b = __float_as_uint(v + 0.0f), ord = (b & 0x80000000u) ? ~b : b | 0x80000000u;
@@ -908,7 +923,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
                 *rs = v;
               }
               if (mi) at = ll_at(at);
-              ll_st(sh.dst + e_col * sh.dst_stride + at, v, tag);
+              ll_st(sh.dst + words + e_col * sh.dst_stride + at, v, tag);
             }
           }
         }
@@ -918,14 +933,14 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     if (mi == 4) break;
     if (mi == 0) { // ---- attention ----
 #pragma unroll 1
-      for (uint32_t i = 0; i < ms.n_items; i++) attn_item<GP>(a, layers[l], ms, red, kv_tiles, kvn, ctl, tag, ms.items[i]);
+      for (uint32_t i = 0; i < ms.n_items; i++) attn_item<GP>(a, layers[l], ms, red, kv_tiles, kvn, ctl, tag, words, ms.items[i]);
       if (a.splits > 1) {
         // rows in several parts: a warp merges eight channels of a (row, head), eight splits at a time with four lanes each
 #pragma unroll 1
         for (uint32_t p = (grid - 1 - cta) + grid * warp; p < M * a.heads * 8; p += grid * WARPS) {
           const uint32_t rh = p >> 3, r = (rh * a.heads_inv) >> 16, used = ms.used[r];
           if (used == 1) continue;
-          const unsigned long long* src = a.b_part + rh * a.splits * PART;
+          const unsigned long long* src = a.b_part + words + rh * a.splits * PART;
           const unsigned long long *col = src + (p & 7) * 8 * a.splits + 2 * t, *mls = src + a.splits * 64 + 2 * min((uint32_t)lane, used - 1);
           const uint32_t s0 = 8 * min((uint32_t)g, used - 1), s1 = 8 * min(g + 8u, used - 1);
           unsigned long long w[6];
@@ -952,7 +967,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
 #pragma unroll
           for (int i = 4; i < 32; i <<= 1) o0 += __shfl_xor_sync(0xffffffffu, o0, i), o1 += __shfl_xor_sync(0xffffffffu, o1, i);
           if (g == 0) {
-            unsigned long long* dst = a.b_attn + r * a.attn_stride + ll_at((rh - r * a.heads) * 64 + (p & 7) * 8 + 2 * t);
+            unsigned long long* dst = a.b_attn + words + r * a.attn_stride + ll_at((rh - r * a.heads) * 64 + (p & 7) * 8 + 2 * t);
             ll_st(dst, o0 / den, tag);
             ll_st(dst + 1, o1 / den, tag);
           }
@@ -968,22 +983,22 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     const unsigned long long ov = __shfl_xor_sync(0xffffffffu, best, o);
     best = ov > best ? ov : best;
   }
-  if ((lane & (ONE ? 31 : 15)) == 0 && best && e_col < M) atomicMax(&a.keys[e_col], best);
+  if ((lane & (ONE ? 31 : 15)) == 0 && best && e_col < M) atomicMax(&a.keys[r0 + e_col], best);
   __threadfence();
   cons_sync();
   if (tid == 0) {
-    const uint32_t n = atomicAdd(&a.state[1], 1u);
+    const uint32_t n = atomicAdd(&a.state[2 * grp + 1], 1u);
     if (n + 1 == grid) {
       __threadfence();
 #pragma unroll 1
       for (uint32_t r = 0; r < M; r++) {
-        const unsigned long long key = atomicExch(&a.keys[r], 0ull);
-        if (a.log) a.log[r] = ms.ids[r];
-        a.out[r] = key ? (int32_t)(0xffffffffu - (uint32_t)key) : 0;
+        const unsigned long long key = atomicExch(&a.keys[r0 + r], 0ull);
+        if (a.log) a.log[r0 + r] = ms.ids[r];
+        a.out[r0 + r] = key ? (int32_t)(0xffffffffu - (uint32_t)key) : 0;
       }
-      a.out[8] = *(volatile int*)a.err_flag;
-      a.state[1] = 0;
-      a.state[0] = tag0 + a.n_layers;
+      a.out[64 + grp] = *(volatile int*)a.err_flag;
+      a.state[2 * grp + 1] = 0;
+      a.state[2 * grp] = tag0 + a.n_layers;
     }
   }
 }
@@ -991,17 +1006,28 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
 struct DgState {
   bool ok = false;
   DgArgs args[4];              // for 1, 2, 4 and 8 padded rows
-  DgLayer* d_layers = nullptr; // the descriptors, likewise
+  void* d_layers = nullptr;    // the tensor maps and the layers' descriptors, for slots of 8 and of 4 lines
   void* words = nullptr;
   uint64_t launches = 0;       // since the words were cleared
   int kind = 0;
 };
 
+// A matrix's slots: 16 rows of up to `slot_lines` lines, then their scales.
+void slot_shape(DgShape& d, bool q8, int mt) {
+  const uint32_t lines = (q8 ? d.k : d.k / 2) / 128, box = std::min(lines, slot_lines(mt));
+  d.nch = (lines + box - 1) / box;
+  d.sc_off = box * 2048;
+  d.sc_pitch = d.nch == 1 ? d.k / 32 : box * (q8 ? 4 : 8);
+  d.sc_bytes = 16 * d.sc_pitch * 2;
+  d.size = al(d.sc_off + d.sc_bytes, 1024); // (the swizzle is a function of the address)
+}
+
 // Shared memory for `mt` padded rows; false where the ring cannot hold a tile of the longest K and one slot more.
 bool layout(DgArgs& a, int kind, int mt, uint32_t max_k) {
   const uint32_t gp = a.heads == a.kv_heads ? 1 : ITEM_HEADS;
-  const uint32_t row_bytes = kind == FC_Q8_0 ? max_k : max_k / 2, nch = (row_bytes + SLOT_ROW - 1) / SLOT_ROW;
-  const uint32_t slot = slot_bytes(kind == FC_Q8_0, mt == 1, std::min(row_bytes, SLOT_ROW));
+  DgShape d{};
+  d.k = max_k;
+  slot_shape(d, kind == FC_Q8_0, mt);
   a.off_desc = al((uint32_t)sizeof(Misc), 128);
   a.off_red = al(a.off_desc + a.n_layers * (uint32_t)sizeof(DgLayer), 128);
   // sums of the warps (two groups of tiles), x and its scales; the attention's per-warp parts lie over all of them
@@ -1009,10 +1035,10 @@ bool layout(DgArgs& a, int kind, int mt, uint32_t max_k) {
   a.off_ys = a.off_x + max_k * 4 * mt;
   a.off_kv = al(std::max(a.off_ys + max_k / 32 * mt * 4, a.off_red + AWARPS * gp * 64 * 4), 128);
   for (a.kv_log = mt <= 2 ? 2 : 1;; a.kv_log--) {
-    a.off_ring = a.off_kv + (2 * KV_TILE << a.kv_log);
-    a.ring_bytes = a.off_ring < SMEM_MAX ? (SMEM_MAX - a.off_ring) / 128 * 128 : 0;
-    if (a.ring_bytes >= std::max(2 * nch + 1, 4u) * slot) return true;
-    if (a.kv_log == 0) return a.ring_bytes >= (nch + 1) * slot;
+    a.off_ring = al(a.off_kv + (2 * KV_TILE << a.kv_log), 1024);
+    a.ring_bytes = a.off_ring + 1024 < SMEM_MAX ? (SMEM_MAX - 1024 - a.off_ring) / 1024 * 1024 : 0;
+    if (a.ring_bytes >= std::max(2 * d.nch + 1, 4u) * d.size) return true;
+    if (a.kv_log == 0) return a.ring_bytes >= (d.nch + 1) * d.size;
   }
 }
 
@@ -1022,8 +1048,8 @@ int launch(FcDevice* dev, DgArgs& a) {
   static OncePerDevice attr;
   if (attr.first(dev->ordinal)) FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(dev->prop.multiProcessorCount), cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = a.off_ring + a.ring_bytes, cfg.stream = dev->stream;
+  cfg.gridDim = dim3(a.sub * ((a.rows + a.group_rows - 1) / a.group_rows)), cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = a.off_ring + a.ring_bytes + 1024, cfg.stream = dev->stream;
   cudaLaunchAttribute at;
   at.id = cudaLaunchAttributeCooperative; // (CTAs wait for one another: all must be resident)
   at.val.cooperative = 1;
@@ -1056,33 +1082,43 @@ void decode_grid_free(FcModel* m) {
   m->dg = nullptr;
 }
 
+// CTAs of a group of a step of `rows` rows.
+static uint32_t group_ctas(const FcModel* m, uint32_t rows) {
+  return (uint32_t)m->dev->prop.multiProcessorCount / ((rows + 7) / 8);
+}
+
 // Whether a step of `rows` rows can run as this kernel, and the set-up on first use.
 bool decode_grid_ready(FcModel* m, uint32_t rows) {
-  if (rows == 0 || rows > 8 || m->n_shards != 1) return false;
-  // (LayerNorm keeps its input in registers: two 256-element parts per warp)
-  if (m->dg) return ((DgState*)m->dg)->ok && (m->arch == ARCH_LLAMA || rows * ((m->dim + 255) / 256) <= 2 * WARPS);
+  if (rows == 0 || rows > 8 * MAX_GROUPS || m->n_shards != 1) return false;
+  if (m->dg) {
+    const uint32_t sub = group_ctas(m, rows), group_rows = std::min(rows, 8u);
+    // (LayerNorm keeps its input in registers: two 256-element parts per warp)
+    return ((DgState*)m->dg)->ok && (m->arch == ARCH_LLAMA || group_rows * ((m->dim + 255) / 256) <= 2 * WARPS) &&
+           (m->dim + 15) / 16 <= MAX_RESID * sub && group_rows * m->heads <= MAX_ITEMS * sub;
+  }
   DgState* st = new DgState();
   m->dg = st;
   const int kind = m->head.w->m.kind;
-  if (kind != FC_Q8_0 && kind != FC_Q4_0) return false;
+  const bool q8 = kind == FC_Q8_0;
+  if (!q8 && kind != FC_Q4_0) return false;
   auto mat_ok = [&](const Linear& l) {
     const QMat& q = l.w->m;
-    const uint32_t row_bytes = kind == FC_Q8_0 ? q.k : q.k / 2;
-    if (q.kind != kind || q.k % 128 || q.k > MAX_K) return false;
-    // (bulk copies are whole 16 bytes: a row's part of the scales where rows are cut, else those of a 16-row tile)
-    if (q.k % 256 && (row_bytes > SLOT_ROW || q.n % 16)) return false;
+    if (q.kind != kind || q.k % (q8 ? 128 : 256) || q.k > MAX_K) return false; // (whole lines)
+    // (copies are whole 16 bytes: a row's scales as a tensor map has them, or those of a 16-row tile where a slot holds the row)
+    if (q.k % 256 && (q.k > slot_lines(8) * 128 || q.n % 16)) return false;
     return (((uintptr_t)q.qs | (uintptr_t)q.sc) & 15) == 0;
   };
-  const uint32_t grid = (uint32_t)m->dev->prop.multiProcessorCount;
   if (m->hd != 64 || m->heads % m->kv_heads || m->rope.rope_dim > 64) return false;
   if (m->dim > MAX_K || m->hidden > MAX_K || m->qd() > MAX_K) return false;
   if (m->arch == ARCH_LLAMA && m->gu_group != 1) return false;
-  if ((m->dim + 15) / 16 > MAX_RESID * grid || 8 * m->heads > MAX_ITEMS * grid) return false;
   if (!mat_ok(m->head)) return false;
   for (auto& l : m->layers)
     if (!mat_ok(l.qkv) || !mat_ok(l.wo) || !mat_ok(l.ff1) || !mat_ok(l.ff2)) return false;
   int coop = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->dev->ordinal) != cudaSuccess || !coop) return false;
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return false;
+  const uint32_t grid = (uint32_t)m->dev->prop.multiProcessorCount, max_k = std::max(m->dim, std::max(m->hidden, m->qd()));
   DgArgs a = DgArgs();
   a.n_layers = m->n_layers, a.dim = m->dim, a.heads = m->heads, a.kv_heads = m->kv_heads, a.ctx = m->ctx;
   a.heads_inv = 65536 / m->heads + 1;
@@ -1090,54 +1126,95 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
   a.tok = m->tok, a.pos_table = m->pos_table;
   a.cos = m->rope.cos, a.sin = m->rope.sin, a.rope_dim = m->rope.rope_dim, a.rope_type = m->rope.type;
   a.eps = m->eps, a.logits = m->logits, a.err_flag = m->dev->d_flag;
-  auto mat = [](const Linear& l, const float* gain, const float* beta) { return DgMat{l.w->m.qs, l.w->m.sc, l.bias, gain, beta}; };
-  std::vector<DgLayer> hl(m->n_layers);
-  for (uint32_t i = 0; i < m->n_layers; i++) {
-    const Layer& l = m->layers[i];
-    hl[i] = DgLayer{{mat(l.qkv, l.norm1_g, l.norm1_b), mat(l.wo, nullptr, nullptr), mat(l.ff1, l.norm2_g, l.norm2_b), mat(l.ff2, nullptr, nullptr)},
-                    l.kv.k,
-                    l.kv.v};
-  }
-  a.head = mat(m->head, m->normf_g, m->normf_b);
-  a.head.bias = nullptr;
   for (int v = 0; v < 4; v++)
-    if (!layout(a, kind, 1 << v, std::max(m->dim, std::max(m->hidden, m->qd())))) return false;
-  // the tagged words, outside the model's plan: a model that fits without them decodes as launches
-  const size_t rows_max = std::min<uint32_t>(8, m->max_streams);
+    if (!layout(a, kind, 1 << v, max_k)) return false;
+  // The tagged words, outside the model's plan: a model that fits without them decodes as launches.
+  const uint32_t groups = (std::min<uint32_t>(8 * MAX_GROUPS, m->max_streams) + 7) / 8, rows_max = std::min<uint32_t>(8, m->max_streams);
   const size_t w_part = (size_t)grid * ITEM_HEADS * PART;
-  const size_t n_words = rows_max * (m->qkv_w() + a.attn_stride + 2 * (size_t)a.x_stride + a.act_stride) + w_part + 16;
-  if (cudaMalloc((void**)&st->d_layers, hl.size() * sizeof(DgLayer)) != cudaSuccess || cudaMalloc(&st->words, n_words * 8) != cudaSuccess ||
-      cudaMemcpyAsync(st->d_layers, hl.data(), hl.size() * sizeof(DgLayer), cudaMemcpyHostToDevice, m->dev->stream) != cudaSuccess ||
+  const size_t g_words = rows_max * (m->qkv_w() + a.attn_stride + 2 * (size_t)a.x_stride + a.act_stride) + w_part;
+  const size_t n_words = groups * g_words + 64 + 8 + 40; // keys, state, out
+  // descriptors: per variant of the slots two tensor maps per matrix, then the layers
+  const size_t n_mats = 4 * (size_t)m->n_layers + 1, maps_bytes = n_mats * 2 * sizeof(CUtensorMap);
+  const size_t var_bytes = (maps_bytes + m->n_layers * sizeof(DgLayer) + 255) & ~(size_t)255;
+  if (cudaMalloc(&st->d_layers, 2 * var_bytes) != cudaSuccess || cudaMalloc(&st->words, n_words * 8) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  std::vector<uint8_t> host(2 * var_bytes);
+  DgMat heads[2];
+  for (int var = 0; var < 2; var++) {
+    uint8_t* at = host.data() + var * var_bytes;
+    const uint8_t* dev_at = (const uint8_t*)st->d_layers + var * var_bytes;
+    size_t next = 0;
+    bool ok = true;
+    auto mat = [&](const Linear& l, const float* gain, const float* beta) {
+      const QMat& q = l.w->m;
+      DgShape d{};
+      d.k = q.k;
+      slot_shape(d, q8, var ? 8 : 1);
+      CUtensorMap tw, ts;
+      memset(&ts, 0, sizeof(ts));
+      const uint32_t row_bytes = q8 ? q.k : q.k / 2;
+      {
+        const cuuint64_t dims[3] = {128, q.n, row_bytes / 128}, strides[2] = {row_bytes, 128};
+        const cuuint32_t box[3] = {128, 16, d.sc_off / 2048}, estr[3] = {1, 1, 1};
+        ok = ok && enc(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void*)q.qs, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+      }
+      if (d.nch > 1) {
+        const cuuint64_t dims[2] = {q.k / 32, q.n}, strides[1] = {q.k / 32 * 2};
+        const cuuint32_t box[2] = {d.sc_pitch, 16}, estr[2] = {1, 1};
+        ok = ok && enc(&ts, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, (void*)q.sc, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+      }
+      memcpy(at + next, &tw, sizeof(tw));
+      memcpy(at + next + sizeof(tw), &ts, sizeof(ts));
+      const DgMat r{dev_at + next, dev_at + next + sizeof(tw), q.sc, l.bias, gain, beta};
+      next += 2 * sizeof(tw);
+      return r;
+    };
+    heads[var] = mat(m->head, m->normf_g, m->normf_b);
+    heads[var].bias = nullptr;
+    std::vector<DgLayer> hl(m->n_layers);
+    for (uint32_t i = 0; i < m->n_layers; i++) {
+      const Layer& l = m->layers[i];
+      hl[i] = DgLayer{{mat(l.qkv, l.norm1_g, l.norm1_b), mat(l.wo, nullptr, nullptr), mat(l.ff1, l.norm2_g, l.norm2_b), mat(l.ff2, nullptr, nullptr)},
+                      l.kv.k,
+                      l.kv.v};
+    }
+    memcpy(at + maps_bytes, hl.data(), hl.size() * sizeof(DgLayer));
+    if (!ok) return false;
+  }
+  if (cudaMemcpyAsync(st->d_layers, host.data(), host.size(), cudaMemcpyHostToDevice, m->dev->stream) != cudaSuccess ||
       cudaMemsetAsync(st->words, 0, n_words * 8, m->dev->stream) != cudaSuccess || cudaStreamSynchronize(m->dev->stream) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  a.layers = st->d_layers;
   unsigned long long* w = (unsigned long long*)st->words;
+  a.group_words = (uint32_t)g_words;
   a.b_part = w, w += w_part;
   a.b_attn = w, w += rows_max * a.attn_stride;
   a.b_x1 = w, w += rows_max * a.x_stride;
   a.b_x2 = w, w += rows_max * a.x_stride;
   a.b_act = w, w += rows_max * a.act_stride;
-  a.b_qkv = w, w += rows_max * m->qkv_w();
-  a.keys = w, w += 8;
-  a.state = (uint32_t*)w, w += 1;
-  a.out = (int32_t*)w; // (nine)
+  a.b_qkv = w;
+  w = (unsigned long long*)st->words + groups * g_words;
+  a.keys = w, w += 64;
+  a.state = (uint32_t*)w, w += 8;
+  a.out = (int32_t*)w;
   for (int v = 0; v < 4; v++) {
     DgArgs& b = st->args[v];
     b = a;
-    layout(b, kind, 1 << v, std::max(m->dim, std::max(m->hidden, m->qd())));
+    layout(b, kind, 1 << v, max_k);
+    b.layers = (const DgLayer*)((uint8_t*)st->d_layers + (v == 3) * var_bytes + maps_bytes);
+    b.head = heads[v == 3];
     auto shape = [&](const Linear& l, const unsigned long long* src, unsigned long long* dst, uint32_t dst_stride) {
       const QMat& q = l.w->m;
-      const bool q8 = kind == FC_Q8_0;
-      const uint32_t row_bytes = q8 ? q.k : q.k / 2;
       DgShape d{src, dst, q.k, q.n};
-      d.tpr = (q.k + 255) / 256, d.tpr_inv = 65536 / d.tpr + 1, d.nu = q.k / 128, d.nch = (row_bytes + SLOT_ROW - 1) / SLOT_ROW;
-      d.pitch = slot_pitch(q8, v == 0, std::min(row_bytes, SLOT_ROW)), d.size = slot_bytes(q8, v == 0, std::min(row_bytes, SLOT_ROW));
-      d.sc_pitch = d.nch == 1 ? q.k / 32 : SLOT_ROW / (q8 ? 32 : 16);
-      // (a group's slots, and one that does not fit before the ring's end; where it can be, the next group's as well)
-      const uint32_t slots = std::min(SLOTS, b.ring_bytes / d.size - 1);
-      d.group = std::max(1u, std::min(tile_group(1 << v), slots / (2 * d.nch)));
+      slot_shape(d, q8, 1 << v);
+      d.tpr = (q.k + 255) / 256, d.tpr_inv = 65536 / d.tpr + 1, d.nu = q.k / 128;
+      // (a group's slots, and where it can be the next group's as well: a ring of one tile and a slot holds one tile's)
+      d.group = std::max(1u, std::min(tile_group(1 << v), std::min(SLOTS, b.ring_bytes / d.size) / (2 * d.nch)));
       d.k_inv = 1.0f / (float)q.k, d.dst_stride = dst_stride;
       return d;
     };
@@ -1153,20 +1230,48 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
   return decode_grid_ready(m, rows);
 }
 
+// Whether a step of these rows is faster as this kernel than as launches. Up to eight rows it always was. Beyond, every
+// group of eight reads all weights (a unit of 16 rows x 128 k costs an SM 0.15 us as Q4_0, 0.17 as Q8_0) and works through
+// its caches on its share of the SMs (2 us per 64-position tile and item), where the launches' step is a chain of some 40 us
+// per layer whatever it holds. Steps at 0 .. 60 positions, us as launches and here: Qwen2-style 24 layers Q8_0, 16 rows 1197 and
+// 712, 32 rows 1316 and 1116, 48 rows 1555 and 1599, 64 rows 1450 and 2017; Llama-style 12 layers Q4_0, 16 rows 464 and 245, 64
+// rows 575 and 503; GPT-2-124M-style Q4_0, 64 rows 732 and 616. At 950 positions: Qwen2-style 16 rows 1177 and 1117, 24 rows
+// 1348 and 1612; GPT-2-124M-style 24 rows 858 and 811, 32 rows 1014 and 1109.
+bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions) {
+  if (!decode_grid_ready(m, rows)) return false;
+  if (rows <= 8) return true;
+  const double sms = m->dev->prop.multiProcessorCount, layers = m->n_layers, groups = (rows + 7) / 8;
+  double units = 0.0, tiles = 0.0, bytes = 0.0;
+  auto add = [&](const Linear& l) { units += (l.w->m.n + 15) / 16 * (l.w->m.k / 128); };
+  for (const auto& l : m->layers) add(l.qkv), add(l.wo), add(l.ff1), add(l.ff2);
+  add(m->head);
+  for (uint32_t r = 0; r < rows; r++) {
+    tiles += positions[r] / KV_POS + 1;
+    bytes += (positions[r] + 1.0) * m->kv_heads * 512;
+  }
+  uint32_t item = 1;
+  for (uint32_t h = 1; h <= ITEM_HEADS; h++)
+    if (m->heads / m->kv_heads % h == 0) item = h;
+  const double here = layers * (10.0 + 2.0 * tiles * (m->heads / item) / sms) + (((DgState*)m->dg)->kind == FC_Q8_0 ? 0.17 : 0.15) * groups * units / sms;
+  const double launches = layers * ((rows <= 16 ? 38.0 : rows <= 32 ? 42.0 : 50.0) + bytes / 4e6) + 1.3e-3 * units;
+  return here < launches;
+}
+
 const int32_t* decode_grid_out(const FcModel* m) { return ((DgState*)m->dg)->args[0].out; }
 
 int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint32_t* positions, const int32_t* tokens, int32_t* log) {
   DgState* st = (DgState*)m->dg;
   FcDevice* dev = m->dev;
   if (st->launches >= (1ull << 31) / (m->n_layers + 1)) { // (before a tag could come round again)
-    FC_CUDA(dev, cudaMemsetAsync(st->words, 0, (size_t)((uint8_t*)st->args[0].keys - (uint8_t*)st->words), dev->stream));
-    FC_CUDA(dev, cudaMemsetAsync(st->args[0].state, 0, 8, dev->stream));
+    FC_CUDA(dev, cudaMemsetAsync(st->words, 0, (size_t)((uint8_t*)st->args[0].out - (uint8_t*)st->words), dev->stream));
     st->launches = 0;
   }
   st->launches++;
   const int v = rows == 1 ? 0 : rows == 2 ? 1 : rows <= 4 ? 2 : 3;
   DgArgs a = st->args[v];
-  a.rows = rows, a.chained = tokens ? 0 : 1, a.log = log;
+  const uint32_t groups = (rows + 7) / 8;
+  a.rows = rows, a.group_rows = (rows + groups - 1) / groups, a.sub = group_ctas(m, rows);
+  a.chained = tokens ? 0 : 1, a.log = log;
   uint32_t longest = 1;
   for (uint32_t r = 0; r < rows; r++) {
     a.tok_in[r] = tokens ? tokens[r] : 0;
@@ -1176,18 +1281,18 @@ int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint
   }
   // Items: as few heads of a group each as the CTAs allow. A row's positions are split only where one CTA would work
   // through more than four 64-position tiles: the merge costs another trip through L2.
-  const uint32_t tiles = (longest + KV_POS - 1) / KV_POS, group = a.heads / a.kv_heads, grid = (uint32_t)dev->prop.multiProcessorCount;
+  const uint32_t tiles = (longest + KV_POS - 1) / KV_POS, group = a.heads / a.kv_heads;
   a.splits = tiles <= 4 ? 1 : std::min(tiles, MAX_SPLITS);
   a.item_heads = 0;
   uint32_t widest = 1;
   for (uint32_t h = 1; h <= std::min(group, ITEM_HEADS); h++)
     if (group % h == 0) {
       widest = h;
-      if (!a.item_heads && rows * (a.heads / h) * a.splits <= grid) a.item_heads = h;
+      if (!a.item_heads && a.group_rows * (a.heads / h) * a.splits <= a.sub) a.item_heads = h;
     }
   if (!a.item_heads) {
     a.item_heads = widest;
-    a.splits = std::max(1u, std::min(a.splits, grid / (rows * (a.heads / widest))));
+    a.splits = std::max(1u, std::min(a.splits, a.sub / (a.group_rows * (a.heads / widest))));
   }
   const bool llama = m->arch == ARCH_LLAMA;
   return st->kind == FC_Q8_0 ? launch_rows<FC_Q8_0>(dev, a, llama) : launch_rows<FC_Q4_0>(dev, a, llama);

@@ -674,11 +674,15 @@ FC_API int fc_model_info(FcModel* m, uint32_t* vocab, uint32_t* ctx, uint32_t* m
 static int finish_grid_steps(FcModel* m, uint32_t n, int32_t* picks, float* logits_out) {
   FcDevice* dev = m->dev;
   int32_t* p = m->pin_dec;
-  FC_CUDA(dev, cudaMemcpyAsync(p, decode_grid_out(m), 36, cudaMemcpyDeviceToHost, dev->stream));
+  FC_CUDA(dev, cudaMemcpyAsync(p, decode_grid_out(m), 288, cudaMemcpyDeviceToHost, dev->stream)); // 64 picks, 8 status words
   if (logits_out)
     FC_CUDA(dev, cudaMemcpyAsync(logits_out, m->logits, (size_t)n * m->vocab * 4, cudaMemcpyDeviceToHost, dev->stream));
   FC_CUDA(dev, cudaStreamSynchronize(dev->stream));
-  if (p[8]) FC_TRY(tc_check_errors(dev));
+  for (int i = 64; i < 72; i++)
+    if (p[i]) {
+      FC_CUDA(dev, cudaMemsetAsync((void*)(decode_grid_out(m) + 64), 0, 32, dev->stream));
+      return tc_check_errors(dev);
+    }
   if (picks) memcpy(picks, p, (size_t)n * 4);
   return FC_OK;
 }
@@ -704,7 +708,7 @@ FC_API int fc_model_feed_batch(FcModel* m, uint32_t n, const uint32_t* stream_id
   // one eager step per batch width it is captured into a CUDA graph and replayed (a decode step is
   // ~50-220 dependent launches of a few microseconds each, so launch overhead, not bandwidth, sets
   // its time at small widths). Fault injection and per-kernel profiling use the eager path.
-  if (!m->pin_dec) FC_CUDA(dev, cudaMallocHost((void**)&m->pin_dec, (size_t)m->max_streams * 16 + 64));
+  if (!m->pin_dec) FC_CUDA(dev, cudaMallocHost((void**)&m->pin_dec, (size_t)m->max_streams * 16 + 288));
   int32_t* p = m->pin_dec;
   for (uint32_t i = 0; i < n; i++) {
     p[i] = tokens[i];
@@ -724,10 +728,10 @@ FC_API int fc_model_feed_batch(FcModel* m, uint32_t n, const uint32_t* stream_id
     m->pos[stream_ids[0]]++;
     return FC_OK;
   }
-  // One to eight streams: the whole step is one persistent kernel (decode_grid.cu).
-  if (decode_grid_ready(m, n)) {
-    uint32_t positions[8];
-    for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]];
+  // One to 64 streams: the whole step is one persistent kernel (decode_grid.cu).
+  uint32_t positions[64];
+  for (uint32_t i = 0; i < n && n <= 64; i++) positions[i] = m->pos[stream_ids[i]];
+  if (n <= 64 && decode_grid_takes(m, n, positions)) {
     FC_TRY(k_decode_grid(m, n, stream_ids, positions, tokens, nullptr));
     FC_TRY(finish_grid_steps(m, n, argmax_out, logits_out));
     for (uint32_t i = 0; i < n; i++) m->pos[stream_ids[i]]++;
@@ -876,11 +880,15 @@ FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream
     m->pos[stream_ids[0]] += steps - 1;
     return FC_OK;
   }
-  if (decode_grid_ready(m, n)) { // a launch per step, each taking the picks of the one before
-    uint32_t positions[8];
+  uint32_t positions[64];
+  for (uint32_t i = 0; i < n && n <= 64; i++) positions[i] = m->pos[stream_ids[i]] + steps / 2; // (half-way)
+  // (the first step may have gone the other way: the chain takes its picks from the host)
+  bool first = true;
+  if (n <= 64 && decode_grid_takes(m, n, positions)) { // a launch per step, each taking the picks of the one before
     for (uint32_t s = 1; s < steps; s++) {
       for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]] + s - 1;
-      FC_TRY(k_decode_grid(m, n, stream_ids, positions, nullptr, m->d_chain_log + (size_t)s * n));
+      FC_TRY(k_decode_grid(m, n, stream_ids, positions, first ? tokens_out : nullptr, m->d_chain_log + (size_t)s * n));
+      first = false;
     }
     if (steps > 2) // the log holds the tokens the steps consumed: the picks of steps 0 .. steps - 2
       FC_CUDA(dev, cudaMemcpyAsync(tokens_out + n, m->d_chain_log + 2 * (size_t)n, (size_t)(steps - 2) * n * 4, cudaMemcpyDeviceToHost, dev->stream));
@@ -894,9 +902,8 @@ FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream
       FC_TRY(fc_model_feed_batch(m, n, stream_ids, tokens_out + (size_t)(s - 1) * n, nullptr, tokens_out + (size_t)s * n));
     return FC_OK;
   }
-  // Steps 1 .. steps-1 run back to back on the device: d_ids / d_pos / d_streams still hold step 0's rows and
-  // d_argmax its picks; each further step starts with the link kernel instead of host copies, and the host
-  // waits once at the end.
+  // Steps 1 .. steps-1 run back to back on the device: d_pos / d_streams hold step 0's rows and d_argmax its picks;
+  // each further step starts with the link kernel instead of host copies, and the host waits once at the end.
   const bool fused_link = m->vocab <= 8192; // the link scans the logits row itself
   auto enqueue_link = [&]() -> int {
     if (fused_link)
@@ -917,6 +924,18 @@ FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream
     if (!fused_link) FC_TRY(k_argmax(dev, m->logits, n, m->vocab, m->d_argmax, m->argmax_scratch));
     return FC_OK;
   };
+  {
+    // (step 0 may have run as one kernel, which leaves these alone)
+    int32_t* p = m->pin_dec;
+    for (uint32_t i = 0; i < n; i++) {
+      p[i] = (int32_t)m->pos[stream_ids[i]] - 1;
+      p[n + i] = (int32_t)stream_ids[i];
+      p[2 * n + i] = tokens_out[i];
+    }
+    FC_CUDA(dev, cudaMemcpyAsync(m->d_pos, p, n * 4, cudaMemcpyHostToDevice, dev->stream));
+    FC_CUDA(dev, cudaMemcpyAsync(m->d_streams, p + n, n * 4, cudaMemcpyHostToDevice, dev->stream));
+    FC_CUDA(dev, cudaMemcpyAsync(m->d_argmax, p + 2 * n, n * 4, cudaMemcpyHostToDevice, dev->stream));
+  }
   if (m->chain_graphs.size() <= n) {
     m->chain_graphs.resize(n + 1, nullptr);
     m->chain_launches.resize(n + 1, 0);

@@ -73,7 +73,7 @@ struct FcModel {
   size_t pass_bytes = 0;  // bound of one scoring pass's workspace (fc_debug_score_pass_bytes; 0: the library's own)
   void* tc = nullptr; // state of the bf16 tensor-core path (built on first use)
   void* dc = nullptr; // state of the one-launch single-stream decode (decode_cluster.cu; probed on first use)
-  void* dg = nullptr; // state of the one-launch decode of one to eight streams (decode_grid.cu; probed on first use)
+  void* dg = nullptr; // state of the one-launch decode of one to 64 streams (decode_grid.cu; probed on first use)
 
   uint32_t qd() const { return heads * hd; }
   uint32_t kvd() const { return kv_heads * hd; }
@@ -116,10 +116,11 @@ int tc_check_errors(FcDevice* dev);
 bool decode_cluster_ready(FcModel* m);
 int k_decode_cluster(FcModel* m, uint32_t stream, uint32_t steps, bool chained);
 void decode_cluster_free(FcModel* m);
-// decode_grid.cu: one decode step of one to eight streams as one kernel. `tokens` null: the step continues the one before
+// decode_grid.cu: one decode step of one to 64 streams as one kernel. `tokens` null: the step continues the one before
 // it, whose picks are its tokens; `log` (device, nullable) receives the tokens the step consumed. The picks and, behind the
-// eighth, the status word of the step are at decode_grid_out (device).
-bool decode_grid_ready(FcModel* m, uint32_t rows);
+// 64th, the eight status words of the step are at decode_grid_out (device).
+bool decode_grid_ready(FcModel* m, uint32_t rows); // it can
+bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions); // and is the faster way
 int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint32_t* positions, const int32_t* tokens, int32_t* log);
 const int32_t* decode_grid_out(const FcModel* m);
 void decode_grid_free(FcModel* m);
