@@ -1,4 +1,4 @@
-// Decode step of one to 64 streams as ONE persistent kernel over all SMs: embedding, every layer (norm, q/k/v
+// Decode steps of one to 64 streams as ONE persistent kernel over all SMs, a chain of greedy ones without leaving it: embedding, every layer (norm, q/k/v
 // product, rotation and cache append, attention, output product, norm, gate/up or fc product, activation, down product),
 // final norm, head and the greedy pick. Op order of GpuLlama::feed / GpuGpt2::feed
 // (ferrum_wgpu/src/models/llama/forward.rs:L18-L72, models/gpt2.rs:L192-L265).
@@ -30,6 +30,9 @@
 // takes 6 cycles an instruction, whatever the number of warps (measured; 3 below). Hence one copy of the product for every
 // stage and of what it does, a kernel per (format, rows, architecture, heads of an item), and descriptors that spare address
 // arithmetic.
+//
+// A step of a chain ends like a grid barrier: the last CTA to arrive takes the picks and publishes them as tagged words, which
+// start the next step; by then every cache append of the step before is visible.
 //
 // A value is overwritten one layer later at the earliest; its writer then depends, through the tags, on every reader
 // of the old one having finished its stage. All CTAs are resident (cooperative launch) and every wait is bounded: one
@@ -105,10 +108,11 @@ struct DgArgs {
   int32_t* out;             // [64] picks, [8] the groups' status words
   float* logits;
   int* err_flag;
-  int32_t* log;             // where the consumed tokens go (nullable)
+  unsigned long long* toks; // tagged words: [64] the tokens of a chain's next step
+  int32_t* log;             // [step][row] the tokens that a chain consumes
   int32_t tok_in[64], pos[64], stream[64];
   uint32_t rows, group_rows, sub; // rows of a group, CTAs of a group
-  uint32_t chained, splits, item_heads, kv_log; // (2^kv_log K/V tiles in flight)
+  uint32_t steps, chained, splits, item_heads, kv_log; // (2^kv_log K/V tiles in flight)
   uint32_t off_desc, off_red, off_x, off_ys, off_kv, off_ring, ring_bytes;
 };
 
@@ -120,13 +124,14 @@ struct Misc { // small per-CTA state
   float slice[(ITEM_HEADS + 2) * 64]; // q heads (scaled), k, v of the attention item's own position
   float pw[AWARPS][8][ITEM_HEADS], cw[AWARPS][ITEM_HEADS];
   float wm[AWARPS][ITEM_HEADS], wl[AWARPS][ITEM_HEADS];
-  int32_t ids[8], pos[8], stream[8];
+  int32_t ids[8], next[8], pos[8], stream[8];
   uint32_t used[8];            // parts that a row's positions are in
   struct Item {
     uint32_t r, h0, kvh, s, c0, c1, append; // row, first head, split, its K/V tiles; whether it appends k and v to the cache
   } items[MAX_ITEMS];
   uint32_t n_items, tiles[5], first[5]; // the CTA's attention items; its tiles of qkv, wo, ff1, ff2, head: T = first, + grid, ..
-  int dead;
+  uint32_t planned, seen;      // steps whose items are there; steps whose items the producer has taken up
+  int dead, stop;
 };
 
 __device__ __forceinline__ unsigned long long ll_ld(const unsigned long long* p) {
@@ -424,17 +429,18 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     for (uint32_t i = 0; i < SLOTS; i++) tc::mbar_init(&ms.full[i], 1), tc::mbar_init(&ms.empty[i], 1);
 #pragma unroll 1
     for (uint32_t i = 0; i < MAX_KV; i++) tc::mbar_init(&ms.kv_full[i], 1), tc::mbar_init(&ms.kv_empty[i], AWARPS);
+    ms.planned = ms.seen = 0;
     tc::fence_barrier_init();
   }
   if (tid < (int)M) {
     ms.ids[tid] = a.chained ? *(volatile int32_t*)(a.out + r0 + tid) : a.tok_in[r0 + tid];
-    ms.pos[tid] = a.pos[r0 + tid], ms.stream[tid] = a.stream[r0 + tid];
+    ms.stream[tid] = a.stream[r0 + tid];
   }
   // (the descriptors are read at every stage: from global memory each would be a trip to L2 in the stage's chain)
 #pragma unroll 1
   for (uint32_t i = tid; i < a.n_layers * (uint32_t)(sizeof(DgLayer) / 8); i += THREADS)
     reinterpret_cast<uint64_t*>(layers)[i] = reinterpret_cast<const uint64_t*>(a.layers)[i];
-  const uint32_t tag0 = *(volatile uint32_t*)(a.state + 2 * grp) + 1; // (words start out as zeros: 0 is no tag)
+  uint32_t tag0 = *(volatile uint32_t*)(a.state + 2 * grp) + 1; // (words start out as zeros: 0 is no tag)
   // Tile T of a stage belongs to CTA (T + start) mod grid; the starts follow one another so that the small stages land on
   // different CTAs. wo and ff2 share theirs: the CTA of a tile keeps its rows of the residual stream.
   if (tid < 5) {
@@ -443,22 +449,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     const uint32_t T = cta >= start ? cta - start : cta + grid - start, n = tiles_of(a.sh[tid].n);
     ms.first[tid] = T;
     ms.tiles[tid] = T < n ? (n - T + grid - 1) / grid : 0u;
-  } else if (tid == 32) {
-    const uint32_t head_groups = a.heads / a.item_heads, group = a.heads / a.kv_heads;
-    uint32_t n = 0;
-#pragma unroll 1
-    for (uint32_t item = cta; item < M * head_groups * a.splits; item += grid) {
-      const uint32_t s = item % a.splits, hg = item / a.splits % head_groups, r = item / (a.splits * head_groups);
-      const uint32_t h0 = hg * a.item_heads, len = (uint32_t)a.pos[r0 + r] + 1;
-      uint32_t c0, c1, used;
-      item_range(len, a.splits, s, c0, c1, used);
-      // (one of the items that hold the row's own position appends it)
-      if (c0 < c1) ms.items[n++] = Misc::Item{r, h0, h0 / group, s, c0, c1, c1 * KV_POS >= len && h0 % group == 0};
-    }
-    ms.n_items = n;
-  } else if (tid >= 64 && tid < 64 + (int)M) {
-    uint32_t c0, c1;
-    item_range((uint32_t)a.pos[r0 + tid - 64] + 1, a.splits, 0, c0, c1, ms.used[tid - 64]);
   }
   __syncthreads();
 
@@ -475,9 +465,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
                    "r"(bytes), "r"(tc::smem_u32(bar))
                    : "memory");
     };
+    uint32_t n_items = 0;
     auto kv_tiles_of = [&](const DgLayer& L) {
 #pragma unroll 1
-      for (uint32_t i = 0; i < ms.n_items; i++) {
+      for (uint32_t i = 0; i < n_items; i++) {
         const Misc::Item& im = ms.items[i];
         const uint32_t len = (uint32_t)ms.pos[im.r] + 1;
         const size_t at = ((size_t)ms.stream[im.r] * a.kv_heads + im.kvh) * a.ctx * 64;
@@ -496,8 +487,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
         }
       }
     };
+    uint32_t step = 0, si = 0;
 #pragma unroll 1
-    for (uint32_t si = 0; si <= 4 * a.n_layers && on; si++) { // qkv, wo, ff1, ff2 of every layer, the head
+    for (; step < a.steps && on; si = si == 4 * a.n_layers ? 0 : si + 1, step += si == 0) { // qkv, wo, ff1, ff2 of every layer, the head
       const uint32_t mi = si == 4 * a.n_layers ? 4 : si & 3;
       const DgMat& W = mi == 4 ? a.head : layers[si >> 2].m[mi];
       const DgShape& sh = a.sh[mi];
@@ -546,6 +538,13 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
                          "l"(W.map_s), "r"(tc::smem_u32(bar)), "r"((int32_t)(c * sh.sc_pitch)), "r"((int32_t)(T * 16))
                          : "memory");
         }
+      if (si == 0 && on) { // (the items of a step, and the caches it reads, are there once its tokens are)
+        for (uint32_t tries = 1; *(volatile uint32_t*)&ms.planned <= step && !ctl.give_up(tries, 8); tries++) __nanosleep(20);
+        __threadfence_block();
+        n_items = *(volatile uint32_t*)&ms.n_items;
+        *(volatile uint32_t*)&ms.seen = step + 1;
+        asm volatile("fence.proxy.async;" ::: "memory");
+      }
       if (mi == 0 && on) kv_tiles_of(layers[si >> 2]);
     }
     // the CTA may not end under a copy in flight: the last use of every slot has landed
@@ -566,6 +565,47 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   // warp per tile, whose halves share the pieces; more: 16 MT threads per tile.
   const uint32_t ewarp = (uint32_t)(WARPS - 1 - warp), etid = ewarp * 32 + lane, e_row = lane & 15;
   const uint32_t e_ti = ONE ? ewarp : etid / PIECE, e_col = ONE ? 0 : (etid >> 4) & (MT - 1);
+  const int g = lane >> 2, t = lane & 3;
+  // Fragment row g is tile row rho: a row's 16-byte chunks are XORed with its low three bits, and the rows whose lanes read
+  // together are to differ where their chunks then do (one row, Q8_0: two rows, every second chunk; Q4_0: two rows, four
+  // neighbouring chunks; more rows, Q8_0: four rows, two neighbouring chunks; Q4_0: eight rows, one chunk).
+  const uint32_t rho = ONE ? (Q8 ? g : (g >> 1) | ((g & 1) << 2)) : (Q8 ? ((g & 3) << 1) | (g >> 2) : g);
+  uint32_t it = 0, kvn = 0, red_par = 0;
+#pragma unroll 1
+  for (uint32_t step = 0;; step++, tag0 += a.n_layers + 1) {
+  // The step's tokens (a chain's: picks of the step before), positions and attention items.
+  if (tid < (int)M) {
+    if (step) {
+      unsigned long long w;
+      uint32_t tries = 0;
+      do {
+        w = ll_ld(a.toks + r0 + tid);
+      } while (!ll_ok(w, tag0) && !ctl.give_up(++tries));
+      __threadfence();
+      ms.ids[tid] = ll_ok(w, tag0) ? (int32_t)(uint32_t)w : 0;
+    }
+    ms.pos[tid] = a.pos[r0 + tid] + step;
+    uint32_t c0, c1;
+    item_range((uint32_t)a.pos[r0 + tid] + step + 1, a.splits, 0, c0, c1, ms.used[tid]);
+  } else if (tid == 32) {
+    const uint32_t head_groups = a.heads / a.item_heads, group = a.heads / a.kv_heads;
+    uint32_t n = 0;
+#pragma unroll 1
+    for (uint32_t item = cta; item < M * head_groups * a.splits; item += grid) {
+      const uint32_t s = item % a.splits, hg = item / a.splits % head_groups, r = item / (a.splits * head_groups);
+      const uint32_t h0 = hg * a.item_heads, len = (uint32_t)a.pos[r0 + r] + step + 1;
+      uint32_t c0, c1, used;
+      item_range(len, a.splits, s, c0, c1, used);
+      // (one of the items that hold the row's own position appends it)
+      if (c0 < c1) ms.items[n++] = Misc::Item{r, h0, h0 / group, s, c0, c1, c1 * KV_POS >= len && h0 % group == 0};
+    }
+    ms.n_items = n;
+  }
+  cons_sync();
+  if (tid == 0) {
+    __threadfence_block();
+    *(volatile uint32_t*)&ms.planned = step + 1;
+  }
   // the embedding, by the CTAs that keep the residual stream: its words carry the tag before the first layer's
   static_assert(tile_group(MT) * (ONE ? 32 : PIECE) <= CONS, "a thread per result of a group");
 #pragma unroll 1
@@ -579,12 +619,6 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     }
   }
 
-  const int g = lane >> 2, t = lane & 3;
-  // Fragment row g is tile row rho: a row's 16-byte chunks are XORed with its low three bits, and the rows whose lanes read
-  // together are to differ where their chunks then do (one row, Q8_0: two rows, every second chunk; Q4_0: two rows, four
-  // neighbouring chunks; more rows, Q8_0: four rows, two neighbouring chunks; Q4_0: eight rows, one chunk).
-  const uint32_t rho = ONE ? (Q8 ? g : (g >> 1) | ((g & 1) << 2)) : (Q8 ? ((g & 3) << 1) | (g >> 2) : g);
-  uint32_t it = 0, kvn = 0, red_par = 0;
   unsigned long long best = 0; // head: the best (logit, index) of this thread's row
   uint32_t mi = 0, l = 0;      // matrix 0 .. 3 of layer l; 4: the head
 #pragma unroll 1
@@ -984,8 +1018,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
     best = ov > best ? ov : best;
   }
   if ((lane & (ONE ? 31 : 15)) == 0 && best && e_col < M) atomicMax(&a.keys[r0 + e_col], best);
+  asm volatile("fence.proxy.async;" ::: "memory"); // (the cache appends, which bulk copies will read)
   __threadfence();
   cons_sync();
+  const bool last = step + 1 == a.steps;
   if (tid == 0) {
     const uint32_t n = atomicAdd(&a.state[2 * grp + 1], 1u);
     if (n + 1 == grid) {
@@ -993,13 +1029,29 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
 #pragma unroll 1
       for (uint32_t r = 0; r < M; r++) {
         const unsigned long long key = atomicExch(&a.keys[r0 + r], 0ull);
-        if (a.log) a.log[r0 + r] = ms.ids[r];
-        a.out[r0 + r] = key ? (int32_t)(0xffffffffu - (uint32_t)key) : 0;
+        const uint32_t pick = key ? 0xffffffffu - (uint32_t)key : 0u;
+        if (a.log) a.log[(size_t)step * a.rows + r0 + r] = ms.ids[r];
+        if (last)
+          a.out[r0 + r] = (int32_t)pick;
+        else
+          ms.next[r] = (int32_t)pick;
       }
-      a.out[64 + grp] = *(volatile int*)a.err_flag;
       a.state[2 * grp + 1] = 0;
-      a.state[2 * grp] = tag0 + a.n_layers;
+      if (last) {
+        a.state[2 * grp] = tag0 + a.n_layers;
+        a.out[64 + grp] = *(volatile int*)a.err_flag;
+      }
+      __threadfence();
+      if (!last)
+#pragma unroll 1
+        for (uint32_t r = 0; r < M; r++) ll_st(a.toks + r0 + r, __int_as_float(ms.next[r]), tag0 + a.n_layers + 1);
     }
+    for (uint32_t tries = 1; *(volatile uint32_t*)&ms.seen <= step && !ctl.give_up(tries, 8); tries++) __nanosleep(20); // (at once)
+    ms.stop = last || *ctl.dead;
+    if (!last && ms.stop) a.out[64 + grp] = 1; // (this CTA does not go on, the others' waits will run out)
+  }
+  cons_sync();
+  if (ms.stop) return;
   }
 }
 
@@ -1008,7 +1060,7 @@ struct DgState {
   DgArgs args[4];              // for 1, 2, 4 and 8 padded rows
   void* d_layers = nullptr;    // the tensor maps and the layers' descriptors, for slots of 8 and of 4 lines
   void* words = nullptr;
-  uint64_t launches = 0;       // since the words were cleared
+  uint64_t tags = 0;           // used since the words were cleared
   int kind = 0;
 };
 
@@ -1132,7 +1184,7 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
   const uint32_t groups = (std::min<uint32_t>(8 * MAX_GROUPS, m->max_streams) + 7) / 8, rows_max = std::min<uint32_t>(8, m->max_streams);
   const size_t w_part = (size_t)grid * ITEM_HEADS * PART;
   const size_t g_words = rows_max * (m->qkv_w() + a.attn_stride + 2 * (size_t)a.x_stride + a.act_stride) + w_part;
-  const size_t n_words = groups * g_words + 64 + 8 + 40; // keys, state, out
+  const size_t n_words = groups * g_words + 64 + 64 + 8 + 40; // next tokens, keys, state, out
   // descriptors: per variant of the slots two tensor maps per matrix, then the layers
   const size_t n_mats = 4 * (size_t)m->n_layers + 1, maps_bytes = n_mats * 2 * sizeof(CUtensorMap);
   const size_t var_bytes = (maps_bytes + m->n_layers * sizeof(DgLayer) + 255) & ~(size_t)255;
@@ -1199,6 +1251,7 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
   a.b_act = w, w += rows_max * a.act_stride;
   a.b_qkv = w;
   w = (unsigned long long*)st->words + groups * g_words;
+  a.toks = w, w += 64;
   a.keys = w, w += 64;
   a.state = (uint32_t*)w, w += 8;
   a.out = (int32_t*)w;
@@ -1259,25 +1312,33 @@ bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions) {
 
 const int32_t* decode_grid_out(const FcModel* m) { return ((DgState*)m->dg)->args[0].out; }
 
-int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint32_t* positions, const int32_t* tokens, int32_t* log) {
+// After a step that reported a wait that gave up: as before the first one.
+int decode_grid_clear(FcModel* m) {
+  DgState* st = (DgState*)m->dg;
+  FC_CUDA(m->dev, cudaMemsetAsync(st->words, 0, (size_t)((uint8_t*)(st->args[0].out + 72) - (uint8_t*)st->words), m->dev->stream));
+  st->tags = 0;
+  return FC_OK;
+}
+
+int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint32_t* positions, const int32_t* tokens, uint32_t steps, int32_t* log) {
   DgState* st = (DgState*)m->dg;
   FcDevice* dev = m->dev;
-  if (st->launches >= (1ull << 31) / (m->n_layers + 1)) { // (before a tag could come round again)
+  st->tags += (uint64_t)steps * (m->n_layers + 1);
+  if (st->tags >= 1ull << 31) { // (before a tag could come round again)
     FC_CUDA(dev, cudaMemsetAsync(st->words, 0, (size_t)((uint8_t*)st->args[0].out - (uint8_t*)st->words), dev->stream));
-    st->launches = 0;
+    st->tags = (uint64_t)steps * (m->n_layers + 1);
   }
-  st->launches++;
   const int v = rows == 1 ? 0 : rows == 2 ? 1 : rows <= 4 ? 2 : 3;
   DgArgs a = st->args[v];
   const uint32_t groups = (rows + 7) / 8;
   a.rows = rows, a.group_rows = (rows + groups - 1) / groups, a.sub = group_ctas(m, rows);
-  a.chained = tokens ? 0 : 1, a.log = log;
+  a.steps = steps, a.chained = tokens ? 0 : 1, a.log = log;
   uint32_t longest = 1;
   for (uint32_t r = 0; r < rows; r++) {
     a.tok_in[r] = tokens ? tokens[r] : 0;
     a.pos[r] = (int32_t)positions[r];
     a.stream[r] = (int32_t)streams[r];
-    longest = std::max(longest, positions[r] + 1);
+    longest = std::max(longest, positions[r] + steps);
   }
   // Items: as few heads of a group each as the CTAs allow. A row's positions are split only where one CTA would work
   // through more than four 64-position tiles: the merge costs another trip through L2.

@@ -125,3 +125,24 @@ def test_a_step_reports_a_wait_that_gave_up_and_the_next_one_works(dev):
     assert g.pos() == 0
     assert np.array_equal(g.feed(3), want)
     g.close()
+
+
+@pytest.mark.parametrize("streams", [1, 3])
+def test_a_chain_over_two_launches_is_the_chain_in_pieces(dev, streams):
+    """A chain runs in the kernel for up to 256 steps; 300 of them against pieces of 1, 100 and 199, from other launches."""
+    cfg, _ = models(QKind.Q8_0)["group2"]
+    m = random_llama(cfg, seed=9, std=0.2)
+    g = CudaLlama(dev, m, QKind.Q8_0, max_streams=streams)
+    first = random_tokens(1, streams, cfg.vocab)
+    before = dev.launch_count()
+    whole = g.decode_greedy(first, 300)
+    assert dev.launch_count() - before == 3
+    for s in range(streams):
+        g.reset(s)
+    tok, parts = first, []
+    for n in (1, 100, 199):
+        parts.append(g.decode_greedy(tok, n))
+        tok = parts[-1][-1]
+    assert np.array_equal(np.concatenate(parts), whole)
+    assert all(g.pos(s) == 300 for s in range(streams))
+    g.close()
