@@ -533,12 +533,11 @@ int k_qgemm_tp(FcDevice* dev, const QMat& w, const __half* x, int epi, const TcA
     v.n = w.n - n0 < slice ? w.n - n0 : slice;
     v.qs = w.qs + qmat_qs_bytes(w.kind, w.k, n0);
     v.sc = (const __half*)((const uint8_t*)w.sc + qmat_sc_bytes(w.kind, w.k, n0));
-    const uint32_t bx = w.k / 16 < 64 ? 32 : 64; // (k is a multiple of 64: at least four threads per row)
-    const dim3 block(bx, 256 / bx), grid((w.k / 16 + bx - 1) / bx, (v.n + block.y - 1) / block.y < 65535 ? (v.n + block.y - 1) / block.y : 65535);
+    const uint32_t eights = (uint32_t)((size_t)v.n * w.k / 8), blocks = (eights + 256 * F16_ITEMS - 1) / (256 * F16_ITEMS); // (a slice: far below 2^32)
     if (w.kind == FC_Q8_0)
-      FC_LAUNCH(dev, "weights_f16", weights_f16_kernel<FC_Q8_0><<<grid, block, 0, dev->stream>>>(v, wf));
+      FC_LAUNCH(dev, "weights_f16", weights_f16_kernel<FC_Q8_0><<<blocks, 256, 0, dev->stream>>>(v, eights, wf));
     else
-      FC_LAUNCH(dev, "weights_f16", weights_f16_kernel<FC_Q4_0><<<grid, block, 0, dev->stream>>>(v, wf));
+      FC_LAUNCH(dev, "weights_f16", weights_f16_kernel<FC_Q4_0><<<blocks, 256, 0, dev->stream>>>(v, eights, wf));
     FC_TRY(half_map(dev, &tw, wf, v.n, w.k, 128));
     TcArgs a = args;
     a.n = v.n;
@@ -652,8 +651,8 @@ int k_qgemm_tx(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl,
 // Whether decoding the weights first pays, by the estimated time of both in ns. Constants measured on K 768..4096 x
 // N 768..32000, 128..16384 rows: a K step of a 128 x 192 tile with in-kernel decoding takes 395 (Q4_0) or 530 (Q8_0: a
 // thread reads twice the bytes), of a 256 x 256 pair tile 415, a tile's own overhead about 800; the decoding pass costs a
-// launch and 1.1 (Q4_0) or 0.65 ps per weight; neither form writes more than 2.65 TB/s. (4096 rows of 4096 x 11008 Q8_0:
-// 464 us with in-kernel decoding, 330 decoded first; 256 rows: 71 and 94.)
+// launch and 0.63 (Q4_0) or 0.65 ps per weight; neither form writes more than 2.65 TB/s. (4096 rows of 4096 x 11008 Q8_0:
+// 464 us with in-kernel decoding, 326 decoded first; 256 rows: 71 and 94.)
 bool tp_takes(const FcDevice* dev, const QMat& w, uint32_t m, int epi) {
   if ((w.kind != FC_Q8_0 && w.kind != FC_Q4_0) || w.k % TC_BK || !m) return false;
   const bool q8 = w.kind == FC_Q8_0;
@@ -670,7 +669,7 @@ bool tp_takes(const FcDevice* dev, const QMat& w, uint32_t m, int epi) {
   const uint64_t out_bytes = (uint64_t)m * w.n * (epi == EPI_LSE ? 0 : epi == EPI_SWIGLU ? 1 : epi == EPI_F16 ? 2 : 4);
   const uint64_t store = out_bytes / 2650;
   ts = ts > store ? ts : store;
-  tp = (tp > store ? tp : store) + launches * 4000 + (uint64_t)w.n * w.k / (q8 ? 1540 : 910);
+  tp = (tp > store ? tp : store) + launches * 4000 + (uint64_t)w.n * w.k / (q8 ? 1540 : 1600);
   return tp < ts;
 }
 size_t tp_workspace_bytes(const QMat& w) { return (size_t)tp_slice_rows(w) * w.k * 2; }

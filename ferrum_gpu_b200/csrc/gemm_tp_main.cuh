@@ -22,37 +22,45 @@
 // acc_empty[b] (leader: 16 epilogue warps). Two accumulator buffers of 256 columns: the epilogue of a tile runs under
 // the next tile's main loop. Every wait is bounded and polls the CTA's abort word.
 
-// Packed rows -> fp16(d q), one rounding: the bits the other kernels' dequantisers produce. A thread decodes half a block
-// (16 weights: 8 or 16 bytes in, two 16-byte stores out, whole sectors); a row's threads are consecutive.
+// Packed rows -> fp16(d q), one rounding: the bits the other kernels' dequantisers produce. Bound by memory: per weight two
+// bytes out and a half or one in. Rows, scales and result lie one behind the other, so the matrix is one run of eights
+// (n k / 8 of them); a thread takes F16_ITEMS eights, 256 apart - all its loads first, every store instruction of a warp 512
+// consecutive bytes. (One half-block per thread and row: as many blocks of one load each, 72 us for the 65 M weights of
+// 32000 x 2048 Q4_0.)
+constexpr int F16_ITEMS = 8;
 template <int KIND>
-__global__ void __launch_bounds__(256) weights_f16_kernel(QMat w, __half* __restrict__ out) {
-  const uint32_t halves = w.k / 16, c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= halves) return;
-  for (uint32_t n = blockIdx.y * blockDim.y + threadIdx.y; n < w.n; n += gridDim.y * blockDim.y) {
-    const uint32_t dd = (uint32_t)__half_as_ushort(w.sc[(size_t)n * (w.k / QK) + c / 2]) * 0x00010001u;
-    uint4 o[2];
+__global__ void __launch_bounds__(256) weights_f16_kernel(QMat w, uint32_t eights, __half* __restrict__ out) {
+  const uint32_t base = blockIdx.x * (256 * F16_ITEMS) + threadIdx.x;
+  uint2 q[F16_ITEMS];
+  uint32_t dd[F16_ITEMS];
+#pragma unroll
+  for (int i = 0; i < F16_ITEMS; i++) {
+    const uint32_t e = min(base + i * 256, eights - 1);
+    if (KIND == FC_Q8_0)
+      q[i] = *reinterpret_cast<const uint2*>(w.qs + (size_t)e * 8);
+    else
+      q[i].x = *reinterpret_cast<const uint32_t*>(w.qs + (size_t)e * 4);
+    dd[i] = (uint32_t)__half_as_ushort(w.sc[e / 4]);
+  }
+#pragma unroll
+  for (int i = 0; i < F16_ITEMS; i++) {
+    const uint32_t d = dd[i] * 0x00010001u;
+    uint4 o;
     if (KIND == FC_Q8_0) {
-      const uint4 q = *reinterpret_cast<const uint4*>(w.qs + (size_t)n * w.k + (size_t)c * 16);
-      auto four = [&](uint32_t v, uint32_t& a, uint32_t& b) {
-        const uint32_t u = v ^ 0x80808080u;
-        a = f16x2_mul(f16x2_sub(__byte_perm(u, 0x64646464u, 0x5140), 0x64806480u), dd);
-        b = f16x2_mul(f16x2_sub(__byte_perm(u, 0x64646464u, 0x5342), 0x64806480u), dd);
-      };
-      four(q.x, o[0].x, o[0].y), four(q.y, o[0].z, o[0].w);
-      four(q.z, o[1].x, o[1].y), four(q.w, o[1].z, o[1].w);
+      const uint32_t u = q[i].x ^ 0x80808080u, v = q[i].y ^ 0x80808080u;
+      o.x = f16x2_mul(f16x2_sub(__byte_perm(u, 0x64646464u, 0x5140), 0x64806480u), d);
+      o.y = f16x2_mul(f16x2_sub(__byte_perm(u, 0x64646464u, 0x5342), 0x64806480u), d);
+      o.z = f16x2_mul(f16x2_sub(__byte_perm(v, 0x64646464u, 0x5140), 0x64806480u), d);
+      o.w = f16x2_mul(f16x2_sub(__byte_perm(v, 0x64646464u, 0x5342), 0x64806480u), d);
     } else {
-      const uint2 q = *reinterpret_cast<const uint2*>(w.qs + (size_t)n * (w.k / 2) + (size_t)c * 8);
-      auto eight = [&](uint32_t v, uint4& a) {
-        const uint32_t v8 = v >> 8;
-        a.x = f16x2_mul(f16x2_sub((v & 0x000f000fu) | 0x64006400u, 0x64086408u), dd);
-        a.y = f16x2_mul(f16x2_sub((v & 0x00f000f0u) | 0x54005400u, 0x54805480u), dd);
-        a.z = f16x2_mul(f16x2_sub((v8 & 0x000f000fu) | 0x64006400u, 0x64086408u), dd);
-        a.w = f16x2_mul(f16x2_sub((v8 & 0x00f000f0u) | 0x54005400u, 0x54805480u), dd);
-      };
-      eight(q.x, o[0]), eight(q.y, o[1]);
+      const uint32_t v = q[i].x, v8 = v >> 8;
+      o.x = f16x2_mul(f16x2_sub((v & 0x000f000fu) | 0x64006400u, 0x64086408u), d);
+      o.y = f16x2_mul(f16x2_sub((v & 0x00f000f0u) | 0x54005400u, 0x54805480u), d);
+      o.z = f16x2_mul(f16x2_sub((v8 & 0x000f000fu) | 0x64006400u, 0x64086408u), d);
+      o.w = f16x2_mul(f16x2_sub((v8 & 0x00f000f0u) | 0x54005400u, 0x54805480u), d);
     }
-    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)n * w.k + (size_t)c * 16);
-    dst[0] = o[0], dst[1] = o[1];
+    const uint32_t e = base + i * 256;
+    if (e < eights) reinterpret_cast<uint4*>(out)[e] = o;
   }
 }
 
