@@ -92,6 +92,26 @@ int fc_post_launch(FcDevice* dev, const char* what);
     FC_TRY(fc_post_launch((dev), (what))); \
   } while (0)
 
+#ifdef __CUDACC__
+// A launch on the device's stream; `early`: it may begin while the kernel before it ends (programmatic dependent launch).
+// The kernel then has to wait (grid_wait) before it reads what other kernels write, or writes what they read; with that
+// first in every kernel of a chain, each begins its waiting while the one before it still works.
+template <typename... P, typename... A>
+void launch_on(FcDevice* dev, bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = dev->stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at, cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#endif
+
 // A kernel's attributes (dynamic shared memory limit) are set per device: a once-flag per device ordinal, one
 // static instance per kernel instantiation.
 struct OncePerDevice {

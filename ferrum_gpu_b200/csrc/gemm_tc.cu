@@ -573,13 +573,13 @@ int k_qgemm_tp(FcDevice* dev, const QMat& w, const __half* x, int epi, const TcA
 
 template <int KIND>
 int launch_tx(FcDevice* dev, const CUtensorMap& txh, const CUtensorMap& txl, const CUtensorMap& tq, const CUtensorMap& tsc,
-              const TxArgs& a, dim3 grid) {
+              const TxArgs& a, dim3 grid, bool early) {
   auto kern = qgemm_tx_kernel<KIND>;
   static OncePerDevice attr;
   if (attr.first(dev->ordinal)) {
     FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TX_SMEM_BYTES));
   }
-  FC_LAUNCH(dev, "qgemm_tx", kern<<<grid, TX_THREADS, TX_SMEM_BYTES, dev->stream>>>(txh, txl, tq, tsc, a));
+  FC_LAUNCH(dev, "qgemm_tx", launch_on(dev, early, kern, grid, TX_THREADS, TX_SMEM_BYTES, txh, txl, tq, tsc, a));
   return FC_OK;
 }
 
@@ -644,8 +644,8 @@ int k_qgemm_tx(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl,
   a.m = m, a.n = w.n, a.k = w.k, a.y = y, a.bias = ep.bias, a.resid = ep.resid, a.act = ep.act, a.err_flag = dev->d_flag;
   const uint32_t tiles = (w.n + TC_BN - 1) / TC_BN, sms = (uint32_t)dev->prop.multiProcessorCount;
   dim3 grid(tiles < sms ? tiles : sms);
-  if (q8) return launch_tx<FC_Q8_0>(dev, maps[0], maps[1], tq, tsc, a, grid);
-  return launch_tx<FC_Q4_0>(dev, maps[0], maps[1], tq, tsc, a, grid);
+  if (q8) return launch_tx<FC_Q8_0>(dev, maps[0], maps[1], tq, tsc, a, grid, ep.ragged);
+  return launch_tx<FC_Q4_0>(dev, maps[0], maps[1], tq, tsc, a, grid, ep.ragged);
 }
 
 // Whether decoding the weights first pays, by the estimated time of both in ns. Constants measured on K 768..4096 x

@@ -162,6 +162,7 @@ __global__ void __launch_bounds__(TX_THREADS, 1)
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_wait(); // (everything above touches only this CTA's own memory)
 
   if (warp < 4) {
     if (warp == 0) {

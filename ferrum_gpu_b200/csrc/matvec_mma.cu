@@ -51,6 +51,7 @@ __device__ __forceinline__ float gelu_f(float x) {
 // x[m][k] f32 -> hi, lo fp16 [mp][k] (rows >= m are zero)
 __global__ void x_split_kernel(const float* __restrict__ x, uint32_t m, uint32_t mp, uint32_t k, __half* __restrict__ xh,
                                __half* __restrict__ xl) {
+  grid_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)mp * k) return;
   const uint32_t r = (uint32_t)(i / k);
@@ -238,6 +239,7 @@ template <int KIND, int NB, int RW, bool RAGGED>
 __global__ void __launch_bounds__(128)
     qmatvec_mma_kernel(QMat w, const __half* __restrict__ xh, const __half* __restrict__ xl, uint32_t m, float* __restrict__ y,
                        float* __restrict__ partial, uint32_t blocks_per_split, Epilogue ep) {
+  grid_wait();
   extern __shared__ __align__(16) __half xs[];
   constexpr int MP = NB * 8;
   constexpr int XROW = XS;            // halves per staged row
@@ -410,6 +412,7 @@ template <int KIND, bool RAGGED>
 __global__ void __launch_bounds__(128)
     qmatvec_mma8_kernel(QMat w, const float* __restrict__ x, uint32_t m, float* __restrict__ y, float* __restrict__ partial,
                         uint32_t blocks_per_split, Epilogue ep) {
+  grid_wait();
   using C = Mma8<KIND>;
   extern __shared__ __align__(16) uint8_t sm8[];
   uint8_t* wq = sm8;
@@ -657,6 +660,7 @@ __global__ void __launch_bounds__(128)
 template <int KIND>
 __global__ void ragged_reduce_kernel(const float* __restrict__ partial, uint32_t splits, uint32_t m, QMat w, const float* __restrict__ x,
                                      const float* __restrict__ x_scale, float* __restrict__ y, const float* __restrict__ bias) {
+  grid_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)m * w.n) return;
   float v = 0.0f;
@@ -671,6 +675,7 @@ __global__ void ragged_reduce_kernel(const float* __restrict__ partial, uint32_t
 // y = epilogue(sum over splits, ascending split index)
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, uint32_t splits, uint32_t m, uint32_t n,
                                      float* __restrict__ y, Epilogue ep) {
+  grid_wait();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)m * n) return;
   float v = 0.0f;
@@ -692,7 +697,7 @@ int launch(FcDevice* dev, const QMat& w, const __half* xh, const __half* xl, uin
     FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
   dim3 grid((w.n + ROWS_PER_CTA * RW - 1) / (ROWS_PER_CTA * RW), splits);
-  FC_LAUNCH(dev, "qmatvec_mma", kern<<<grid, 128, smem, dev->stream>>>(w, xh, xl, m, y, partial, bps, ep));
+  FC_LAUNCH(dev, "qmatvec_mma", launch_on(dev, ep.ragged, kern, grid, 128, smem, w, xh, xl, m, y, partial, bps, ep));
   return FC_OK;
 }
 
@@ -731,7 +736,7 @@ int ragged_reduce(FcDevice* dev, const QMat& w, const float* x, uint32_t m, cons
   if (ep.act != ACT_NONE || ep.resid) return fc_fail(dev, FC_ERR_ARG, "a product of a ragged width stands alone");
   const size_t tot = (size_t)m * w.n;
   FC_LAUNCH(dev, "splitk_reduce",
-            ragged_reduce_kernel<KIND><<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w, x, x_scale, y, ep.bias));
+            launch_on(dev, ep.ragged, ragged_reduce_kernel<KIND>, (unsigned)((tot + 255) / 256), 256, 0, partial, splits, m, w, x, x_scale, y, ep.bias));
   return FC_OK;
 }
 int pick_ragged_reduce(FcDevice* dev, const QMat& w, const float* x, uint32_t m, const float* partial, uint32_t splits, const float* x_scale,
@@ -751,7 +756,7 @@ int launch_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t m, float*
   auto kern = qmatvec_mma8_kernel<KIND, RAGGED>;
   static OncePerDevice attr;
   if (attr.first(dev->ordinal)) FC_CUDA(dev, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Mma8<KIND>::SMEM));
-  FC_LAUNCH(dev, "qmatvec_mma8", kern<<<grid, 128, Mma8<KIND>::SMEM, dev->stream>>>(w, x, m, y, part, bps, ep));
+  FC_LAUNCH(dev, "qmatvec_mma8", launch_on(dev, ep.ragged, kern, grid, 128, Mma8<KIND>::SMEM, w, x, m, y, part, bps, ep));
   return FC_OK;
 }
 template <bool RAGGED>
@@ -817,7 +822,7 @@ static int k_qmatvec_mma8(FcDevice* dev, const QMat& w, const float* x, uint32_t
   if (splits > 1) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
-              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep));
+              launch_on(dev, ep.ragged, splitk_reduce_kernel, (unsigned)((tot + 255) / 256), 256, 0, partial, splits, m, w.n, y, ep));
   }
   return FC_OK;
 }
@@ -878,7 +883,7 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
     FC_LAUNCH(dev, "norm_split",
               norm_split_kernel<<<mp, 256, 0, dev->stream>>>(x, m, w.k, ep.norm, ep.norm_g, ep.norm_b, ep.norm_eps, xh, xl, pend, nullptr));
   else
-    FC_LAUNCH(dev, "x_split", x_split_kernel<<<(unsigned)((total + 255) / 256), 256, 0, dev->stream>>>(x, m, mp, w.k, xh, xl));
+    FC_LAUNCH(dev, "x_split", launch_on(dev, ep.ragged, x_split_kernel, (unsigned)((total + 255) / 256), 256, 0, x, m, mp, w.k, xh, xl));
   if (tx) return k_qgemm_tx(dev, w, xh, xl, mp, m, y, ep);
   // split K until the grid covers the SMs about twice: whole 128-k slices per split, the last split may be
   // shorter (K = 2816 is 22 slices: 11 splits of 2, where a power-of-two rule stops at 2 splits of 11)
@@ -907,7 +912,7 @@ int k_qmatvec_mma(FcDevice* dev, const QMat& w, const float* x, uint32_t m, floa
   if (part) {
     const size_t tot = (size_t)m * w.n;
     FC_LAUNCH(dev, "splitk_reduce",
-              splitk_reduce_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, dev->stream>>>(partial, splits, m, w.n, y, ep));
+              launch_on(dev, ep.ragged, splitk_reduce_kernel, (unsigned)((tot + 255) / 256), 256, 0, partial, splits, m, w.n, y, ep));
   }
   return FC_OK;
 }
