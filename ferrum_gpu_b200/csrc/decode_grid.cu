@@ -34,8 +34,9 @@
 // A step of a chain ends like a grid barrier: the last CTA to arrive takes the picks and publishes them as tagged words, which
 // start the next step; by then every cache append of the step before is visible.
 //
-// A value is overwritten one layer later at the earliest; its writer then depends, through the tags, on every reader
-// of the old one having finished its stage. All CTAs are resident (cooperative launch) and every wait is bounded: one
+// A value is overwritten one layer later at the earliest (a token one step later); its writer then depends, through the tags,
+// on every reader of the old one having finished its stage. A word belongs to one group of CTAs for good: tags count per group,
+// and only one that never comes round again tells a word from what an earlier launch left there. All CTAs are resident (cooperative launch) and every wait is bounded: one
 // that gives up raises the device's status word, everybody's waits end at once, and the step reports it.
 #include <algorithm>
 #include <cstring>
@@ -108,7 +109,9 @@ struct DgArgs {
   int32_t* out;             // [64] picks, [8] the groups' status words
   float* logits;
   int* err_flag;
-  unsigned long long* toks; // tagged words: [64] the tokens of a chain's next step
+  // tagged words: [group][8] the tokens of a chain's next step. By group and not by row of the batch: tags count per group, and
+  // the group of a row depends on how many rows there are (row 5 of 8 is in group 0, of 10 in group 1).
+  unsigned long long* toks;
   int32_t* log;             // [step][row] the tokens that a chain consumes
   int32_t tok_in[64], pos[64], stream[64];
   uint32_t rows, group_rows, sub; // rows of a group, CTAs of a group
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
       unsigned long long w;
       uint32_t tries = 0;
       do {
-        w = ll_ld(a.toks + r0 + tid);
+        w = ll_ld(a.toks + grp * 8 + tid);
       } while (!ll_ok(w, tag0) && !ctl.give_up(++tries));
       __threadfence();
       ms.ids[tid] = ll_ok(w, tag0) ? (int32_t)(uint32_t)w : 0;
@@ -1044,7 +1047,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
       __threadfence();
       if (!last)
 #pragma unroll 1
-        for (uint32_t r = 0; r < M; r++) ll_st(a.toks + r0 + r, __int_as_float(ms.next[r]), tag0 + a.n_layers + 1);
+        for (uint32_t r = 0; r < M; r++) ll_st(a.toks + grp * 8 + r, __int_as_float(ms.next[r]), tag0 + a.n_layers + 1);
     }
     for (uint32_t tries = 1; *(volatile uint32_t*)&ms.seen <= step && !ctl.give_up(tries, 8); tries++) __nanosleep(20); // (at once)
     ms.stop = last || *ctl.dead;

@@ -1,0 +1,47 @@
+"""Chains of greedy steps in the one-kernel decode (csrc/decode_grid.cu) when the number of streams changes between them: which
+group of rows a stream belongs to depends on how many there are, so what one call left behind must mean nothing to the next."""
+import random
+
+import numpy as np
+import pytest
+
+from ferrum_gpu_b200 import CudaLlama, QKind
+from ferrum_gpu_b200.hostmodel import LlamaConfig, random_llama, random_tokens
+
+pytestmark = pytest.mark.gpu
+
+CFG = LlamaConfig(vocab=1000, ctx=64, dim=256, heads=4, kv_heads=2, head_dim=64, layers=2, hidden=256, rope_dim=64)
+
+
+def drawn(seed, calls):
+    rng = random.Random(seed)
+    return [(rng.randint(1, 24), rng.randint(1, 16)) for _ in range(calls)]
+
+
+# (streams, steps) of every call. Tags advance by three (layers + 1) a step: in the first two the second call waits for a tag
+# that the first one left at the rows of another group; among the drawn ones three calls do.
+@pytest.mark.parametrize("calls", [[(8, 3), (10, 3)], [(16, 3), (17, 3)], [(8, 3), (9, 4), (20, 3), (17, 5)], drawn(14, 60)],
+                         ids=["8_10", "16_17", "8_9_20_17", "drawn"])
+def test_chains_of_changing_widths_are_their_steps(dev, calls):
+    m = random_llama(CFG, seed=9, std=0.2)
+    g = CudaLlama(dev, m, QKind.Q8_0, max_streams=24)
+    ref = CudaLlama(dev, m, QKind.Q8_0, max_streams=24)
+    for i, (streams, steps) in enumerate(calls):
+        first = random_tokens(100 + i, streams, CFG.vocab)
+        for s in range(streams):
+            g.reset(s)
+            ref.reset(s)
+        slots = list(range(streams))
+        before = dev.launch_count()
+        got = g.decode_greedy(first, steps, streams=slots)
+        assert dev.launch_count() - before == min(steps, 2), "the one-kernel route"
+        tok = first
+        for step in range(steps):
+            tok, _ = ref.feed_batch(tok, streams=slots)
+            assert np.array_equal(tok, got[step]), (i, streams, step)
+        # the caches that both left behind
+        _, a = g.feed_batch(tok, streams=slots, want_logits=True)
+        _, b = ref.feed_batch(tok, streams=slots, want_logits=True)
+        assert np.array_equal(a, b), (i, streams)
+    g.close()
+    ref.close()
