@@ -133,7 +133,7 @@ struct Misc { // small per-CTA state
     uint32_t r, h0, kvh, s, c0, c1, append; // row, first head, split, its K/V tiles; whether it appends k and v to the cache
   } items[MAX_ITEMS];
   uint32_t n_items, tiles[5], first[5]; // the CTA's attention items; its tiles of qkv, wo, ff1, ff2, head: T = first, + grid, ..
-  uint32_t planned, seen;      // steps whose items are there; steps whose items the producer has taken up
+  uint32_t planned, seen;      // steps whose items and positions are there; steps whose the producer has no more use for
   int dead, stop;
 };
 
@@ -545,10 +545,15 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
         for (uint32_t tries = 1; *(volatile uint32_t*)&ms.planned <= step && !ctl.give_up(tries, 8); tries++) __nanosleep(20);
         __threadfence_block();
         n_items = *(volatile uint32_t*)&ms.n_items;
-        *(volatile uint32_t*)&ms.seen = step + 1;
         asm volatile("fence.proxy.async;" ::: "memory");
       }
-      if (mi == 0 && on) kv_tiles_of(layers[si >> 2]);
+      if (mi == 0 && on) {
+        kv_tiles_of(layers[si >> 2]);
+        if (on && (si >> 2) + 1 == a.n_layers) { // (behind the last read of the step's items: the consumers write the next step's over them)
+          __threadfence_block();
+          *(volatile uint32_t*)&ms.seen = step + 1;
+        }
+      }
     }
     // the CTA may not end under a copy in flight: the last use of every slot has landed
 #pragma unroll 1

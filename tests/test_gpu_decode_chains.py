@@ -45,3 +45,29 @@ def test_chains_of_changing_widths_are_their_steps(dev, calls):
         assert np.array_equal(a, b), (i, streams)
     g.close()
     ref.close()
+
+
+@pytest.mark.parametrize("kind", [QKind.Q8_0, QKind.Q4_0])
+def test_a_chain_where_most_ctas_have_attention_and_nothing_after_it(dev, kind):
+    """48 heads of one or three streams are 48 or 144 attention items, and everything behind them 65 tiles of a few
+    CTAs: the others go from a step's last item straight to the next step's plan, which lies where their copies' was."""
+    cfg = LlamaConfig(vocab=16, ctx=320, dim=256, heads=48, kv_heads=48, head_dim=64, layers=1, hidden=256, rope_dim=64)
+    m = random_llama(cfg, seed=3, std=0.3)
+    g = CudaLlama(dev, m, kind, max_streams=3)
+    ref = CudaLlama(dev, m, kind, max_streams=3)
+    for streams in (1, 3):
+        slots = list(range(streams))
+        first = random_tokens(5, streams, cfg.vocab)
+        for s in slots:
+            g.reset(s)
+            ref.reset(s)
+        got = g.decode_greedy(first, 240, streams=slots)
+        tok = first
+        for step in range(240):
+            tok, _ = ref.feed_batch(tok, streams=slots)
+            assert np.array_equal(tok, got[step]), (streams, step)
+        _, a = g.feed_batch(tok, streams=slots, want_logits=True)
+        _, b = ref.feed_batch(tok, streams=slots, want_logits=True)
+        assert np.array_equal(a, b)
+    g.close()
+    ref.close()
