@@ -1027,10 +1027,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   }
   if ((lane & (ONE ? 31 : 15)) == 0 && best && e_col < M) atomicMax(&a.keys[r0 + e_col], best);
   asm volatile("fence.proxy.async;" ::: "memory"); // (the cache appends, which bulk copies will read)
-  __threadfence();
   cons_sync();
   const bool last = step + 1 == a.steps;
   if (tid == 0) {
+    __threadfence(); // (behind the barrier: it orders what every thread of the CTA wrote before the count)
     const uint32_t n = atomicAdd(&a.state[2 * grp + 1], 1u);
     if (n + 1 == grid) {
       __threadfence();
