@@ -208,7 +208,9 @@ __device__ __forceinline__ void codes8(uint32_t w, uint32_t w2, uint32_t (&p)[4]
   }
 }
 
-// Bounded waits that end early once somebody in the CTA gave up; other CTAs run into their own limit at about the same time.
+// Bounded waits that end early once somebody in the CTA gave up; other CTAs run into their own limit at about the same time. Who
+// gave up goes on with whatever is there: values may be anything, addresses may not come from words that the wait vouches for.
+// (Nor does a barrier's parity vouch for them then: a whole ring past the producer it counts as complete.)
 struct Ctl {
   volatile int* dead;
   int* err;
@@ -429,7 +431,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   if (tid == 0) {
     ms.dead = *(volatile int*)a.err_flag != 0; // an earlier launch gave up: do not wait again
 #pragma unroll 1
-    for (uint32_t i = 0; i < SLOTS; i++) tc::mbar_init(&ms.full[i], 1), tc::mbar_init(&ms.empty[i], 1);
+    for (uint32_t i = 0; i < SLOTS; i++) tc::mbar_init(&ms.full[i], 1), tc::mbar_init(&ms.empty[i], 1), ms.slot_at[i] = 0;
 #pragma unroll 1
     for (uint32_t i = 0; i < MAX_KV; i++) tc::mbar_init(&ms.kv_full[i], 1), tc::mbar_init(&ms.kv_empty[i], AWARPS);
     ms.planned = ms.seen = 0;
@@ -544,7 +546,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
       if (si == 0 && on) { // (the items of a step, and the caches it reads, are there once its tokens are)
         for (uint32_t tries = 1; *(volatile uint32_t*)&ms.planned <= step && !ctl.give_up(tries, 8); tries++) __nanosleep(20);
         __threadfence_block();
-        n_items = *(volatile uint32_t*)&ms.n_items;
+        // (no plan: somebody gave up before there was one, and what lies in its place is anything)
+        on = *(volatile uint32_t*)&ms.planned > step && *ctl.dead == 0;
+        n_items = on ? *(volatile uint32_t*)&ms.n_items : 0;
         asm volatile("fence.proxy.async;" ::: "memory");
       }
       if (mi == 0 && on) {
@@ -660,7 +664,8 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
           if (works) {
             const uint32_t c = kg / UPC, si = it + u_ti * sh.nch + c, b0 = (kg - c * UPC) * 4; // (first block, within the slot)
             ctl.mbar(&ms.full[si % SLOTS], (si / SLOTS) & 1);
-            const uint8_t* slot = ring + ms.slot_at[si % SLOTS];
+            // (once somebody gave up, the place may be that of an earlier, smaller slot, or the first zero: inside the ring either way)
+            const uint8_t* slot = ring + min(ms.slot_at[si % SLOTS], a.ring_bytes - sh.size);
             const uint32_t sc_pitch = sh.sc_pitch;
             const __half* sp = reinterpret_cast<const __half*>(slot + sh.sc_off) + rho * sc_pitch + b0;
             const uint8_t* wp = slot + (b0 / (128 / BLK)) * 2048 + rho * 128; // the unit's line (Q4_0: half a line) of row rho

@@ -681,7 +681,8 @@ static int finish_grid_steps(FcModel* m, uint32_t n, int32_t* picks, float* logi
   for (int i = 64; i < 72; i++)
     if (p[i]) {
       FC_TRY(decode_grid_clear(m));
-      return tc_check_errors(dev);
+      FC_TRY(tc_check_errors(dev));
+      return fc_fail(dev, FC_ERR_TIMEOUT, "a decode step gave up a bounded wait"); // (its status was read elsewhere already)
     }
   if (picks) memcpy(picks, p, (size_t)n * 4);
   return FC_OK;
