@@ -1068,8 +1068,10 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
   }
 }
 
+enum { DG_UNTRIED, DG_READY, DG_NO_ROOM, DG_UNFIT };
 struct DgState {
-  bool ok = false;
+  int set_up = DG_UNTRIED;
+  uint32_t asked = 0, retry = 64; // without room: questions since the last try, and after how many the next one is
   DgArgs args[4];              // for 1, 2, 4 and 8 padded rows
   void* d_layers = nullptr;    // the tensor maps and the layers' descriptors, for slots of 8 and of 4 lines
   void* words = nullptr;
@@ -1152,20 +1154,11 @@ static uint32_t group_ctas(const FcModel* m, uint32_t rows) {
   return (uint32_t)m->dev->prop.multiProcessorCount / ((rows + 7) / 8);
 }
 
-// Whether a step of `rows` rows can run as this kernel, and the set-up on first use.
-bool decode_grid_ready(FcModel* m, uint32_t rows) {
-  if (rows == 0 || rows > 8 * MAX_GROUPS || m->n_shards != 1) return false;
-  if (m->dg) {
-    const uint32_t sub = group_ctas(m, rows), group_rows = std::min(rows, 8u);
-    // (LayerNorm keeps its input in registers: two 256-element parts per warp)
-    return ((DgState*)m->dg)->ok && (m->arch == ARCH_LLAMA || group_rows * ((m->dim + 255) / 256) <= 2 * WARPS) &&
-           (m->dim + 15) / 16 <= MAX_RESID * sub && group_rows * m->heads <= MAX_ITEMS * sub;
-  }
-  DgState* st = new DgState();
-  m->dg = st;
+// The set-up. On failure the caller frees what it had taken.
+static int decode_grid_set_up(FcModel* m, DgState* st) {
   const int kind = m->head.w->m.kind;
   const bool q8 = kind == FC_Q8_0;
-  if (!q8 && kind != FC_Q4_0) return false;
+  if (!q8 && kind != FC_Q4_0) return DG_UNFIT;
   auto mat_ok = [&](const Linear& l) {
     const QMat& q = l.w->m;
     if (q.kind != kind || q.k % (q8 ? 128 : 256) || q.k > MAX_K) return false; // (whole lines)
@@ -1173,16 +1166,16 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
     if (q.k % 256 && (q.k > slot_lines(8) * 128 || q.n % 16)) return false;
     return (((uintptr_t)q.qs | (uintptr_t)q.sc) & 15) == 0;
   };
-  if (m->hd != 64 || m->heads % m->kv_heads || m->rope.rope_dim > 64) return false;
-  if (m->dim > MAX_K || m->hidden > MAX_K || m->qd() > MAX_K) return false;
-  if (m->arch == ARCH_LLAMA && m->gu_group != 1) return false;
-  if (!mat_ok(m->head)) return false;
+  if (m->hd != 64 || m->heads % m->kv_heads || m->rope.rope_dim > 64) return DG_UNFIT;
+  if (m->dim > MAX_K || m->hidden > MAX_K || m->qd() > MAX_K) return DG_UNFIT;
+  if (m->arch == ARCH_LLAMA && m->gu_group != 1) return DG_UNFIT;
+  if (!mat_ok(m->head)) return DG_UNFIT;
   for (auto& l : m->layers)
-    if (!mat_ok(l.qkv) || !mat_ok(l.wo) || !mat_ok(l.ff1) || !mat_ok(l.ff2)) return false;
+    if (!mat_ok(l.qkv) || !mat_ok(l.wo) || !mat_ok(l.ff1) || !mat_ok(l.ff2)) return DG_UNFIT;
   int coop = 0;
-  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->dev->ordinal) != cudaSuccess || !coop) return false;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, m->dev->ordinal) != cudaSuccess || !coop) return DG_UNFIT;
   EncodeTiledFn enc = encode_fn();
-  if (!enc) return false;
+  if (!enc) return DG_UNFIT;
   const uint32_t grid = (uint32_t)m->dev->prop.multiProcessorCount, max_k = std::max(m->dim, std::max(m->hidden, m->qd()));
   DgArgs a = DgArgs();
   a.n_layers = m->n_layers, a.dim = m->dim, a.heads = m->heads, a.kv_heads = m->kv_heads, a.ctx = m->ctx;
@@ -1192,7 +1185,7 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
   a.cos = m->rope.cos, a.sin = m->rope.sin, a.rope_dim = m->rope.rope_dim, a.rope_type = m->rope.type;
   a.eps = m->eps, a.logits = m->logits, a.err_flag = m->dev->d_flag;
   for (int v = 0; v < 4; v++)
-    if (!layout(a, kind, 1 << v, max_k)) return false;
+    if (!layout(a, kind, 1 << v, max_k)) return DG_UNFIT;
   // The tagged words, outside the model's plan: a model that fits without them decodes as launches.
   const uint32_t groups = (std::min<uint32_t>(8 * MAX_GROUPS, m->max_streams) + 7) / 8, rows_max = std::min<uint32_t>(8, m->max_streams);
   const size_t w_part = (size_t)grid * ITEM_HEADS * PART;
@@ -1201,9 +1194,9 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
   // descriptors: per variant of the slots two tensor maps per matrix, then the layers
   const size_t n_mats = 4 * (size_t)m->n_layers + 1, maps_bytes = n_mats * 2 * sizeof(CUtensorMap);
   const size_t var_bytes = (maps_bytes + m->n_layers * sizeof(DgLayer) + 255) & ~(size_t)255;
-  if (cudaMalloc(&st->d_layers, 2 * var_bytes) != cudaSuccess || cudaMalloc(&st->words, n_words * 8) != cudaSuccess) {
+  if (device_malloc(m->dev, &st->d_layers, 2 * var_bytes) != cudaSuccess || device_malloc(m->dev, &st->words, n_words * 8) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return DG_NO_ROOM;
   }
   std::vector<uint8_t> host(2 * var_bytes);
   DgMat heads[2];
@@ -1248,12 +1241,12 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
                       l.kv.v};
     }
     memcpy(at + maps_bytes, hl.data(), hl.size() * sizeof(DgLayer));
-    if (!ok) return false;
+    if (!ok) return DG_UNFIT;
   }
   if (cudaMemcpyAsync(st->d_layers, host.data(), host.size(), cudaMemcpyHostToDevice, m->dev->stream) != cudaSuccess ||
       cudaMemsetAsync(st->words, 0, n_words * 8, m->dev->stream) != cudaSuccess || cudaStreamSynchronize(m->dev->stream) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return DG_UNFIT;
   }
   unsigned long long* w = (unsigned long long*)st->words;
   a.group_words = (uint32_t)g_words;
@@ -1292,8 +1285,30 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
     b.sh[4] = shape(m->head, a.b_x2, nullptr, 0);
   }
   st->kind = kind;
-  st->ok = true;
-  return decode_grid_ready(m, rows);
+  return DG_READY;
+}
+
+// Whether a step of `rows` rows can run as this kernel. The set-up is made on first use, and tried again now and then where there
+// was no room for it (a try gives back what the scratch pool holds and waits for the stream).
+bool decode_grid_ready(FcModel* m, uint32_t rows) {
+  if (rows == 0 || rows > 8 * MAX_GROUPS || m->n_shards != 1) return false;
+  DgState* st = (DgState*)m->dg;
+  if (!st) m->dg = st = new DgState();
+  if (st->set_up == DG_UNTRIED || (st->set_up == DG_NO_ROOM && ++st->asked == st->retry)) {
+    st->asked = 0;
+    if (st->set_up == DG_NO_ROOM) st->retry = std::min(2 * st->retry, 4096u);
+    st->set_up = decode_grid_set_up(m, st);
+    if (st->set_up != DG_READY) {
+      if (st->d_layers) cudaFree(st->d_layers);
+      if (st->words) cudaFree(st->words);
+      st->d_layers = st->words = nullptr;
+    }
+  }
+  if (st->set_up != DG_READY) return false;
+  const uint32_t sub = group_ctas(m, rows), group_rows = std::min(rows, 8u);
+  // (LayerNorm keeps its input in registers: two 256-element parts per warp)
+  return (m->arch == ARCH_LLAMA || group_rows * ((m->dim + 255) / 256) <= 2 * WARPS) && (m->dim + 15) / 16 <= MAX_RESID * sub &&
+         group_rows * m->heads <= MAX_ITEMS * sub;
 }
 
 // Whether a step of these rows is faster as this kernel than as launches. Up to eight rows it always was. Beyond, every
