@@ -1311,8 +1311,40 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
          group_rows * m->heads <= MAX_ITEMS * sub;
 }
 
-// Whether a step of these rows is faster as this kernel than as launches. Up to eight rows it always was. Beyond, every
-// group of eight reads all weights (a unit of 16 rows x 128 k costs an SM 0.15 us as Q4_0, 0.17 as Q8_0) and works through
+// How the attention of steps that reach `longest` positions is cut into items: as few heads of a group each as the CTAs allow. A
+// row's positions are split only where one CTA would work through more than four 64-position tiles: the merge costs another trip
+// through L2.
+struct DgPlan {
+  uint32_t splits, item_heads;
+};
+static DgPlan decode_grid_plan(const FcModel* m, uint32_t group_rows, uint32_t sub, uint32_t longest) {
+  const uint32_t tiles = (longest + KV_POS - 1) / KV_POS, group = m->heads / m->kv_heads;
+  DgPlan p{tiles <= 4 ? 1 : std::min(tiles, MAX_SPLITS), 0};
+  uint32_t widest = 1;
+  for (uint32_t h = 1; h <= std::min(group, ITEM_HEADS); h++)
+    if (group % h == 0) {
+      widest = h;
+      if (!p.item_heads && group_rows * (m->heads / h) * p.splits <= sub) p.item_heads = h;
+    }
+  if (!p.item_heads) {
+    p.item_heads = widest;
+    p.splits = std::max(1u, std::min(p.splits, sub / (group_rows * (m->heads / widest))));
+  }
+  return p;
+}
+
+// Whether a step of these rows is faster as this kernel than as launches; figures in us, measured through decode_greedy. One row
+// always was (MHA of 48 heads at 3900 positions: 56 a layer here, 87 as launches; 12 heads: 21 and 169).
+//
+// Two to eight rows: the launches are a chain of some 33 per layer whose attention reads the caches at 5 TB/s with all SMs; here a
+// CTA works through its items' tiles one after the other (0.73 per 64-position tile, 0.95 for heads of a group together; from three
+// rows on twice that where the widths leave room for one tile in flight), so long caches of many heads go as launches. Per layer, here
+// and as launches: 48 heads of 48 as Q8_0, 8 rows at 0 positions 80 and 82, at 500 111 and 102, at 3900 328 and 235, 4 rows at 1000
+// 89 and 103, at 2000 132 and 123; 12 of 12 as Q4_0, 8 rows at 1000 45 and 48, at 2000 66 and 59; 16 of 2 as Q8_0, 8 rows at 2000
+// 44 and 49, at 3900 58 and 53; 32 of 8 as Q4_0, 8 rows at 1000 56 and 62, at 2000 71 and 68. Of 172 such pairs (2 to 8 rows, 0 to
+// 3900 positions, seven models) the estimates below pick the slower side of two, which differ by 1 %.
+//
+// More rows: every group of eight reads all weights (a unit of 16 rows x 128 k costs an SM 0.15 us as Q4_0, 0.17 as Q8_0) and works through
 // its caches on its share of the SMs (2 us per 64-position tile and item), where the launches' step is a chain of some 40 us
 // per layer whatever it holds. Steps at 0 .. 60 positions, us as launches and here: Qwen2-style 24 layers Q8_0, 16 rows 1197 and
 // 712, 32 rows 1316 and 1116, 48 rows 1555 and 1599, 64 rows 1450 and 2017; Llama-style 12 layers Q4_0, 16 rows 464 and 245, 64
@@ -1320,15 +1352,27 @@ bool decode_grid_ready(FcModel* m, uint32_t rows) {
 // 1348 and 1612; GPT-2-124M-style 24 rows 858 and 811, 32 rows 1014 and 1109.
 bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions) {
   if (!decode_grid_ready(m, rows)) return false;
-  if (rows <= 8) return true;
+  if (rows == 1) return true;
   const double sms = m->dev->prop.multiProcessorCount, layers = m->n_layers, groups = (rows + 7) / 8;
   double units = 0.0, tiles = 0.0, bytes = 0.0;
   auto add = [&](const Linear& l) { units += (l.w->m.n + 15) / 16 * (l.w->m.k / 128); };
   for (const auto& l : m->layers) add(l.qkv), add(l.wo), add(l.ff1), add(l.ff2);
   add(m->head);
+  uint32_t longest = 0;
   for (uint32_t r = 0; r < rows; r++) {
     tiles += positions[r] / KV_POS + 1;
     bytes += (positions[r] + 1.0) * m->kv_heads * 512;
+    longest = std::max(longest, positions[r] + 1);
+  }
+  if (rows <= 8) {
+    const uint32_t sub = group_ctas(m, rows), longest_tiles = (longest + KV_POS - 1) / KV_POS;
+    const DgPlan p = decode_grid_plan(m, rows, sub, longest);
+    const uint32_t items = rows * (m->heads / p.item_heads) * p.splits, each = (longest_tiles + p.splits - 1) / p.splits;
+    const bool one_tile = rows > 2 && ((DgState*)m->dg)->args[rows <= 4 ? 2 : 3].kv_log == 0;
+    const double tile = (p.item_heads == 1 ? 0.73 : 0.95) * (one_tile ? 1.9 : 1.0);
+    const double here = layers * (10.0 + (items + sub - 1) / sub * each * tile + (p.splits > 1 ? 5.0 : 0.0)) + (rows <= 4 ? 0.12 : 0.25) * units / sms;
+    const double launches = layers * (33.0 + 1.5e-3 * longest + bytes / 5.3e6) + 1.2e-3 * units;
+    return here < launches;
   }
   uint32_t item = 1;
   for (uint32_t h = 1; h <= ITEM_HEADS; h++)
@@ -1368,21 +1412,8 @@ int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint
     a.stream[r] = (int32_t)streams[r];
     longest = std::max(longest, positions[r] + steps);
   }
-  // Items: as few heads of a group each as the CTAs allow. A row's positions are split only where one CTA would work
-  // through more than four 64-position tiles: the merge costs another trip through L2.
-  const uint32_t tiles = (longest + KV_POS - 1) / KV_POS, group = a.heads / a.kv_heads;
-  a.splits = tiles <= 4 ? 1 : std::min(tiles, MAX_SPLITS);
-  a.item_heads = 0;
-  uint32_t widest = 1;
-  for (uint32_t h = 1; h <= std::min(group, ITEM_HEADS); h++)
-    if (group % h == 0) {
-      widest = h;
-      if (!a.item_heads && a.group_rows * (a.heads / h) * a.splits <= a.sub) a.item_heads = h;
-    }
-  if (!a.item_heads) {
-    a.item_heads = widest;
-    a.splits = std::max(1u, std::min(a.splits, a.sub / (a.group_rows * (a.heads / widest))));
-  }
+  const DgPlan plan = decode_grid_plan(m, a.group_rows, a.sub, longest);
+  a.splits = plan.splits, a.item_heads = plan.item_heads;
   const bool llama = m->arch == ARCH_LLAMA;
   return st->kind == FC_Q8_0 ? launch_rows<FC_Q8_0>(dev, a, llama) : launch_rows<FC_Q4_0>(dev, a, llama);
 }
