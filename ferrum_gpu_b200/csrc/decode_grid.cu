@@ -1076,6 +1076,7 @@ struct DgState {
   void* d_layers = nullptr;    // the tensor maps and the layers' descriptors, for slots of 8 and of 4 lines
   void* words = nullptr;
   uint64_t tags = 0;           // used since the words were cleared
+  double units = 0.0;          // of 16 rows x 128 k, in all matrices
   int kind = 0;
 };
 
@@ -1285,6 +1286,9 @@ static int decode_grid_set_up(FcModel* m, DgState* st) {
     b.sh[4] = shape(m->head, a.b_x2, nullptr, 0);
   }
   st->kind = kind;
+  auto add = [&](const Linear& l) { st->units += (l.w->m.n + 15) / 16 * (l.w->m.k / 128); };
+  for (const auto& l : m->layers) add(l.qkv), add(l.wo), add(l.ff1), add(l.ff2);
+  add(m->head);
   return DG_READY;
 }
 
@@ -1354,10 +1358,8 @@ bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions) {
   if (!decode_grid_ready(m, rows)) return false;
   if (rows == 1) return true;
   const double sms = m->dev->prop.multiProcessorCount, layers = m->n_layers, groups = (rows + 7) / 8;
-  double units = 0.0, tiles = 0.0, bytes = 0.0;
-  auto add = [&](const Linear& l) { units += (l.w->m.n + 15) / 16 * (l.w->m.k / 128); };
-  for (const auto& l : m->layers) add(l.qkv), add(l.wo), add(l.ff1), add(l.ff2);
-  add(m->head);
+  const double units = ((DgState*)m->dg)->units;
+  double tiles = 0.0, bytes = 0.0;
   uint32_t longest = 0;
   for (uint32_t r = 0; r < rows; r++) {
     tiles += positions[r] / KV_POS + 1;
@@ -1382,6 +1384,29 @@ bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions) {
   return here < launches;
 }
 
+// Of `steps` steps that follow one another, the first of them at `positions`: how many go the way the first one goes, in one kernel or
+// as launches; and, in one kernel, how many have its cut of the attention. A chain is cut there, so that it is its single steps bit for bit.
+uint32_t decode_grid_steps(FcModel* m, uint32_t rows, const uint32_t* positions, uint32_t steps, bool* takes) {
+  uint32_t at[8 * MAX_GROUPS], n = 0;
+  *takes = rows <= 8 * MAX_GROUPS && decode_grid_takes(m, rows, positions);
+  if (rows == 1 || rows > 8 * MAX_GROUPS || !decode_grid_ready(m, rows)) return steps;
+  for (bool same = true; same && ++n < steps;) {
+    for (uint32_t r = 0; r < rows; r++) at[r] = positions[r] + n;
+    same = decode_grid_takes(m, rows, at) == *takes;
+  }
+  return n;
+}
+static uint32_t decode_grid_same_plan(const FcModel* m, uint32_t group_rows, uint32_t sub, uint32_t longest, uint32_t steps) {
+  const DgPlan first = decode_grid_plan(m, group_rows, sub, longest);
+  uint32_t n = 0;
+  do {
+    n += KV_POS - (longest + n - 1) % KV_POS; // (a plan holds for whole tiles)
+    const DgPlan p = decode_grid_plan(m, group_rows, sub, longest + n);
+    if (p.splits != first.splits || p.item_heads != first.item_heads) break;
+  } while (n < steps);
+  return std::min(n, steps);
+}
+
 const int32_t* decode_grid_out(const FcModel* m) { return ((DgState*)m->dg)->args[0].out; }
 
 // After a step that reported a wait that gave up: as before the first one.
@@ -1395,25 +1420,29 @@ int decode_grid_clear(FcModel* m) {
 int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint32_t* positions, const int32_t* tokens, uint32_t steps, int32_t* log) {
   DgState* st = (DgState*)m->dg;
   FcDevice* dev = m->dev;
-  st->tags += (uint64_t)steps * (m->n_layers + 1);
-  if (st->tags >= 1ull << 31) { // (before a tag could come round again)
-    FC_CUDA(dev, cudaMemsetAsync(st->words, 0, (size_t)((uint8_t*)st->args[0].out - (uint8_t*)st->words), dev->stream));
-    st->tags = (uint64_t)steps * (m->n_layers + 1);
-  }
   const int v = rows == 1 ? 0 : rows == 2 ? 1 : rows <= 4 ? 2 : 3;
   DgArgs a = st->args[v];
   const uint32_t groups = (rows + 7) / 8;
   a.rows = rows, a.group_rows = (rows + groups - 1) / groups, a.sub = group_ctas(m, rows);
-  a.steps = steps, a.chained = tokens ? 0 : 1, a.log = log;
-  uint32_t longest = 1;
+  uint32_t longest = 0;
   for (uint32_t r = 0; r < rows; r++) {
     a.tok_in[r] = tokens ? tokens[r] : 0;
-    a.pos[r] = (int32_t)positions[r];
     a.stream[r] = (int32_t)streams[r];
-    longest = std::max(longest, positions[r] + steps);
+    longest = std::max(longest, positions[r] + 1);
   }
-  const DgPlan plan = decode_grid_plan(m, a.group_rows, a.sub, longest);
-  a.splits = plan.splits, a.item_heads = plan.item_heads;
   const bool llama = m->arch == ARCH_LLAMA;
-  return st->kind == FC_Q8_0 ? launch_rows<FC_Q8_0>(dev, a, llama) : launch_rows<FC_Q4_0>(dev, a, llama);
+  for (uint32_t s = 0; s < steps; s += a.steps) { // a launch for as long as the cut of the attention holds, up to 256 steps
+    a.steps = std::min(256u, decode_grid_same_plan(m, a.group_rows, a.sub, longest + s, steps - s));
+    st->tags += (uint64_t)a.steps * (m->n_layers + 1);
+    if (st->tags >= 1ull << 31) { // (before a tag could come round again)
+      FC_CUDA(dev, cudaMemsetAsync(st->words, 0, (size_t)((uint8_t*)st->args[0].out - (uint8_t*)st->words), dev->stream));
+      st->tags = (uint64_t)a.steps * (m->n_layers + 1);
+    }
+    for (uint32_t r = 0; r < rows; r++) a.pos[r] = (int32_t)(positions[r] + s);
+    a.chained = tokens && s == 0 ? 0 : 1, a.log = log ? log + (size_t)s * rows : nullptr;
+    const DgPlan plan = decode_grid_plan(m, a.group_rows, a.sub, longest + s);
+    a.splits = plan.splits, a.item_heads = plan.item_heads;
+    FC_TRY(st->kind == FC_Q8_0 ? launch_rows<FC_Q8_0>(dev, a, llama) : launch_rows<FC_Q4_0>(dev, a, llama));
+  }
+  return FC_OK;
 }

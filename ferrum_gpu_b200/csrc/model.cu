@@ -856,6 +856,9 @@ __global__ void __launch_bounds__(256)
   for (uint32_t i = threadIdx.x; i < d; i += blockDim.x) x[(size_t)r * d + i] = ps ? src[i] + ps[i] : src[i];
 }
 
+// `steps` - 1 further greedy steps that all go the same way; the first picks of `tokens_out` are there already.
+static int continue_greedy(FcModel* m, uint32_t n, const uint32_t* stream_ids, uint32_t steps, int32_t* tokens_out, bool grid);
+
 FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream_ids, const int32_t* first_tokens, uint32_t steps,
                                   int32_t* tokens_out) {
   if (!m || !stream_ids || !first_tokens || !tokens_out) return FC_ERR_ARG;
@@ -870,7 +873,21 @@ FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream
   }
   // the first step takes its tokens from the host like any other (and checks streams and ids)
   FC_TRY(fc_model_feed_batch(m, n, stream_ids, first_tokens, nullptr, tokens_out));
-  if (steps == 1) return FC_OK;
+  for (uint32_t done = 1; done < steps;) {
+    bool grid = false;
+    uint32_t more = steps - done, positions[64];
+    if (n <= 64) {
+      for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]];
+      more = decode_grid_steps(m, n, positions, more, &grid);
+    }
+    FC_TRY(continue_greedy(m, n, stream_ids, more + 1, tokens_out + (size_t)(done - 1) * n, grid));
+    done += more;
+  }
+  return FC_OK;
+}
+
+static int continue_greedy(FcModel* m, uint32_t n, const uint32_t* stream_ids, uint32_t steps, int32_t* tokens_out, bool grid) {
+  FcDevice* dev = m->dev;
   if (n == 1 && m->n_shards == 1 && !decode_grid_ready(m, 1) && decode_cluster_ready(m)) {
     // the remaining steps in one launch: the kernel takes each pick as the next token itself
     FC_CUDA(dev, cudaMemsetAsync(m->d_chain_cnt, 0, 4, dev->stream));
@@ -882,17 +899,10 @@ FC_API int fc_model_decode_greedy(FcModel* m, uint32_t n, const uint32_t* stream
     m->pos[stream_ids[0]] += steps - 1;
     return FC_OK;
   }
-  uint32_t positions[64];
-  for (uint32_t i = 0; i < n && n <= 64; i++) positions[i] = m->pos[stream_ids[i]] + steps / 2; // (half-way)
-  if (n <= 64 && decode_grid_takes(m, n, positions)) {
-    // The remaining steps in one launch per 256 of them; the first one's tokens come from the host (the step before may
-    // have run as launches).
-    const uint32_t most = 256;
-    for (uint32_t s = 1; s < steps; s += most) {
-      for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]] + s - 1;
-      FC_TRY(k_decode_grid(m, n, stream_ids, positions, s == 1 ? tokens_out : nullptr, std::min(most, steps - s),
-                           m->d_chain_log + (size_t)(s - 1) * n));
-    }
+  if (grid) { // (the first step's tokens come from the host: the step before may have run as launches)
+    uint32_t positions[64];
+    for (uint32_t i = 0; i < n; i++) positions[i] = m->pos[stream_ids[i]];
+    FC_TRY(k_decode_grid(m, n, stream_ids, positions, tokens_out, steps - 1, m->d_chain_log));
     if (steps > 2) // the log holds the tokens the steps consumed: the picks of steps 0 .. steps - 2
       FC_CUDA(dev, cudaMemcpyAsync(tokens_out + n, m->d_chain_log + n, (size_t)(steps - 2) * n * 4, cudaMemcpyDeviceToHost, dev->stream));
     FC_TRY(finish_grid_steps(m, n, tokens_out + (size_t)(steps - 1) * n, nullptr));

@@ -116,11 +116,12 @@ int tc_check_errors(FcDevice* dev);
 bool decode_cluster_ready(FcModel* m);
 int k_decode_cluster(FcModel* m, uint32_t stream, uint32_t steps, bool chained);
 void decode_cluster_free(FcModel* m);
-// decode_grid.cu: `steps` greedy decode steps of one to 64 streams as one kernel. `tokens` null: they continue the step before,
+// decode_grid.cu: `steps` greedy decode steps of one to 64 streams as one kernel (a chain as few). `tokens` null: they continue the step before,
 // whose picks are the first one's tokens; `log` (device, nullable; [steps][rows]) receives the tokens the steps consumed. The
 // last picks and, behind the 64th, the eight status words of the run are at decode_grid_out (device).
 bool decode_grid_ready(FcModel* m, uint32_t rows); // it can
 bool decode_grid_takes(FcModel* m, uint32_t rows, const uint32_t* positions); // and is the faster way
+uint32_t decode_grid_steps(FcModel* m, uint32_t rows, const uint32_t* positions, uint32_t steps, bool* takes); // and how many of a chain do alike
 int k_decode_grid(FcModel* m, uint32_t rows, const uint32_t* streams, const uint32_t* positions, const int32_t* tokens, uint32_t steps, int32_t* log);
 int decode_grid_clear(FcModel* m);
 const int32_t* decode_grid_out(const FcModel* m);

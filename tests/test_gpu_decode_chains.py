@@ -71,3 +71,47 @@ def test_a_chain_where_most_ctas_have_attention_and_nothing_after_it(dev, kind):
         assert np.array_equal(a, b)
     g.close()
     ref.close()
+
+
+# heads, K/V heads, streams, tokens before the chain, its steps, a few of the launches it may take
+@pytest.mark.parametrize("heads, kv_heads, streams, prompt, steps", [
+    (4, 2, 1, 250, 20),    # past the 256 positions beyond which the attention is split
+    (4, 2, 3, 310, 140),   # a split more every 64 positions
+    (12, 12, 8, 1760, 120), # from one kernel to launches
+    (12, 4, 12, 250, 20),
+], ids=["split", "splits", "to_launches", "groups"])
+def test_a_chain_is_its_single_steps_bit_for_bit(dev, heads, kv_heads, streams, prompt, steps):
+    """How a step runs and how its attention is cut depends on its positions; a chain changes where its single steps would."""
+    cfg = LlamaConfig(vocab=500, ctx=2000, dim=256 * (heads // 4), heads=heads, kv_heads=kv_heads, head_dim=64, layers=2,
+                      hidden=3072 if heads == 12 else 512, rope_dim=64)
+    m = random_llama(cfg, seed=2, std=0.05)
+    g = CudaLlama(dev, m, QKind.Q4_0, max_streams=streams)
+    ids = random_tokens(8, prompt, cfg.vocab)
+    first = random_tokens(9, streams, cfg.vocab)
+    slots = list(range(streams))
+
+    def start():
+        for s in slots:
+            g.reset(s)
+            for at in range(0, prompt - 3 * s, 1000):
+                g.prefill(ids[at:min(at + 1000, prompt - 3 * s)], stream=s)
+
+    start()
+    before = dev.launch_count()
+    chain = g.decode_greedy(first, steps, streams=slots)
+    launches = dev.launch_count() - before
+    _, after = g.feed_batch(chain[-1], streams=slots, want_logits=True)
+    start()
+    tok, single = first, set()
+    for step in range(steps):
+        before = dev.launch_count()
+        tok, _ = g.feed_batch(tok, streams=slots)
+        single.add(dev.launch_count() - before)
+        assert np.array_equal(tok, chain[step]), step
+    # (the caches, down to the last bit of what the chain's attention gave the layer above)
+    assert np.array_equal(g.feed_batch(tok, streams=slots, want_logits=True)[1], after)
+    if (heads, kv_heads) == (12, 12):
+        assert min(single) == 1 < max(single), "some steps as one kernel, some as launches"
+    elif streams <= 8:
+        assert single == {1} and launches <= 2 + steps // 64 + 1
+    g.close()
