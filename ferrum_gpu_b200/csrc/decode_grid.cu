@@ -728,22 +728,35 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
               if (e < k) u = *reinterpret_cast<const float4*>(p + e), w = *reinterpret_cast<const float4*>(p + e + 4);
               v[0] = u.x, v[1] = u.y, v[2] = u.z, v[3] = u.w, v[4] = w.x, v[5] = w.y, v[6] = w.z, v[7] = w.w;
             };
-            // two fp16 terms of every element, at the power of two that brings its 32-block's largest into [2^14, 2^15)
+            // Two fp16 terms of every element, at the power of two that brings its 32-block's largest into [2^14, 2^15). One row keeps
+            // the low terms 2^11 larger: 22 bits of every element down to 2^-28 of the largest. A block with a smaller one that is
+            // not zero, with one that is not finite, or of magnitudes whose scale would leave the normal floats goes as it is (its
+            // scale says so) and is multiplied in f32.
             auto stage = [&](uint32_t task, const float (&x)[8]) {
               const uint32_t r = row_of(task), b = (task - r * tpr) * 8 + g; // (lane = block, quarter)
-              float am = fmaxf(fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3]))),
-                               fmaxf(fmaxf(fabsf(x[4]), fabsf(x[5])), fmaxf(fabsf(x[6]), fabsf(x[7]))));
-              am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
-              am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-              const uint32_t ex = min(max(__float_as_uint(am) & 0x7f800000u, 15u << 23), 254u << 23);
+              uint32_t mx = 0, mn = 0xffffffffu; // (of the bits; a zero is not the smallest)
+#pragma unroll
+              for (int i = 0; i < 8; i++) {
+                const uint32_t u = __float_as_uint(x[i]) & 0x7fffffffu;
+                mx = max(mx, u);
+                if (ONE) mn = min(mn, u - 1);
+              }
+              mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+              mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+              const uint32_t ex = min(max(mx & 0x7f800000u, 15u << 23), 254u << 23);
               const float up = __uint_as_float((268u << 23) - ex);
+              bool held = true;
+              if (ONE) {
+                const bool bad = (mx != 0 && mx - (63u << 23) >= (161u << 23)) || mn < ex - (28u << 23) - 1;
+                held = (__ballot_sync(0xffffffffu, bad) >> (lane & 28) & 15u) == 0;
+              }
               uint32_t hi[4], lo[4];
 #pragma unroll
               for (int i = 0; i < 4; i++) {
                 const float v0 = x[2 * i] * up, v1 = x[2 * i + 1] * up;
                 const __half2 h = __floats2half2_rn(v0, v1);
                 const float2 f = __half22float2(h);
-                const __half2 d = __floats2half2_rn(v0 - f.x, v1 - f.y);
+                const __half2 d = ONE ? __floats2half2_rn((v0 - f.x) * 2048.0f, (v1 - f.y) * 2048.0f) : __floats2half2_rn(v0 - f.x, v1 - f.y);
                 hi[i] = *reinterpret_cast<const uint32_t*>(&h), lo[i] = *reinterpret_cast<const uint32_t*>(&d);
               }
               if (b * 32 < k) {
@@ -752,6 +765,11 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
                 *reinterpret_cast<uint4*>(at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                 *reinterpret_cast<uint4*>(at + (ONE ? 64 : MT * 64)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                 if (t == 0) ysm[b * MT + r] = __uint_as_float(ex - (14u << 23));
+                if (ONE && !held) {
+                  *reinterpret_cast<float4*>(at) = make_float4(x[0], x[1], x[2], x[3]);
+                  *reinterpret_cast<float4*>(at + 64) = make_float4(x[4], x[5], x[6], x[7]);
+                  if (t == 0) ysm[b] = __uint_as_float(0x7fffffffu);
+                }
               }
             };
             auto warp_sum = [&](float v) {
@@ -843,6 +861,7 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
                 if (t == (g >> 1)) xb[j] = *reinterpret_cast<const uint4*>(xs + kg * (4 * XBLK) + j * 128 + (g & 1) * 64 + t * 16);
               }
               const float ys = ysm[kg * 4 + t];
+              const bool plain = __any_sync(0xffffffffu, ys != ys); // a block of the unit is multiplied in f32
               float cc[2][4];
 #pragma unroll
               for (int j = 0; j < 2; j++) cc[j][0] = cc[j][1] = cc[j][2] = cc[j][3] = 0.0f;
@@ -860,10 +879,35 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
                 dg_mma(cc[0], pa[0], pb[0], pa[1], pb[1], xb[j].x, xb[j].y);
                 dg_mma(cc[1], pa[2], pb[2], pa[3], pb[3], xb[j].z, xb[j].w);
               }
-              const float dg = __half2float(__ushort_as_half((unsigned short)sraw[0])) * ys;
-              const float dg8 = __half2float(__ushort_as_half((unsigned short)sraw[1])) * ys;
-              acc[0] = fmaf((cc[0][1] + cc[1][1]) + (cc[0][0] + cc[1][0]), dg, acc[0]); // (the small terms first)
-              acc[2] = fmaf((cc[0][3] + cc[1][3]) + (cc[0][2] + cc[1][2]), dg8, acc[2]);
+              float d = __half2float(__ushort_as_half((unsigned short)sraw[0])), d8 = __half2float(__ushort_as_half((unsigned short)sraw[1]));
+              float s = fmaf(cc[0][1] + cc[1][1], 0x1p-11f, cc[0][0] + cc[1][0]), s8 = fmaf(cc[0][3] + cc[1][3], 0x1p-11f, cc[0][2] + cc[1][2]);
+              if (!plain) {
+                d *= ys, d8 *= ys;
+              } else if (ys == ys) {
+                d *= ys, d8 *= ys;
+              } else { // this lane's block lies there as it is (of the sums above only the block's own columns saw it)
+                const uint32_t c = kg / UPC, si = it + u_ti * sh.nch + c, b0 = (kg - c * UPC) * 4;
+                const uint8_t* wp = ring + min(ms.slot_at[si % SLOTS], a.ring_bytes - sh.size) + (b0 / (128 / BLK)) * 2048 + rho * 128;
+                const uint8_t* xp = xs + kg * (4 * XBLK) + t * 16;
+                constexpr int PER = Q8 ? 4 : 8; // codes of a word
+                s = s8 = 0.0f;
+#pragma unroll 1
+                for (uint32_t e = 0; e < 32; e += PER) {
+                  const uint32_t chunk = Q8 ? 2 * t + (e >> 4) : (b0 & 4) + t, word = Q8 ? (e >> 2) & 3 : e >> 3;
+                  const uint32_t* p = reinterpret_cast<const uint32_t*>(wp + (chunk ^ (rho & 7)) * 16) + word;
+                  const uint32_t w = p[0], w8 = p[256];
+#pragma unroll
+                  for (uint32_t j = 0; j < PER; j++) {
+                    const float xe = *reinterpret_cast<const float*>(xp + (e >> 3) * 128 + ((e + j) & 4) * 16 + (j & 3) * 4);
+                    // (Q4_0: element j of a word's eight at nibble (j >> 1) + 4 (j & 1))
+                    const uint32_t sft = Q8 ? 8 * j : 4 * (j >> 1) + 16 * (j & 1);
+                    s = fmaf(xe, Q8 ? (float)(int8_t)(w >> sft) : (float)(int)(w >> sft & 15) - 8.0f, s);
+                    s8 = fmaf(xe, Q8 ? (float)(int8_t)(w8 >> sft) : (float)(int)(w8 >> sft & 15) - 8.0f, s8);
+                  }
+                }
+              }
+              acc[0] = fmaf(s, d, acc[0]);
+              acc[2] = fmaf(s8, d8, acc[2]);
             } else {
               const uint8_t* xp = xs + kg * (4 * XBLK) + (WIDE ? g : (g >> 2) * MT + (g & (MT - 1))) * 64 + t * 16;
               const float* yp = ysm + kg * 4 * MT + ((2 * t) & (MT - 1));
