@@ -37,7 +37,9 @@
 // A value is overwritten one layer later at the earliest (a token one step later); its writer then depends, through the tags,
 // on every reader of the old one having finished its stage. A word belongs to one group of CTAs for good: tags count per group,
 // and only one that never comes round again tells a word from what an earlier launch left there. All CTAs are resident (cooperative launch) and every wait is bounded: one
-// that gives up raises the device's status word, everybody's waits end at once, and the step reports it.
+// that gives up raises the device's status word and ends its CTA's other waits; the other CTAs, which miss what that one had to
+// send, run into their own limits (1.5 s) at about the same time, and the step reports it. A word raised before the launch ends all
+// waits at once.
 #include <algorithm>
 #include <cstring>
 
@@ -731,7 +733,9 @@ __global__ void __launch_bounds__(THREADS, 1) decode_grid_kernel(const __grid_co
             // Two fp16 terms of every element, at the power of two that brings its 32-block's largest into [2^14, 2^15). One row keeps
             // the low terms 2^11 larger: 22 bits of every element down to 2^-28 of the largest. A block with a smaller one that is
             // not zero, with one that is not finite, or of magnitudes whose scale would leave the normal floats goes as it is (its
-            // scale says so) and is multiplied in f32.
+            // scale says so) and is multiplied in f32. (Terms alone put the logits of a model with a constant 2^30 beside its
+            // activations off by 1e-3. The check and the factor cost 0.2 to 1.1 % of a step: 60.3 -> 60.8 us, 384 wide; asking for
+            // the smallest element first and looking closer behind a vote cost 2.4 %.)
             auto stage = [&](uint32_t task, const float (&x)[8]) {
               const uint32_t r = row_of(task), b = (task - r * tpr) * 8 + g; // (lane = block, quarter)
               uint32_t mx = 0, mn = 0xffffffffu; // (of the bits; a zero is not the smallest)
